@@ -84,6 +84,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_binding = None
 
 
 def load():
@@ -100,6 +101,19 @@ def load():
             fn.restype, fn.argtypes = res, args
         _lib = lib
     return _lib
+
+
+def binding():
+    """The PyTorch binding (csrc/gct_torch.cpp): the operators as single C calls on tensors.  Raises if it has not been
+    built."""
+    global _binding
+    if _binding is None:
+        load()
+        import torch  # noqa: F401  (its libraries must be in the process before the binding is)
+        from . import _gct_torch
+        _gct_torch.set_error_class(GctError)
+        _binding = _gct_torch
+    return _binding
 
 
 def check(rc):

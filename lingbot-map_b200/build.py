@@ -1,4 +1,5 @@
-"""Build the C-ABI library libgct_b200.so for sm_100a with nvcc (in-tree, next to this file)."""
+"""Build the C-ABI library libgct_b200.so for sm_100a with nvcc and the PyTorch binding _gct_torch.so on top of it with
+g++ (both in-tree, next to this file)."""
 import os
 import shutil
 import subprocess
@@ -9,6 +10,8 @@ SOURCES = ["csrc/gct_attn_sm100.cu", "csrc/gct_elementwise.cu", "csrc/gct_manage
            "csrc/gct_exchange.cu", "csrc/gct_decode.cu", "csrc/gct_render.cu"]
 HEADERS = ["csrc/gct_common.h", "../include/gct_b200.h"]
 LIB = os.path.join(HERE, "libgct_b200.so")
+BINDING_SOURCE = "csrc/gct_torch.cpp"
+BINDING = os.path.join(HERE, "_gct_torch.so")
 
 
 def _nvcc():
@@ -18,26 +21,50 @@ def _nvcc():
     raise RuntimeError("nvcc not found; set NVCC or put the CUDA toolkit on PATH")
 
 
-def needs_build():
-    if not os.path.exists(LIB):
+def _older(target, sources):
+    if not os.path.exists(target):
         return True
-    t = os.path.getmtime(LIB)
-    return any(os.path.getmtime(os.path.join(HERE, s)) > t for s in SOURCES + HEADERS)
+    t = os.path.getmtime(target)
+    return any(os.path.getmtime(os.path.join(HERE, s)) > t for s in sources)
+
+
+def needs_build():
+    return _older(LIB, SOURCES + HEADERS) or _older(BINDING, [BINDING_SOURCE] + HEADERS)
+
+
+def _run(cmd, what):
+    r = subprocess.run(cmd, cwd=HERE, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"{what} failed:\n" + r.stdout + r.stderr)
+    return r.stderr
+
+
+def _build_binding():
+    """The binding holds no device code; it finds libgct_b200.so beside itself ($ORIGIN)."""
+    import sysconfig
+    import torch
+    from torch.utils import cpp_extension
+    includes = cpp_extension.include_paths() + [sysconfig.get_paths()["include"], os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
+    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
+    cmd += [x for i in includes for x in ("-isystem", i)]
+    cmd += [BINDING_SOURCE, "-o", BINDING, f"-L{HERE}", "-l:libgct_b200.so", "-Wl,-rpath,$ORIGIN", f"-L{torch_lib}", "-ltorch", "-ltorch_cpu",
+            "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda"]
+    _run(cmd, "the C++ compiler")
 
 
 def build(force=False, verbose=False):
-    """Compile every CUDA source of the package into libgct_b200.so.  Returns the library path."""
-    if not force and not needs_build():
-        return LIB
-    cmd = [_nvcc(), "-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
-           "-Xcompiler", "-fPIC", "-shared", "-cudart", "static", "-o", LIB] + SOURCES
-    if verbose:
-        cmd.insert(1, "-Xptxas=-v")
-    r = subprocess.run(cmd, cwd=HERE, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + r.stdout + r.stderr)
-    if verbose:
-        print(r.stderr)
+    """Compile every source of the package into libgct_b200.so and _gct_torch.so.  Returns the library path."""
+    if force or _older(LIB, SOURCES + HEADERS):
+        cmd = [_nvcc(), "-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
+               "-Xcompiler", "-fPIC", "-shared", "-cudart", "static", "-o", LIB] + SOURCES
+        if verbose:
+            cmd.insert(1, "-Xptxas=-v")
+        log = _run(cmd, "nvcc")
+        if verbose:
+            print(log)
+    if force or _older(BINDING, [BINDING_SOURCE] + HEADERS):
+        _build_binding()
     return LIB
 
 

@@ -50,6 +50,7 @@ class B200KVCacheManager:
         if head_dim != 64:
             raise ValueError("B200 backend supports head_dim == 64 (ViT-L) only")
         self._lib = _lib.load()
+        self._native = _lib.binding()
         self._handle = C.c_void_p()
         cfg = _lib.MgrConfig(num_blocks, tokens_per_frame, num_heads, head_dim, num_special_tokens,
                              scale_frames, sliding_window, max_total_frames)
@@ -58,6 +59,8 @@ class B200KVCacheManager:
         if rc == _lib.ERR_INVALID and tokens_per_frame <= num_special_tokens:
             raise AssertionError(self._lib.gct_last_error().decode())      # flashinfer_cache.py:113-115
         _lib.check(rc)
+        self._h = self._handle.value            # the handle as the binding takes it
+        self._dev_index = None
 
         self.num_blocks = num_blocks
         self.num_special_tokens = num_special_tokens
@@ -82,6 +85,7 @@ class B200KVCacheManager:
         if not bookkeeping_only:
             if self.device is None or self.device.type != "cuda":
                 raise RuntimeError("B200KVCacheManager needs a CUDA device (there is no CPU path)")
+            self._dev_index = torch.cuda.current_device() if self.device.index is None else self.device.index
             with torch.cuda.device(self.device):
                 # pools are zero-initialised: rows past the valid length of the last special page are
                 # read (and masked) by the attention kernel and must hold finite values
@@ -129,16 +133,12 @@ class B200KVCacheManager:
         assert k.shape[0] - self.num_special_tokens == self.patches_per_frame, (
             f"block {block_idx}: expected {self.patches_per_frame} patch tokens, "
             f"got {k.shape[0] - self.num_special_tokens} (tokens_per_frame={k.shape[0]})")
-        k = self._check_frame_tensor(k, "k")
-        v = self._check_frame_tensor(v, "v")
-        with torch.cuda.device(self.device):      # the C ABI works on the current device
-            self._check(self._lib.gct_mgr_append(self._handle, block_idx, k.data_ptr(), _dtype_code(k),
-                                                 v.data_ptr(), _dtype_code(v), _stream_ptr(self.device)))
+        self._native.append(self._h, self._dev_index, block_idx, k, v)
 
     def append_frame_bookkeeping(self, block_idx: int) -> None:
         """append_frame without device writes (dry runs; KV-sharded replicas that do not own the page).  Whoever
         fills the pages directly calls rescan_key_norms() afterwards to re-enable the bounded attention mode."""
-        self._check(self._lib.gct_mgr_append_bookkeeping(self._handle, block_idx))
+        self._native.append_bookkeeping(self._h, block_idx)
 
     def rescan_key_norms(self, block_idx: Optional[int] = None) -> None:
         """Recompute the per-head maximum key norm of a block (all blocks by default) from its pool, after pages
@@ -169,31 +169,20 @@ class B200KVCacheManager:
         """qkv Linear output [tokens_per_frame, 3*H*D] -> LayerNorm(q,k), RoPE, bf16; K/V go straight into
         their pages, q is returned as [tokens_per_frame, H, D] bf16 (attention.py:413-426 + append_frame)."""
         self._require_device()
-        if qkv.dim() != 2 or qkv.shape[0] != self.tokens_per_frame or qkv.shape[1] != 3 * self.num_heads * self.head_dim:
-            raise ValueError(f"qkv must be [{self.tokens_per_frame}, {3 * self.num_heads * self.head_dim}]")
-        if qkv.stride(1) != 1:
-            qkv = qkv.contiguous()
-        if q_out is None:
-            q_out = torch.empty(self.tokens_per_frame, self.num_heads, self.head_dim, dtype=torch.bfloat16,
-                                device=self.device)
-        ptr = lambda t: None if t is None else t.data_ptr()
-        with torch.cuda.device(self.device):
-            self._check(self._lib.gct_mgr_append_fused(
-                self._handle, block_idx, qkv.data_ptr(), _dtype_code(qkv), qkv.stride(0), ptr(q_norm_w), ptr(q_norm_b),
-                ptr(k_norm_w), ptr(k_norm_b), ptr(rope_cs), rope_mode, q_out.data_ptr(), _stream_ptr(self.device)))
-        return q_out
+        return self._native.append_fused(self._h, self._dev_index, block_idx, qkv, q_norm_w, q_norm_b, k_norm_w, k_norm_b, rope_cs,
+                                         rope_mode, q_out)
 
     def evict_frames(self, block_idx: int, scale_frames: int, sliding_window: int, cross_frame_special: bool = True,
                      include_scale_frames: bool = True, camera_only: bool = False, num_register_tokens: int = 4) -> None:
         """Recycle window pages beyond ``sliding_window``; no-op while deferred - flashinfer_cache.py:229-254."""
-        self._check(self._lib.gct_mgr_evict(self._handle, block_idx, sliding_window))
+        self._native.evict(self._h, block_idx, sliding_window)
 
     def execute_deferred_eviction(self, block_idx: int, scale_frames: int, sliding_window: int, **kwargs) -> None:
         self._check(self._lib.gct_mgr_exec_deferred(self._handle, block_idx, sliding_window))
 
     def rollback_last_frame(self, block_idx: int) -> None:
         """Undo the most recent append_frame - flashinfer_cache.py:268-301."""
-        self._check(self._lib.gct_mgr_rollback(self._handle, block_idx))
+        self._native.rollback(self._h, block_idx)
 
     def reset(self) -> None:
         self._check(self._lib.gct_mgr_reset(self._handle))
@@ -299,18 +288,8 @@ class B200KVCacheManager:
         q [q_len, H, D] (float32 or bfloat16) -> out [q_len, H, D] bfloat16.  Like the reference, the page
         table is planned when block_idx == 0 and reused by the other blocks of the same frame."""
         self._require_device()
-        if self._stats(block_idx)[0] == 0:
-            return torch.zeros_like(q)                              # :368-370
-        q = self._check_frame_tensor(q, "q")
-        if block_idx == 0:
-            self.plan()
-        out = torch.empty(q.shape, dtype=torch.bfloat16, device=self.device)
-        lse = torch.empty(q.shape[0], self.num_heads, dtype=torch.float32, device=self.device) if return_lse else None
-        with torch.cuda.device(self.device):
-            self._check(self._lib.gct_mgr_attention(self._handle, block_idx, q.data_ptr(), _dtype_code(q), q.shape[0],
-                                                    out.data_ptr(), None if lse is None else lse.data_ptr(),
-                                                    _stream_ptr(self.device)))
-        return (out, lse) if return_lse else out
+        out = self._native.attention(self._h, self._dev_index, block_idx, q, return_lse)
+        return torch.zeros_like(q) if out is None else out          # nothing cached yet: :368-370
 
     def compute_attention_partial(self, block_idx: int, q: Tensor, out: Optional[Tensor] = None,
                                   lse: Optional[Tensor] = None):

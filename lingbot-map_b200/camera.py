@@ -18,7 +18,6 @@ import torch
 from torch import Tensor
 
 from . import _lib
-from .cache import _stream_ptr
 
 
 class DecodeCache:
@@ -53,30 +52,24 @@ class DecodeCache:
         n = q.shape[0]
         if store and self.count + n > self.capacity:
             self._grow(self.count + n)
-        out = torch.empty_like(q)
-        lib = _lib.load()
-        ws, stream = self.workspace, _stream_ptr(self.device)
-        with torch.cuda.device(self.device):
-            if n <= 8:
-                _lib.check(lib.gct_decode_attention(
-                    q.data_ptr(), k_new.data_ptr(), v_new.data_ptr(), n, self.k.data_ptr(), self.v.data_ptr(),
-                    self.count, self.capacity, 1 if store else 0, self.heads, self.head_dim, out.data_ptr(),
-                    ws.data_ptr(), ws.numel(), stream))
-            else:
-                # a scale phase of more than 8 frames: the kernel takes 8 query tokens per launch.  Each chunk of
-                # queries gets its own rows as "new" rows and all other rows (cached + the rest of this call) as the
-                # cache; the order of the keys inside a softmax does not matter.  The append is a plain copy.
-                for lo in range(0, n, 8):
-                    hi = min(lo + 8, n)
-                    ok = torch.cat([self.k[:self.count], k_new[:lo], k_new[hi:]])
-                    ov = torch.cat([self.v[:self.count], v_new[:lo], v_new[hi:]])
-                    qc, kc, vc = q[lo:hi].contiguous(), k_new[lo:hi].contiguous(), v_new[lo:hi].contiguous()
-                    _lib.check(lib.gct_decode_attention(
-                        qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), hi - lo, ok.data_ptr(), ov.data_ptr(), ok.shape[0],
-                        ok.shape[0], 0, self.heads, self.head_dim, out[lo:hi].data_ptr(), ws.data_ptr(), ws.numel(), stream))
-                if store:
-                    self.k[self.count:self.count + n].copy_(k_new)
-                    self.v[self.count:self.count + n].copy_(v_new)
+        native = _lib.binding()
+        if n <= 8:
+            out = native.decode_attention(q, k_new, v_new, self.k, self.v, self.count, store, self.workspace)
+        else:
+            # a scale phase of more than 8 frames: the kernel takes 8 query tokens per launch.  Each chunk of
+            # queries gets its own rows as "new" rows and all other rows (cached + the rest of this call) as the
+            # cache; the order of the keys inside a softmax does not matter.  The append is a plain copy.
+            outs = []
+            for lo in range(0, n, 8):
+                hi = min(lo + 8, n)
+                ok = torch.cat([self.k[:self.count], k_new[:lo], k_new[hi:]])
+                ov = torch.cat([self.v[:self.count], v_new[:lo], v_new[hi:]])
+                outs.append(native.decode_attention(q[lo:hi].contiguous(), k_new[lo:hi].contiguous(), v_new[lo:hi].contiguous(), ok, ov,
+                                                    ok.shape[0], False, self.workspace))
+            out = torch.cat(outs)
+            if store:
+                self.k[self.count:self.count + n].copy_(k_new)
+                self.v[self.count:self.count + n].copy_(v_new)
         if store:
             self.count += n
         return out

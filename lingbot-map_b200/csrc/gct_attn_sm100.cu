@@ -1060,20 +1060,24 @@ namespace {
 
 // Finish time, in KV blocks of one two-tile CTA, of `n_long` CTAs of `len_long` blocks followed by `n_short` CTAs of
 // `len_short` blocks handed out in that order to `sms` SMs, each to the SM that is free first; every CTA pays
-// `fixed` blocks of prologue and epilogue.
+// `fixed` blocks of prologue and epilogue.  After the long CTAs the SMs are free at one of two times, early or late, and
+// each then finishes a short CTA every `len_short + fixed`: the n_short-th of these finish times is the answer.  (A heap
+// over the SMs gives the same number but costs microseconds per candidate, milliseconds per new cache length.)
 double list_schedule(int n_long, double len_long, int n_short, double len_short, int sms, double fixed) {
-  // the long CTAs are equal: after them n_long % sms SMs have run one more than the others
-  const int full = n_long / sms, extra = n_long % sms;
-  std::vector<double> heap(static_cast<size_t>(sms));           // min-heap of the SMs' finish times
-  for (int i = 0; i < sms; ++i) heap[i] = (full + (i < extra ? 1 : 0)) * (len_long + fixed);
-  auto cmp = [](double x, double y) { return x > y; };
-  std::make_heap(heap.begin(), heap.end(), cmp);
-  for (int i = 0; i < n_short; ++i) {
-    std::pop_heap(heap.begin(), heap.end(), cmp);
-    heap.back() += len_short + fixed;
-    std::push_heap(heap.begin(), heap.end(), cmp);
+  const int full = n_long / sms, n_late = n_long % sms, n_early = sms - n_late;
+  double early = full * (len_long + fixed), late = (full + 1) * (len_long + fixed);
+  const double end_long = n_late > 0 ? late : early, step = len_short + fixed;
+  double t = 0.0;
+  for (int done = 0; done < n_short;) {
+    if (n_late == 0 || early <= late) {
+      t = early += step;
+      done += n_early;
+    } else {
+      t = late += step;
+      done += n_late;
+    }
   }
-  return *std::max_element(heap.begin(), heap.end());
+  return std::max(t, end_long);
 }
 
 struct SplitPlanKey {

@@ -33,6 +33,7 @@ int fail(int code, const std::string& msg);
 #ifndef GCT_PDL
 #define GCT_PDL 1
 #endif
+#ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() {
 #if GCT_PDL
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -53,6 +54,7 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
+#endif  // __CUDACC__
 
 constexpr int kHeadDim = 64;
 constexpr int kBlockN = 128;   // KV tokens per attention block (one UMMA N tile)
@@ -112,9 +114,11 @@ struct PrepLaunch {
   int src_dtype_v = GCT_BF16;
   int64_t src_token_stride = 0, src_head_stride = 64;
   int tokens = 0, heads = 0, tokens_per_frame = 0;
-  const float* qn_w = nullptr; const float* qn_b = nullptr;   // null: no LayerNorm
-  const float* kn_w = nullptr; const float* kn_b = nullptr;
-  const float* rope_cs = nullptr;    // [tokens_per_frame, 32, 2] cos,sin; null or mode NONE: no rotation
+  const void* qn_w = nullptr; const void* qn_b = nullptr;   // null: no LayerNorm
+  const void* kn_w = nullptr; const void* kn_b = nullptr;
+  int norm_dtype = GCT_F32;          // dtype of the four norm parameters
+  const void* rope_cs = nullptr;     // [tokens_per_frame, 32, 2] cos,sin; null or mode NONE: no rotation
+  bool rope_f64 = false;             // the table holds doubles (a complex128 tensor) instead of floats; 3-D mode only
   int rope_mode = GCT_ROPE_NONE;
   __nv_bfloat16* q_out = nullptr;    // [tokens, H, 64] or null
   // K/V destination, dense: [tokens, H, 64]
@@ -128,6 +132,21 @@ struct PrepLaunch {
   float* key_norm_max = nullptr;     // [H] running maximum of the 2-norms of the K rows written (paged destination)
 };
 int launch_prep(const PrepLaunch& p, cudaStream_t stream);
+
+// ---- calls behind the PyTorch binding (gct_torch.cpp) ------------------------------------
+// Same work as the C entry points of gct_b200.h; these take what PyTorch holds as it is (norm parameters in bf16, a
+// complex128 rotation table) and let the binding size its scratch before the call.
+const gct_mgr_config_t& mgr_config(const gct_mgr_t* m);
+// src: q_src / k_src / v_src, strides, dtypes, norm parameters, rotation and q_out filled in; the destination pages come
+// from the bookkeeping of this append.
+int mgr_append(gct_mgr_t* m, int block, PrepLaunch src, cudaStream_t stream);
+// (q tiles per CTA, splits) of a dense attention call with at most max_splits partial results.
+int dense_attention_plan(int batch, int n_q, int n_kv, int heads, int max_splits, int* q_tiles_per_cta, int* splits);
+// splits > 1: part_o [splits, batch * n_q * heads, 64] and part_lse [splits, batch * n_q * heads] are scratch.
+int dense_attention_run(const void* q, const void* k, const void* v, void* out, int batch, int n_q, int n_kv, int heads,
+                        const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3], int q_tiles_per_cta,
+                        int splits, float* part_o, float* part_lse, int* status, cudaStream_t stream);
+
 
 // key_norm_max[head] = max over all K rows of the pool [pages, 2, page_size, heads, 64] of their 2-norm
 int launch_scan_keys(const __nv_bfloat16* pool, int num_pages, int page_size, int heads, float* key_norm_max,

@@ -62,7 +62,7 @@ __device__ __forceinline__ float row_sum(float x) {
 
 // cs: the eight (cos, sin) pairs this lane needs.  3-D: entries 4s..4s+3 (pairs of its 8 elements), only
 // cs[0..3] used.  2-D: entries 16*half + 8*(s&1) + i for its elements i = 0..7.
-__device__ __forceinline__ void norm_rope8(Row8& x, const float* w, const float* bia, const float2 (&cs)[8],
+__device__ __forceinline__ void norm_rope8(Row8& x, const void* w, const void* bia, int norm_dtype, const float2 (&cs)[8],
                                            int rope_mode, int part) {
   if (w != nullptr) {
     float sum = 0.f;
@@ -76,12 +76,9 @@ __device__ __forceinline__ void norm_rope8(Row8& x, const float* w, const float*
       sq += x.v[i] * x.v[i];
     }
     const float rstd = rsqrtf(row_sum(sq) * (1.f / 64.f) + 1e-5f);
-    const float4 w0 = *reinterpret_cast<const float4*>(w + 8 * part), w1 = *reinterpret_cast<const float4*>(w + 8 * part + 4);
-    const float4 b0 = *reinterpret_cast<const float4*>(bia + 8 * part), b1 = *reinterpret_cast<const float4*>(bia + 8 * part + 4);
-    const float ww[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-    const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+    const Row8 ww = load8(w, norm_dtype, 8 * part), bb = load8(bia, norm_dtype, 8 * part);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) x.v[i] = x.v[i] * rstd * ww[i] + bb[i];
+    for (int i = 0; i < 8; ++i) x.v[i] = x.v[i] * rstd * ww.v[i] + bb.v[i];
   }
   if (rope_mode == GCT_ROPE_3D) {
 #pragma unroll
@@ -119,15 +116,25 @@ __global__ void __launch_bounds__(256) gct_prep_kernel(const PrepLaunch p) {
   // rotation coefficients of this lane
   float2 cs[8];
   if (p.rope_mode == GCT_ROPE_3D) {
-    const float4* t = reinterpret_cast<const float4*>(p.rope_cs + (static_cast<size_t>(tf) * 32 + 4 * part) * 2);
-    const float4 a = t[0], b = t[1];
-    cs[0] = make_float2(a.x, a.y);
-    cs[1] = make_float2(a.z, a.w);
-    cs[2] = make_float2(b.x, b.y);
-    cs[3] = make_float2(b.z, b.w);
+    const size_t e = (static_cast<size_t>(tf) * 32 + 4 * part) * 2;
+    if (p.rope_f64) {
+      const double2* t = reinterpret_cast<const double2*>(static_cast<const double*>(p.rope_cs) + e);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const double2 d = t[i];
+        cs[i] = make_float2(static_cast<float>(d.x), static_cast<float>(d.y));
+      }
+    } else {
+      const float4* t = reinterpret_cast<const float4*>(static_cast<const float*>(p.rope_cs) + e);
+      const float4 a = t[0], b = t[1];
+      cs[0] = make_float2(a.x, a.y);
+      cs[1] = make_float2(a.z, a.w);
+      cs[2] = make_float2(b.x, b.y);
+      cs[3] = make_float2(b.z, b.w);
+    }
   } else if (p.rope_mode == GCT_ROPE_2D) {
     const int entry = (part >> 2) * 16 + (part & 1) * 8;      // 16*half + (e' % 16) for this lane's first element
-    const float4* t = reinterpret_cast<const float4*>(p.rope_cs + (static_cast<size_t>(tf) * 32 + entry) * 2);
+    const float4* t = reinterpret_cast<const float4*>(static_cast<const float*>(p.rope_cs) + (static_cast<size_t>(tf) * 32 + entry) * 2);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const float4 a = t[i];
@@ -175,11 +182,11 @@ __global__ void __launch_bounds__(256) gct_prep_kernel(const PrepLaunch p) {
     v = load8(p.v_src, p.src_dtype_v, src);
   }
   if (do_q) {
-    norm_rope8(q, p.qn_w, p.qn_b, cs, p.rope_mode, part);
+    norm_rope8(q, p.qn_w, p.qn_b, p.norm_dtype, cs, p.rope_mode, part);
     if (active) store8(p.q_out + static_cast<size_t>(token) * p.heads * kHeadDim + dst, q);
   }
   if (do_kv) {
-    norm_rope8(k, p.kn_w, p.kn_b, cs, p.rope_mode, part);
+    norm_rope8(k, p.kn_w, p.kn_b, p.norm_dtype, cs, p.rope_mode, part);
     if (active) {
       store8(k_row + dst, k);
       store8(v_row + dst, v);
@@ -337,6 +344,7 @@ __global__ void gct_rope2d_table_kernel(int pph, int ppw, int ns, float base, fl
 int launch_prep(const PrepLaunch& p, cudaStream_t stream) {
   if (p.tokens <= 0 || p.heads <= 0 || p.tokens_per_frame <= 0) return fail(GCT_ERR_INVALID, "prep: bad shape");
   if (p.rope_mode != GCT_ROPE_NONE && p.rope_cs == nullptr) return fail(GCT_ERR_INVALID, "prep: rope table missing");
+  if (p.rope_mode == GCT_ROPE_2D && p.rope_f64) return fail(GCT_ERR_INVALID, "prep: the 2-D table is float");
   if ((p.src_token_stride | p.src_head_stride) & 7)
     return fail(GCT_ERR_INVALID, "prep: source strides must be multiples of 8 elements (16-byte vector loads)");
   auto misaligned = [](const void* q) { return q != nullptr && (reinterpret_cast<uintptr_t>(q) & 15) != 0; };

@@ -363,6 +363,32 @@ int gct_mgr_append_bookkeeping(gct_mgr_t* m, int block) {
   return rc;
 }
 
+// The three parts of a qkv row [3*H*64] as sources of the prologue kernel.
+static int fill_qkv_source(PrepLaunch* p, const char* who, const void* qkv, int qkv_dtype, int64_t row_stride, int heads,
+                           const float* qn_w, const float* qn_b, const float* kn_w, const float* kn_b, const float* rope_cs,
+                           int rope_mode) {
+  if (qkv == nullptr) return fail(GCT_ERR_INVALID, std::string(who) + ": null argument");
+  if (qkv_dtype != GCT_F32 && qkv_dtype != GCT_BF16) return fail(GCT_ERR_INVALID, std::string(who) + ": dtype");
+  if ((qn_w == nullptr) != (qn_b == nullptr) || (kn_w == nullptr) != (kn_b == nullptr))
+    return fail(GCT_ERR_INVALID, std::string(who) + ": norm weight and bias must come together");
+  const int64_t C = static_cast<int64_t>(heads) * kHeadDim;
+  if (row_stride < 3 * C) return fail(GCT_ERR_INVALID, std::string(who) + ": row stride smaller than 3*H*64");
+  const size_t esz = qkv_dtype == GCT_F32 ? 4 : 2;
+  p->q_src = qkv;
+  p->k_src = static_cast<const uint8_t*>(qkv) + C * esz;
+  p->v_src = static_cast<const uint8_t*>(qkv) + 2 * C * esz;
+  p->src_dtype_qk = p->src_dtype_v = qkv_dtype;
+  p->src_token_stride = row_stride;
+  p->src_head_stride = kHeadDim;
+  p->qn_w = qn_w;
+  p->qn_b = qn_b;
+  p->kn_w = kn_w;
+  p->kn_b = kn_b;
+  p->rope_cs = rope_cs;
+  p->rope_mode = rope_mode;
+  return GCT_OK;
+}
+
 static int check_bound(const gct_mgr* m) {
   if (m == nullptr) return fail(GCT_ERR_INVALID, "null manager");
   if (!m->bound) return fail(GCT_ERR_INVALID, "manager has no device memory bound (gct_mgr_bind)");
@@ -401,27 +427,41 @@ static void fill_paged_dst(const gct_mgr* m, int block, const AppendPlan& pl, Pr
   p->heads = m->cfg.num_heads;
 }
 
+}  // extern "C"
+
+namespace gct {
+const gct_mgr_config_t& mgr_config(const gct_mgr_t* m) { return m->cfg; }
+
+int mgr_append(gct_mgr_t* m, int block, PrepLaunch p, cudaStream_t stream) {
+  int rc = check_bound(m);
+  if (rc != GCT_OK) return rc;
+  AppendPlan pl;
+  rc = append_bookkeeping(m, block, &pl);
+  if (rc != GCT_OK) return rc;
+  fill_paged_dst(m, block, pl, &p);
+  rc = track_key_norms(m, block, &p, stream);
+  if (rc != GCT_OK) return rc;
+  m->launches += 1;
+  return launch_prep(p, stream);
+}
+}  // namespace gct
+
+extern "C" {
+
 int gct_mgr_append(gct_mgr_t* m, int block, const void* k_dev, int k_dtype, const void* v_dev, int v_dtype, void* stream) {
   int rc = check_bound(m);
   if (rc != GCT_OK) return rc;
   if (k_dev == nullptr || v_dev == nullptr) return fail(GCT_ERR_INVALID, "gct_mgr_append: null K/V");
   if ((k_dtype != GCT_F32 && k_dtype != GCT_BF16) || (v_dtype != GCT_F32 && v_dtype != GCT_BF16))
     return fail(GCT_ERR_INVALID, "gct_mgr_append: dtype must be GCT_F32 or GCT_BF16");
-  AppendPlan pl;
-  rc = append_bookkeeping(m, block, &pl);
-  if (rc != GCT_OK) return rc;
   PrepLaunch p;
-  fill_paged_dst(m, block, pl, &p);
   p.k_src = k_dev;
   p.v_src = v_dev;
   p.src_dtype_qk = k_dtype;
   p.src_dtype_v = v_dtype;
   p.src_token_stride = static_cast<int64_t>(m->cfg.num_heads) * kHeadDim;
   p.src_head_stride = kHeadDim;
-  rc = track_key_norms(m, block, &p, static_cast<cudaStream_t>(stream));
-  if (rc != GCT_OK) return rc;
-  m->launches += 1;
-  return launch_prep(p, static_cast<cudaStream_t>(stream));
+  return mgr_append(m, block, p, static_cast<cudaStream_t>(stream));
 }
 
 int gct_mgr_append_fused(gct_mgr_t* m, int block, const void* qkv_dev, int qkv_dtype, int64_t qkv_row_stride,
@@ -429,35 +469,13 @@ int gct_mgr_append_fused(gct_mgr_t* m, int block, const void* qkv_dev, int qkv_d
                          const float* rope_cs_dev, int rope_mode, void* q_out_dev, void* stream) {
   int rc = check_bound(m);
   if (rc != GCT_OK) return rc;
-  if (qkv_dev == nullptr || q_out_dev == nullptr) return fail(GCT_ERR_INVALID, "gct_mgr_append_fused: null argument");
-  if (qkv_dtype != GCT_F32 && qkv_dtype != GCT_BF16) return fail(GCT_ERR_INVALID, "gct_mgr_append_fused: dtype");
-  if ((qn_w_dev == nullptr) != (qn_b_dev == nullptr) || (kn_w_dev == nullptr) != (kn_b_dev == nullptr))
-    return fail(GCT_ERR_INVALID, "gct_mgr_append_fused: norm weight and bias must come together");
-  const int64_t C = static_cast<int64_t>(m->cfg.num_heads) * kHeadDim;
-  if (qkv_row_stride < 3 * C) return fail(GCT_ERR_INVALID, "gct_mgr_append_fused: row stride smaller than 3*H*64");
-  AppendPlan pl;
-  rc = append_bookkeeping(m, block, &pl);
-  if (rc != GCT_OK) return rc;
+  if (q_out_dev == nullptr) return fail(GCT_ERR_INVALID, "gct_mgr_append_fused: null argument");
   PrepLaunch p;
-  fill_paged_dst(m, block, pl, &p);
-  const size_t esz = qkv_dtype == GCT_F32 ? 4 : 2;
-  p.q_src = qkv_dev;
-  p.k_src = static_cast<const uint8_t*>(qkv_dev) + C * esz;
-  p.v_src = static_cast<const uint8_t*>(qkv_dev) + 2 * C * esz;
-  p.src_dtype_qk = p.src_dtype_v = qkv_dtype;
-  p.src_token_stride = qkv_row_stride;
-  p.src_head_stride = kHeadDim;
-  p.qn_w = qn_w_dev;
-  p.qn_b = qn_b_dev;
-  p.kn_w = kn_w_dev;
-  p.kn_b = kn_b_dev;
-  p.rope_cs = rope_cs_dev;
-  p.rope_mode = rope_mode;
-  p.q_out = static_cast<__nv_bfloat16*>(q_out_dev);
-  rc = track_key_norms(m, block, &p, static_cast<cudaStream_t>(stream));
+  rc = fill_qkv_source(&p, "gct_mgr_append_fused", qkv_dev, qkv_dtype, qkv_row_stride, m->cfg.num_heads, qn_w_dev, qn_b_dev,
+                       kn_w_dev, kn_b_dev, rope_cs_dev, rope_mode);
   if (rc != GCT_OK) return rc;
-  m->launches += 1;
-  return launch_prep(p, static_cast<cudaStream_t>(stream));
+  p.q_out = static_cast<__nv_bfloat16*>(q_out_dev);
+  return mgr_append(m, block, p, static_cast<cudaStream_t>(stream));
 }
 
 static void evict_now(gct_mgr* m, int block, int sliding_window) {
@@ -786,6 +804,52 @@ int gct_attn_launch_shape(int n_q, int heads, int kv_blocks, int num_sms, int ma
   return GCT_OK;
 }
 
+}  // extern "C"
+
+namespace gct {
+int dense_attention_plan(int batch, int n_q, int n_kv, int heads, int max_splits, int* q_tiles_per_cta, int* splits) {
+  if (batch <= 0 || n_q <= 0 || n_kv <= 0 || heads <= 0) return fail(GCT_ERR_INVALID, "dense attention: bad shape");
+  int sms = 148;
+  const int rc = device_sm_count(&sms);
+  if (rc != GCT_OK) return rc;
+  choose_attention_config((n_q + kTileM - 1) / kTileM, heads * batch, (n_kv + kBlockN - 1) / kBlockN, sms, std::max(max_splits, 1),
+                          q_tiles_per_cta, splits);
+  return GCT_OK;
+}
+
+int dense_attention_run(const void* q, const void* k, const void* v, void* out, int batch, int n_q, int n_kv, int heads,
+                        const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3], int q_tiles_per_cta,
+                        int splits, float* part_o, float* part_lse, int* status, cudaStream_t stream) {
+  AttnLaunch a;
+  // strides are (batch, token, head) in elements
+  int rc = make_tensor_map(&a.tm_q, q, heads, n_q, batch, q_strides[2], q_strides[1], q_strides[0]);
+  if (rc != GCT_OK) return rc;
+  rc = make_tensor_map(&a.tm_k, k, heads, n_kv, batch, k_strides[2], k_strides[1], k_strides[0]);
+  if (rc != GCT_OK) return rc;
+  rc = make_tensor_map(&a.tm_v, v, heads, n_kv, batch, v_strides[2], v_strides[1], v_strides[0]);
+  if (rc != GCT_OK) return rc;
+  a.page_table = nullptr;
+  a.n_pages = 1;
+  a.page_len = n_kv;
+  a.last_page_len = n_kv;
+  a.n_q = n_q;
+  a.heads = heads;
+  a.batch = batch;
+  a.status = status;
+  a.q_tiles_per_cta = q_tiles_per_cta;
+  a.splits = splits;
+  a.final_bf16 = splits == 1;
+  a.out = static_cast<__nv_bfloat16*>(out);
+  a.part_o = part_o;
+  a.part_lse = part_lse;
+  rc = launch_attention(a, stream);
+  if (rc != GCT_OK || splits == 1) return rc;
+  return launch_merge(part_o, part_lse, splits, static_cast<int64_t>(batch) * n_q * heads, a.out, nullptr, nullptr, stream);
+}
+}  // namespace gct
+
+extern "C" {
+
 int gct_attn_dense(const void* q_dev, const void* k_dev, const void* v_dev, void* out_dev, int batch, int n_q, int n_kv,
                    int heads, const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3],
                    void* workspace_dev, size_t workspace_bytes, void* stream) {
@@ -795,73 +859,30 @@ int gct_attn_dense(const void* q_dev, const void* k_dev, const void* v_dev, void
   if (batch <= 0 || n_q <= 0 || n_kv <= 0 || heads <= 0) return fail(GCT_ERR_INVALID, "gct_attn_dense: bad shape");
   if (workspace_dev == nullptr || workspace_bytes < 256 || (reinterpret_cast<uintptr_t>(workspace_dev) & 255))
     return fail(GCT_ERR_CAPACITY, "gct_attn_dense: needs a 256-byte aligned workspace of at least 256 bytes (status word)");
-  AttnLaunch a;
-  // strides are (batch, token, head) in elements
-  int rc = make_tensor_map(&a.tm_q, q_dev, heads, n_q, batch, q_strides[2], q_strides[1], q_strides[0]);
-  if (rc != GCT_OK) return rc;
-  rc = make_tensor_map(&a.tm_k, k_dev, heads, n_kv, batch, k_strides[2], k_strides[1], k_strides[0]);
-  if (rc != GCT_OK) return rc;
-  rc = make_tensor_map(&a.tm_v, v_dev, heads, n_kv, batch, v_strides[2], v_strides[1], v_strides[0]);
-  if (rc != GCT_OK) return rc;
-  a.page_table = nullptr;
-  a.n_pages = 1;
-  a.page_len = n_kv;
-  a.last_page_len = n_kv;
-  a.n_q = n_q;
-  a.heads = heads;
-  a.batch = batch;
-  a.status = static_cast<int*>(workspace_dev);
-  const int total_blocks = (n_kv + kBlockN - 1) / kBlockN;
   const size_t rows = static_cast<size_t>(batch) * n_q * heads;
   const size_t per_split = rows * kHeadDim * 4 + rows * 4;
-  const int max_splits = static_cast<int>(std::min<size_t>((workspace_bytes - 256) / per_split, kMaxSplitsCap));
-  int sms = 148;
-  rc = device_sm_count(&sms);
+  int qt = 1, splits = 1;
+  const int rc = dense_attention_plan(batch, n_q, n_kv, heads,
+                                      static_cast<int>(std::min<size_t>((workspace_bytes - 256) / per_split, kMaxSplitsCap)), &qt, &splits);
   if (rc != GCT_OK) return rc;
-  choose_attention_config((n_q + kTileM - 1) / kTileM, heads * batch, total_blocks, sms, std::max(max_splits, 1),
-                          &a.q_tiles_per_cta, &a.splits);
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (a.splits == 1) {
-    a.final_bf16 = true;
-    a.out = static_cast<__nv_bfloat16*>(out_dev);
-    return launch_attention(a, s);
-  }
-  a.final_bf16 = false;
-  a.part_o = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace_dev) + 256);
-  a.part_lse = a.part_o + static_cast<size_t>(a.splits) * rows * kHeadDim;
-  rc = launch_attention(a, s);
-  if (rc != GCT_OK) return rc;
-  return launch_merge(a.part_o, a.part_lse, a.splits, static_cast<int64_t>(rows), static_cast<__nv_bfloat16*>(out_dev),
-                      nullptr, nullptr, s);
+  float* part_o = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace_dev) + 256);
+  return dense_attention_run(q_dev, k_dev, v_dev, out_dev, batch, n_q, n_kv, heads, q_strides, k_strides, v_strides, qt, splits, part_o,
+                             part_o + static_cast<size_t>(splits) * rows * kHeadDim, static_cast<int*>(workspace_dev),
+                             static_cast<cudaStream_t>(stream));
 }
 
 int gct_prep_qkv(const void* qkv_dev, int qkv_dtype, int64_t qkv_row_stride, int tokens, int tokens_per_frame, int heads,
                  const float* qn_w_dev, const float* qn_b_dev, const float* kn_w_dev, const float* kn_b_dev,
                  const float* rope_cs_dev, int rope_mode, void* q_out_dev, void* k_out_dev, void* v_out_dev, void* stream) {
-  if (qkv_dev == nullptr || q_out_dev == nullptr || k_out_dev == nullptr || v_out_dev == nullptr)
+  if (q_out_dev == nullptr || k_out_dev == nullptr || v_out_dev == nullptr)
     return fail(GCT_ERR_INVALID, "gct_prep_qkv: null argument");
-  if (qkv_dtype != GCT_F32 && qkv_dtype != GCT_BF16) return fail(GCT_ERR_INVALID, "gct_prep_qkv: dtype");
-  if ((qn_w_dev == nullptr) != (qn_b_dev == nullptr) || (kn_w_dev == nullptr) != (kn_b_dev == nullptr))
-    return fail(GCT_ERR_INVALID, "gct_prep_qkv: norm weight and bias must come together");
-  const int64_t C = static_cast<int64_t>(heads) * kHeadDim;
-  if (qkv_row_stride < 3 * C) return fail(GCT_ERR_INVALID, "gct_prep_qkv: row stride smaller than 3*H*64");
   PrepLaunch p;
-  const size_t esz = qkv_dtype == GCT_F32 ? 4 : 2;
-  p.q_src = qkv_dev;
-  p.k_src = static_cast<const uint8_t*>(qkv_dev) + C * esz;
-  p.v_src = static_cast<const uint8_t*>(qkv_dev) + 2 * C * esz;
-  p.src_dtype_qk = p.src_dtype_v = qkv_dtype;
-  p.src_token_stride = qkv_row_stride;
-  p.src_head_stride = kHeadDim;
+  const int rc = fill_qkv_source(&p, "gct_prep_qkv", qkv_dev, qkv_dtype, qkv_row_stride, heads, qn_w_dev, qn_b_dev, kn_w_dev,
+                                 kn_b_dev, rope_cs_dev, rope_mode);
+  if (rc != GCT_OK) return rc;
   p.tokens = tokens;
   p.tokens_per_frame = tokens_per_frame;
   p.heads = heads;
-  p.qn_w = qn_w_dev;
-  p.qn_b = qn_b_dev;
-  p.kn_w = kn_w_dev;
-  p.kn_b = kn_b_dev;
-  p.rope_cs = rope_cs_dev;
-  p.rope_mode = rope_mode;
   p.q_out = static_cast<__nv_bfloat16*>(q_out_dev);
   p.k_out = static_cast<__nv_bfloat16*>(k_out_dev);
   p.v_out = static_cast<__nv_bfloat16*>(v_out_dev);

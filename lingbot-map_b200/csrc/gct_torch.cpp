@@ -1,0 +1,476 @@
+// PyTorch binding: one C call per operator.
+//
+// The operators are small (a few microseconds of GPU work for a short cache), so what the host does around a launch is
+// part of their time: through ctypes an operator spent 10-20 us in Python on argument conversion, device guards, stream
+// look-ups and one torch.empty per output (96 us per layer pair of a streamed frame, against about 100 us of kernels at the
+// start of a sequence).  These functions are plain CPython vector-call functions over at::Tensor: they check, allocate
+// from PyTorch's caching allocator, take the current stream and launch.  The computing stays behind the C ABI of
+// libgct_b200.so, which this module is linked against; nothing here includes a kernel.
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <atomic>
+#include <mutex>
+
+#include "gct_common.h"
+
+namespace {
+
+using at::Tensor;
+using gct::kHeadDim;
+
+PyObject* g_error_class = nullptr;      // _lib.GctError(code, message)
+
+// An exception of the given Python type, thrown through C++ frames and set at the boundary.
+struct Raise {
+  PyObject* type;
+  std::string msg;
+};
+[[noreturn]] void value_error(const std::string& m) { throw Raise{PyExc_ValueError, m}; }
+[[noreturn]] void type_error(const std::string& m) { throw Raise{PyExc_TypeError, m}; }
+[[noreturn]] void runtime_error(const std::string& m) { throw Raise{PyExc_RuntimeError, m}; }
+struct Failed {                          // a C ABI status code other than GCT_OK
+  int code;
+};
+void check(int rc) {
+  if (rc != GCT_OK) throw Failed{rc};
+}
+
+template <typename F>
+PyObject* guarded(F&& f) {
+  try {
+    return f();
+  } catch (const Raise& r) {
+    PyErr_SetString(r.type, r.msg.c_str());
+  } catch (const Failed& e) {
+    const char* text = gct_last_error();
+    if (e.code == GCT_ERR_POOL_EXHAUSTED || e.code == GCT_ERR_UNDERFLOW) {
+      PyErr_SetString(PyExc_AssertionError, text);      // the reference signals these with `assert`
+    } else if (g_error_class != nullptr) {
+      PyObject* exc = PyObject_CallFunction(g_error_class, "is", e.code, text);
+      if (exc != nullptr) {
+        PyErr_SetObject(g_error_class, exc);
+        Py_DECREF(exc);
+      }
+    } else {
+      PyErr_SetString(PyExc_RuntimeError, text);
+    }
+  } catch (python_error& e) {
+    e.restore();
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+  }
+  return nullptr;
+}
+
+void need(Py_ssize_t got, Py_ssize_t want, const char* who) {
+  if (got != want) type_error(std::string(who) + ": wrong number of arguments");
+}
+const Tensor& tensor(PyObject* o, const char* name) {
+  if (!THPVariable_Check(o)) type_error(std::string(name) + " must be a tensor");
+  return THPVariable_Unpack(o);
+}
+const Tensor* optional_tensor(PyObject* o, const char* name) { return o == Py_None ? nullptr : &tensor(o, name); }
+int64_t integer(PyObject* o) {
+  const long long v = PyLong_AsLongLong(o);
+  if (v == -1 && PyErr_Occurred()) throw python_error();
+  return v;
+}
+double real(PyObject* o) {
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred()) throw python_error();
+  return v;
+}
+gct_mgr_t* manager(PyObject* o) { return reinterpret_cast<gct_mgr_t*>(static_cast<uintptr_t>(PyLong_AsUnsignedLongLong(o))); }
+
+void need_cuda(const Tensor& t, const char* name) {
+  if (!t.is_cuda()) runtime_error(std::string(name) + " must be a CUDA tensor: the B200 backend has no CPU path");
+}
+int dtype_code(const Tensor& t) {
+  if (t.scalar_type() == at::kFloat) return GCT_F32;
+  if (t.scalar_type() == at::kBFloat16) return GCT_BF16;
+  type_error(std::string("unsupported dtype ") + c10::toString(t.scalar_type()) + ": the B200 backend takes float32 or bfloat16");
+}
+Tensor empty(at::IntArrayRef size, at::ScalarType dtype, const Tensor& like) {
+  return at::detail::empty_cuda(size, dtype, like.device(), c10::nullopt);
+}
+cudaStream_t stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+PyObject* wrap(Tensor t) { return THPVariable_Wrap(std::move(t)); }
+const __nv_bfloat16* bf16(const Tensor& t) { return static_cast<const __nv_bfloat16*>(t.data_ptr()); }
+
+// Status word of the operators that have no manager, one per device for the life of the process.
+int* status_of(const Tensor& like) {
+  static std::atomic<int*> words[64];
+  static std::mutex mu;
+  const int dev = like.device().index();
+  if (dev < 0 || dev >= 64) value_error("device ordinal out of range");
+  int* p = words[dev].load(std::memory_order_acquire);
+  if (p == nullptr) {
+    std::lock_guard<std::mutex> lock(mu);
+    p = words[dev].load(std::memory_order_relaxed);
+    if (p == nullptr) {
+      Tensor* word = new Tensor(at::zeros({64}, at::TensorOptions().dtype(at::kInt).device(like.device())));
+      p = word->data_ptr<int>();
+      words[dev].store(p, std::memory_order_release);
+    }
+  }
+  return p;
+}
+
+// LayerNorm parameters and rotation table as the prologue kernel takes them.  `keep` holds tensors that had to be
+// converted (a norm parameter that is neither fp32 nor bf16, or not of the dtype of the others) until the launch is queued.
+struct NormRope {
+  Tensor keep[5];
+  void fill(gct::PrepLaunch* p, PyObject* const* norm, PyObject* cs, int64_t mode) {
+    const Tensor* t[4];
+    static const char* names[4] = {"q_norm_w", "q_norm_b", "k_norm_w", "k_norm_b"};
+    bool all_bf16 = true;
+    for (int i = 0; i < 4; ++i) {
+      t[i] = optional_tensor(norm[i], names[i]);
+      if (t[i] != nullptr) {
+        need_cuda(*t[i], names[i]);
+        if (t[i]->numel() != kHeadDim) value_error(std::string(names[i]) + " must have 64 elements");
+        all_bf16 &= t[i]->scalar_type() == at::kBFloat16;
+      }
+    }
+    if ((t[0] == nullptr) != (t[1] == nullptr) || (t[2] == nullptr) != (t[3] == nullptr)) {
+      gct::set_error("norm weight and bias must come together");
+      throw Failed{GCT_ERR_INVALID};
+    }
+    const void* ptr[4] = {nullptr, nullptr, nullptr, nullptr};
+    for (int i = 0; i < 4; ++i) {
+      if (t[i] == nullptr) continue;
+      const at::ScalarType want = all_bf16 ? at::kBFloat16 : at::kFloat;
+      if (t[i]->scalar_type() == want && t[i]->is_contiguous()) {
+        ptr[i] = t[i]->data_ptr();
+      } else {
+        keep[i] = t[i]->detach().to(want).contiguous();
+        ptr[i] = keep[i].data_ptr();
+      }
+    }
+    p->qn_w = ptr[0];
+    p->qn_b = ptr[1];
+    p->kn_w = ptr[2];
+    p->kn_b = ptr[3];
+    p->norm_dtype = all_bf16 ? GCT_BF16 : GCT_F32;
+    p->rope_mode = static_cast<int>(mode);
+    const Tensor* c = optional_tensor(cs, "rope_cs");
+    if (c == nullptr || mode == GCT_ROPE_NONE) return;
+    need_cuda(*c, "rope_cs");
+    const bool is_complex = c->scalar_type() == at::kComplexFloat || c->scalar_type() == at::kComplexDouble;
+    if (c->numel() < static_cast<int64_t>(p->tokens_per_frame) * (is_complex ? 32 : 64)) value_error("rope_cs holds too few rows");
+    Tensor table = *c;
+    if (mode == GCT_ROPE_2D || !(is_complex || c->scalar_type() == at::kFloat)) {
+      if (c->scalar_type() != at::kFloat) table = is_complex ? at::view_as_real(c->to(at::kComplexFloat)) : c->to(at::kFloat);
+    }
+    if (!table.is_contiguous()) table = table.contiguous();
+    p->rope_f64 = table.scalar_type() == at::kComplexDouble;
+    p->rope_cs = table.data_ptr();
+    keep[4] = std::move(table);
+  }
+};
+
+void fill_qkv(gct::PrepLaunch* p, const Tensor& qkv, int64_t heads) {
+  const size_t esz = qkv.element_size();
+  const int64_t C = heads * kHeadDim;
+  const uint8_t* base = static_cast<const uint8_t*>(qkv.data_ptr());
+  p->q_src = base;
+  p->k_src = base + C * esz;
+  p->v_src = base + 2 * C * esz;
+  p->src_dtype_qk = p->src_dtype_v = dtype_code(qkv);
+  p->src_token_stride = qkv.stride(0);
+  p->src_head_stride = kHeadDim;
+}
+
+struct Qkv {
+  Tensor q, k, v;
+};
+Qkv prep(Tensor qkv, int64_t heads, int64_t tokens_per_frame, PyObject* const* norm, PyObject* cs, int64_t mode) {
+  need_cuda(qkv, "qkv");
+  if (qkv.dim() != 2 || qkv.size(1) != 3 * heads * kHeadDim) value_error("qkv must be [tokens, 3*H*64]");
+  if (qkv.stride(1) != 1) qkv = qkv.contiguous();
+  c10::cuda::CUDAGuard guard(qkv.device());
+  gct::PrepLaunch p;
+  fill_qkv(&p, qkv, heads);
+  p.tokens = static_cast<int>(qkv.size(0));
+  p.tokens_per_frame = static_cast<int>(tokens_per_frame);
+  p.heads = static_cast<int>(heads);
+  NormRope nr;
+  nr.fill(&p, norm, cs, mode);
+  Qkv r{empty({qkv.size(0), heads, kHeadDim}, at::kBFloat16, qkv), empty({qkv.size(0), heads, kHeadDim}, at::kBFloat16, qkv),
+        empty({qkv.size(0), heads, kHeadDim}, at::kBFloat16, qkv)};
+  p.q_out = const_cast<__nv_bfloat16*>(bf16(r.q));
+  p.k_out = const_cast<__nv_bfloat16*>(bf16(r.k));
+  p.v_out = const_cast<__nv_bfloat16*>(bf16(r.v));
+  check(gct::launch_prep(p, stream_of(qkv)));
+  return r;
+}
+
+// prep_qkv(qkv, heads, tokens_per_frame, qw, qb, kw, kb, rope_cs, rope_mode) -> (q, k, v)
+PyObject* py_prep_qkv(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 9, "prep_qkv");
+    Qkv r = prep(tensor(a[0], "qkv"), integer(a[1]), integer(a[2]), a + 3, a[7], integer(a[8]));
+    PyObject* out = PyTuple_New(3);
+    if (out == nullptr) throw python_error();
+    PyTuple_SET_ITEM(out, 0, wrap(std::move(r.q)));
+    PyTuple_SET_ITEM(out, 1, wrap(std::move(r.k)));
+    PyTuple_SET_ITEM(out, 2, wrap(std::move(r.v)));
+    return out;
+  });
+}
+
+// Split-KV partials come from the caching allocator, and only when a call splits: calls on several streams or threads
+// do not share them, and the allocator takes them back when the call returns.
+constexpr int kDenseMaxSplits = 8;
+Tensor dense(const Tensor& q, const Tensor& k, const Tensor& v, Tensor out) {
+  const Tensor* t[3] = {&q, &k, &v};
+  static const char* names[3] = {"q", "k", "v"};
+  for (int i = 0; i < 3; ++i) {
+    need_cuda(*t[i], names[i]);
+    if (t[i]->scalar_type() != at::kBFloat16 || t[i]->dim() != 4 || t[i]->size(3) != kHeadDim || t[i]->stride(3) != 1)
+      value_error(std::string(names[i]) + " must be bf16 [B, N, H, 64] with contiguous head_dim");
+  }
+  const int64_t B = q.size(0), Nq = q.size(1), H = q.size(2), Nkv = k.size(1);
+  if (k.sizes() != v.sizes() || k.size(0) != B || k.size(2) != H) value_error("k/v shape mismatch");
+  c10::cuda::CUDAGuard guard(q.device());
+  if (!out.defined()) out = empty({B, Nq, H, kHeadDim}, at::kBFloat16, q);
+  int qt = 1, splits = 1;
+  check(gct::dense_attention_plan(static_cast<int>(B), static_cast<int>(Nq), static_cast<int>(Nkv), static_cast<int>(H), kDenseMaxSplits, &qt,
+                                  &splits));
+  const int64_t rows = B * Nq * H;
+  Tensor scratch;
+  float* part = nullptr;
+  if (splits > 1) {
+    scratch = empty({splits * rows * (kHeadDim + 1)}, at::kFloat, q);
+    part = scratch.data_ptr<float>();
+  }
+  const int64_t qs[3] = {q.stride(0), q.stride(1), q.stride(2)}, ks[3] = {k.stride(0), k.stride(1), k.stride(2)},
+                vs[3] = {v.stride(0), v.stride(1), v.stride(2)};
+  check(gct::dense_attention_run(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), static_cast<int>(B), static_cast<int>(Nq),
+                                 static_cast<int>(Nkv), static_cast<int>(H), qs, ks, vs, qt, splits, part,
+                                 part == nullptr ? nullptr : part + splits * rows * kHeadDim, status_of(q), stream_of(q)));
+  return out;
+}
+
+// dense_attention(q, k, v, out | None) -> out
+PyObject* py_dense_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 4, "dense_attention");
+    const Tensor* out = optional_tensor(a[3], "out");
+    return wrap(dense(tensor(a[0], "q"), tensor(a[1], "k"), tensor(a[2], "v"), out == nullptr ? Tensor() : *out));
+  });
+}
+
+// operator_status(device_index) -> value of the status word; waits for the device
+PyObject* py_operator_status(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 1, "operator_status");
+    const c10::Device dev(c10::kCUDA, static_cast<c10::DeviceIndex>(integer(a[0])));
+    c10::cuda::CUDAGuard guard(dev);
+    const Tensor like = at::detail::empty_cuda({0}, at::kInt, dev, c10::nullopt);
+    int* word = status_of(like);
+    return PyLong_FromLong(at::from_blob(word, {1}, at::TensorOptions().dtype(at::kInt).device(dev)).item<int>());
+  });
+}
+
+// ---- cache manager ----------------------------------------------------------------------------
+
+// [tokens, H, 64] rows of one frame, contiguous
+Tensor frame_rows(const Tensor& t, const char* name, const gct_mgr_config_t& cfg, int64_t device) {
+  if (!t.is_cuda() || t.device().index() != device)
+    value_error(std::string(name) + " lives on " + t.device().str() + ", the cache on cuda:" + std::to_string(device));
+  if (t.dim() != 3 || t.size(1) != cfg.num_heads || t.size(2) != kHeadDim)
+    value_error(std::string(name) + " must be [tokens, " + std::to_string(cfg.num_heads) + ", 64]");
+  return t.is_contiguous() ? t : t.contiguous();
+}
+
+// append(manager, device, block, k, v)
+PyObject* py_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 5, "append");
+    gct_mgr_t* m = manager(a[0]);
+    const int64_t dev = integer(a[1]);
+    const Tensor k = frame_rows(tensor(a[3], "k"), "k", gct::mgr_config(m), dev), v = frame_rows(tensor(a[4], "v"), "v", gct::mgr_config(m), dev);
+    if (k.size(0) != gct::mgr_config(m).tokens_per_frame || v.size(0) != k.size(0)) value_error("k and v must hold the tokens of one frame");
+    c10::cuda::CUDAGuard guard(k.device());
+    check(gct_mgr_append(m, static_cast<int>(integer(a[2])), k.data_ptr(), dtype_code(k), v.data_ptr(), dtype_code(v), stream_of(k)));
+    Py_RETURN_NONE;
+  });
+}
+
+Tensor append_fused(gct_mgr_t* m, int64_t device, int64_t block, Tensor qkv, PyObject* const* norm, PyObject* cs, int64_t mode, Tensor q_out) {
+  const gct_mgr_config_t& cfg = gct::mgr_config(m);
+  const int64_t T = cfg.tokens_per_frame, H = cfg.num_heads;
+  if (qkv.dim() != 2 || qkv.size(0) != T || qkv.size(1) != 3 * H * kHeadDim)
+    value_error("qkv must be [" + std::to_string(T) + ", " + std::to_string(3 * H * kHeadDim) + "]");
+  if (!qkv.is_cuda() || qkv.device().index() != device) value_error("qkv lives on " + qkv.device().str() + ", the cache on cuda:" + std::to_string(device));
+  if (qkv.stride(1) != 1) qkv = qkv.contiguous();
+  c10::cuda::CUDAGuard guard(qkv.device());
+  gct::PrepLaunch p;
+  fill_qkv(&p, qkv, H);
+  p.tokens_per_frame = static_cast<int>(T);
+  NormRope nr;
+  nr.fill(&p, norm, cs, mode);
+  if (!q_out.defined()) q_out = empty({T, H, kHeadDim}, at::kBFloat16, qkv);
+  p.q_out = static_cast<__nv_bfloat16*>(q_out.data_ptr());
+  check(gct::mgr_append(m, static_cast<int>(block), p, stream_of(qkv)));
+  return q_out;
+}
+
+// append_fused(manager, device, block, qkv, qw, qb, kw, kb, rope_cs, rope_mode, q_out | None) -> q
+PyObject* py_append_fused(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 11, "append_fused");
+    const Tensor* q_out = optional_tensor(a[10], "q_out");
+    return wrap(append_fused(manager(a[0]), integer(a[1]), integer(a[2]), tensor(a[3], "qkv"), a + 4, a[8], integer(a[9]),
+                             q_out == nullptr ? Tensor() : *q_out));
+  });
+}
+
+struct Attended {
+  Tensor out, lse;
+};
+// Planning may wait for an upload eight plans back: other Python threads run meanwhile.
+struct WithoutGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+// The page table is planned at block 0 and reused by the other blocks of the frame.
+Attended attend(gct_mgr_t* m, int64_t device, int64_t block, const Tensor& q_in, bool want_lse) {
+  const gct_mgr_config_t& cfg = gct::mgr_config(m);
+  const Tensor q = frame_rows(q_in, "q", cfg, device);
+  c10::cuda::CUDAGuard guard(q.device());
+  cudaStream_t s = stream_of(q);
+  if (block == 0) {
+    WithoutGil free_others;
+    check(gct_mgr_plan(m, 0, -1, s));
+  }
+  Attended r;
+  r.out = empty(q.sizes(), at::kBFloat16, q);
+  if (want_lse) r.lse = empty({q.size(0), q.size(1)}, at::kFloat, q);
+  check(gct_mgr_attention(m, static_cast<int>(block), q.data_ptr(), dtype_code(q), static_cast<int>(q.size(0)), r.out.data_ptr(),
+                          want_lse ? r.lse.data_ptr<float>() : nullptr, s));
+  return r;
+}
+
+// attention(manager, device, block, q, want_lse) -> out | (out, lse) | None (nothing cached yet)
+PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 5, "attention");
+    gct_mgr_t* m = manager(a[0]);
+    int64_t stats[6];
+    check(gct_mgr_stats(m, static_cast<int>(integer(a[2])), stats));
+    if (stats[0] == 0) Py_RETURN_NONE;
+    const bool want_lse = PyObject_IsTrue(a[4]) == 1;
+    Attended r = attend(m, integer(a[1]), integer(a[2]), tensor(a[3], "q"), want_lse);
+    if (!want_lse) return wrap(std::move(r.out));
+    PyObject* out = PyTuple_New(2);
+    if (out == nullptr) throw python_error();
+    PyTuple_SET_ITEM(out, 0, wrap(std::move(r.out)));
+    PyTuple_SET_ITEM(out, 1, wrap(std::move(r.lse)));
+    return out;
+  });
+}
+
+// The bookkeeping calls of every layer of every frame.
+PyObject* py_append_bookkeeping(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 2, "append_bookkeeping");
+    check(gct_mgr_append_bookkeeping(manager(a[0]), static_cast<int>(integer(a[1]))));
+    Py_RETURN_NONE;
+  });
+}
+PyObject* py_evict(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 3, "evict");
+    check(gct_mgr_evict(manager(a[0]), static_cast<int>(integer(a[1])), static_cast<int>(integer(a[2]))));
+    Py_RETURN_NONE;
+  });
+}
+PyObject* py_rollback(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 2, "rollback");
+    check(gct_mgr_rollback(manager(a[0]), static_cast<int>(integer(a[1]))));
+    Py_RETURN_NONE;
+  });
+}
+
+// ---- camera head, rotation tables ---------------------------------------------------------------
+
+// decode_attention(q, k_new, v_new, cache_k, cache_v, cached, store, workspace) -> out
+PyObject* py_decode_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 8, "decode_attention");
+    const Tensor &ck = tensor(a[3], "cache_k"), &cv = tensor(a[4], "cache_v"), &ws = tensor(a[7], "workspace");
+    auto rows = [&](PyObject* o, const char* name) {
+      const Tensor& t = tensor(o, name);
+      return t.is_contiguous() ? t : t.contiguous();
+    };
+    const Tensor q = rows(a[0], "q"), k = rows(a[1], "k_new"), v = rows(a[2], "v_new");
+    const Tensor* all[5] = {&q, &k, &v, &ck, &cv};
+    for (const Tensor* t : all) {
+      need_cuda(*t, "decode attention: every tensor");
+      if (t->scalar_type() != at::kFloat || t->dim() != 3 || !t->is_contiguous() || t->size(1) != ck.size(1) || t->size(2) != ck.size(2) ||
+          t->device() != ck.device())
+        value_error("decode attention: tensors must be contiguous float32 [rows, H, D] on one device");
+    }
+    if (k.size(0) != q.size(0) || v.size(0) != q.size(0)) value_error("decode attention: q, k and v must have the same number of rows");
+    c10::cuda::CUDAGuard guard(q.device());
+    Tensor out = empty(q.sizes(), at::kFloat, q);
+    check(gct_decode_attention(q.data_ptr<float>(), k.data_ptr<float>(), v.data_ptr<float>(), static_cast<int>(q.size(0)), ck.data_ptr<float>(),
+                               cv.data_ptr<float>(), static_cast<int>(integer(a[5])), static_cast<int>(ck.size(0)), PyObject_IsTrue(a[6]) == 1,
+                               static_cast<int>(ck.size(1)), static_cast<int>(ck.size(2)), out.data_ptr<float>(), ws.data_ptr(), ws.nbytes(),
+                               stream_of(q)));
+    return wrap(std::move(out));
+  });
+}
+
+// rope3d_table(frame_index, pph, ppw, num_special, out)
+PyObject* py_rope3d_table(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 5, "rope3d_table");
+    const Tensor& out = tensor(a[4], "out");
+    need_cuda(out, "out");
+    const int64_t pph = integer(a[1]), ppw = integer(a[2]), ns = integer(a[3]);
+    if (out.scalar_type() != at::kFloat || !out.is_contiguous() || out.numel() < (ns + pph * ppw) * 64)
+      value_error("out must be contiguous float32 [tokens, 32, 2]");
+    c10::cuda::CUDAGuard guard(out.device());
+    check(gct_rope3d_table(static_cast<int>(integer(a[0])), static_cast<int>(pph), static_cast<int>(ppw), static_cast<int>(ns),
+                           out.data_ptr<float>(), stream_of(out)));
+    Py_RETURN_NONE;
+  });
+}
+
+// set_error_class(GctError)
+PyObject* py_set_error_class(PyObject*, PyObject* cls) {
+  Py_INCREF(cls);
+  Py_XDECREF(g_error_class);
+  g_error_class = cls;
+  Py_RETURN_NONE;
+}
+
+#define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr}
+PyMethodDef g_methods[] = {FAST(prep_qkv),
+                           FAST(dense_attention),
+                           FAST(operator_status),
+                           FAST(append),
+                           FAST(append_fused),
+                           FAST(attention),
+                           FAST(append_bookkeeping),
+                           FAST(evict),
+                           FAST(rollback),
+                           FAST(decode_attention),
+                           FAST(rope3d_table),
+                           {"set_error_class", py_set_error_class, METH_O, nullptr},
+                           {nullptr, nullptr, 0, nullptr}};
+PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_gct_torch", "PyTorch binding of libgct_b200.so", -1, g_methods,
+                        nullptr,               nullptr,      nullptr,                             nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__gct_torch() { return PyModule_Create(&g_module); }

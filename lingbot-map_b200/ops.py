@@ -6,33 +6,15 @@ Dense attention and the prologue are also registered as torch.library custom ope
 (`gct_b200::dense_attention`, `gct_b200::prep_qkv`) with shape-only fake implementations: the reference
 wraps whole frame blocks and `attn_pre` in torch.compile (demo.py:177-186, gct_profile.py:47-57), and a
 custom operator is traced as one opaque node instead of breaking the graph at the ctypes call."""
-import ctypes as C
 from typing import Optional
 
 import torch
 from torch import Tensor
 
 from . import _lib
-from .cache import _dtype_code, _stream_ptr
+from .cache import _stream_ptr
 
-_workspaces = {}
-
-
-def _workspace(device, nbytes: int) -> Tensor:
-    """Per-device scratch (status word + split-KV partials) for calls that have no manager.
-
-    One buffer per device, shared by every stream and thread: two dense-attention calls whose GPU work overlaps in
-    time (different streams, or several host threads) race on the split-KV partials and must be serialised by the
-    caller.  When the buffer has to grow, the status word a kernel may have set in the old one is carried over, so
-    device_status() keeps reporting it."""
-    key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
-    ws = _workspaces.get(key)
-    if ws is None or ws.numel() < nbytes:
-        new = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        if ws is not None:
-            new[:4].copy_(ws[:4])               # stream-ordered after every kernel that used the old buffer
-        _workspaces[key] = ws = new
-    return ws
+_native = _lib.binding()
 
 
 def _require_cuda(t: Tensor, name: str):
@@ -47,28 +29,7 @@ def dense_attention(q: Tensor, k: Tensor, v: Tensor, out: Optional[Tensor] = Non
     multiples of 8 elements) -> [B, Nq, H, 64] bf16 contiguous."""
     if out is None and torch.compiler.is_compiling():
         return torch.ops.gct_b200.dense_attention(q, k, v)      # one opaque node in the traced graph
-    return _dense_attention_impl(q, k, v, out)                  # eager: straight to the C ABI
-
-
-def _dense_attention_impl(q: Tensor, k: Tensor, v: Tensor, out: Optional[Tensor] = None) -> Tensor:
-    for t, n in ((q, "q"), (k, "k"), (v, "v")):
-        _require_cuda(t, n)
-        if t.dtype != torch.bfloat16 or t.dim() != 4 or t.shape[-1] != 64 or t.stride(-1) != 1:
-            raise ValueError(f"{n} must be bf16 [B, N, H, 64] with contiguous head_dim")
-    B, Nq, H, _ = q.shape
-    Nkv = k.shape[1]
-    if k.shape != v.shape or k.shape[0] != B or k.shape[2] != H:
-        raise ValueError("k/v shape mismatch")
-    if out is None:
-        out = torch.empty(B, Nq, H, 64, dtype=torch.bfloat16, device=q.device)
-    lib = _lib.load()
-    rows = B * Nq * H
-    ws = _workspace(q.device, 256 + 8 * rows * (64 * 4 + 4))
-    st = lambda t: (C.c_int64 * 3)(t.stride(0), t.stride(1), t.stride(2))
-    with torch.cuda.device(q.device):
-        _lib.check(lib.gct_attn_dense(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), B, Nq, Nkv, H,
-                                      st(q), st(k), st(v), ws.data_ptr(), ws.numel(), _stream_ptr(q.device)))
-    return out
+    return _native.dense_attention(q, k, v, out)                # eager: straight to the C ABI
 
 
 def prep_qkv(qkv: Tensor, heads: int, tokens_per_frame: int, q_norm_w, q_norm_b, k_norm_w, k_norm_b,
@@ -79,30 +40,12 @@ def prep_qkv(qkv: Tensor, heads: int, tokens_per_frame: int, q_norm_w, q_norm_b,
     if torch.compiler.is_compiling():
         return torch.ops.gct_b200.prep_qkv(qkv, heads, tokens_per_frame, q_norm_w, q_norm_b, k_norm_w, k_norm_b, rope_cs,
                                            rope_mode)
-    return _prep_qkv_impl(qkv, heads, tokens_per_frame, q_norm_w, q_norm_b, k_norm_w, k_norm_b, rope_cs, rope_mode)
-
-
-def _prep_qkv_impl(qkv: Tensor, heads: int, tokens_per_frame: int, q_norm_w, q_norm_b, k_norm_w, k_norm_b,
-                   rope_cs: Optional[Tensor], rope_mode: int):
-    _require_cuda(qkv, "qkv")
-    if qkv.dim() != 2 or qkv.shape[1] != 3 * heads * 64:
-        raise ValueError("qkv must be [tokens, 3*H*64]")
-    if qkv.stride(1) != 1:
-        qkv = qkv.contiguous()
-    T = qkv.shape[0]
-    q, k, v = (torch.empty(T, heads, 64, dtype=torch.bfloat16, device=qkv.device) for _ in range(3))
-    ptr = lambda t: None if t is None else t.data_ptr()
-    with torch.cuda.device(qkv.device):
-        _lib.check(_lib.load().gct_prep_qkv(
-            qkv.data_ptr(), _dtype_code(qkv), qkv.stride(0), T, tokens_per_frame, heads, ptr(q_norm_w), ptr(q_norm_b),
-            ptr(k_norm_w), ptr(k_norm_b), ptr(rope_cs), rope_mode, q.data_ptr(), k.data_ptr(), v.data_ptr(),
-            _stream_ptr(qkv.device)))
-    return q, k, v
+    return _native.prep_qkv(qkv, heads, tokens_per_frame, q_norm_w, q_norm_b, k_norm_w, k_norm_b, rope_cs, rope_mode)
 
 
 @torch.library.custom_op("gct_b200::dense_attention", mutates_args=())
 def _dense_attention_op(q: Tensor, k: Tensor, v: Tensor) -> Tensor:
-    return _dense_attention_impl(q, k, v, None)
+    return _native.dense_attention(q, k, v, None)
 
 
 @_dense_attention_op.register_fake
@@ -114,7 +57,7 @@ def _dense_attention_fake(q: Tensor, k: Tensor, v: Tensor) -> Tensor:
 def _prep_qkv_op(qkv: Tensor, heads: int, tokens_per_frame: int, q_norm_w: Optional[Tensor], q_norm_b: Optional[Tensor],
                  k_norm_w: Optional[Tensor], k_norm_b: Optional[Tensor], rope_cs: Optional[Tensor],
                  rope_mode: int) -> tuple[Tensor, Tensor, Tensor]:
-    return _prep_qkv_impl(qkv, heads, tokens_per_frame, q_norm_w, q_norm_b, k_norm_w, k_norm_b, rope_cs, rope_mode)
+    return _native.prep_qkv(qkv, heads, tokens_per_frame, q_norm_w, q_norm_b, k_norm_w, k_norm_b, rope_cs, rope_mode)
 
 
 @_prep_qkv_op.register_fake
@@ -128,9 +71,7 @@ def rope3d_table(frame_index: int, pph: int, ppw: int, num_special: int, device,
     n = num_special + pph * ppw
     if out is None:
         out = torch.empty(n, 32, 2, dtype=torch.float32, device=device)
-    _require_cuda(out, "out")
-    with torch.cuda.device(out.device):
-        _lib.check(_lib.load().gct_rope3d_table(frame_index, pph, ppw, num_special, out.data_ptr(), _stream_ptr(out.device)))
+    _native.rope3d_table(frame_index, pph, ppw, num_special, out)
     return out
 
 
@@ -159,8 +100,5 @@ def lse_merge(parts: Tensor, lse: Tensor, return_lse: bool = False):
 def device_status(device) -> int:
     """Status word of the manager-less operators on `device` (0 = ok; 1 = a bounded wait timed out,
     2 = an index check failed).  Synchronises the device."""
-    key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
-    ws = _workspaces.get(key)
-    if ws is None:
-        return 0
-    return int(ws[:4].view(torch.int32).item())
+    index = torch.device(device).index
+    return _native.operator_status(torch.cuda.current_device() if index is None else index)
