@@ -19,6 +19,8 @@ from torch import Tensor
 
 from . import _lib
 
+_native = _lib.binding()
+
 
 class DecodeCache:
     """K and V rows of one (refinement iteration, block) pair: [capacity, H, D] fp32, `count` rows valid."""
@@ -52,9 +54,8 @@ class DecodeCache:
         n = q.shape[0]
         if store and self.count + n > self.capacity:
             self._grow(self.count + n)
-        native = _lib.binding()
         if n <= 8:
-            out = native.decode_attention(q, k_new, v_new, self.k, self.v, self.count, store, self.workspace)
+            out = _native.decode_attention(q, k_new, v_new, self.k, self.v, self.count, store, self.workspace)
         else:
             # a scale phase of more than 8 frames: the kernel takes 8 query tokens per launch.  Each chunk of
             # queries gets its own rows as "new" rows and all other rows (cached + the rest of this call) as the
@@ -64,7 +65,7 @@ class DecodeCache:
                 hi = min(lo + 8, n)
                 ok = torch.cat([self.k[:self.count], k_new[:lo], k_new[hi:]])
                 ov = torch.cat([self.v[:self.count], v_new[:lo], v_new[hi:]])
-                outs.append(native.decode_attention(q[lo:hi].contiguous(), k_new[lo:hi].contiguous(), v_new[lo:hi].contiguous(), ok, ov,
+                outs.append(_native.decode_attention(q[lo:hi].contiguous(), k_new[lo:hi].contiguous(), v_new[lo:hi].contiguous(), ok, ov,
                                                     ok.shape[0], False, self.workspace))
             out = torch.cat(outs)
             if store:

@@ -56,6 +56,9 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 }
 #endif  // __CUDACC__
 
+// SM count of the current device (looked up once per device).
+int device_sm_count(int* out);
+
 constexpr int kHeadDim = 64;
 constexpr int kBlockN = 128;   // KV tokens per attention block (one UMMA N tile)
 constexpr int kTileM = 128;    // query rows per UMMA tile

@@ -55,7 +55,7 @@ int make_tensor_map(CUtensorMap* out, const void* base, int heads, int64_t token
 }
 
 // SM count of the current device, cached per device ordinal.
-static int device_sm_count(int* out) {
+int device_sm_count(int* out) {
   constexpr int kMaxDevices = 64;
   static std::mutex mu;
   static int cached[kMaxDevices] = {0};
