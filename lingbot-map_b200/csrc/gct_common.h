@@ -109,6 +109,18 @@ int make_tensor_map(CUtensorMap* out, const void* base, int heads, int64_t token
 void choose_attention_config(int n_q_tiles, int heads_x_batch, int total_blocks, int num_sms, int max_splits,
                              int* q_tiles_per_cta, int* splits, int* split_len = nullptr);
 
+// Frustum culling with the camera on the host (packed) or, to spare two synchronising copies, in device memory with the given
+// strides (row and column of R, step of t).
+int frustum_cull(const float* pts, int64_t n, const float* R, const float* t, const int* device_strides, float fx, float fy, float cx,
+                 float cy, int width, int height, float near_plane, float far_plane, uint8_t* visible, cudaStream_t stream);
+// Voxelisation of up to kVoxelMaxPoints points: sort (scratch of `bytes`; `report`: pinned host memory of tiles + 1 ints;
+// waits for the stream), then, with outputs sized by the number of voxels, gather.
+constexpr int64_t kVoxelMaxPoints = 256 * 2048;
+int voxel_sort_layout(int64_t n, size_t* bytes, int* tiles);
+int voxel_sort(const float* xyz, float voxel_size, int64_t n, void* scratch, int32_t* report, int64_t* voxels_out, cudaStream_t stream);
+int voxel_gather(const float* xyz, const float* rgb, float voxel_size, int64_t n, void* scratch, float* centers, float* colors,
+                 int64_t* codes, cudaStream_t stream);
+
 // ---- elementwise kernels ---------------------------------------------------------------
 struct PrepLaunch {
   // sources: rows of 64 elements; element strides between tokens and heads

@@ -347,8 +347,12 @@ Attended attend(gct_mgr_t* m, int64_t device, int64_t block, const Tensor& q_in,
   c10::cuda::CUDAGuard guard(q.device());
   cudaStream_t s = stream_of(q);
   if (block == 0) {
-    WithoutGil free_others;
-    check(gct_mgr_plan(m, 0, -1, s));
+    int rc;
+    {
+      WithoutGil free_others;
+      rc = gct_mgr_plan(m, 0, -1, s);
+    }
+    check(rc);
   }
   Attended r;
   r.out = empty(q.sizes(), at::kBFloat16, q);
@@ -446,6 +450,82 @@ PyObject* py_rope3d_table(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+// ---- point clouds -------------------------------------------------------------------------------
+
+Tensor float_rows(const Tensor& t, const char* name) {
+  need_cuda(t, name);
+  Tensor r = t.is_contiguous() ? t : t.contiguous();
+  return r.scalar_type() == at::kFloat ? r : r.to(at::kFloat);
+}
+
+// frustum_cull(pts, R_cw, t_cw, fx, fy, cx, cy, W, H, near, far) -> bool mask
+PyObject* py_frustum_cull(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 11, "frustum_cull");
+    const Tensor pts = float_rows(tensor(a[0], "pts"), "pts");
+    Tensor R = tensor(a[1], "R_cw").detach(), t = tensor(a[2], "t_cw").detach();
+    if (R.numel() != 9 || t.numel() != 3) value_error("R_cw must hold 9 values, t_cw 3");
+    c10::cuda::CUDAGuard guard(pts.device());
+    const bool on_device = R.is_cuda() || t.is_cuda();
+    // a camera of which one half is on the device goes there whole: a copy to the device does not wait, one back does
+    auto place = [&](Tensor x) {
+      if (x.scalar_type() != at::kFloat) x = x.to(at::kFloat);
+      if (on_device && x.device() != pts.device()) x = x.to(pts.device());
+      return on_device || x.is_contiguous() ? x : x.contiguous();
+    };
+    R = place(R);
+    t = place(t);
+    if (R.dim() != 2) R = R.reshape({3, 3});
+    if (t.dim() != 1) t = t.reshape({3});
+    const int strides[3] = {static_cast<int>(R.stride(0)), static_cast<int>(R.stride(1)), static_cast<int>(t.stride(0))};
+    const int64_t count = pts.size(0);
+    Tensor visible = empty({count}, at::kBool, pts);
+    if (count > 0)
+      check(gct::frustum_cull(pts.data_ptr<float>(), count, R.data_ptr<float>(), t.data_ptr<float>(), on_device ? strides : nullptr, static_cast<float>(real(a[3])),
+                              static_cast<float>(real(a[4])), static_cast<float>(real(a[5])), static_cast<float>(real(a[6])),
+                              static_cast<int>(integer(a[7])), static_cast<int>(integer(a[8])), static_cast<float>(real(a[9])),
+                              static_cast<float>(real(a[10])), static_cast<uint8_t*>(visible.data_ptr()), stream_of(pts)));
+    return wrap(std::move(visible));
+  });
+}
+
+// voxelize_frame(xyz, rgb, voxel_size) -> (centers, colors, codes) | None (more points than the sort takes)
+PyObject* py_voxelize_frame(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 3, "voxelize_frame");
+    const Tensor &in_xyz = tensor(a[0], "pts_xyz"), &in_rgb = tensor(a[1], "pts_rgb");
+    need_cuda(in_xyz, "pts_xyz");
+    const int64_t count = in_xyz.size(0);
+    if (count < 1 || count > gct::kVoxelMaxPoints) Py_RETURN_NONE;
+    const Tensor xyz = float_rows(in_xyz, "pts_xyz"), rgb = float_rows(in_rgb, "pts_rgb");
+    if (xyz.numel() != 3 * count || rgb.numel() != 3 * count) value_error("pts_xyz and pts_rgb must be [N, 3]");
+    const float voxel = static_cast<float>(real(a[2]));
+    c10::cuda::CUDAGuard guard(xyz.device());
+    cudaStream_t s = stream_of(xyz);
+    size_t bytes = 0;
+    int tiles = 0;
+    check(gct::voxel_sort_layout(count, &bytes, &tiles));
+    Tensor scratch = empty({static_cast<int64_t>(bytes)}, at::kByte, xyz);
+    Tensor report = at::empty({tiles + 1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+    int64_t voxels = 0;
+    int rc;
+    {
+      WithoutGil free_others;      // waits: the outputs are sized by the number of voxels
+      rc = gct::voxel_sort(xyz.data_ptr<float>(), voxel, count, scratch.data_ptr(), report.data_ptr<int32_t>(), &voxels, s);
+    }
+    check(rc);
+    Tensor centers = empty({voxels, 3}, at::kFloat, xyz), colors = empty({voxels, 3}, at::kFloat, xyz), codes = empty({voxels}, at::kLong, xyz);
+    check(gct::voxel_gather(xyz.data_ptr<float>(), rgb.data_ptr<float>(), voxel, count, scratch.data_ptr(), centers.data_ptr<float>(),
+                            colors.data_ptr<float>(), codes.data_ptr<int64_t>(), s));
+    PyObject* out = PyTuple_New(3);
+    if (out == nullptr) throw python_error();
+    PyTuple_SET_ITEM(out, 0, wrap(std::move(centers)));
+    PyTuple_SET_ITEM(out, 1, wrap(std::move(colors)));
+    PyTuple_SET_ITEM(out, 2, wrap(std::move(codes)));
+    return out;
+  });
+}
+
 // set_error_class(GctError)
 PyObject* py_set_error_class(PyObject*, PyObject* cls) {
   Py_INCREF(cls);
@@ -466,6 +546,8 @@ PyMethodDef g_methods[] = {FAST(prep_qkv),
                            FAST(rollback),
                            FAST(decode_attention),
                            FAST(rope3d_table),
+                           FAST(frustum_cull),
+                           FAST(voxelize_frame),
                            {"set_error_class", py_set_error_class, METH_O, nullptr},
                            {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_gct_torch", "PyTorch binding of libgct_b200.so", -1, g_methods,

@@ -1,15 +1,15 @@
 """Point-cloud helpers of the reference's offline renderer on this library's kernels.
 
 Same call signatures as demo_render/render_cuda_ext/render_cuda_ext/_api.py (`frustum_cull`, `voxelize_frame`);
-the sort, gather and compaction around the Morton kernel are the same tensor-library calls the reference makes
-(voxel_morton.cu:98-114 uses at::sort / index_select / nonzero).  The renderer itself (Open3D / Filament) needs a
+a frame's cloud is voxelised by this library's own sort and gather, a larger one by the tensor-library calls
+the reference makes around its Morton kernel (voxel_morton.cu:98-114 uses at::sort / index_select / nonzero).  The renderer itself (Open3D / Filament) needs a
 graphics API and is not part of this package."""
-import ctypes as C
-
 import torch
 
 from . import _lib
 from .cache import _stream_ptr
+
+_native = _lib.binding()
 
 
 def frustum_cull(pts: torch.Tensor, R_cw: torch.Tensor, t_cw: torch.Tensor, fx: float, fy: float, cx: float, cy: float,
@@ -17,16 +17,7 @@ def frustum_cull(pts: torch.Tensor, R_cw: torch.Tensor, t_cw: torch.Tensor, fx: 
     """Visible mask [N] bool of points [N, 3] fp32 for the camera (R_cw, t_cw), frustum_cull.cu:35-53."""
     if not pts.is_cuda:
         raise RuntimeError("pts must be a CUDA tensor: there is no CPU path")
-    pts = pts.contiguous().float()
-    n = pts.shape[0]
-    vis = torch.zeros(n, dtype=torch.uint8, device=pts.device)
-    if n:
-        R = (C.c_float * 9)(*[float(x) for x in R_cw.detach().float().cpu().reshape(-1).tolist()])
-        t = (C.c_float * 3)(*[float(x) for x in t_cw.detach().float().cpu().reshape(-1).tolist()])
-        with torch.cuda.device(pts.device):
-            _lib.check(_lib.load().gct_frustum_cull(pts.data_ptr(), n, R, t, fx, fy, cx, cy, W, H, near_plane, far_plane,
-                                                    vis.data_ptr(), _stream_ptr(pts.device)))
-    return vis.bool()
+    return _native.frustum_cull(pts, R_cw, t_cw, fx, fy, cx, cy, W, H, near_plane, far_plane)
 
 
 def voxelize_frame(pts_xyz: torch.Tensor, pts_rgb: torch.Tensor, voxel_size: float):
@@ -38,6 +29,10 @@ def voxelize_frame(pts_xyz: torch.Tensor, pts_rgb: torch.Tensor, voxel_size: flo
     n = pts_xyz.shape[0]
     if n == 0:
         return (torch.zeros(0, 3, device=dev), torch.zeros(0, 3, device=dev), torch.zeros(0, dtype=torch.int64, device=dev))
+    out = _native.voxelize_frame(pts_xyz, pts_rgb, voxel_size)
+    if out is not None:
+        return out
+    # a cloud of many frames (over 524,288 points): the tensor library's sort around the Morton kernel
     xyz, rgb = pts_xyz.contiguous().float(), pts_rgb.contiguous().float()
     codes = torch.empty(n, dtype=torch.int64, device=dev)
     centers = torch.empty(n, 3, dtype=torch.float32, device=dev)

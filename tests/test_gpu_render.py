@@ -66,3 +66,46 @@ def test_large_cloud_properties():
     idx = torch.arange(0, n, 9973, device=DEV)
     want = R.frustum_cull(xyz[idx].cpu().numpy(), Rm, t, *args)
     assert np.array_equal(vis[idx].cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("n", [1, 2047, 2048, 2049, 2 * 2048 + 1, 65536])
+@pytest.mark.parametrize("extent", [3, 100, 5000, 2 ** 20 - 1])
+def test_voxelize_frame_sort_edges(n, extent):
+    """The frame-sized sort at the edges of its tiles (2048 points) and for clouds whose voxel indices need from one pass
+    (within +-7) over the five that are launched first (below 2^12) to all eight (2^20); every index twice, so that the
+    order among equal keys shows in the colours."""
+    rs = np.random.RandomState(n + extent)
+    idx = rs.randint(-extent, extent + 1, (n, 3))
+    idx[n // 2:] = idx[:n - n // 2]
+    xyz = (idx + 0.5).astype(np.float32)                   # voxel size 1: exact
+    rgb = rs.rand(n, 3).astype(np.float32)
+    c, col, codes = RO.voxelize_frame(torch.from_numpy(xyz).to(DEV), torch.from_numpy(rgb).to(DEV), 1.0)
+    wc, wcol, wcodes = R.voxelize_frame(xyz, rgb, 1.0)
+    assert np.array_equal(codes.cpu().numpy(), wcodes)
+    assert np.array_equal(c.cpu().numpy(), wc)
+    assert np.array_equal(col.cpu().numpy(), wcol)
+
+
+@pytest.mark.parametrize("depths", [(0.5, 5.0), (1e-38, 1e-36), (1e36, 3e38)])
+@pytest.mark.parametrize("camera_on", ["cpu", "cuda:0"])
+def test_frustum_cull_on_image_borders(depths, camera_on):
+    """Points whose projections lie within a few rounding steps of the image borders, where the test without divisions must
+    hand over to the exact one, and depths whose reciprocal leaves the float range.  Transposed and strided cameras."""
+    rs = np.random.RandomState(3)
+    n, (fx, fy, cx, cy, W, H) = 40000, (300.0, 310.0, 259.0, 189.0, 518, 378)
+    z = np.exp(rs.uniform(np.log(depths[0]), np.log(depths[1]), n)).astype(np.float32)
+    u = rs.choice([-1.0, 0.0, W, W - 1, 200.5], n) + rs.randint(-3, 4, n) * rs.choice([0.0, 3e-8, 3e-5, 1e-3, 0.3], n)
+    v = rs.choice([-1.0, 0.0, H, H - 1, 100.5], n) + rs.randint(-3, 4, n) * rs.choice([0.0, 3e-8, 3e-5, 1e-3, 0.3], n)
+    with np.errstate(over="ignore"):
+        cam = np.stack([((u - cx) / fx * z).astype(np.float32), ((v - cy) / fy * z).astype(np.float32), z], axis=1)
+    perm = np.array([[0, 1, 0], [0, 0, 1], [1, 0, 0]], np.float32)        # exact in floats; its transpose is not itself
+    pts = np.ascontiguousarray(cam @ perm)
+    t = np.zeros(3, np.float32)
+    args = (fx, fy, cx, cy, W, H, depths[0] * 0.9, min(depths[1] * 1.1, 3.3e38))
+    Rm = torch.from_numpy(np.ascontiguousarray(perm.T)).to(camera_on).t()
+    tt = torch.zeros(6, device=camera_on)[::2]
+    got = RO.frustum_cull(torch.from_numpy(pts).to(DEV), Rm, tt, *args).cpu().numpy()
+    with np.errstate(all="ignore"):
+        want = R.frustum_cull(pts, perm, t, *args)
+    assert np.array_equal(got, want)
+    assert 0.02 < want.mean() < 0.98
