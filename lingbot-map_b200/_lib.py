@@ -109,9 +109,9 @@ def binding():
     global _binding
     if _binding is None:
         load()
-        import torch  # noqa: F401  (its libraries must be in the process before the binding is)
+        import torch        # its libraries must be in the process before the binding is
         from . import _gct_torch
-        _gct_torch.set_error_class(GctError)
+        _gct_torch.set_classes(GctError, torch.nn.Parameter)
         _binding = _gct_torch
     return _binding
 

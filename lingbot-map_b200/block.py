@@ -15,9 +15,28 @@ from typing import Callable, Optional
 
 import torch
 from torch import Tensor, nn
+from torch.nn.modules import module as _nn_module
 
 from . import _lib, ops
 from .cache import B200KVCacheManager
+
+_native = _lib.binding()
+
+
+def _stock(m: nn.Module, cls) -> bool:
+    """m is a plain `cls`: nothing hooks into it and its forward has not been rebound on the instance."""
+    return type(m) is cls and not m._forward_hooks and not m._forward_pre_hooks and "forward" not in m.__dict__
+
+
+def _stock_dropout(m: nn.Module) -> bool:
+    return (_stock(m, nn.Identity) or _stock(m, nn.Dropout)) and (type(m) is nn.Identity or m.p == 0.0 or not m.training)
+
+
+def _may_fuse() -> bool:
+    """Whole layers run as one native call in eager inference only: under torch.compile the modules are traced, with
+    gradients enabled the Linear layers record them, and global hooks want to see every module."""
+    return not (torch.is_grad_enabled() or torch.compiler.is_compiling() or _nn_module._global_forward_hooks
+                or _nn_module._global_forward_pre_hooks)
 
 
 def _reference_classes():
@@ -102,6 +121,29 @@ class _AttentionBase(nn.Module):
         f = lambda p: p.detach().to(torch.float32).contiguous()
         return f(self.q_norm.weight), f(self.q_norm.bias), f(self.k_norm.weight), f(self.k_norm.bias)
 
+    def _layer_params(self):
+        """(qkv weight and bias, the four q/k norm parameters, proj weight and bias) when the sub-modules are the stock
+        ones, else None."""
+        mods = self._modules
+        qkv, proj, qn, kn = mods["qkv"], mods["proj"], mods["q_norm"], mods["k_norm"]
+        if not (_stock(qkv, nn.Linear) and _stock(proj, nn.Linear) and _stock_dropout(mods["proj_drop"])):
+            return None
+        if _stock(qn, nn.Identity) and _stock(kn, nn.Identity):
+            norm = (None, None, None, None)
+        elif _stock(qn, nn.LayerNorm) and _stock(kn, nn.LayerNorm):
+            norm = (qn.weight, qn.bias, kn.weight, kn.bias)
+            if any(p is None for p in norm):
+                return None
+        else:
+            return None
+        return (qkv.weight, qkv.bias) + norm + (proj.weight, proj.bias)
+
+    def _rope_kind(self, pos, enable_3d_rope):
+        """(rope mode, base frequency) for the native layers."""
+        if self.rope is None or pos is None:
+            return _lib.ROPE_NONE, 0.0
+        return (_lib.ROPE_3D, 0.0) if enable_3d_rope else (_lib.ROPE_2D, float(getattr(self.rope, "base_frequency", 100.0)))
+
     def _rope_args(self, pos, enable_3d_rope):
         if self.rope is None or pos is None:
             return None, _lib.ROPE_NONE
@@ -131,6 +173,12 @@ class B200FrameAttention(_AttentionBase):
 
     def forward(self, x: Tensor, pos=None, num_patches=None, num_special=None, num_frames=None,
                 enable_3d_rope=False) -> Tensor:
+        if _may_fuse():
+            params = self._layer_params()
+            if params is not None:
+                y = _native.frame_layer(x, params, self.num_heads, pos, *self._rope_kind(pos, enable_3d_rope))
+                if y is not NotImplemented:
+                    return y
         out, _, _ = self._dense(x, pos, enable_3d_rope, tokens_per_frame=x.shape[1])
         return self.proj_drop(self.proj(out.to(x.dtype) if x.dtype != torch.bfloat16 else out))
 
@@ -280,6 +328,10 @@ class B200Block(nn.Module):
                 enable_3d_rope=enable_3d_rope, kv_cache=kv_cache, global_idx=global_idx,
                 num_frame_per_block=num_frame_per_block, num_frame_for_scale=num_frame_for_scale,
                 num_register_tokens=num_register_tokens)
+        if _may_fuse():
+            y = self._fused_forward(x, pos, num_frames, enable_3d_rope, kv_cache, global_idx)
+            if y is not NotImplemented:
+                return y
         is_streaming = kv_cache is not None and (num_frames is None or num_frames <= 1)
         if is_streaming:
             if "attn_pre" in self.__dict__:      # rebound by the caller (compile_model): keep its compiled region
@@ -298,6 +350,33 @@ class B200Block(nn.Module):
                                        num_frame_for_scale=num_frame_for_scale,
                                        num_register_tokens=num_register_tokens))
         return self.ffn_residual(x)
+
+    def _fused_forward(self, x, pos, num_frames, enable_3d_rope, manager, global_idx):
+        """The forward below as one native call where every sub-module is the stock one; NotImplemented elsewhere.  An
+        attn_pre rebound on the instance keeps the module code, a rebound ffn_residual is called."""
+        mods, own = self._modules, self.__dict__
+        attn, norm1, ls1, ls2 = mods["attn"], mods["norm1"], mods["ls1"], mods["ls2"]
+        if not (_stock(attn, B200Attention) and _stock(norm1, nn.LayerNorm) and (_stock(ls1, LayerScale) or _stock(ls1, nn.Identity))
+                and "attn_pre" not in own and (manager is None or type(manager) is B200KVCacheManager and manager._bound)):
+            return NotImplemented
+        params = attn._layer_params()
+        if params is None:
+            return NotImplemented
+        norm2, mlp = mods["norm2"], mods["mlp"]
+        ffn = "ffn_residual" not in own and _stock(mlp, Mlp) and _stock(norm2, nn.LayerNorm) and (_stock(ls2, LayerScale) or _stock(ls2, nn.Identity))
+        fc1 = fc2 = None
+        if ffn:
+            parts = mlp._modules
+            fc1, fc2, act = parts["fc1"], parts["fc2"], parts["act"]
+            ffn = (_stock(fc1, nn.Linear) and _stock(fc2, nn.Linear) and _stock(act, nn.GELU) and act.approximate == "none"
+                   and _stock_dropout(parts["drop"]))
+        tail = ((norm2.weight, norm2.bias, fc1.weight, fc1.bias, fc2.weight, fc2.bias, getattr(ls2, "gamma", None)) if ffn
+                else (None,) * 7)
+        handle, device, skip = (0, 0, False) if manager is None else (manager._h, manager._dev_index, bool(manager._skip_append))
+        y = _native.block_layer(x, (norm1.weight, norm1.bias) + params + (getattr(ls1, "gamma", None),) + tail, norm1.eps,
+                                norm2.eps if ffn else 0.0, attn.num_heads, ffn, pos, *attn._rope_kind(pos, enable_3d_rope), handle, device,
+                                global_idx, attn.kv_cache_sliding_window, num_frames or 1, skip)
+        return y if ffn or y is NotImplemented else self.ffn_residual(y)
 
     def ffn_residual(self, x: Tensor) -> Tensor:
         return x + self.ls2(self.mlp(self.norm2(x)))

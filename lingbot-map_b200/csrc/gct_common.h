@@ -163,6 +163,28 @@ int dense_attention_run(const void* q, const void* k, const void* v, void* out, 
                         int splits, float* part_o, float* part_lse, int* status, cudaStream_t stream);
 
 
+// Residual sum and LayerNorm of rows: v = x + gamma * y to sum_out (y null: v = x, nothing stored), LayerNorm(v) to norm_out
+// (null: not wanted).
+constexpr int kRowMaxCols = 2048;
+struct RowLaunch {
+  int64_t rows = 0;
+  int cols = 0;
+  const void* x = nullptr;
+  int x_dtype = GCT_BF16;
+  const __nv_bfloat16* y = nullptr;
+  const void* gamma = nullptr;       // [cols]; null: 1
+  int gamma_dtype = GCT_F32;
+  void* sum_out = nullptr;
+  int sum_dtype = GCT_BF16;
+  const void* norm_w = nullptr; const void* norm_b = nullptr;
+  int norm_dtype = GCT_F32;
+  float eps = 1e-5f;
+  __nv_bfloat16* norm_out = nullptr;
+};
+int launch_residual_norm(const RowLaunch& p, cudaStream_t stream);
+// Table of the 2-D rotation [tokens, 32, 2] from integer positions [tokens, 2] with the given strides.
+int launch_rope2d_positions(const int64_t* pos, int64_t token_stride, int64_t axis_stride, int tokens, float base, float* cs, cudaStream_t stream);
+
 // key_norm_max[head] = max over all K rows of the pool [pages, 2, page_size, heads, 64] of their 2-norm
 int launch_scan_keys(const __nv_bfloat16* pool, int num_pages, int page_size, int heads, float* key_norm_max,
                      cudaStream_t stream);

@@ -207,6 +207,97 @@ __global__ void __launch_bounds__(256) gct_prep_kernel(const PrepLaunch p) {
   }
 }
 
+// v = x + gamma * y per row, stored in x's precision, and LayerNorm(v) as bf16: the residual sums and norms of a block
+// (lingbot_map/layers/block.py:217-310) in one pass over the row, which as separate tensor operations were four to
+// six launches of 2-7 us each (scale, add, norm in fp32, cast to bf16 for the next Linear).  One warp per row, the row in
+// registers: 12 MB for 1005 x 1024 in bf16, so the time is one round trip to memory.
+template <int kChunks>                    // 8-element chunks per lane: columns <= 256 * kChunks
+__global__ void __launch_bounds__(128) gct_residual_norm_kernel(const RowLaunch p) {
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const int64_t row = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  if (row >= p.rows) return;
+  const size_t base = static_cast<size_t>(row) * p.cols;
+  Row8 v[kChunks];
+  float sum = 0.f;
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c) {
+    const int col = 8 * (32 * c + lane);
+    if (col < p.cols) v[c] = load8(p.x, p.x_dtype, base + col);
+  }
+  if (p.y != nullptr) {
+#pragma unroll
+    for (int c = 0; c < kChunks; ++c) {
+      const int col = 8 * (32 * c + lane);
+      if (col >= p.cols) continue;
+      const Row8 y = load8(p.y, GCT_BF16, base + col);
+      if (p.gamma != nullptr) {
+        const Row8 g = load8(p.gamma, p.gamma_dtype, col);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[c].v[i] = fmaf(y.v[i], g.v[i], v[c].v[i]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[c].v[i] += y.v[i];
+      }
+      if (p.sum_dtype == GCT_F32) {
+        float4* d = reinterpret_cast<float4*>(static_cast<float*>(p.sum_out) + base + col);
+        d[0] = make_float4(v[c].v[0], v[c].v[1], v[c].v[2], v[c].v[3]);
+        d[1] = make_float4(v[c].v[4], v[c].v[5], v[c].v[6], v[c].v[7]);
+      } else {
+        store8(static_cast<__nv_bfloat16*>(p.sum_out) + base + col, v[c]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[c].v[i] = __bfloat162float(__float2bfloat16_rn(v[c].v[i]));      // the norm is that of the stored sum
+      }
+    }
+  }
+  if (p.norm_out == nullptr) return;
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c)
+    if (8 * (32 * c + lane) < p.cols)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) sum += v[c].v[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  const float mean = sum / p.cols;
+  float sq = 0.f;
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c)
+    if (8 * (32 * c + lane) < p.cols)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        v[c].v[i] -= mean;
+        sq = fmaf(v[c].v[i], v[c].v[i], sq);
+      }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+  const float rstd = rsqrtf(sq / p.cols + p.eps);
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c) {
+    const int col = 8 * (32 * c + lane);
+    if (col >= p.cols) continue;
+    Row8 r;
+    const Row8 w = load8(p.norm_w, p.norm_dtype, col), b = load8(p.norm_b, p.norm_dtype, col);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) r.v[i] = fmaf(v[c].v[i] * rstd, w.v[i], b.v[i]);
+    store8(p.norm_out + base + col, r);
+  }
+}
+
+// cos/sin table of the 2-D rotation from integer (y, x) positions [tokens, 2] (lingbot_map/layers/rope.py:105-119): entry
+// 16 * axis + j is the angle position * base^(-2j/32) in fp32.
+__global__ void gct_rope2d_positions_kernel(const int64_t* __restrict__ pos, int64_t token_stride, int64_t axis_stride, int tokens, float base,
+                                            float* __restrict__ cs) {
+  pdl_wait();
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= tokens * 32) return;
+  const int token = idx >> 5, axis = (idx >> 4) & 1, j = idx & 15;
+  const float inv = 1.0f / powf(base, static_cast<float>(2 * j) / 32.0f);
+  const float ang = static_cast<float>(pos[token * token_stride + axis * axis_stride]) * inv;
+  float sn, cn;
+  sincosf(ang, &sn, &cn);
+  *reinterpret_cast<float2*>(cs + 2 * idx) = make_float2(cn, sn);
+}
+
 __global__ void gct_cast_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, int64_t n4) {
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4; i += stride) {
@@ -356,6 +447,25 @@ int launch_prep(const PrepLaunch& p, cudaStream_t stream) {
   const long long warps = static_cast<long long>(p.tokens) * head_groups;
   const int blocks = static_cast<int>((warps * 32 + 255) / 256);
   GCT_CUDA_CHECK(launch_pdl(gct_prep_kernel, dim3(blocks), dim3(256), 0, stream, p));
+  return GCT_OK;
+}
+
+int launch_residual_norm(const RowLaunch& p, cudaStream_t stream) {
+  if (p.rows <= 0 || p.cols <= 0 || p.cols % 8 != 0 || p.cols > kRowMaxCols) return fail(GCT_ERR_INVALID, "residual norm: bad shape");
+  auto misaligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) != 0; };
+  if (misaligned(p.x) || misaligned(p.y) || misaligned(p.gamma) || misaligned(p.norm_w) || misaligned(p.norm_b) || misaligned(p.sum_out) ||
+      misaligned(p.norm_out))
+    return fail(GCT_ERR_INVALID, "residual norm: tensors must be 16-byte aligned");
+  const dim3 grid(static_cast<unsigned>((p.rows + 3) / 4)), block(128);
+  const int chunks = (p.cols + 255) / 256;
+  auto kernel = chunks <= 1 ? gct_residual_norm_kernel<1> : chunks <= 2 ? gct_residual_norm_kernel<2> : chunks <= 4 ? gct_residual_norm_kernel<4> : gct_residual_norm_kernel<8>;
+  GCT_CUDA_CHECK(launch_pdl(kernel, grid, block, 0, stream, p));
+  return GCT_OK;
+}
+
+int launch_rope2d_positions(const int64_t* pos, int64_t token_stride, int64_t axis_stride, int tokens, float base, float* cs, cudaStream_t stream) {
+  const dim3 grid((tokens * 32 + 255) / 256), block(256);
+  GCT_CUDA_CHECK(launch_pdl(gct_rope2d_positions_kernel, grid, block, 0, stream, pos, token_stride, axis_stride, tokens, base, cs));
   return GCT_OK;
 }
 

@@ -7,6 +7,7 @@
 // from PyTorch's caching allocator, take the current stream and launch.  The computing stays behind the C ABI of
 // libgct_b200.so, which this module is linked against; nothing here includes a kernel.
 #include <ATen/ATen.h>
+#include <ATen/autocast_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -404,6 +405,230 @@ PyObject* py_rollback(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+// ---- whole layers -------------------------------------------------------------------------------
+//
+// The streaming forward of the frame attention layer and of the global block in one call each: this library's kernels
+// around the library GEMMs of the Linear layers.  As modules, a layer pair was some fifty launches and as many Python
+// round trips (0.8 ms of host time for 0.2-0.6 ms of GPU work): casts of activations and norm parameters for autocast, the
+// rotation tables element by element, norms, scales and sums one operation each.  The caller (block.py) makes sure that the
+// modules are the stock ones; what is left to check here returns NotImplemented, and the module code runs instead.
+
+PyObject* g_parameter_class = nullptr;
+
+struct NotStock {};
+// A plain tensor or parameter (no tensor subclass), or nothing.
+const Tensor* stock(PyObject* o) {
+  if (o == Py_None) return nullptr;
+  if (!THPVariable_CheckExact(o) && reinterpret_cast<PyObject*>(Py_TYPE(o)) != g_parameter_class) throw NotStock{};
+  return &THPVariable_Unpack(o);
+}
+
+// bf16 is what the Linear layers compute in: under autocast whatever the parameters are, else only if all of it is bf16.
+struct Precision {
+  bool autocast;
+  Precision(const Tensor& x) {
+    autocast = at::autocast::is_autocast_enabled(at::kCUDA);
+    const bool known = x.scalar_type() == at::kFloat || x.scalar_type() == at::kBFloat16;
+    if (!known || (autocast ? at::autocast::get_autocast_dtype(at::kCUDA) != at::kBFloat16 : x.scalar_type() != at::kBFloat16)) throw NotStock{};
+  }
+  // a Linear parameter in bf16, from autocast's own cache where it keeps one
+  Tensor linear(PyObject* o) const {
+    const Tensor* t = stock(o);
+    if (t == nullptr) return Tensor();
+    if (!t->is_cuda()) throw NotStock{};
+    if (t->scalar_type() == at::kBFloat16) return *t;
+    if (!autocast || t->scalar_type() != at::kFloat) throw NotStock{};
+    return at::autocast::cached_cast(at::kBFloat16, *t, c10::kCUDA);
+  }
+  // a norm or scale parameter of `n` values as it is
+  const Tensor* row(PyObject* o, int64_t n) const {
+    const Tensor* t = stock(o);
+    if (t == nullptr) return nullptr;
+    const bool bf = t->scalar_type() == at::kBFloat16;
+    if (!t->is_cuda() || t->numel() != n || !t->is_contiguous() || !(bf || (autocast && t->scalar_type() == at::kFloat))) throw NotStock{};
+    return t;
+  }
+};
+
+Tensor linear(const Tensor& rows, const Tensor& w, const Tensor& b) {
+  return b.defined() ? at::addmm(b, rows, w.t()) : at::mm(rows, w.t());
+}
+
+// Norm of the rows of x as bf16; with y, of the sum x + gamma * y, which is returned in *sum.
+Tensor residual_norm(const Tensor& x, const Tensor* y, const Tensor* gamma, Tensor* sum, const Tensor* w, const Tensor* b, double eps) {
+  gct::RowLaunch p;
+  p.rows = x.size(0);
+  p.cols = static_cast<int>(x.size(1));
+  p.x = x.data_ptr();
+  p.x_dtype = dtype_code(x);
+  if (y != nullptr) {
+    p.y = bf16(*y);
+    if (gamma != nullptr) {
+      p.gamma = gamma->data_ptr();
+      p.gamma_dtype = dtype_code(*gamma);
+    }
+    const bool f32 = p.x_dtype == GCT_F32 || (gamma != nullptr && p.gamma_dtype == GCT_F32);
+    *sum = empty(x.sizes(), f32 ? at::kFloat : at::kBFloat16, x);
+    p.sum_out = sum->data_ptr();
+    p.sum_dtype = f32 ? GCT_F32 : GCT_BF16;
+  }
+  Tensor out;
+  if (w != nullptr) {
+    out = empty(x.sizes(), at::kBFloat16, x);
+    p.norm_w = w->data_ptr();
+    p.norm_b = b->data_ptr();
+    p.norm_dtype = dtype_code(*w);
+    p.eps = static_cast<float>(eps);
+    p.norm_out = static_cast<__nv_bfloat16*>(out.data_ptr());
+  }
+  check(gct::launch_residual_norm(p, stream_of(x)));
+  return out;
+}
+
+// Rotation table for `tokens` tokens from what the modules pass as positions.
+Tensor rotation(PyObject* pos, int64_t mode, double base, int64_t tokens) {
+  const Tensor* p = stock(pos);
+  if (mode == GCT_ROPE_NONE || p == nullptr) return Tensor();
+  if (!p->is_cuda()) throw NotStock{};
+  if (mode == GCT_ROPE_3D) {
+    if (!p->is_complex() || p->numel() != tokens * 32) throw NotStock{};
+    return *p;
+  }
+  if (p->scalar_type() != at::kLong || p->dim() != 3 || p->size(1) != tokens || p->size(2) != 2) throw NotStock{};
+  Tensor cs = empty({tokens, 32, 2}, at::kFloat, *p);
+  check(gct::launch_rope2d_positions(p->data_ptr<int64_t>(), p->stride(1), p->stride(2), static_cast<int>(tokens), static_cast<float>(base),
+                                     cs.data_ptr<float>(), stream_of(*p)));
+  return cs;
+}
+
+// PyObject handles around the table for the prologue (which takes Python arguments as they come).
+struct Held {
+  PyObject* o;
+  explicit Held(const Tensor& t) : o(t.defined() ? THPVariable_Wrap(t) : Py_NewRef(Py_None)) {}
+  ~Held() { Py_DECREF(o); }
+};
+
+template <typename F>
+PyObject* layer(F&& f) {
+  return guarded([&]() -> PyObject* {
+    try {
+      return f();
+    } catch (const NotStock&) {
+      Py_RETURN_NOTIMPLEMENTED;
+    }
+  });
+}
+
+// frame_layer(x, (qkv_w, qkv_b, qn_w, qn_b, kn_w, kn_b, proj_w, proj_b), heads, pos, rope_mode, rope_base) -> y
+PyObject* py_frame_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return layer([&]() -> PyObject* {
+    need(n, 6, "frame_layer");
+    const Tensor* px = stock(a[0]);
+    if (px == nullptr || !px->is_cuda() || px->dim() != 3 || PyTuple_GET_SIZE(a[1]) != 8) throw NotStock{};
+    const Precision prec(*px);
+    PyObject* const* w = &PyTuple_GET_ITEM(a[1], 0);
+    const int64_t B = px->size(0), N = px->size(1), C = px->size(2), heads = integer(a[2]), mode = integer(a[4]);
+    if (B < 1 || N < 1 || C != heads * kHeadDim) throw NotStock{};
+    const Tensor qkv_w = prec.linear(w[0]), qkv_b = prec.linear(w[1]), proj_w = prec.linear(w[6]), proj_b = prec.linear(w[7]);
+    for (int i = 2; i < 6; ++i) prec.row(w[i], kHeadDim);
+    c10::cuda::CUDAGuard guard(px->device());
+    at::AutoDispatchBelowADInplaceOrView below;
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::DispatchKey::AutocastCUDA);
+    const Held cs(rotation(a[3], mode, real(a[5]), N));
+    Tensor rows = px->reshape({B * N, C});
+    if (rows.scalar_type() != at::kBFloat16) rows = rows.to(at::kBFloat16);
+    Qkv r = prep(linear(rows, qkv_w, qkv_b), heads, N, w + 2, cs.o, cs.o == Py_None ? GCT_ROPE_NONE : mode);
+    const Tensor o = dense(r.q.view({B, N, heads, kHeadDim}), r.k.view({B, N, heads, kHeadDim}), r.v.view({B, N, heads, kHeadDim}), Tensor());
+    return wrap(linear(o.view({B * N, C}), proj_w, proj_b).view({B, N, C}));
+  });
+}
+
+// block_layer(x, (n1_w, n1_b, qkv_w, qkv_b, qn_w, qn_b, kn_w, kn_b, proj_w, proj_b, gamma1, n2_w, n2_b, fc1_w, fc1_b, fc2_w, fc2_b,
+//             gamma2), eps1, eps2, heads, with_ffn, pos, rope_mode, rope_base, manager | 0, device, block, window, frames, skip_append) -> y
+// manager and frames <= 1: one streamed frame on the paged cache.  manager and frames > 1: the scale pass, all tokens attend to
+// each other, then every frame is appended.  No manager: dense attention per batch entry.
+PyObject* py_block_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return layer([&]() -> PyObject* {
+    need(n, 15, "block_layer");
+    const Tensor* px = stock(a[0]);
+    if (px == nullptr || !px->is_cuda() || px->dim() != 3 || PyTuple_GET_SIZE(a[1]) != 18) throw NotStock{};
+    const Precision prec(*px);
+    PyObject* const* w = &PyTuple_GET_ITEM(a[1], 0);
+    const int64_t B = px->size(0), N = px->size(1), C = px->size(2), heads = integer(a[4]), mode = integer(a[7]);
+    const bool with_ffn = PyObject_IsTrue(a[5]) == 1, skip = PyObject_IsTrue(a[14]) == 1;
+    gct_mgr_t* m = manager(a[9]);
+    const int64_t device = integer(a[10]), block = integer(a[11]), window = integer(a[12]), frames = integer(a[13]);
+    if (B < 1 || N < 1 || C != heads * kHeadDim || C > gct::kRowMaxCols) throw NotStock{};
+    if (m != nullptr) {
+      const gct_mgr_config_t& cfg = gct::mgr_config(m);
+      if (B != 1 || N != std::max<int64_t>(frames, 1) * cfg.tokens_per_frame || heads != cfg.num_heads || device != px->device().index() ||
+          (frames > 1 && skip))
+        throw NotStock{};
+    }
+    const Tensor qkv_w = prec.linear(w[2]), qkv_b = prec.linear(w[3]), proj_w = prec.linear(w[8]), proj_b = prec.linear(w[9]);
+    for (int i = 4; i < 8; ++i) prec.row(w[i], kHeadDim);
+    const Tensor *n1w = prec.row(w[0], C), *n1b = prec.row(w[1], C), *g1 = prec.row(w[10], C);
+    const Tensor *n2w = nullptr, *n2b = nullptr, *g2 = nullptr;
+    Tensor fc1_w, fc1_b, fc2_w, fc2_b;
+    if (n1w == nullptr || n1b == nullptr || n1w->scalar_type() != n1b->scalar_type()) throw NotStock{};
+    if (with_ffn) {
+      n2w = prec.row(w[11], C);
+      n2b = prec.row(w[12], C);
+      g2 = prec.row(w[17], C);
+      fc1_w = prec.linear(w[13]);
+      fc1_b = prec.linear(w[14]);
+      fc2_w = prec.linear(w[15]);
+      fc2_b = prec.linear(w[16]);
+      if (n2w == nullptr || n2b == nullptr || n2w->scalar_type() != n2b->scalar_type() || !fc1_w.defined() || !fc2_w.defined()) throw NotStock{};
+    }
+    c10::cuda::CUDAGuard guard(px->device());
+    at::AutoDispatchBelowADInplaceOrView below;
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::DispatchKey::AutocastCUDA);
+    const Held cs(rotation(a[6], mode, real(a[8]), N));
+    const int64_t rope = cs.o == Py_None ? GCT_ROPE_NONE : mode;
+    const Tensor x = px->reshape({B * N, C});
+    const Tensor normed = residual_norm(x, nullptr, nullptr, nullptr, n1w, n1b, real(a[2]));
+    const Tensor qkv = linear(normed, qkv_w, qkv_b);
+    const int blk = static_cast<int>(block);
+    Tensor o;
+    if (m != nullptr && frames <= 1) {
+      int deferred = 0;
+      if (skip) {
+        check(gct_mgr_get_defer(m, &deferred));
+        check(gct_mgr_set_defer(m, 1));
+      }
+      const Tensor q = append_fused(m, device, block, qkv, w + 4, cs.o, rope, Tensor());
+      if (!skip) check(gct_mgr_evict(m, blk, static_cast<int>(window)));
+      o = attend(m, device, block, q, false).out;
+      if (skip) {
+        check(gct_mgr_rollback(m, blk));
+        check(gct_mgr_set_defer(m, deferred));
+      }
+    } else {
+      Qkv r = prep(qkv, heads, N, w + 4, cs.o, rope);
+      o = dense(r.q.view({B, N, heads, kHeadDim}), r.k.view({B, N, heads, kHeadDim}), r.v.view({B, N, heads, kHeadDim}), Tensor());
+      if (m != nullptr) {
+        const int64_t step = gct::mgr_config(m).tokens_per_frame * C;
+        for (int64_t f = 0; f < frames; ++f) {
+          check(gct_mgr_append(m, blk, bf16(r.k) + f * step, GCT_BF16, bf16(r.v) + f * step, GCT_BF16, stream_of(x)));
+          check(gct_mgr_evict(m, blk, static_cast<int>(window)));
+        }
+      }
+    }
+    const Tensor attn = linear(o.view({B * N, C}), proj_w, proj_b);
+    Tensor sum;
+    const Tensor normed2 = residual_norm(x, &attn, g1, &sum, n2w, n2b, real(a[3]));
+    if (with_ffn) {
+      const Tensor h = at::gelu(linear(normed2, fc1_w, fc1_b));
+      const Tensor f = linear(h, fc2_w, fc2_b);
+      Tensor out;
+      residual_norm(sum, &f, g2, &out, nullptr, nullptr, 0.0);
+      sum = out;
+    }
+    return wrap(sum.view({B, N, C}));
+  });
+}
+
 // ---- camera head, rotation tables ---------------------------------------------------------------
 
 // decode_attention(q, k_new, v_new, cache_k, cache_v, cached, store, workspace) -> out
@@ -526,12 +751,14 @@ PyObject* py_voxelize_frame(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
-// set_error_class(GctError)
-PyObject* py_set_error_class(PyObject*, PyObject* cls) {
-  Py_INCREF(cls);
-  Py_XDECREF(g_error_class);
-  g_error_class = cls;
-  Py_RETURN_NONE;
+// set_classes(GctError, torch.nn.Parameter)
+PyObject* py_set_classes(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 2, "set_classes");
+    Py_XSETREF(g_error_class, Py_NewRef(a[0]));
+    Py_XSETREF(g_parameter_class, Py_NewRef(a[1]));
+    Py_RETURN_NONE;
+  });
 }
 
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr}
@@ -548,7 +775,9 @@ PyMethodDef g_methods[] = {FAST(prep_qkv),
                            FAST(rope3d_table),
                            FAST(frustum_cull),
                            FAST(voxelize_frame),
-                           {"set_error_class", py_set_error_class, METH_O, nullptr},
+                           FAST(frame_layer),
+                           FAST(block_layer),
+                           FAST(set_classes),
                            {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_gct_torch", "PyTorch binding of libgct_b200.so", -1, g_methods,
                         nullptr,               nullptr,      nullptr,                             nullptr};

@@ -179,3 +179,76 @@ def test_plain_attention_without_norm_and_rope():
         ref = torch.nn.functional.scaled_dot_product_attention(qkv[0], qkv[1], qkv[2])
         ref = fa.proj(ref.transpose(1, 2).reshape(2, N, dim))
     close(y, ref.double().cpu().numpy(), "plain attention")
+
+
+@pytest.mark.parametrize("dim,H,weights,x_dtype,rope", [(128, 2, "bf16", "bf16", "3d"), (192, 3, "f32", "f32", "3d"), (576, 9, "bf16", "f32", "none"),
+                                                        (1024, 16, "f32", "bf16", "2d"), (128, 2, "bf16", "bf16", "no autocast")])
+@pytest.mark.parametrize("scaled", [True, False])
+def test_layers_as_one_call_equal_the_module_code(monkeypatch, dim, H, weights, x_dtype, rope, scaled):
+    """B200Block and B200FrameAttention as single native calls against the same modules run operation by operation: scale
+    pass, keyframes with eviction, a non-keyframe, batch mode without a cache, a rebound ffn_residual; columns from half a
+    warp's chunk up to four, row counts that leave warps idle, and every combination of parameter and activation precision.
+
+    Both sides round the same intermediates to bf16, the native call fewer of them (scale and sum in one step), and return
+    bf16 or fp32; results may differ by two bf16 rounding steps at the largest magnitude of the output, 2 * 2^-7 * max."""
+    from lingbot_map_b200 import block as block_mod
+    pph, ppw, ns, scale, window = 3, 5, 6, 2, 2
+    T = ns + pph * ppw
+    dt = {"bf16": torch.bfloat16, "f32": torch.float32}
+    blk = P.B200Block(dim=dim, num_heads=H, init_values=0.5 if scaled else None, qk_norm=scaled, rope=None if rope == "none" else Rope2dStub(),
+                      kv_cache_sliding_window=window, kv_cache_scale_frames=scale).eval().to(DEV)
+    fa = P.B200FrameAttention(dim, num_heads=H, qk_norm=scaled, rope=None if rope == "none" else Rope2dStub()).eval().to(DEV)
+    seeded.fill_module_(blk, 3)
+    seeded.fill_module_(fa, 4)
+    blk, fa = blk.to(dt[weights]), fa.to(dt[weights])
+    three_d = rope not in ("2d", "none")
+    y, x = torch.meshgrid(torch.arange(1, pph + 1), torch.arange(1, ppw + 1), indexing="ij")
+    pos2d = torch.cat([torch.zeros(ns, 2, dtype=torch.int64), torch.stack([y, x], -1).reshape(-1, 2)])[None].to(DEV)
+    calls = []
+    real = block_mod._native.block_layer
+
+    class Counting:
+        def __getattr__(self, name):
+            return getattr(_lib_native, name)
+
+        def block_layer(self, *a):
+            calls.append("block")
+            r = real(*a)
+            assert r is not NotImplemented
+            return r
+
+        def frame_layer(self, *a):
+            calls.append("frame")
+            r = _lib_native.frame_layer(*a)
+            assert r is not NotImplemented
+            return r
+
+    _lib_native = block_mod._native
+    monkeypatch.setattr(block_mod, "_native", Counting())
+
+    def run(fused):
+        monkeypatch.setattr(block_mod, "_may_fuse", lambda: fused)
+        mgr = P.B200KVCacheManager(1, scale + window + 16, T, H, 64, device=DEV, scale_frames=scale, sliding_window=window, max_total_frames=40)
+        kw = dict(num_patches=T - ns, num_special=ns, enable_3d_rope=three_d, global_idx=0, num_frame_for_scale=scale)
+        pos = lambda f, n: rope3d_pos(f, n, pph, ppw, ns) if three_d else pos2d.repeat(1, n, 1)
+        data = lambda i, *s: torch.from_numpy(seeded.randn(i, *s, dim)).to(DEV).to(dt[x_dtype])
+        out = [fa(data(1, 3, T), pos=pos2d.expand(3, -1, -1)), blk(data(2, 2, T), pos=pos(0, 1), **kw),
+               blk(data(3, 1, scale * T), pos=pos(0, scale), num_frames=scale, kv_cache=mgr, **kw)]
+        for i in range(5):
+            mgr._skip_append = i == 2
+            out.append(blk(data(4 + i, 1, T), pos=pos(scale + i, 1), num_frames=1, kv_cache=mgr, **kw))
+        blk.ffn_residual = lambda v: 2 * v
+        out.append(blk(data(9, 1, T), pos=pos(9, 1), num_frames=1, kv_cache=mgr, **kw))
+        del blk.__dict__["ffn_residual"]
+        assert mgr.device_status() == 0
+        return out, mgr.build_visible_page_table(0), mgr._gather_kv(0)
+
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16, enabled=rope != "no autocast"):
+        got, table, kv = run(True)
+        want, wtable, wkv = run(False)
+    assert calls == ["frame"] + ["block"] * 8
+    assert table == wtable
+    for i, (a, b) in enumerate(zip(got + list(kv), want + list(wkv))):
+        assert a.dtype == b.dtype and a.shape == b.shape, i
+        d, top = float((a.float() - b.float()).abs().max()), float(b.float().abs().max())
+        assert d <= 2 * 2 ** -7 * top, (i, d, top)
