@@ -24,8 +24,19 @@ _native = _lib.binding()
 
 
 def _stock(m: nn.Module, cls) -> bool:
-    """m is a plain `cls`: nothing hooks into it and its forward has not been rebound on the instance."""
-    return type(m) is cls and not m._forward_hooks and not m._forward_pre_hooks and "forward" not in m.__dict__
+    """m is a plain `cls`: nothing hooks into it, it has not been compiled in place and its forward has not been rebound on the
+    instance."""
+    return (type(m) is cls and not m._forward_hooks and not m._forward_pre_hooks and m._compiled_call_impl is None
+            and "forward" not in m.__dict__)
+
+
+def _rebound(obj, names: frozenset) -> bool:
+    """One of the methods that a native layer passes by has been replaced on the instance (by a profiler, for instance)."""
+    return not names.isdisjoint(obj.__dict__)
+
+
+_ATTENTION_STEPS = frozenset(("prepare_qkv", "stream_frame", "_dense", "_qkv_rows", "_norm_params", "_rope_args", "_evict"))
+_MANAGER_STEPS = frozenset(("append_frame", "append_frame_fused", "evict_frames", "compute_attention", "rollback_last_frame", "plan"))
 
 
 def _stock_dropout(m: nn.Module) -> bool:
@@ -34,9 +45,9 @@ def _stock_dropout(m: nn.Module) -> bool:
 
 def _may_fuse() -> bool:
     """Whole layers run as one native call in eager inference only: under torch.compile the modules are traced, with
-    gradients enabled the Linear layers record them, and global hooks want to see every module."""
+    gradients enabled the Linear layers record them, and global hooks and torch.jit.trace want to see every module."""
     return not (torch.is_grad_enabled() or torch.compiler.is_compiling() or _nn_module._global_forward_hooks
-                or _nn_module._global_forward_pre_hooks)
+                or _nn_module._global_forward_pre_hooks or torch._C._get_tracing_state() is not None)
 
 
 def _reference_classes():
@@ -126,7 +137,8 @@ class _AttentionBase(nn.Module):
         ones, else None."""
         mods = self._modules
         qkv, proj, qn, kn = mods["qkv"], mods["proj"], mods["q_norm"], mods["k_norm"]
-        if not (_stock(qkv, nn.Linear) and _stock(proj, nn.Linear) and _stock_dropout(mods["proj_drop"])):
+        if (not (_stock(qkv, nn.Linear) and _stock(proj, nn.Linear) and _stock_dropout(mods["proj_drop"]))
+                or _rebound(self, _ATTENTION_STEPS)):
             return None
         if _stock(qn, nn.Identity) and _stock(kn, nn.Identity):
             norm = (None, None, None, None)
@@ -173,7 +185,7 @@ class B200FrameAttention(_AttentionBase):
 
     def forward(self, x: Tensor, pos=None, num_patches=None, num_special=None, num_frames=None,
                 enable_3d_rope=False) -> Tensor:
-        if _may_fuse():
+        if type(self) is B200FrameAttention and _may_fuse():      # a subclass may replace any step
             params = self._layer_params()
             if params is not None:
                 y = _native.frame_layer(x, params, self.num_heads, pos, *self._rope_kind(pos, enable_3d_rope))
@@ -328,7 +340,7 @@ class B200Block(nn.Module):
                 enable_3d_rope=enable_3d_rope, kv_cache=kv_cache, global_idx=global_idx,
                 num_frame_per_block=num_frame_per_block, num_frame_for_scale=num_frame_for_scale,
                 num_register_tokens=num_register_tokens)
-        if _may_fuse():
+        if type(self) is B200Block and _may_fuse():               # a subclass may replace any step
             y = self._fused_forward(x, pos, num_frames, enable_3d_rope, kv_cache, global_idx)
             if y is not NotImplemented:
                 return y
@@ -357,7 +369,8 @@ class B200Block(nn.Module):
         mods, own = self._modules, self.__dict__
         attn, norm1, ls1, ls2 = mods["attn"], mods["norm1"], mods["ls1"], mods["ls2"]
         if not (_stock(attn, B200Attention) and _stock(norm1, nn.LayerNorm) and (_stock(ls1, LayerScale) or _stock(ls1, nn.Identity))
-                and "attn_pre" not in own and (manager is None or type(manager) is B200KVCacheManager and manager._bound)):
+                and "attn_pre" not in own
+                and (manager is None or type(manager) is B200KVCacheManager and manager._bound and not _rebound(manager, _MANAGER_STEPS))):
             return NotImplemented
         params = attn._layer_params()
         if params is None:

@@ -77,7 +77,8 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, kQ == 1 ? 2 : 1) gct_decode
   const size_t row_stride = static_cast<size_t>(a.heads) * D;
   const size_t head_off = static_cast<size_t>(h) * D + lane * kPer;
 
-  // rows [j, j + kGroup) of K and V; past the end of the range the last row again (its weight is set to zero)
+  // rows [j, j + kGroup) of K and V; past the end of the range the last K row again (its weight is set to zero) and zeros for
+  // V, whose last row may hold an infinity
   auto load_group = [&](int j, V(&kv)[kGroup], V(&vv)[kGroup]) {
 #pragma unroll
     for (int u = 0; u < kGroup; ++u) {
@@ -85,7 +86,7 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, kQ == 1 ? 2 : 1) gct_decode
       const float* kp = r < a.cached ? a.cache_k + static_cast<size_t>(r) * row_stride : a.k_new + static_cast<size_t>(r - a.cached) * row_stride;
       const float* vp = r < a.cached ? a.cache_v + static_cast<size_t>(r) * row_stride : a.v_new + static_cast<size_t>(r - a.cached) * row_stride;
       kv[u] = *reinterpret_cast<const V*>(kp + head_off);
-      vv[u] = *reinterpret_cast<const V*>(vp + head_off);
+      vv[u] = j + u < j1 ? *reinterpret_cast<const V*>(vp + head_off) : LaneVec<D>::zero();
     }
   };
   constexpr int kStep = kDecodeWarps * kGroup;

@@ -9,6 +9,7 @@
 #include <ATen/ATen.h>
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -39,6 +40,18 @@ struct Failed {                          // a C ABI status code other than GCT_O
 };
 void check(int rc) {
   if (rc != GCT_OK) throw Failed{rc};
+}
+
+// What may wait runs without the interpreter lock, as the ctypes calls and PyTorch's own operators do: a launch while the
+// stream's queue is full, a plan behind an upload eight plans back, a cudaMalloc.
+struct WithoutGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+template <typename F>
+auto unlocked(F&& f) {
+  WithoutGil free_others;
+  return f();
 }
 
 template <typename F>
@@ -122,16 +135,23 @@ int* status_of(const Tensor& like) {
   return p;
 }
 
+// The four q/k norm parameters (null: none), from Python's arguments.
+struct Norm {
+  const Tensor* t[4];
+  explicit Norm(PyObject* const* o) {
+    for (int i = 0; i < 4; ++i) t[i] = optional_tensor(o[i], "a norm parameter");
+  }
+};
+
 // LayerNorm parameters and rotation table as the prologue kernel takes them.  `keep` holds tensors that had to be
 // converted (a norm parameter that is neither fp32 nor bf16, or not of the dtype of the others) until the launch is queued.
 struct NormRope {
   Tensor keep[5];
-  void fill(gct::PrepLaunch* p, PyObject* const* norm, PyObject* cs, int64_t mode) {
-    const Tensor* t[4];
+  void fill(gct::PrepLaunch* p, const Norm& norm, const Tensor* c, int64_t mode) {
+    const Tensor* const* t = norm.t;
     static const char* names[4] = {"q_norm_w", "q_norm_b", "k_norm_w", "k_norm_b"};
     bool all_bf16 = true;
     for (int i = 0; i < 4; ++i) {
-      t[i] = optional_tensor(norm[i], names[i]);
       if (t[i] != nullptr) {
         need_cuda(*t[i], names[i]);
         if (t[i]->numel() != kHeadDim) value_error(std::string(names[i]) + " must have 64 elements");
@@ -146,10 +166,12 @@ struct NormRope {
     for (int i = 0; i < 4; ++i) {
       if (t[i] == nullptr) continue;
       const at::ScalarType want = all_bf16 ? at::kBFloat16 : at::kFloat;
-      if (t[i]->scalar_type() == want && t[i]->is_contiguous()) {
+      // the kernel loads 16 bytes at a time: a bf16 parameter at another address (a slice of a flat buffer) is copied
+      const bool in_place = t[i]->is_contiguous() && (want == at::kFloat || (reinterpret_cast<uintptr_t>(t[i]->data_ptr()) & 15) == 0);
+      if (t[i]->scalar_type() == want && in_place) {
         ptr[i] = t[i]->data_ptr();
       } else {
-        keep[i] = t[i]->detach().to(want).contiguous();
+        keep[i] = t[i]->detach().to(want).clone(at::MemoryFormat::Contiguous);
         ptr[i] = keep[i].data_ptr();
       }
     }
@@ -159,12 +181,11 @@ struct NormRope {
     p->kn_b = ptr[3];
     p->norm_dtype = all_bf16 ? GCT_BF16 : GCT_F32;
     p->rope_mode = static_cast<int>(mode);
-    const Tensor* c = optional_tensor(cs, "rope_cs");
     if (c == nullptr || mode == GCT_ROPE_NONE) return;
     need_cuda(*c, "rope_cs");
     const bool is_complex = c->scalar_type() == at::kComplexFloat || c->scalar_type() == at::kComplexDouble;
     if (c->numel() < static_cast<int64_t>(p->tokens_per_frame) * (is_complex ? 32 : 64)) value_error("rope_cs holds too few rows");
-    Tensor table = *c;
+    Tensor table = c->is_conj() ? c->resolve_conj() : *c;
     if (mode == GCT_ROPE_2D || !(is_complex || c->scalar_type() == at::kFloat)) {
       if (c->scalar_type() != at::kFloat) table = is_complex ? at::view_as_real(c->to(at::kComplexFloat)) : c->to(at::kFloat);
     }
@@ -178,6 +199,10 @@ struct NormRope {
 void fill_qkv(gct::PrepLaunch* p, const Tensor& qkv, int64_t heads) {
   const size_t esz = qkv.element_size();
   const int64_t C = heads * kHeadDim;
+  if (qkv.stride(0) < 3 * C) {
+    gct::set_error("qkv: row stride smaller than 3*H*64");
+    throw Failed{GCT_ERR_INVALID};
+  }
   const uint8_t* base = static_cast<const uint8_t*>(qkv.data_ptr());
   p->q_src = base;
   p->k_src = base + C * esz;
@@ -190,7 +215,7 @@ void fill_qkv(gct::PrepLaunch* p, const Tensor& qkv, int64_t heads) {
 struct Qkv {
   Tensor q, k, v;
 };
-Qkv prep(Tensor qkv, int64_t heads, int64_t tokens_per_frame, PyObject* const* norm, PyObject* cs, int64_t mode) {
+Qkv prep(Tensor qkv, int64_t heads, int64_t tokens_per_frame, const Norm& norm, const Tensor* cs, int64_t mode) {
   need_cuda(qkv, "qkv");
   if (qkv.dim() != 2 || qkv.size(1) != 3 * heads * kHeadDim) value_error("qkv must be [tokens, 3*H*64]");
   if (qkv.stride(1) != 1) qkv = qkv.contiguous();
@@ -215,7 +240,10 @@ Qkv prep(Tensor qkv, int64_t heads, int64_t tokens_per_frame, PyObject* const* n
 PyObject* py_prep_qkv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     need(n, 9, "prep_qkv");
-    Qkv r = prep(tensor(a[0], "qkv"), integer(a[1]), integer(a[2]), a + 3, a[7], integer(a[8]));
+    const Tensor &qkv = tensor(a[0], "qkv"), *cs = optional_tensor(a[7], "rope_cs");
+    const int64_t heads = integer(a[1]), tokens_per_frame = integer(a[2]), mode = integer(a[8]);
+    const Norm norm(a + 3);
+    Qkv r = unlocked([&] { return prep(qkv, heads, tokens_per_frame, norm, cs, mode); });
     PyObject* out = PyTuple_New(3);
     if (out == nullptr) throw python_error();
     PyTuple_SET_ITEM(out, 0, wrap(std::move(r.q)));
@@ -262,8 +290,8 @@ Tensor dense(const Tensor& q, const Tensor& k, const Tensor& v, Tensor out) {
 PyObject* py_dense_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     need(n, 4, "dense_attention");
-    const Tensor* out = optional_tensor(a[3], "out");
-    return wrap(dense(tensor(a[0], "q"), tensor(a[1], "k"), tensor(a[2], "v"), out == nullptr ? Tensor() : *out));
+    const Tensor &q = tensor(a[0], "q"), &k = tensor(a[1], "k"), &v = tensor(a[2], "v"), *out = optional_tensor(a[3], "out");
+    return wrap(unlocked([&] { return dense(q, k, v, out == nullptr ? Tensor() : *out); }));
   });
 }
 
@@ -299,12 +327,13 @@ PyObject* py_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor k = frame_rows(tensor(a[3], "k"), "k", gct::mgr_config(m), dev), v = frame_rows(tensor(a[4], "v"), "v", gct::mgr_config(m), dev);
     if (k.size(0) != gct::mgr_config(m).tokens_per_frame || v.size(0) != k.size(0)) value_error("k and v must hold the tokens of one frame");
     c10::cuda::CUDAGuard guard(k.device());
-    check(gct_mgr_append(m, static_cast<int>(integer(a[2])), k.data_ptr(), dtype_code(k), v.data_ptr(), dtype_code(v), stream_of(k)));
+    const int block = static_cast<int>(integer(a[2]));
+    check(unlocked([&] { return gct_mgr_append(m, block, k.data_ptr(), dtype_code(k), v.data_ptr(), dtype_code(v), stream_of(k)); }));
     Py_RETURN_NONE;
   });
 }
 
-Tensor append_fused(gct_mgr_t* m, int64_t device, int64_t block, Tensor qkv, PyObject* const* norm, PyObject* cs, int64_t mode, Tensor q_out) {
+Tensor append_fused(gct_mgr_t* m, int64_t device, int64_t block, Tensor qkv, const Norm& norm, const Tensor* cs, int64_t mode, Tensor q_out) {
   const gct_mgr_config_t& cfg = gct::mgr_config(m);
   const int64_t T = cfg.tokens_per_frame, H = cfg.num_heads;
   if (qkv.dim() != 2 || qkv.size(0) != T || qkv.size(1) != 3 * H * kHeadDim)
@@ -327,19 +356,16 @@ Tensor append_fused(gct_mgr_t* m, int64_t device, int64_t block, Tensor qkv, PyO
 PyObject* py_append_fused(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     need(n, 11, "append_fused");
-    const Tensor* q_out = optional_tensor(a[10], "q_out");
-    return wrap(append_fused(manager(a[0]), integer(a[1]), integer(a[2]), tensor(a[3], "qkv"), a + 4, a[8], integer(a[9]),
-                             q_out == nullptr ? Tensor() : *q_out));
+    const Tensor &qkv = tensor(a[3], "qkv"), *cs = optional_tensor(a[8], "rope_cs"), *q_out = optional_tensor(a[10], "q_out");
+    const int64_t device = integer(a[1]), block = integer(a[2]), mode = integer(a[9]);
+    gct_mgr_t* m = manager(a[0]);
+    const Norm norm(a + 4);
+    return wrap(unlocked([&] { return append_fused(m, device, block, qkv, norm, cs, mode, q_out == nullptr ? Tensor() : *q_out); }));
   });
 }
 
 struct Attended {
   Tensor out, lse;
-};
-// Planning may wait for an upload eight plans back: other Python threads run meanwhile.
-struct WithoutGil {
-  PyThreadState* state = PyEval_SaveThread();
-  ~WithoutGil() { PyEval_RestoreThread(state); }
 };
 // The page table is planned at block 0 and reused by the other blocks of the frame.
 Attended attend(gct_mgr_t* m, int64_t device, int64_t block, const Tensor& q_in, bool want_lse) {
@@ -347,14 +373,7 @@ Attended attend(gct_mgr_t* m, int64_t device, int64_t block, const Tensor& q_in,
   const Tensor q = frame_rows(q_in, "q", cfg, device);
   c10::cuda::CUDAGuard guard(q.device());
   cudaStream_t s = stream_of(q);
-  if (block == 0) {
-    int rc;
-    {
-      WithoutGil free_others;
-      rc = gct_mgr_plan(m, 0, -1, s);
-    }
-    check(rc);
-  }
+  if (block == 0) check(gct_mgr_plan(m, 0, -1, s));
   Attended r;
   r.out = empty(q.sizes(), at::kBFloat16, q);
   if (want_lse) r.lse = empty({q.size(0), q.size(1)}, at::kFloat, q);
@@ -372,7 +391,9 @@ PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
     check(gct_mgr_stats(m, static_cast<int>(integer(a[2])), stats));
     if (stats[0] == 0) Py_RETURN_NONE;
     const bool want_lse = PyObject_IsTrue(a[4]) == 1;
-    Attended r = attend(m, integer(a[1]), integer(a[2]), tensor(a[3], "q"), want_lse);
+    const Tensor& q = tensor(a[3], "q");
+    const int64_t device = integer(a[1]), block = integer(a[2]);
+    Attended r = unlocked([&] { return attend(m, device, block, q, want_lse); });
     if (!want_lse) return wrap(std::move(r.out));
     PyObject* out = PyTuple_New(2);
     if (out == nullptr) throw python_error();
@@ -416,12 +437,16 @@ PyObject* py_rollback(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* g_parameter_class = nullptr;
 
 struct NotStock {};
-// A plain tensor or parameter (no tensor subclass), or nothing.
+// A plain tensor or parameter, or nothing.  Not plain: tensor subclasses, lazily conjugated or negated views (their memory holds
+// other values), and tensors that carry a forward-mode tangent (the modules propagate it through the residual sums).
 const Tensor* stock(PyObject* o) {
   if (o == Py_None) return nullptr;
   if (!THPVariable_CheckExact(o) && reinterpret_cast<PyObject*>(Py_TYPE(o)) != g_parameter_class) throw NotStock{};
-  return &THPVariable_Unpack(o);
+  const Tensor& t = THPVariable_Unpack(o);
+  if (t.is_conj() || t.is_neg() || t._fw_grad(0).defined()) throw NotStock{};
+  return &t;
 }
+bool aligned16(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
 
 // bf16 is what the Linear layers compute in: under autocast whatever the parameters are, else only if all of it is bf16.
 struct Precision {
@@ -445,7 +470,7 @@ struct Precision {
     const Tensor* t = stock(o);
     if (t == nullptr) return nullptr;
     const bool bf = t->scalar_type() == at::kBFloat16;
-    if (!t->is_cuda() || t->numel() != n || !t->is_contiguous() || !(bf || (autocast && t->scalar_type() == at::kFloat))) throw NotStock{};
+    if (!t->is_cuda() || t->numel() != n || !t->is_contiguous() || !(bf || (autocast && t->scalar_type() == at::kFloat)) || !aligned16(*t)) throw NotStock{};
     return t;
   }
 };
@@ -486,8 +511,7 @@ Tensor residual_norm(const Tensor& x, const Tensor* y, const Tensor* gamma, Tens
 }
 
 // Rotation table for `tokens` tokens from what the modules pass as positions.
-Tensor rotation(PyObject* pos, int64_t mode, double base, int64_t tokens) {
-  const Tensor* p = stock(pos);
+Tensor rotation(const Tensor* p, int64_t mode, double base, int64_t tokens) {
   if (mode == GCT_ROPE_NONE || p == nullptr) return Tensor();
   if (!p->is_cuda()) throw NotStock{};
   if (mode == GCT_ROPE_3D) {
@@ -500,13 +524,6 @@ Tensor rotation(PyObject* pos, int64_t mode, double base, int64_t tokens) {
                                      cs.data_ptr<float>(), stream_of(*p)));
   return cs;
 }
-
-// PyObject handles around the table for the prologue (which takes Python arguments as they come).
-struct Held {
-  PyObject* o;
-  explicit Held(const Tensor& t) : o(t.defined() ? THPVariable_Wrap(t) : Py_NewRef(Py_None)) {}
-  ~Held() { Py_DECREF(o); }
-};
 
 template <typename F>
 PyObject* layer(F&& f) {
@@ -531,15 +548,20 @@ PyObject* py_frame_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (B < 1 || N < 1 || C != heads * kHeadDim) throw NotStock{};
     const Tensor qkv_w = prec.linear(w[0]), qkv_b = prec.linear(w[1]), proj_w = prec.linear(w[6]), proj_b = prec.linear(w[7]);
     for (int i = 2; i < 6; ++i) prec.row(w[i], kHeadDim);
-    c10::cuda::CUDAGuard guard(px->device());
-    at::AutoDispatchBelowADInplaceOrView below;
-    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::DispatchKey::AutocastCUDA);
-    const Held cs(rotation(a[3], mode, real(a[5]), N));
-    Tensor rows = px->reshape({B * N, C});
-    if (rows.scalar_type() != at::kBFloat16) rows = rows.to(at::kBFloat16);
-    Qkv r = prep(linear(rows, qkv_w, qkv_b), heads, N, w + 2, cs.o, cs.o == Py_None ? GCT_ROPE_NONE : mode);
-    const Tensor o = dense(r.q.view({B, N, heads, kHeadDim}), r.k.view({B, N, heads, kHeadDim}), r.v.view({B, N, heads, kHeadDim}), Tensor());
-    return wrap(linear(o.view({B * N, C}), proj_w, proj_b).view({B, N, C}));
+    const Norm norm(w + 2);
+    const Tensor* pos = stock(a[3]);
+    const double base = real(a[5]);
+    return wrap(unlocked([&]() -> Tensor {
+      c10::cuda::CUDAGuard guard(px->device());
+      at::AutoDispatchBelowADInplaceOrView below;
+      c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::DispatchKey::AutocastCUDA);
+      const Tensor cs = rotation(pos, mode, base, N);
+      Tensor rows = px->reshape({B * N, C});
+      if (rows.scalar_type() != at::kBFloat16) rows = rows.to(at::kBFloat16);
+      Qkv r = prep(linear(rows, qkv_w, qkv_b), heads, N, norm, cs.defined() ? &cs : nullptr, cs.defined() ? mode : GCT_ROPE_NONE);
+      const Tensor o = dense(r.q.view({B, N, heads, kHeadDim}), r.k.view({B, N, heads, kHeadDim}), r.v.view({B, N, heads, kHeadDim}), Tensor());
+      return linear(o.view({B * N, C}), proj_w, proj_b).view({B, N, C});
+    }));
   });
 }
 
@@ -570,7 +592,7 @@ PyObject* py_block_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor *n1w = prec.row(w[0], C), *n1b = prec.row(w[1], C), *g1 = prec.row(w[10], C);
     const Tensor *n2w = nullptr, *n2b = nullptr, *g2 = nullptr;
     Tensor fc1_w, fc1_b, fc2_w, fc2_b;
-    if (n1w == nullptr || n1b == nullptr || n1w->scalar_type() != n1b->scalar_type()) throw NotStock{};
+    if (n1w == nullptr || n1b == nullptr || n1w->scalar_type() != n1b->scalar_type() || proj_w.dim() != 2 || proj_w.size(0) != C) throw NotStock{};
     if (with_ffn) {
       n2w = prec.row(w[11], C);
       n2b = prec.row(w[12], C);
@@ -579,53 +601,62 @@ PyObject* py_block_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
       fc1_b = prec.linear(w[14]);
       fc2_w = prec.linear(w[15]);
       fc2_b = prec.linear(w[16]);
-      if (n2w == nullptr || n2b == nullptr || n2w->scalar_type() != n2b->scalar_type() || !fc1_w.defined() || !fc2_w.defined()) throw NotStock{};
+      if (n2w == nullptr || n2b == nullptr || n2w->scalar_type() != n2b->scalar_type() || !fc1_w.defined() || !fc2_w.defined() ||
+          fc2_w.dim() != 2 || fc2_w.size(0) != C)
+        throw NotStock{};
     }
-    c10::cuda::CUDAGuard guard(px->device());
-    at::AutoDispatchBelowADInplaceOrView below;
-    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::DispatchKey::AutocastCUDA);
-    const Held cs(rotation(a[6], mode, real(a[8]), N));
-    const int64_t rope = cs.o == Py_None ? GCT_ROPE_NONE : mode;
-    const Tensor x = px->reshape({B * N, C});
-    const Tensor normed = residual_norm(x, nullptr, nullptr, nullptr, n1w, n1b, real(a[2]));
-    const Tensor qkv = linear(normed, qkv_w, qkv_b);
-    const int blk = static_cast<int>(block);
-    Tensor o;
-    if (m != nullptr && frames <= 1) {
-      int deferred = 0;
-      if (skip) {
-        check(gct_mgr_get_defer(m, &deferred));
-        check(gct_mgr_set_defer(m, 1));
-      }
-      const Tensor q = append_fused(m, device, block, qkv, w + 4, cs.o, rope, Tensor());
-      if (!skip) check(gct_mgr_evict(m, blk, static_cast<int>(window)));
-      o = attend(m, device, block, q, false).out;
-      if (skip) {
-        check(gct_mgr_rollback(m, blk));
-        check(gct_mgr_set_defer(m, deferred));
-      }
-    } else {
-      Qkv r = prep(qkv, heads, N, w + 4, cs.o, rope);
-      o = dense(r.q.view({B, N, heads, kHeadDim}), r.k.view({B, N, heads, kHeadDim}), r.v.view({B, N, heads, kHeadDim}), Tensor());
-      if (m != nullptr) {
-        const int64_t step = gct::mgr_config(m).tokens_per_frame * C;
-        for (int64_t f = 0; f < frames; ++f) {
-          check(gct_mgr_append(m, blk, bf16(r.k) + f * step, GCT_BF16, bf16(r.v) + f * step, GCT_BF16, stream_of(x)));
-          check(gct_mgr_evict(m, blk, static_cast<int>(window)));
+    const Norm norm(w + 4);
+    const Tensor* pos = stock(a[6]);
+    const double eps1 = real(a[2]), eps2 = real(a[3]), base = real(a[8]);
+    return wrap(unlocked([&]() -> Tensor {
+      c10::cuda::CUDAGuard guard(px->device());
+      at::AutoDispatchBelowADInplaceOrView below;
+      c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::DispatchKey::AutocastCUDA);
+      const Tensor table = rotation(pos, mode, base, N);
+      const Tensor* cs = table.defined() ? &table : nullptr;
+      const int64_t rope = table.defined() ? mode : GCT_ROPE_NONE;
+      Tensor x = px->reshape({B * N, C});
+      if (!aligned16(x)) x = x.clone();
+      const Tensor normed = residual_norm(x, nullptr, nullptr, nullptr, n1w, n1b, eps1);
+      const Tensor qkv = linear(normed, qkv_w, qkv_b);
+      const int blk = static_cast<int>(block);
+      Tensor o;
+      if (m != nullptr && frames <= 1) {
+        int deferred = 0;
+        if (skip) {
+          check(gct_mgr_get_defer(m, &deferred));
+          check(gct_mgr_set_defer(m, 1));
+        }
+        const Tensor q = append_fused(m, device, block, qkv, norm, cs, rope, Tensor());
+        if (!skip) check(gct_mgr_evict(m, blk, static_cast<int>(window)));
+        o = attend(m, device, block, q, false).out;
+        if (skip) {
+          check(gct_mgr_rollback(m, blk));
+          check(gct_mgr_set_defer(m, deferred));
+        }
+      } else {
+        Qkv r = prep(qkv, heads, N, norm, cs, rope);
+        o = dense(r.q.view({B, N, heads, kHeadDim}), r.k.view({B, N, heads, kHeadDim}), r.v.view({B, N, heads, kHeadDim}), Tensor());
+        if (m != nullptr) {
+          const int64_t step = gct::mgr_config(m).tokens_per_frame * C;
+          for (int64_t f = 0; f < frames; ++f) {
+            check(gct_mgr_append(m, blk, bf16(r.k) + f * step, GCT_BF16, bf16(r.v) + f * step, GCT_BF16, stream_of(x)));
+            check(gct_mgr_evict(m, blk, static_cast<int>(window)));
+          }
         }
       }
-    }
-    const Tensor attn = linear(o.view({B * N, C}), proj_w, proj_b);
-    Tensor sum;
-    const Tensor normed2 = residual_norm(x, &attn, g1, &sum, n2w, n2b, real(a[3]));
-    if (with_ffn) {
-      const Tensor h = at::gelu(linear(normed2, fc1_w, fc1_b));
-      const Tensor f = linear(h, fc2_w, fc2_b);
-      Tensor out;
-      residual_norm(sum, &f, g2, &out, nullptr, nullptr, 0.0);
-      sum = out;
-    }
-    return wrap(sum.view({B, N, C}));
+      const Tensor attn = linear(o.view({B * N, C}), proj_w, proj_b);
+      Tensor sum;
+      const Tensor normed2 = residual_norm(x, &attn, g1, &sum, n2w, n2b, eps2);
+      if (with_ffn) {
+        const Tensor h = at::gelu(linear(normed2, fc1_w, fc1_b));
+        const Tensor f = linear(h, fc2_w, fc2_b);
+        Tensor out;
+        residual_norm(sum, &f, g2, &out, nullptr, nullptr, 0.0);
+        sum = out;
+      }
+      return sum.view({B, N, C});
+    }));
   });
 }
 
@@ -651,10 +682,11 @@ PyObject* py_decode_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (k.size(0) != q.size(0) || v.size(0) != q.size(0)) value_error("decode attention: q, k and v must have the same number of rows");
     c10::cuda::CUDAGuard guard(q.device());
     Tensor out = empty(q.sizes(), at::kFloat, q);
-    check(gct_decode_attention(q.data_ptr<float>(), k.data_ptr<float>(), v.data_ptr<float>(), static_cast<int>(q.size(0)), ck.data_ptr<float>(),
-                               cv.data_ptr<float>(), static_cast<int>(integer(a[5])), static_cast<int>(ck.size(0)), PyObject_IsTrue(a[6]) == 1,
+    const int cached = static_cast<int>(integer(a[5])), store = PyObject_IsTrue(a[6]) == 1;
+    check(unlocked([&] { return gct_decode_attention(q.data_ptr<float>(), k.data_ptr<float>(), v.data_ptr<float>(), static_cast<int>(q.size(0)), ck.data_ptr<float>(),
+                               cv.data_ptr<float>(), cached, static_cast<int>(ck.size(0)), store,
                                static_cast<int>(ck.size(1)), static_cast<int>(ck.size(2)), out.data_ptr<float>(), ws.data_ptr(), ws.nbytes(),
-                               stream_of(q)));
+                               stream_of(q)); }));
     return wrap(std::move(out));
   });
 }
@@ -702,6 +734,9 @@ PyObject* py_frustum_cull(PyObject*, PyObject* const* a, Py_ssize_t n) {
     t = place(t);
     if (R.dim() != 2) R = R.reshape({3, 3});
     if (t.dim() != 1) t = t.reshape({3});
+    // their owner may free them on another stream as soon as this returns, as it could when the call waited for a copy
+    for (const Tensor* c : {&R, &t})
+      if (c->is_cuda()) c10::cuda::CUDACachingAllocator::recordStream(c->storage().data_ptr(), c10::cuda::getCurrentCUDAStream(pts.device().index()));
     const int strides[3] = {static_cast<int>(R.stride(0)), static_cast<int>(R.stride(1)), static_cast<int>(t.stride(0))};
     const int64_t count = pts.size(0);
     Tensor visible = empty({count}, at::kBool, pts);
@@ -723,7 +758,7 @@ PyObject* py_voxelize_frame(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int64_t count = in_xyz.size(0);
     if (count < 1 || count > gct::kVoxelMaxPoints) Py_RETURN_NONE;
     const Tensor xyz = float_rows(in_xyz, "pts_xyz"), rgb = float_rows(in_rgb, "pts_rgb");
-    if (xyz.numel() != 3 * count || rgb.numel() != 3 * count) value_error("pts_xyz and pts_rgb must be [N, 3]");
+    if (xyz.numel() < 3 * count || rgb.numel() < 3 * count) value_error("pts_xyz and pts_rgb must be [N, 3]");
     const float voxel = static_cast<float>(real(a[2]));
     c10::cuda::CUDAGuard guard(xyz.device());
     cudaStream_t s = stream_of(xyz);

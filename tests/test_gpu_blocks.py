@@ -252,3 +252,50 @@ def test_layers_as_one_call_equal_the_module_code(monkeypatch, dim, H, weights, 
         assert a.dtype == b.dtype and a.shape == b.shape, i
         d, top = float((a.float() - b.float()).abs().max()), float(b.float().abs().max())
         assert d <= 2 * 2 ** -7 * top, (i, d, top)
+
+
+def _layer_pair(dim=128, H=2):
+    blk = P.B200Block(dim=dim, num_heads=H, init_values=0.5, qk_norm=True, rope=Rope2dStub()).eval().to(DEV)
+    fa = P.B200FrameAttention(dim, num_heads=H, qk_norm=True, rope=Rope2dStub()).eval().to(DEV)
+    seeded.fill_module_(blk, 3)
+    seeded.fill_module_(fa, 4)
+    return blk.to(torch.bfloat16), fa.to(torch.bfloat16)
+
+
+def _off_alignment(t):
+    """The same values one element off a 16-byte boundary, as a slice of a flat parameter buffer lies."""
+    flat = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    flat[1:].copy_(t.reshape(-1))
+    return flat[1:].view(t.shape)
+
+
+@pytest.mark.parametrize("what", ["norm", "gamma", "qk norm", "input", "conjugated positions"])
+def test_layers_take_what_the_modules_take(what):
+    """Parameters and inputs off the 16-byte alignment of the vector loads, and positions whose conjugation is still to be
+    done: as one native call or through the modules, with the result of the aligned, resolved tensors.  Where the modules run instead
+    of the native layer a value may be rounded to bf16 once more on the way: two rounding steps, 2 * 2^-7 * max."""
+    blk, fa = _layer_pair()
+    pph, ppw, ns = 3, 5, 6
+    x = torch.from_numpy(seeded.randn(11, 1, ns + pph * ppw, 128)).to(DEV).bfloat16()
+    pos = rope3d_pos(3, 1, pph, ppw, ns)
+    kw = dict(num_patches=pph * ppw, num_special=ns, enable_3d_rope=True)
+
+    def run(x, pos):
+        with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+            return [blk(x, pos=pos, **kw), fa(x, pos=pos, enable_3d_rope=True)]
+
+    want = run(x, pos)
+    if what == "norm":
+        blk.norm1.weight.data, blk.norm2.bias.data = _off_alignment(blk.norm1.weight.data), _off_alignment(blk.norm2.bias.data)
+    elif what == "gamma":
+        blk.ls1.gamma.data, blk.ls2.gamma.data = _off_alignment(blk.ls1.gamma.data), _off_alignment(blk.ls2.gamma.data)
+    elif what == "qk norm":
+        for m in (blk.attn, fa):
+            m.q_norm.weight.data, m.k_norm.bias.data = _off_alignment(m.q_norm.weight.data), _off_alignment(m.k_norm.bias.data)
+    elif what == "input":
+        x = _off_alignment(x)
+    else:
+        pos = torch.conj(torch.conj_physical(pos))
+        assert pos.is_conj()
+    for got, ref in zip(run(x, pos), want):
+        assert float((got.float() - ref.float()).abs().max()) <= 2 * 2 ** -7 * float(ref.float().abs().max())

@@ -72,6 +72,22 @@ def test_more_than_eight_new_tokens_in_one_call():
     assert c.count == 23 and np.abs(got - want).max() <= 2e-5
 
 
+@pytest.mark.parametrize("cached", [0, 1, 2, 3, 33, 70])
+def test_infinite_value_of_the_last_key_stays_infinite(cached):
+    """A group of four keys that reaches past the end of a range must not multiply the last value row by a weight of zero."""
+    H, D = 2, 128
+    c = P.DecodeCache(H, D, DEV, capacity=128)
+    rs = np.random.RandomState(cached)
+    t = lambda *s: torch.from_numpy(rs.standard_normal(s).astype(np.float32)).to(DEV)
+    for _ in range(cached):
+        c.attend(t(1, H, D), t(1, H, D), t(1, H, D), True)
+    v = t(1, H, D)
+    v[0, :, 5] = float("inf")
+    out = c.attend(t(1, H, D), t(1, H, D), v, False).cpu()
+    assert bool((out[0, :, 5] == float("inf")).all())
+    assert bool(torch.isfinite(out[0, :, :5]).all() and torch.isfinite(out[0, :, 6:]).all())
+
+
 @pytest.mark.skipif(not os.path.isdir(os.path.join(REF, "lingbot_map")), reason="reference package not installed under baseline/_ref")
 def test_camera_head_stream_matches_reference():
     if REF not in sys.path:
