@@ -2,20 +2,12 @@
 // K/V rows written straight into their cache pages, fp32->bf16 cast, split-KV merge, RoPE tables.
 #include <math.h>
 
+#include <type_traits>
+
 #include "gct_common.h"
 
 namespace gct {
 namespace {
-
-// One warp per (token, group of four heads): lanes 8h..8h+7 own head h of the group, lane part s = lane & 7
-// owns the eight consecutive elements 8s..8s+7 of the 64-wide row (one 16-byte bf16 or two 16-byte fp32
-// loads), so a warp moves 512 contiguous bytes per tensor and all of q, k, v are in flight at once.
-//   LayerNorm(64), eps 1e-5, affine            lingbot_map/layers/attention.py:58-59,415
-//   3-D RoPE: pair (2m,2m+1) rotated by angle m lingbot_map/layers/rope.py:450-461
-//   2-D RoPE: inside each 32-wide half pair (j, j+16) rotated by angle j; table entry 16*half + j
-//                                              lingbot_map/layers/rope.py:134-157,191-198
-//   page write of K/V rows                     lingbot_map/layers/flashinfer_cache.py:503-505,547-549
-constexpr int kHeadsPerWarp = 4;
 
 struct Row8 {
   float v[8];
@@ -60,88 +52,177 @@ __device__ __forceinline__ float row_sum(float x) {
   return x;
 }
 
-// cs: the eight (cos, sin) pairs this lane needs.  3-D: entries 4s..4s+3 (pairs of its 8 elements), only
-// cs[0..3] used.  2-D: entries 16*half + 8*(s&1) + i for its elements i = 0..7.
-__device__ __forceinline__ void norm_rope8(Row8& x, const void* w, const void* bia, int norm_dtype, const float2 (&cs)[8],
-                                           int rope_mode, int part) {
-  if (w != nullptr) {
-    float sum = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) sum += x.v[i];
-    const float mean = row_sum(sum) * (1.f / 64.f);
-    float sq = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      x.v[i] -= mean;
-      sq += x.v[i] * x.v[i];
-    }
-    const float rstd = rsqrtf(row_sum(sq) * (1.f / 64.f) + 1e-5f);
-    const Row8 ww = load8(w, norm_dtype, 8 * part), bb = load8(bia, norm_dtype, 8 * part);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) x.v[i] = x.v[i] * rstd * ww.v[i] + bb.v[i];
+// ---- q/k LayerNorm + RoPE + bf16 + page write ------------------------------------------------------
+//   LayerNorm(64), eps 1e-5, affine            lingbot_map/layers/attention.py:58-59,415
+//   3-D RoPE: pair (2m,2m+1) rotated by angle m lingbot_map/layers/rope.py:450-461
+//   2-D RoPE: inside each 32-wide half pair (j, j+16) rotated by angle j; table entry 16*half + j
+//                                              lingbot_map/layers/rope.py:134-157,191-198
+//   page write of K/V rows                     lingbot_map/layers/flashinfer_cache.py:503-505,547-549
+//
+// Four lanes per (token, head) row of 64, rows handed to the lanes in order (any number of heads fills the warps).  Lane part s
+// owns elements [e, e+8) and [e+16, e+24) with e = 32*(s/2) + 8*(s%2): the partners of both rotations are then its own, the
+// only exchanges are the two steps of each LayerNorm sum, and q, k and v are six 16-byte loads in flight (twelve in fp32).
+// With one frame (12 MB, 1005 rows of 16 heads) the kernel is one round trip to memory and its launch; with many it is bound by
+// memory and by instructions.  What it is built around: types and rotation are template parameters, because a branch on the
+// type at each load makes the loads wait for one another; norm parameters are read once per CTA into shared memory under the
+// row loads.  With eight lanes per row and types at
+// run time (31 shuffles per four heads instead of 10 per eight, three round trips in a row) one frame took 8.5 us (2-D) and 9.9 us (3-D,
+// pages), now 6.0 and 6.4 us; eight frames (99 MB) 31.5 us, now 21.2 us (4.7 TB/s).
+constexpr int kPrepThreads = 128;
+constexpr int kRope3dF64 = 3;            // GCT_ROPE_3D on a table of doubles
+
+template <bool kF32>
+struct RawRow;                           // a lane's sixteen elements as loaded
+template <>
+struct RawRow<false> {
+  uint4 u[2];
+  __device__ __forceinline__ void load(const void* base, size_t e) {
+    const __nv_bfloat16* p = static_cast<const __nv_bfloat16*>(base) + e;
+    u[0] = *reinterpret_cast<const uint4*>(p);
+    u[1] = *reinterpret_cast<const uint4*>(p + 16);
   }
-  if (rope_mode == GCT_ROPE_3D) {
+  __device__ __forceinline__ void floats(float (&x)[16]) const {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float a = x.v[2 * i] * cs[i].x - x.v[2 * i + 1] * cs[i].y;
-      const float b = x.v[2 * i] * cs[i].y + x.v[2 * i + 1] * cs[i].x;
-      x.v[2 * i] = a;
-      x.v[2 * i + 1] = b;
-    }
-  } else if (rope_mode == GCT_ROPE_2D) {
-    // element e' = 8*(part & 3) + i inside its 32-wide half; its partner e' +/- 16 lives two lanes away.
-    // First 16 of a half: out = x*cos - partner*sin; last 16: out = x*cos + partner*sin.
-    const float sgn = (part & 2) ? 1.f : -1.f;
+    for (int c = 0; c < 2; ++c) {
+      const uint32_t w[4] = {u[c].x, u[c].y, u[c].z, u[c].w};
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float partner = __shfl_xor_sync(0xffffffffu, x.v[i], 2);
-      x.v[i] = x.v[i] * cs[i].x + sgn * partner * cs[i].y;
+      for (int i = 0; i < 4; ++i) {
+        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
+        x[8 * c + 2 * i] = f.x;
+        x[8 * c + 2 * i + 1] = f.y;
+      }
     }
+  }
+};
+template <>
+struct RawRow<true> {
+  float4 u[4];
+  __device__ __forceinline__ void load(const void* base, size_t e) {
+    const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(base) + e);
+    u[0] = p[0];
+    u[1] = p[1];
+    u[2] = p[4];
+    u[3] = p[5];
+  }
+  __device__ __forceinline__ void floats(float (&x)[16]) const {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      x[4 * c] = u[c].x;
+      x[4 * c + 1] = u[c].y;
+      x[4 * c + 2] = u[c].z;
+      x[4 * c + 3] = u[c].w;
+    }
+  }
+};
+
+__device__ __forceinline__ void store16(__nv_bfloat16* dst, const float (&x)[16]) {
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    Row8 r;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) r.v[i] = x[8 * c + i];
+    store8(dst + 16 * c, r);
   }
 }
 
-__global__ void __launch_bounds__(256) gct_prep_kernel(const PrepLaunch p) {
-  pdl_wait();
-  const int lane = threadIdx.x & 31;
-  const int part = lane & 7;
-  const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int head_groups = (p.heads + kHeadsPerWarp - 1) / kHeadsPerWarp;
-  const int token = wid / head_groups;
-  if (token >= p.tokens) return;
-  const int h = (wid - token * head_groups) * kHeadsPerWarp + (lane >> 3);
-  const bool active = h < p.heads;          // inactive lanes still take part in the shuffles
-  const int hh = active ? h : p.heads - 1;
-  const int tf = token % p.tokens_per_frame;
+// sum over the four lanes of a row
+__device__ __forceinline__ float quad_sum(float x) {
+  x += __shfl_xor_sync(0xffffffffu, x, 1);
+  x += __shfl_xor_sync(0xffffffffu, x, 2);
+  return x;
+}
 
+// w, bia: 64 floats each in shared memory, already offset by the lane's first element.
+__device__ __forceinline__ void norm16(float (&x)[16], const float* w, const float* bia) {
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int i = 0; i < 16; ++i) s[i & 3] += x[i];
+  const float mean = quad_sum((s[0] + s[1]) + (s[2] + s[3])) * (1.f / 64.f);
+  float sq[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    x[i] -= mean;
+    sq[i & 3] += x[i] * x[i];
+  }
+  const float rstd = rsqrtf(quad_sum((sq[0] + sq[1]) + (sq[2] + sq[3])) * (1.f / 64.f) + 1e-5f);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const int at = 4 * (c & 1) + 16 * (c >> 1);
+    const float4 ww = *reinterpret_cast<const float4*>(w + at), bb = *reinterpret_cast<const float4*>(bia + at);
+    x[4 * c] = x[4 * c] * rstd * ww.x + bb.x;
+    x[4 * c + 1] = x[4 * c + 1] * rstd * ww.y + bb.y;
+    x[4 * c + 2] = x[4 * c + 2] * rstd * ww.z + bb.z;
+    x[4 * c + 3] = x[4 * c + 3] * rstd * ww.w + bb.w;
+  }
+}
+
+// cs: 3-D: cs[i] rotates the pair of elements 2i, 2i+1 of the sixteen; 2-D: cs[i] the elements i and i + 8.
+template <int kMode>
+__device__ __forceinline__ void rotate16(float (&x)[16], const float2 (&cs)[8]) {
+  if constexpr (kMode == GCT_ROPE_NONE) return;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int lo = kMode == GCT_ROPE_2D ? i : 2 * i, hi = kMode == GCT_ROPE_2D ? i + 8 : 2 * i + 1;
+    const float a = x[lo] * cs[i].x - x[hi] * cs[i].y;
+    const float b = x[lo] * cs[i].y + x[hi] * cs[i].x;
+    x[lo] = a;
+    x[hi] = b;
+  }
+}
+
+// kMode: rotation; kQkF32, kVF32: types of the sources of q and k, and of v.
+template <int kMode, bool kQkF32, bool kVF32>
+__global__ void __launch_bounds__(kPrepThreads) gct_prep_kernel(const PrepLaunch p) {
+  __shared__ __align__(16) float s_norm[4][kHeadDim];       // q weight, q bias, k weight, k bias
+  pdl_wait();
+  const int part = threadIdx.x & 3, e0 = 32 * (part >> 1) + 8 * (part & 1);
+  const int rows = p.tokens * p.heads;
+  const int row = (blockIdx.x * kPrepThreads + threadIdx.x) >> 2;
+  const bool active = row < rows;           // inactive lanes (all four of a row) still take part in the shuffles
+  const int r = active ? row : rows - 1;
+  const int token = r / p.heads, h = r - token * p.heads;
+  const bool do_q = p.q_src != nullptr && p.q_out != nullptr, do_kv = p.k_out != nullptr || p.pool != nullptr;
+  const size_t src = static_cast<size_t>(token) * p.src_token_stride + static_cast<size_t>(h) * p.src_head_stride + e0;
+  RawRow<kQkF32> rq, rk;
+  RawRow<kVF32> rv;
+  if (do_q) rq.load(p.q_src, src);
+  if (do_kv) {
+    rk.load(p.k_src, src);
+    rv.load(p.v_src, src);
+  }
   // rotation coefficients of this lane
   float2 cs[8];
-  if (p.rope_mode == GCT_ROPE_3D) {
-    const size_t e = (static_cast<size_t>(tf) * 32 + 4 * part) * 2;
-    if (p.rope_f64) {
-      const double2* t = reinterpret_cast<const double2*>(static_cast<const double*>(p.rope_cs) + e);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const double2 d = t[i];
-        cs[i] = make_float2(static_cast<float>(d.x), static_cast<float>(d.y));
-      }
-    } else {
-      const float4* t = reinterpret_cast<const float4*>(static_cast<const float*>(p.rope_cs) + e);
-      const float4 a = t[0], b = t[1];
-      cs[0] = make_float2(a.x, a.y);
-      cs[1] = make_float2(a.z, a.w);
-      cs[2] = make_float2(b.x, b.y);
-      cs[3] = make_float2(b.z, b.w);
-    }
-  } else if (p.rope_mode == GCT_ROPE_2D) {
-    const int entry = (part >> 2) * 16 + (part & 1) * 8;      // 16*half + (e' % 16) for this lane's first element
-    const float4* t = reinterpret_cast<const float4*>(static_cast<const float*>(p.rope_cs) + (static_cast<size_t>(tf) * 32 + entry) * 2);
+  if constexpr (kMode != GCT_ROPE_NONE) {
+    const size_t entry = static_cast<size_t>(token % p.tokens_per_frame) * 32 + (kMode == GCT_ROPE_2D ? 16 * (part >> 1) + 8 * (part & 1) : e0 / 2);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const float4 a = t[i];
-      cs[2 * i] = make_float2(a.x, a.y);
-      cs[2 * i + 1] = make_float2(a.z, a.w);
+      const size_t at = 2 * (entry + (kMode == GCT_ROPE_2D ? 2 * i : 2 * (i & 1) + 8 * (i >> 1)));      // two entries
+      if constexpr (kMode == kRope3dF64) {
+        const double2* t = reinterpret_cast<const double2*>(static_cast<const double*>(p.rope_cs) + at);
+        const double2 c0 = t[0], c1 = t[1];
+        cs[2 * i] = make_float2(static_cast<float>(c0.x), static_cast<float>(c0.y));
+        cs[2 * i + 1] = make_float2(static_cast<float>(c1.x), static_cast<float>(c1.y));
+      } else {
+        const float4 c = *reinterpret_cast<const float4*>(static_cast<const float*>(p.rope_cs) + at);
+        cs[2 * i] = make_float2(c.x, c.y);
+        cs[2 * i + 1] = make_float2(c.z, c.w);
+      }
     }
   }
+  // the running maximum as it was: older than the atomics below, so at worst one of them is issued in vain
+  unsigned int seen = 0;
+  if (do_kv && p.key_norm_max != nullptr) seen = *reinterpret_cast<volatile unsigned int*>(p.key_norm_max + h);
+  // norm parameters, one element per array and thread of half a CTA
+  {
+    const int i = threadIdx.x & 63, which = threadIdx.x >> 6;
+    const void* const w = which ? p.kn_w : p.qn_w;
+    const void* const b = which ? p.kn_b : p.qn_b;
+    if (w != nullptr) {
+      s_norm[2 * which][i] = p.norm_dtype == GCT_F32 ? static_cast<const float*>(w)[i] : __bfloat162float(static_cast<const __nv_bfloat16*>(w)[i]);
+      s_norm[2 * which + 1][i] = p.norm_dtype == GCT_F32 ? static_cast<const float*>(b)[i] : __bfloat162float(static_cast<const __nv_bfloat16*>(b)[i]);
+    }
+  }
+  __syncthreads();
 
   // destination rows of K and V for this token
   __nv_bfloat16* k_row = nullptr;
@@ -162,48 +243,40 @@ __global__ void __launch_bounds__(256) gct_prep_kernel(const PrepLaunch p) {
       slot = token - p.sp_n0;
     }
     if (page < 0 || page >= p.num_pages || slot < 0 || slot >= p.page_size) {
-      if (lane == 0) atomicCAS(p.status, 0, kStatusBadIndex);
-      return;
+      if (active && part == 0) atomicCAS(p.status, 0, kStatusBadIndex);
+    } else {
+      const size_t page_elems = static_cast<size_t>(p.page_size) * p.heads * kHeadDim;
+      k_row = p.pool + (static_cast<size_t>(page) * 2) * page_elems + static_cast<size_t>(slot) * p.heads * kHeadDim;
+      v_row = k_row + page_elems;
     }
-    const size_t page_elems = static_cast<size_t>(p.page_size) * p.heads * kHeadDim;
-    k_row = p.pool + (static_cast<size_t>(page) * 2) * page_elems + static_cast<size_t>(slot) * p.heads * kHeadDim;
-    v_row = k_row + page_elems;
   }
+  const bool in_range = !do_kv || k_row != nullptr;         // a token without a valid page writes nothing
 
-  const size_t src = static_cast<size_t>(token) * p.src_token_stride + static_cast<size_t>(hh) * p.src_head_stride +
-                     8 * part;
-  const size_t dst = static_cast<size_t>(hh) * kHeadDim + 8 * part;
-  const bool do_q = p.q_src != nullptr && p.q_out != nullptr;
-  const bool do_kv = k_row != nullptr;
-  Row8 q, k, v;
-  if (do_q) q = load8(p.q_src, p.src_dtype_qk, src);
-  if (do_kv) {
-    k = load8(p.k_src, p.src_dtype_qk, src);
-    v = load8(p.v_src, p.src_dtype_v, src);
-  }
+  const size_t dst = static_cast<size_t>(h) * kHeadDim + e0;
+  float x[16];
   if (do_q) {
-    norm_rope8(q, p.qn_w, p.qn_b, p.norm_dtype, cs, p.rope_mode, part);
-    if (active) store8(p.q_out + static_cast<size_t>(token) * p.heads * kHeadDim + dst, q);
+    rq.floats(x);
+    if (p.qn_w != nullptr) norm16(x, s_norm[0] + e0, s_norm[1] + e0);
+    rotate16<kMode>(x, cs);
+    if (active && in_range) store16(p.q_out + static_cast<size_t>(token) * p.heads * kHeadDim + dst, x);
   }
   if (do_kv) {
-    norm_rope8(k, p.kn_w, p.kn_b, p.norm_dtype, cs, p.rope_mode, part);
-    if (active) {
-      store8(k_row + dst, k);
-      store8(v_row + dst, v);
-    }
+    rk.floats(x);
+    if (p.kn_w != nullptr) norm16(x, s_norm[2] + e0, s_norm[3] + e0);
+    rotate16<kMode>(x, cs);
+    if (active && in_range) store16(k_row + dst, x);
     if (p.key_norm_max != nullptr) {
       // running maximum of |k| per head (an upper bound: fp32 values, inflated for the bf16 rounding).  Positive
-      // floats order like their bit patterns; the plain read first keeps atomics rare once the maximum settles.
-      float sq = 0.f;
+      // floats order like their bit patterns; the look at the maximum above keeps atomics rare once it settles.
+      float sq[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int i = 0; i < 8; ++i) sq += k.v[i] * k.v[i];
-      const float nrm = sqrtf(row_sum(sq)) * 1.004f;
-      if (active && part == 0) {
-        unsigned int* slot = reinterpret_cast<unsigned int*>(p.key_norm_max + hh);
-        if (!(nrm <= __uint_as_float(*reinterpret_cast<volatile unsigned int*>(slot))))   // also taken for NaN
-          atomicMax(slot, nrm == nrm ? __float_as_uint(nrm) : 0x7f800000u);
-      }
+      for (int i = 0; i < 16; ++i) sq[i & 3] += x[i] * x[i];
+      const float nrm = sqrtf(quad_sum((sq[0] + sq[1]) + (sq[2] + sq[3]))) * 1.004f;
+      if (active && in_range && part == 0 && !(nrm <= __uint_as_float(seen)))        // also taken for NaN
+        atomicMax(reinterpret_cast<unsigned int*>(p.key_norm_max + h), nrm == nrm ? __float_as_uint(nrm) : 0x7f800000u);
     }
+    rv.floats(x);
+    if (active && in_range) store16(v_row + dst, x);
   }
 }
 
@@ -443,10 +516,19 @@ int launch_prep(const PrepLaunch& p, cudaStream_t stream) {
       misaligned(p.v_out) || misaligned(p.pool) || misaligned(p.qn_w) || misaligned(p.qn_b) || misaligned(p.kn_w) ||
       misaligned(p.kn_b) || misaligned(p.rope_cs))
     return fail(GCT_ERR_INVALID, "prep: tensors must be 16-byte aligned");
-  const int head_groups = (p.heads + kHeadsPerWarp - 1) / kHeadsPerWarp;
-  const long long warps = static_cast<long long>(p.tokens) * head_groups;
-  const int blocks = static_cast<int>((warps * 32 + 255) / 256);
-  GCT_CUDA_CHECK(launch_pdl(gct_prep_kernel, dim3(blocks), dim3(256), 0, stream, p));
+  const long long rows = static_cast<long long>(p.tokens) * p.heads;
+  if (rows > (1ll << 28)) return fail(GCT_ERR_INVALID, "prep: too many rows");
+  const dim3 grid(static_cast<unsigned>((rows * 4 + kPrepThreads - 1) / kPrepThreads)), block(kPrepThreads);
+  const bool qk32 = p.src_dtype_qk == GCT_F32, v32 = p.src_dtype_v == GCT_F32;
+  auto pick = [&](auto mode) {
+    constexpr int m = decltype(mode)::value;
+    return qk32 ? (v32 ? gct_prep_kernel<m, true, true> : gct_prep_kernel<m, true, false>)
+                : (v32 ? gct_prep_kernel<m, false, true> : gct_prep_kernel<m, false, false>);
+  };
+  auto kernel = p.rope_mode == GCT_ROPE_3D ? (p.rope_f64 ? pick(std::integral_constant<int, kRope3dF64>()) : pick(std::integral_constant<int, GCT_ROPE_3D>()))
+                : p.rope_mode == GCT_ROPE_2D ? pick(std::integral_constant<int, GCT_ROPE_2D>())
+                                             : pick(std::integral_constant<int, GCT_ROPE_NONE>());
+  GCT_CUDA_CHECK(launch_pdl(kernel, grid, block, 0, stream, p));
   return GCT_OK;
 }
 

@@ -242,6 +242,40 @@ def test_append_fused_equals_prep_then_append():
     assert len(a2.all_special_pages[0]) == 6 and a2.compute_last_page_len(0) == 1
 
 
+@pytest.mark.parametrize("tokens,tpf,H", [(1, 1, 1), (7, 7, 3), (33, 11, 2), (40, 20, 16), (1005, 1005, 5)])
+@pytest.mark.parametrize("rope", ["none", "2d", "3d", "3d f64"])
+@pytest.mark.parametrize("src,norm", [("f32", "f32"), ("bf16", "bf16"), ("bf16", "none"), ("f32", "bf16")])
+def test_prologue_types_rotations_and_ragged_rows(tokens, tpf, H, rope, src, norm):
+    """Every instantiation of the prologue, at row counts that fill no warp, one CTA partly and several, against float64: the
+    result is rounded to bf16 once (2^-8 of the value after a rotation of fp32 values of size <= 8, error below 1e-4)."""
+    g = torch.Generator(device=DEV).manual_seed(tokens * 31 + H)
+    rand = lambda *n: torch.randn(*n, device=DEV, generator=g)
+    dt = {"f32": torch.float32, "bf16": torch.bfloat16}
+    qkv = torch.cat([rand(tokens, 3 * H * 64), rand(tokens, 8)], dim=1).to(dt[src])[:, :3 * H * 64]        # rows further apart than they are long
+    par = [None] * 4 if norm == "none" else [(1 + 0.1 * rand(64)).to(dt[norm]), (0.1 * rand(64)).to(dt[norm]), (1 + 0.1 * rand(64)).to(dt[norm]),
+                                             (0.1 * rand(64)).to(dt[norm])]
+    ang = rand(tpf, 32).double()
+    cs = torch.stack([ang.cos(), ang.sin()], -1)
+    mode, table = {"none": (_lib.ROPE_NONE, None), "2d": (_lib.ROPE_2D, cs.float()), "3d": (_lib.ROPE_3D, cs.float()),
+                   "3d f64": (_lib.ROPE_3D, torch.view_as_complex(cs))}[rope]
+    got = P.ops.prep_qkv(qkv, H, tpf, *par, table, mode)
+    parts = qkv.double().reshape(tokens, 3, H, 64).unbind(1)
+    c, sn = (x[torch.arange(tokens, device=DEV) % tpf][:, None] for x in (ang.cos(), ang.sin()))
+    for i, x in enumerate(parts):
+        if i < 2:
+            if par[0] is not None:
+                x = torch.nn.functional.layer_norm(x, (64,), par[2 * i].double(), par[2 * i + 1].double(), 1e-5)
+            if rope.startswith("3d"):
+                a, b = x[..., 0::2], x[..., 1::2]
+                x = torch.stack([a * c - b * sn, a * sn + b * c], -1).reshape(tokens, H, 64)
+            elif rope == "2d":
+                y = x.reshape(tokens, H, 2, 2, 16)
+                a, b = y[:, :, :, 0], y[:, :, :, 1]
+                c2, s2 = c.reshape(tokens, 1, 2, 16), sn.reshape(tokens, 1, 2, 16)
+                x = torch.stack([a * c2 - b * s2, a * s2 + b * c2], 3).reshape(tokens, H, 64)
+        assert bool(((got[i].double() - x).abs() <= 2 ** -8 * x.abs() + 1e-4).all()), i
+
+
 # ---------------------------------------------------------------- production geometry
 def test_full_geometry_properties():
     """378x518 geometry: 1005 tokens/frame, 16 heads, page 999, scale 8 + window 64, 80 keyframes.
