@@ -276,6 +276,28 @@ def test_prologue_types_rotations_and_ragged_rows(tokens, tpf, H, rope, src, nor
         assert bool(((got[i].double() - x).abs() <= 2 ** -8 * x.abs() + 1e-4).all()), i
 
 
+@pytest.mark.parametrize("groups", [1, 2, 3, 4, 5, 8, 9, 17])
+@pytest.mark.parametrize("shift", [0, 2])
+def test_merge_of_any_number_of_partials(groups, shift):
+    """Partials of 16-byte and of 8-byte alignment (every group off by `shift` floats), weights over many orders of magnitude,
+    a group without keys; against float64: bf16 rounding of the result plus 1e-5 for the fp32 sums and the fast exponential."""
+    n_q, H = 5, 3
+    rows = n_q * H
+    g = torch.Generator(device=DEV).manual_seed(groups)
+    flat = torch.randn(groups, rows * 64 + shift, device=DEV, generator=g)
+    lse = 4 * torch.randn(groups, rows, device=DEV, generator=g)
+    if groups > 1:
+        lse[groups // 2] = float("-inf")
+    out = torch.empty(n_q, H, 64, dtype=torch.bfloat16, device=DEV)
+    lse_out = torch.empty(rows, device=DEV)
+    _lib.check(_lib.load().gct_lse_merge_strided(flat.data_ptr(), lse.data_ptr(), groups, n_q, H, flat.shape[1], rows, out.data_ptr(),
+                                                 lse_out.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    w = torch.softmax(lse.double(), 0)
+    want = (w[:, :, None] * flat[:, :rows * 64].double().reshape(groups, rows, 64)).sum(0)
+    assert bool(((out.double().reshape(rows, 64) - want).abs() <= 2 ** -8 * want.abs() + 1e-5).all())
+    assert float((lse_out.double() - torch.logsumexp(lse.double(), 0)).abs().max()) <= 1e-5
+
+
 # ---------------------------------------------------------------- production geometry
 def test_full_geometry_properties():
     """378x518 geometry: 1005 tokens/frame, 16 heads, page 999, scale 8 + window 64, 80 keyframes.
