@@ -280,80 +280,117 @@ __global__ void __launch_bounds__(kPrepThreads) gct_prep_kernel(const PrepLaunch
   }
 }
 
+// Eight consecutive elements as loaded, of either type: all loads of a thread are issued before the first conversion, which a
+// branch on the type around load and conversion would prevent.
+struct Raw8 {
+  uint4 a, b;
+  __device__ __forceinline__ void load(const void* base, int dtype, size_t elem) {
+    const uint4* p = reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(base) + elem * (dtype == GCT_F32 ? 4 : 2));
+    a = p[0];
+    if (dtype == GCT_F32) b = p[1];
+  }
+  __device__ __forceinline__ Row8 floats(int dtype) const {
+    Row8 r;
+    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    if (dtype == GCT_F32) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) r.v[i] = __uint_as_float(w[i]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        r.v[2 * i] = __uint_as_float(w[i] << 16);
+        r.v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+      }
+    }
+    return r;
+  }
+};
+
 // v = x + gamma * y per row, stored in x's precision, and LayerNorm(v) as bf16: the residual sums and norms of a block
 // (lingbot_map/layers/block.py:217-310) in one pass over the row, which as separate tensor operations were four to
-// six launches of 2-7 us each (scale, add, norm in fp32, cast to bf16 for the next Linear).  One warp per row, the row in
-// registers: 12 MB for 1005 x 1024 in bf16, so the time is one round trip to memory.
-template <int kChunks>                    // 8-element chunks per lane: columns <= 256 * kChunks
-__global__ void __launch_bounds__(128) gct_residual_norm_kernel(const RowLaunch p) {
+// six launches of 2-7 us each (scale, add, norm in fp32, cast to bf16 for the next Linear).
+//
+// A frame is 1005 rows of 1024 (6-12 MB), so the time is the chain load - mean - variance - store and how many rows are in
+// flight.  Eight elements per thread and as many threads per row as that takes (whole warps; kThreads), everything the thread
+// needs loaded first.  One warp per row, with the parameters fetched after the sums, took
+// 5.6 us (norm alone), 9.2 us (sum and norm) and 6.4 us (sum alone), now 4.0, 4.8 and 3.6 us.
+template <int kThreads>                   // threads per row: 32, 64, 128 or 256; columns <= 8 * kThreads
+__global__ void __launch_bounds__(kThreads > 128 ? kThreads : 128) gct_residual_norm_kernel(const RowLaunch p) {
+  constexpr int kRows = kThreads >= 128 ? 1 : 128 / kThreads, kWarps = kThreads / 32;      // rows per CTA, warps per row
+  __shared__ float s_part[2][kRows][kWarps];
   pdl_wait();
-  const int lane = threadIdx.x & 31;
-  const int64_t row = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  if (row >= p.rows) return;
-  const size_t base = static_cast<size_t>(row) * p.cols;
-  Row8 v[kChunks];
-  float sum = 0.f;
-#pragma unroll
-  for (int c = 0; c < kChunks; ++c) {
-    const int col = 8 * (32 * c + lane);
-    if (col < p.cols) v[c] = load8(p.x, p.x_dtype, base + col);
+  const int in_row = threadIdx.x % kThreads, local = threadIdx.x / kThreads, lane = threadIdx.x & 31, warp = in_row >> 5;
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * kRows + local;
+  const int col = 8 * in_row;
+  const bool active = row < p.rows && col < p.cols;
+  const size_t at = static_cast<size_t>(row) * p.cols + col;
+  const bool with_y = p.y != nullptr, with_gamma = with_y && p.gamma != nullptr, with_norm = p.norm_out != nullptr;
+  Raw8 x, y, g, w, b;
+  if (active) {
+    x.load(p.x, p.x_dtype, at);
+    if (with_y) y.load(p.y, GCT_BF16, at);
+    if (with_gamma) g.load(p.gamma, p.gamma_dtype, col);
+    if (with_norm) {
+      w.load(p.norm_w, p.norm_dtype, col);
+      b.load(p.norm_b, p.norm_dtype, col);
+    }
   }
-  if (p.y != nullptr) {
+  Row8 v = {};
+  if (active) {
+    v = x.floats(p.x_dtype);
+    if (with_y) {
+      const Row8 yy = y.floats(GCT_BF16);
+      if (with_gamma) {
+        const Row8 gg = g.floats(p.gamma_dtype);
 #pragma unroll
-    for (int c = 0; c < kChunks; ++c) {
-      const int col = 8 * (32 * c + lane);
-      if (col >= p.cols) continue;
-      const Row8 y = load8(p.y, GCT_BF16, base + col);
-      if (p.gamma != nullptr) {
-        const Row8 g = load8(p.gamma, p.gamma_dtype, col);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[c].v[i] = fmaf(y.v[i], g.v[i], v[c].v[i]);
+        for (int i = 0; i < 8; ++i) v.v[i] = fmaf(yy.v[i], gg.v[i], v.v[i]);
       } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[c].v[i] += y.v[i];
+        for (int i = 0; i < 8; ++i) v.v[i] += yy.v[i];
       }
       if (p.sum_dtype == GCT_F32) {
-        float4* d = reinterpret_cast<float4*>(static_cast<float*>(p.sum_out) + base + col);
-        d[0] = make_float4(v[c].v[0], v[c].v[1], v[c].v[2], v[c].v[3]);
-        d[1] = make_float4(v[c].v[4], v[c].v[5], v[c].v[6], v[c].v[7]);
+        float4* d = reinterpret_cast<float4*>(static_cast<float*>(p.sum_out) + at);
+        d[0] = make_float4(v.v[0], v.v[1], v.v[2], v.v[3]);
+        d[1] = make_float4(v.v[4], v.v[5], v.v[6], v.v[7]);
       } else {
-        store8(static_cast<__nv_bfloat16*>(p.sum_out) + base + col, v[c]);
+        store8(static_cast<__nv_bfloat16*>(p.sum_out) + at, v);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[c].v[i] = __bfloat162float(__float2bfloat16_rn(v[c].v[i]));      // the norm is that of the stored sum
+        for (int i = 0; i < 8; ++i) v.v[i] = __bfloat162float(__float2bfloat16_rn(v.v[i]));      // the norm is that of the stored sum
       }
     }
   }
-  if (p.norm_out == nullptr) return;
+  if (!with_norm) return;
+  // sum over the threads of a row (idle ones add zero); every thread of the CTA comes here
+  auto total = [&](float t, int step) -> float {
 #pragma unroll
-  for (int c = 0; c < kChunks; ++c)
-    if (8 * (32 * c + lane) < p.cols)
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if constexpr (kWarps > 1) {
+      if (lane == 0) s_part[step][local][warp] = t;
+      __syncthreads();
+      t = 0.f;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) sum += v[c].v[i];
+      for (int i = 0; i < kWarps; ++i) t += s_part[step][local][i];
+    }
+    return t;
+  };
+  float sum = 0.f, sq = 0.f;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  const float mean = sum / p.cols;
-  float sq = 0.f;
+  for (int i = 0; i < 8; ++i) sum += v.v[i];
+  const float mean = total(sum, 0) / p.cols;
+  if (active) {
 #pragma unroll
-  for (int c = 0; c < kChunks; ++c)
-    if (8 * (32 * c + lane) < p.cols)
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        v[c].v[i] -= mean;
-        sq = fmaf(v[c].v[i], v[c].v[i], sq);
-      }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-  const float rstd = rsqrtf(sq / p.cols + p.eps);
-#pragma unroll
-  for (int c = 0; c < kChunks; ++c) {
-    const int col = 8 * (32 * c + lane);
-    if (col >= p.cols) continue;
-    Row8 r;
-    const Row8 w = load8(p.norm_w, p.norm_dtype, col), b = load8(p.norm_b, p.norm_dtype, col);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) r.v[i] = fmaf(v[c].v[i] * rstd, w.v[i], b.v[i]);
-    store8(p.norm_out + base + col, r);
+    for (int i = 0; i < 8; ++i) {
+      v.v[i] -= mean;
+      sq = fmaf(v.v[i], v.v[i], sq);
+    }
   }
+  const float rstd = rsqrtf(total(sq, 1) / p.cols + p.eps);
+  if (!active) return;
+  const Row8 ww = w.floats(p.norm_dtype), bb = b.floats(p.norm_dtype);
+  Row8 r;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) r.v[i] = fmaf(v.v[i] * rstd, ww.v[i], bb.v[i]);
+  store8(p.norm_out + at, r);
 }
 
 // cos/sin table of the 2-D rotation from integer (y, x) positions [tokens, 2] (lingbot_map/layers/rope.py:105-119): entry
@@ -587,9 +624,13 @@ int launch_residual_norm(const RowLaunch& p, cudaStream_t stream) {
   if (misaligned(p.x) || misaligned(p.y) || misaligned(p.gamma) || misaligned(p.norm_w) || misaligned(p.norm_b) || misaligned(p.sum_out) ||
       misaligned(p.norm_out))
     return fail(GCT_ERR_INVALID, "residual norm: tensors must be 16-byte aligned");
-  const dim3 grid(static_cast<unsigned>((p.rows + 3) / 4)), block(128);
-  const int chunks = (p.cols + 255) / 256;
-  auto kernel = chunks <= 1 ? gct_residual_norm_kernel<1> : chunks <= 2 ? gct_residual_norm_kernel<2> : chunks <= 4 ? gct_residual_norm_kernel<4> : gct_residual_norm_kernel<8>;
+  // threads per row: eight columns each, whole warps; short rows share a CTA of 128
+  const int threads = p.cols <= 256 ? 32 : p.cols <= 512 ? 64 : p.cols <= 1024 ? 128 : 256;
+  const int64_t rows_per_cta = threads >= 128 ? 1 : 128 / threads, ctas = (p.rows + rows_per_cta - 1) / rows_per_cta;
+  if (ctas > 0x7fffffff) return fail(GCT_ERR_INVALID, "residual norm: too many rows");
+  const dim3 grid(static_cast<unsigned>(ctas)), block(threads > 128 ? threads : 128);
+  auto kernel = threads == 32 ? gct_residual_norm_kernel<32> : threads == 64 ? gct_residual_norm_kernel<64>
+                : threads == 128 ? gct_residual_norm_kernel<128> : gct_residual_norm_kernel<256>;
   GCT_CUDA_CHECK(launch_pdl(kernel, grid, block, 0, stream, p));
   return GCT_OK;
 }

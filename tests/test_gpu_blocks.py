@@ -182,12 +182,13 @@ def test_plain_attention_without_norm_and_rope():
 
 
 @pytest.mark.parametrize("dim,H,weights,x_dtype,rope", [(128, 2, "bf16", "bf16", "3d"), (192, 3, "f32", "f32", "3d"), (576, 9, "bf16", "f32", "none"),
-                                                        (1024, 16, "f32", "bf16", "2d"), (128, 2, "bf16", "bf16", "no autocast")])
+                                                        (1024, 16, "f32", "bf16", "2d"), (128, 2, "bf16", "bf16", "no autocast"),
+                                                        (320, 5, "bf16", "f32", "3d"), (1088, 17, "f32", "bf16", "none"), (2048, 32, "bf16", "f32", "3d")])
 @pytest.mark.parametrize("scaled", [True, False])
 def test_layers_as_one_call_equal_the_module_code(monkeypatch, dim, H, weights, x_dtype, rope, scaled):
     """B200Block and B200FrameAttention as single native calls against the same modules run operation by operation: scale
-    pass, keyframes with eviction, a non-keyframe, batch mode without a cache, a rebound ffn_residual; columns from half a
-    warp's chunk up to four, row counts that leave warps idle, and every combination of parameter and activation precision.
+    pass, keyframes with eviction, a non-keyframe, batch mode without a cache, a rebound ffn_residual; columns for one to
+    eight warps per row, row counts that leave warps idle, and every combination of parameter and activation precision.
 
     Both sides round the same intermediates to bf16, the native call fewer of them (scale and sum in one step), and return
     bf16 or fp32; results may differ by two bf16 rounding steps at the largest magnitude of the output, 2 * 2^-7 * max."""
