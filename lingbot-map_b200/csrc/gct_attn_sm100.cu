@@ -1096,14 +1096,26 @@ struct SplitPlan {
 void choose_attention_config(int n_q_tiles, int heads_x_batch, int total_blocks, int num_sms, int max_splits,
                              int* q_tiles_per_cta, int* splits, int* split_len) {
   // Cost model in units of "one KV block for one CTA": a CTA with two query tiles takes about as long
-  // per block as one with a single tile takes for 0.6 blocks-worth of its pair; every CTA pays a fixed
-  // prologue/epilogue of about two blocks, and a split result needs the merge kernel afterwards (a launch
+  // per block as one with a single tile takes for 0.6 blocks-worth of its pair; every wave of CTAs pays for
+  // its prologue and epilogue, and a split result needs the merge kernel afterwards (a launch
   // of its own, about five blocks).  Pick the cheapest (tiles per CTA, splits).
 #ifndef GCT_MERGE_COST
 #define GCT_MERGE_COST 5.0
 #endif
   constexpr double kMergeCost = GCT_MERGE_COST;
-  constexpr double kFixed = 2.0;
+  // Paged calls (split_len != nullptr): a call that fits one wave pays about five blocks once; in a call of several waves
+  // every wave costs about fifteen blocks beside its KV blocks (set-up, pipeline fill, epilogue, and at the board's power limit a
+  // lower clock the fuller the SMs are: idle SMs are not lost time there).  Measured, 64 (head, tile pair) items, us for 2 ranges
+  // (128 CTAs) against the 9 that a fixed cost of two blocks chose: 250 KV blocks 168 : 195, 371 242 : 268, 385 254 : 280,
+  // 527 338 : 360, 600 385 : 402.  One tile per CTA (0.6 of the work): measured for one wave only.
+  const bool paged = split_len != nullptr;
+  auto fixed = [paged](int qt, bool one_wave) { return !paged ? 2.0 : one_wave ? (qt == 2 ? 5.0 : 4.0) : (qt == 2 ? 15.0 : 9.0); };
+  // Long ranges + a short one fill the SMs that equal ranges leave idle.  The paged kernel alone, back to back at the power limit,
+  // takes about as long as with two equal ranges (us: 71 KV blocks 54.8 : 56.7, 193 134 : 132, 285 190 : 192, 600 392 : 385); inside
+  // a frame, beside the other kernels, it is faster: 24 layers at 600 blocks 9.7-10.0 ms against 10.5 with two and with nine
+  // equal ranges, two layer pairs as modules 949-974 : 1013 us.  Not beyond a thousand blocks: nine long ranges and a short one were
+  // 0.6 % slower there than nine equal ones (1057 blocks, back to back).
+  constexpr int kUnevenMaxBlocks = 1000;
   // the plan of the previous call with the same arguments (a frame asks 24 times for the same one)
   static thread_local SplitPlanKey last_key = {-1, -1, -1, -1, -1};
   static thread_local SplitPlan last_plan = {1, 1, 0};
@@ -1114,7 +1126,8 @@ void choose_attention_config(int n_q_tiles, int heads_x_batch, int total_blocks,
     *split_len = last_plan.split_len;
     return;
   }
-  double best = 1e300;
+  double best = 1e300, uneven = 1e300;
+  int uneven_qt = 1, uneven_s = 1, uneven_len = 0;
   int best_qt = 1, best_s = 1, best_len = 0;
   for (int qt = 2; qt >= 1; --qt) {
     const long long items = static_cast<long long>((n_q_tiles + qt - 1) / qt) * heads_x_batch;
@@ -1124,7 +1137,7 @@ void choose_attention_config(int n_q_tiles, int heads_x_batch, int total_blocks,
       const long long ctas = items * s;
       const long long waves = (ctas + num_sms - 1) / num_sms;
       const int blocks = (total_blocks + s - 1) / s;
-      const double cost = static_cast<double>(waves) * (blocks * per_block + kFixed) + (s > 1 ? kMergeCost : 0.0);
+      const double cost = static_cast<double>(waves) * (blocks * per_block + fixed(qt, waves == 1)) + (s > 1 ? kMergeCost : 0.0);
       if (cost < best - 1e-9) {
         best = cost;
         best_qt = qt;
@@ -1133,7 +1146,7 @@ void choose_attention_config(int n_q_tiles, int heads_x_batch, int total_blocks,
       }
     }
     // s - 1 long ranges and a short one, the short CTAs last: try a few lengths of the short range per s
-    if (split_len == nullptr || items * 2 > 4096) continue;
+    if (!paged || total_blocks > kUnevenMaxBlocks || items * 2 > 4096) continue;
     for (int s = 2; s <= smax; ++s) {
       const int even = (total_blocks + s - 1) / s;
       for (int step = 1; step <= 12; ++step) {
@@ -1143,17 +1156,20 @@ void choose_attention_config(int n_q_tiles, int heads_x_batch, int total_blocks,
         const int real_rest = total_blocks - (s - 1) * len;
         if (len < 1 || real_rest < 1 || real_rest > len) continue;
         const double cost = list_schedule(static_cast<int>(items * (s - 1)), len * per_block, static_cast<int>(items),
-                                          real_rest * per_block, num_sms, kFixed) + kMergeCost;
-        // only for a clear gain over the best plan so far: a long back-to-back run at the board's power limit gains
-        // nothing from filling idle SMs (measured 0.6 % slower at 1057 blocks, where the model promises 2.5 %)
-        if (cost < best * 0.96) {
-          best = cost;
-          best_qt = qt;
-          best_s = s;
-          best_len = len;
+                                          real_rest * per_block, num_sms, fixed(qt, items * (s - 1) <= num_sms)) + kMergeCost;
+        if (cost < uneven) {
+          uneven = cost;
+          uneven_qt = qt;
+          uneven_s = s;
+          uneven_len = len;
         }
       }
     }
+  }
+  if (uneven < best * 0.96) {                  // only for a clear gain over the best equal ranges
+    best_qt = uneven_qt;
+    best_s = uneven_s;
+    best_len = uneven_len;
   }
   *q_tiles_per_cta = best_qt;
   *splits = best_s;
