@@ -139,6 +139,20 @@ def test_compute_needs_device():
         P.ops.dense_attention(*(torch.zeros(1, 4, 1, 64, dtype=torch.bfloat16) for _ in range(3)))
 
 
+@pytest.mark.parametrize("n_q,heads,blocks", [(1005, 16, 81), (783, 16, 92), (1005, 16, 250), (1005, 16, 600), (894, 16, 527)])
+def test_launch_shape_fills_one_wave_below_a_thousand_blocks(n_q, heads, blocks):
+    """64 (head, tile pair) items: two long ranges in one wave and a short one on the SMs they leave free, which ends no later
+    than the long ones by more than the plan's fixed cost; one equal cut more would start further waves."""
+    import ctypes as C
+    qt, s, ln = C.c_int(), C.c_int(), C.c_int()
+    _lib.check(_lib.load().gct_attn_launch_shape(n_q, heads, blocks, 148, 16, C.byref(qt), C.byref(s), C.byref(ln)))
+    items = heads * -(-n_q // 256)
+    assert (qt.value, s.value) == (2, 3) and items * 2 <= 148
+    rest = blocks - 2 * ln.value
+    rounds = -(-items // (148 - 2 * items))
+    assert 1 <= rest <= ln.value and rounds * (rest + 5) <= ln.value + 5 + (rest + 5)
+
+
 def test_launch_shape_covers_the_kv_blocks():
     """Host arithmetic of the paged attention launch: every plan covers the KV blocks exactly once with non-empty
     ranges; equal ranges at the benchmark's size, long ranges plus a short one where equal ranges would leave SMs idle
