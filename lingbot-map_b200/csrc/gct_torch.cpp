@@ -479,8 +479,9 @@ Tensor linear(const Tensor& rows, const Tensor& w, const Tensor& b) {
   return b.defined() ? at::addmm(b, rows, w.t()) : at::mm(rows, w.t());
 }
 
-// Norm of the rows of x as bf16; with y, of the sum x + gamma * y, which is returned in *sum.
+// Norm of the rows of x as bf16; with y, of the sum x + gamma * y, which is returned in *sum.  The kernel takes dense rows.
 Tensor residual_norm(const Tensor& x, const Tensor* y, const Tensor* gamma, Tensor* sum, const Tensor* w, const Tensor* b, double eps) {
+  if (!x.is_contiguous() || (y != nullptr && (!y->is_contiguous() || y->sizes() != x.sizes()))) runtime_error("residual norm: rows must be contiguous");
   gct::RowLaunch p;
   p.rows = x.size(0);
   p.cols = static_cast<int>(x.size(1));
@@ -616,7 +617,8 @@ PyObject* py_block_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
       const Tensor* cs = table.defined() ? &table : nullptr;
       const int64_t rope = table.defined() ? mode : GCT_ROPE_NONE;
       Tensor x = px->reshape({B * N, C});
-      if (!aligned16(x)) x = x.clone();
+      // reshape hands back a view wherever strides allow (a column slice, every other token, a transposed or expanded input)
+      if (!x.is_contiguous() || !aligned16(x)) x = x.clone(at::MemoryFormat::Contiguous);
       const Tensor normed = residual_norm(x, nullptr, nullptr, nullptr, n1w, n1b, eps1);
       const Tensor qkv = linear(normed, qkv_w, qkv_b);
       const int blk = static_cast<int>(block);

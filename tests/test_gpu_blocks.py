@@ -300,3 +300,48 @@ def test_layers_take_what_the_modules_take(what):
         assert pos.is_conj()
     for got, ref in zip(run(x, pos), want):
         assert float((got.float() - ref.float()).abs().max()) <= 2 * 2 ** -7 * float(ref.float().abs().max())
+
+
+def _strided(t, form):
+    """The values of t [B, N, C] in memory of another layout."""
+    B, N, C = t.shape
+    if form == "columns":                       # a slice of wider rows
+        return torch.cat([t, t.flip(-1)], dim=-1)[..., :C]
+    if form == "every other token":
+        return torch.stack([t, t.flip(-1)], dim=2).reshape(B, 2 * N, C)[:, ::2]
+    if form == "transposed":                    # what flatten(2).transpose(1, 2) of a feature map gives
+        return t.transpose(1, 2).contiguous().transpose(1, 2)
+    if form == "transposed, off alignment":
+        return _off_alignment(t.transpose(1, 2).contiguous()).transpose(1, 2)
+    if form == "batches apart":
+        return torch.cat([t, t.flip(-1)], dim=1)[:, :N]
+    return t[:, :1].expand(B, N, C)             # one row for every token
+
+
+@pytest.mark.parametrize("form", ["columns", "every other token", "transposed", "transposed, off alignment", "batches apart", "expanded"])
+@pytest.mark.parametrize("how", ["batch of 1", "batch of 2", "scale pass", "streamed", "non-keyframe"])
+@pytest.mark.parametrize("x_dtype", ["bf16", "f32"])
+def test_block_takes_inputs_of_any_strides(form, how, x_dtype):
+    """Output and cache pages of a strided input equal those of its contiguous copy, bit for bit: both run the same kernels on
+    the same rows."""
+    blk, fa = _layer_pair()
+    pph, ppw, ns, scale = 3, 5, 6, 2
+    T, frames = ns + pph * ppw, scale if how == "scale pass" else 1
+    x = torch.from_numpy(seeded.randn(13, 2 if how == "batch of 2" else 1, frames * T, 128)).to(DEV).to({"bf16": torch.bfloat16, "f32": torch.float32}[x_dtype])
+    x = _strided(x, form)
+    kw = dict(num_patches=T - ns, num_special=ns, enable_3d_rope=True, num_frames=frames, global_idx=0, pos=rope3d_pos(0, frames, pph, ppw, ns))
+
+    def run(x):
+        mgr = None
+        if not how.startswith("batch"):
+            mgr = P.B200KVCacheManager(1, scale + 2 + 16, T, 2, 64, device=DEV, scale_frames=scale, sliding_window=2, max_total_frames=40)
+            mgr._skip_append = how == "non-keyframe"
+        with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+            y = blk(x, kv_cache=mgr, **kw)
+            return [y, fa(x, pos=kw["pos"], enable_3d_rope=True)] + ([] if mgr is None else [mgr.kv_caches[0].clone()])
+
+    got, want = run(x), run(x.clone(memory_format=torch.contiguous_format))
+    assert torch.equal(got[0], want[0]) and all(torch.equal(a, b) for a, b in zip(got[2:], want[2:]))
+    # the frame layer's first matrix product reads x with its strides: its sums may run in another order (one bf16 rounding
+    # step of an intermediate, as everywhere in this file two steps of the largest output)
+    assert float((got[1].float() - want[1].float()).abs().max()) <= 2 * 2 ** -7 * float(want[1].float().abs().max())
