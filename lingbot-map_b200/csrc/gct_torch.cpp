@@ -104,6 +104,10 @@ gct_mgr_t* manager(PyObject* o) { return reinterpret_cast<gct_mgr_t*>(static_cas
 void need_cuda(const Tensor& t, const char* name) {
   if (!t.is_cuda()) runtime_error(std::string(name) + " must be a CUDA tensor: the B200 backend has no CPU path");
 }
+void need_beside(const Tensor& t, const char* name, const Tensor& rows) {
+  need_cuda(t, name);
+  if (t.device() != rows.device()) value_error(std::string(name) + " lives on " + t.device().str() + ", the rows on " + rows.device().str());
+}
 int dtype_code(const Tensor& t) {
   if (t.scalar_type() == at::kFloat) return GCT_F32;
   if (t.scalar_type() == at::kBFloat16) return GCT_BF16;
@@ -147,13 +151,14 @@ struct Norm {
 // converted (a norm parameter that is neither fp32 nor bf16, or not of the dtype of the others) until the launch is queued.
 struct NormRope {
   Tensor keep[5];
-  void fill(gct::PrepLaunch* p, const Norm& norm, const Tensor* c, int64_t mode) {
+  // Everything has to lie on the device of the rows: the kernel gets addresses.
+  void fill(gct::PrepLaunch* p, const Norm& norm, const Tensor* c, int64_t mode, const Tensor& rows) {
     const Tensor* const* t = norm.t;
     static const char* names[4] = {"q_norm_w", "q_norm_b", "k_norm_w", "k_norm_b"};
     bool all_bf16 = true;
     for (int i = 0; i < 4; ++i) {
       if (t[i] != nullptr) {
-        need_cuda(*t[i], names[i]);
+        need_beside(*t[i], names[i], rows);
         if (t[i]->numel() != kHeadDim) value_error(std::string(names[i]) + " must have 64 elements");
         all_bf16 &= t[i]->scalar_type() == at::kBFloat16;
       }
@@ -182,7 +187,7 @@ struct NormRope {
     p->norm_dtype = all_bf16 ? GCT_BF16 : GCT_F32;
     p->rope_mode = static_cast<int>(mode);
     if (c == nullptr || mode == GCT_ROPE_NONE) return;
-    need_cuda(*c, "rope_cs");
+    need_beside(*c, "rope_cs", rows);
     const bool is_complex = c->scalar_type() == at::kComplexFloat || c->scalar_type() == at::kComplexDouble;
     if (c->numel() < static_cast<int64_t>(p->tokens_per_frame) * (is_complex ? 32 : 64)) value_error("rope_cs holds too few rows");
     Tensor table = c->is_conj() ? c->resolve_conj() : *c;
@@ -226,7 +231,7 @@ Qkv prep(Tensor qkv, int64_t heads, int64_t tokens_per_frame, const Norm& norm, 
   p.tokens_per_frame = static_cast<int>(tokens_per_frame);
   p.heads = static_cast<int>(heads);
   NormRope nr;
-  nr.fill(&p, norm, cs, mode);
+  nr.fill(&p, norm, cs, mode, qkv);
   Qkv r{empty({qkv.size(0), heads, kHeadDim}, at::kBFloat16, qkv), empty({qkv.size(0), heads, kHeadDim}, at::kBFloat16, qkv),
         empty({qkv.size(0), heads, kHeadDim}, at::kBFloat16, qkv)};
   p.q_out = const_cast<__nv_bfloat16*>(bf16(r.q));
@@ -260,7 +265,7 @@ Tensor dense(const Tensor& q, const Tensor& k, const Tensor& v, Tensor out) {
   const Tensor* t[3] = {&q, &k, &v};
   static const char* names[3] = {"q", "k", "v"};
   for (int i = 0; i < 3; ++i) {
-    need_cuda(*t[i], names[i]);
+    need_beside(*t[i], names[i], q);
     if (t[i]->scalar_type() != at::kBFloat16 || t[i]->dim() != 4 || t[i]->size(3) != kHeadDim || t[i]->stride(3) != 1)
       value_error(std::string(names[i]) + " must be bf16 [B, N, H, 64] with contiguous head_dim");
   }
@@ -345,7 +350,7 @@ Tensor append_fused(gct_mgr_t* m, int64_t device, int64_t block, Tensor qkv, con
   fill_qkv(&p, qkv, H);
   p.tokens_per_frame = static_cast<int>(T);
   NormRope nr;
-  nr.fill(&p, norm, cs, mode);
+  nr.fill(&p, norm, cs, mode, qkv);
   if (!q_out.defined()) q_out = empty({T, H, kHeadDim}, at::kBFloat16, qkv);
   p.q_out = static_cast<__nv_bfloat16*>(q_out.data_ptr());
   check(gct::mgr_append(m, static_cast<int>(block), p, stream_of(qkv)));
@@ -449,9 +454,11 @@ const Tensor* stock(PyObject* o) {
 bool aligned16(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
 
 // bf16 is what the Linear layers compute in: under autocast whatever the parameters are, else only if all of it is bf16.
+// A parameter on another device than x is the modules' to refuse.
 struct Precision {
   bool autocast;
-  Precision(const Tensor& x) {
+  c10::Device device;
+  Precision(const Tensor& x) : device(x.device()) {
     autocast = at::autocast::is_autocast_enabled(at::kCUDA);
     const bool known = x.scalar_type() == at::kFloat || x.scalar_type() == at::kBFloat16;
     if (!known || (autocast ? at::autocast::get_autocast_dtype(at::kCUDA) != at::kBFloat16 : x.scalar_type() != at::kBFloat16)) throw NotStock{};
@@ -460,7 +467,7 @@ struct Precision {
   Tensor linear(PyObject* o) const {
     const Tensor* t = stock(o);
     if (t == nullptr) return Tensor();
-    if (!t->is_cuda()) throw NotStock{};
+    if (t->device() != device) throw NotStock{};
     if (t->scalar_type() == at::kBFloat16) return *t;
     if (!autocast || t->scalar_type() != at::kFloat) throw NotStock{};
     return at::autocast::cached_cast(at::kBFloat16, *t, c10::kCUDA);
@@ -470,7 +477,7 @@ struct Precision {
     const Tensor* t = stock(o);
     if (t == nullptr) return nullptr;
     const bool bf = t->scalar_type() == at::kBFloat16;
-    if (!t->is_cuda() || t->numel() != n || !t->is_contiguous() || !(bf || (autocast && t->scalar_type() == at::kFloat)) || !aligned16(*t)) throw NotStock{};
+    if (t->device() != device || t->numel() != n || !t->is_contiguous() || !(bf || (autocast && t->scalar_type() == at::kFloat)) || !aligned16(*t)) throw NotStock{};
     return t;
   }
 };
@@ -511,10 +518,10 @@ Tensor residual_norm(const Tensor& x, const Tensor* y, const Tensor* gamma, Tens
   return out;
 }
 
-// Rotation table for `tokens` tokens from what the modules pass as positions.
-Tensor rotation(const Tensor* p, int64_t mode, double base, int64_t tokens) {
+// Rotation table for the `tokens` tokens of x from what the modules pass as positions.
+Tensor rotation(const Tensor* p, int64_t mode, double base, int64_t tokens, const Tensor& x) {
   if (mode == GCT_ROPE_NONE || p == nullptr) return Tensor();
-  if (!p->is_cuda()) throw NotStock{};
+  if (p->device() != x.device()) throw NotStock{};
   if (mode == GCT_ROPE_3D) {
     if (!p->is_complex() || p->numel() != tokens * 32) throw NotStock{};
     return *p;
@@ -556,7 +563,7 @@ PyObject* py_frame_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
       c10::cuda::CUDAGuard guard(px->device());
       at::AutoDispatchBelowADInplaceOrView below;
       c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::DispatchKey::AutocastCUDA);
-      const Tensor cs = rotation(pos, mode, base, N);
+      const Tensor cs = rotation(pos, mode, base, N, *px);
       Tensor rows = px->reshape({B * N, C});
       if (rows.scalar_type() != at::kBFloat16) rows = rows.to(at::kBFloat16);
       Qkv r = prep(linear(rows, qkv_w, qkv_b), heads, N, norm, cs.defined() ? &cs : nullptr, cs.defined() ? mode : GCT_ROPE_NONE);
@@ -613,7 +620,7 @@ PyObject* py_block_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
       c10::cuda::CUDAGuard guard(px->device());
       at::AutoDispatchBelowADInplaceOrView below;
       c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::DispatchKey::AutocastCUDA);
-      const Tensor table = rotation(pos, mode, base, N);
+      const Tensor table = rotation(pos, mode, base, N, *px);
       const Tensor* cs = table.defined() ? &table : nullptr;
       const int64_t rope = table.defined() ? mode : GCT_ROPE_NONE;
       Tensor x = px->reshape({B * N, C});
@@ -760,6 +767,7 @@ PyObject* py_voxelize_frame(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int64_t count = in_xyz.size(0);
     if (count < 1 || count > gct::kVoxelMaxPoints) Py_RETURN_NONE;
     const Tensor xyz = float_rows(in_xyz, "pts_xyz"), rgb = float_rows(in_rgb, "pts_rgb");
+    need_beside(rgb, "pts_rgb", xyz);
     if (xyz.numel() < 3 * count || rgb.numel() < 3 * count) value_error("pts_xyz and pts_rgb must be [N, 3]");
     const float voxel = static_cast<float>(real(a[2]));
     c10::cuda::CUDAGuard guard(xyz.device());

@@ -345,3 +345,46 @@ def test_block_takes_inputs_of_any_strides(form, how, x_dtype):
     # the frame layer's first matrix product reads x with its strides: its sums may run in another order (one bf16 rounding
     # step of an intermediate, as everywhere in this file two steps of the largest output)
     assert float((got[1].float() - want[1].float()).abs().max()) <= 2 * 2 ** -7 * float(want[1].float().abs().max())
+
+
+@pytest.mark.parametrize("where", ["norm1.weight", "norm1.bias", "attn.qkv.weight", "attn.qkv.bias", "attn.q_norm.weight", "attn.k_norm.bias", "attn.proj.weight",
+                                   "ls1.gamma", "norm2.weight", "norm2.bias", "mlp.fc1.weight", "mlp.fc2.bias", "ls2.gamma", "positions"])
+@pytest.mark.parametrize("three_d", [True, False])
+def test_layers_refuse_what_lies_on_another_device(monkeypatch, where, three_d):
+    """A parameter or positions on another device than the input: nothing is launched with its address, the native call hands
+    over to the modules (NotImplemented) and these raise.  The host stands for any other device: the rule compares devices."""
+    from lingbot_map_b200 import block as block_mod
+    blk, fa = _layer_pair()
+    pph, ppw, ns = 3, 5, 6
+    T = ns + pph * ppw
+    x = torch.from_numpy(seeded.randn(11, 1, T, 128)).to(DEV).bfloat16()
+    pos = rope3d_pos(3, 1, pph, ppw, ns) if three_d else torch.ones(1, T, 2, dtype=torch.int64, device=DEV)
+    answers, real = [], block_mod._native
+
+    class Watching:
+        def __getattr__(self, name):
+            def call(*a):
+                r = getattr(real, name)(*a)
+                answers.append((name, r is NotImplemented))
+                return r
+            return call
+
+    monkeypatch.setattr(block_mod, "_native", Watching())
+    if where == "positions":
+        pos = pos.cpu()
+    else:
+        path, name = where.rsplit(".", 1)
+        p = getattr(blk.get_submodule(path), name)
+        p.data = p.data.cpu()
+        if where.startswith("attn."):
+            p = getattr(fa.get_submodule(path[5:]), name)
+            p.data = p.data.cpu()
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        with pytest.raises((RuntimeError, ValueError)):
+            blk(x, pos=pos, enable_3d_rope=three_d)
+        assert answers == [("block_layer", True)]
+        if where.startswith("attn.") or where == "positions":
+            with pytest.raises((RuntimeError, ValueError)):
+                fa(x, pos=pos, enable_3d_rope=three_d)
+            assert answers[1:] == [("frame_layer", True)]
+    torch.cuda.synchronize()
