@@ -40,7 +40,8 @@ __device__ bool cull_exact(float x, float y, float z, const CullArgs& a) {
   return u >= 0 && u < a.W && v >= 0 && v < a.H;
 }
 
-// Most points without a division.  The image is the open interval (-1, size) per axis (truncation maps (-1, 0] to pixel 0);
+// Most points without a division.  An image of size >= 1 is the open interval (-1, size) per axis (truncation maps (-1, 0] to pixel 0;
+// an empty one has no such interval, and the host sets the limits so that every point is out);
 // with the coordinate taken from its middle, |px / pz * f + (c - mid)| against half its width decides.  The product with an
 // approximate reciprocal is off by less than 2^-20 relative, which near a border is less than 2^-20 (|c| + size + 1);
 // in_ and out_ keep ten times that away from the border.  In between, and for anything not finite, `undecided` is set.
@@ -493,6 +494,7 @@ int frustum_cull(const float* pts, int64_t n, const float* R, const float* t, co
     *mid = c - middle;
     *in = half - margin;
     *out = half + margin;
+    if (size <= 0) *in = *out = -1.f;                      // no pixel: out wherever the projection is a number
   };
   axis(cx, width, &a.mid_u, &a.in_u, &a.out_u);
   axis(cy, height, &a.mid_v, &a.in_v, &a.out_v);

@@ -109,3 +109,19 @@ def test_frustum_cull_on_image_borders(depths, camera_on):
         want = R.frustum_cull(pts, perm, t, *args)
     assert np.array_equal(got, want)
     assert 0.02 < want.mean() < 0.98
+
+
+@pytest.mark.parametrize("W,H", [(0, 378), (518, 0), (0, 0), (-3, 378), (1, 1)])
+def test_frustum_cull_of_an_empty_image(W, H):
+    """An image without pixels sees nothing, also of the points that project into (-1, 0), which truncation maps to pixel 0; one
+    pixel sees those."""
+    rs = np.random.RandomState(5)
+    n = 4003
+    z = rs.uniform(0.5, 5.0, n).astype(np.float32)
+    uv = rs.uniform(-2.0, 2.0, (2, n)).astype(np.float32)
+    pts = np.ascontiguousarray(np.stack([uv[0] * z / 300, uv[1] * z / 310, z], axis=1).astype(np.float32))
+    eye, zero = np.eye(3, dtype=np.float32), np.zeros(3, np.float32)
+    args = (300.0, 310.0, 0.0, 0.0, W, H, 0.1, 10.0)
+    got = RO.frustum_cull(torch.from_numpy(pts).to(DEV), torch.from_numpy(eye), torch.from_numpy(zero), *args).cpu().numpy()
+    assert np.array_equal(got, R.frustum_cull(pts, eye, zero, *args))
+    assert got.any() == (W > 0 and H > 0)
