@@ -741,7 +741,8 @@ PyObject* py_frustum_cull(PyObject*, PyObject* const* a, Py_ssize_t n) {
     };
     R = place(R);
     t = place(t);
-    if (R.dim() != 2) R = R.reshape({3, 3});
+    // the kernel steps through R by row and column strides: nine values of any other shape ([1, 9], a flat [9]) are taken in order
+    if (R.sizes() != at::IntArrayRef({3, 3})) R = R.reshape({3, 3});
     if (t.dim() != 1) t = t.reshape({3});
     // their owner may free them on another stream as soon as this returns, as it could when the call waited for a copy
     for (const Tensor* c : {&R, &t})

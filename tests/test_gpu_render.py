@@ -125,3 +125,21 @@ def test_frustum_cull_of_an_empty_image(W, H):
     got = RO.frustum_cull(torch.from_numpy(pts).to(DEV), torch.from_numpy(eye), torch.from_numpy(zero), *args).cpu().numpy()
     assert np.array_equal(got, R.frustum_cull(pts, eye, zero, *args))
     assert got.any() == (W > 0 and H > 0)
+
+
+@pytest.mark.parametrize("camera_on", ["cpu", "cuda:0"])
+@pytest.mark.parametrize("r_shape", [(3, 3), (9,), (1, 9), (9, 1), (1, 3, 3), (3, 3, 1), (3, 1, 3)])
+@pytest.mark.parametrize("t_shape", [(3,), (1, 3), (3, 1)])
+def test_frustum_cull_takes_a_camera_of_any_shape(camera_on, r_shape, t_shape):
+    """Nine and three values in any shape, on the host or on the device, also as every other value of a buffer."""
+    rs = np.random.RandomState(8)
+    n, args = 5003, (300.0, 310.0, 259.0, 189.0, 518, 378, 0.1, 6.0)
+    pts = (3 * rs.standard_normal((n, 3))).astype(np.float32)
+    q, _ = np.linalg.qr(rs.standard_normal((3, 3)))
+    Rm, t = q.astype(np.float32), (0.5 * rs.standard_normal(3)).astype(np.float32)
+    want = R.frustum_cull(pts, Rm, t, *args)
+    dense = torch.from_numpy(Rm).to(camera_on).reshape(r_shape)
+    apart = torch.stack([dense, 7 + dense], dim=-1)[..., 0]
+    for r in (dense, apart):
+        got = RO.frustum_cull(torch.from_numpy(pts).to(DEV), r, torch.from_numpy(t).to(camera_on).reshape(t_shape), *args).cpu().numpy()
+        assert np.array_equal(got, want)
