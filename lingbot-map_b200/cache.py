@@ -288,7 +288,9 @@ class B200KVCacheManager:
         q [q_len, H, D] (float32 or bfloat16) -> out [q_len, H, D] bfloat16.  Like the reference, the page
         table is planned when block_idx == 0 and reused by the other blocks of the same frame."""
         self._require_device()
-        out = self._native.attention(self._h, self._dev_index, block_idx, q, return_lse)
+        # a plan() of a subclass, or put in its place (to attend over a page range, to time it), is the one that is called
+        stock = type(self).plan is _STOCK_PLAN and "plan" not in self.__dict__
+        out = self._native.attention(self._h, self._dev_index, block_idx, q, return_lse, None if stock else self.plan)
         return torch.zeros_like(q) if out is None else out          # nothing cached yet: :368-370
 
     def compute_attention_partial(self, block_idx: int, q: Tensor, out: Optional[Tensor] = None,
@@ -335,3 +337,6 @@ class B200KVCacheManager:
         n = C.c_int64()
         self._check(self._lib.gct_mgr_launch_count(self._handle, C.byref(n)))
         return n.value
+
+
+_STOCK_PLAN = B200KVCacheManager.plan

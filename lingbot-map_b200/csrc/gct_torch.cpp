@@ -372,13 +372,13 @@ PyObject* py_append_fused(PyObject*, PyObject* const* a, Py_ssize_t n) {
 struct Attended {
   Tensor out, lse;
 };
-// The page table is planned at block 0 and reused by the other blocks of the frame.
-Attended attend(gct_mgr_t* m, int64_t device, int64_t block, const Tensor& q_in, bool want_lse) {
+// The page table is planned at block 0 and reused by the other blocks of the frame; `planned`: the caller has done it.
+Attended attend(gct_mgr_t* m, int64_t device, int64_t block, const Tensor& q_in, bool want_lse, bool planned = false) {
   const gct_mgr_config_t& cfg = gct::mgr_config(m);
   const Tensor q = frame_rows(q_in, "q", cfg, device);
   c10::cuda::CUDAGuard guard(q.device());
   cudaStream_t s = stream_of(q);
-  if (block == 0) check(gct_mgr_plan(m, 0, -1, s));
+  if (block == 0 && !planned) check(gct_mgr_plan(m, 0, -1, s));
   Attended r;
   r.out = empty(q.sizes(), at::kBFloat16, q);
   if (want_lse) r.lse = empty({q.size(0), q.size(1)}, at::kFloat, q);
@@ -387,10 +387,11 @@ Attended attend(gct_mgr_t* m, int64_t device, int64_t block, const Tensor& q_in,
   return r;
 }
 
-// attention(manager, device, block, q, want_lse) -> out | (out, lse) | None (nothing cached yet)
+// attention(manager, device, block, q, want_lse, plan | None) -> out | (out, lse) | None (nothing cached yet)
+// plan: called at block 0 in place of the plan over all visible pages.
 PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
-    need(n, 5, "attention");
+    need(n, 6, "attention");
     gct_mgr_t* m = manager(a[0]);
     int64_t stats[6];
     check(gct_mgr_stats(m, static_cast<int>(integer(a[2])), stats));
@@ -398,7 +399,14 @@ PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const bool want_lse = PyObject_IsTrue(a[4]) == 1;
     const Tensor& q = tensor(a[3], "q");
     const int64_t device = integer(a[1]), block = integer(a[2]);
-    Attended r = unlocked([&] { return attend(m, device, block, q, want_lse); });
+    const bool planned = a[5] != Py_None;
+    if (planned && block == 0) {
+      frame_rows(q, "q", gct::mgr_config(m), device);      // a tensor that is refused is refused before the plan changes
+      PyObject* done = PyObject_CallNoArgs(a[5]);
+      if (done == nullptr) throw python_error();
+      Py_DECREF(done);
+    }
+    Attended r = unlocked([&] { return attend(m, device, block, q, want_lse, planned); });
     if (!want_lse) return wrap(std::move(r.out));
     PyObject* out = PyTuple_New(2);
     if (out == nullptr) throw python_error();

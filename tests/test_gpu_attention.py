@@ -298,6 +298,44 @@ def test_merge_of_any_number_of_partials(groups, shift):
     assert float((lse_out.double() - torch.logsumexp(lse.double(), 0)).abs().max()) <= 1e-5
 
 
+@pytest.mark.parametrize("how", ["subclass", "instance", "class"])
+def test_a_replaced_plan_is_the_one_that_is_called(monkeypatch, how):
+    """compute_attention plans at block 0 through the manager's own plan(): one that attends to a page range only gives the
+    result of that range (bf16 rounding of the fp32 partial result: 2^-8 of the value), at block 0 and at the block after it."""
+    calls = []
+
+    def pages(self, *a):
+        calls.append(a)
+        stock(self, 0, 2)
+
+    stock = P.B200KVCacheManager.plan
+
+    class Ranged(P.B200KVCacheManager):
+        plan = pages
+
+    tpf, H = 262, 2
+    m = (Ranged if how == "subclass" else P.B200KVCacheManager)(2, 16, tpf, H, 64, device=DEV, scale_frames=2, sliding_window=4, max_total_frames=40)
+    for t in range(4):
+        for b in range(2):
+            m.append_frame(b, bf(seeded.randn(1000 + 10 * t + b, tpf, H, 64)), bf(seeded.randn(2000 + 10 * t + b, tpf, H, 64)))
+    q = bf(seeded.randn(3, tpf, H, 64))
+    full = m.compute_attention(0, q)
+    if how == "instance":
+        m.plan = lambda *a: pages(m, *a)
+    elif how == "class":
+        monkeypatch.setattr(P.B200KVCacheManager, "plan", pages)
+    calls.clear()
+    got = [m.compute_attention(b, q) for b in range(2)]
+    assert calls == [()]
+    for b in range(2):
+        want, _ = m.compute_attention_partial(b, q)
+        assert bool(((got[b].float() - want).abs() <= 2 ** -8 * want.abs() + 1e-5).all())
+    assert how == "subclass" or float((got[0].float() - full.float()).abs().max()) > 0.05
+    with pytest.raises(ValueError):                 # refused before the plan changes
+        m.compute_attention(0, q[:, :1])
+    assert calls == [()]
+
+
 # ---------------------------------------------------------------- production geometry
 def test_full_geometry_properties():
     """378x518 geometry: 1005 tokens/frame, 16 heads, page 999, scale 8 + window 64, 80 keyframes.
