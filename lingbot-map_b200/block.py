@@ -16,6 +16,7 @@ from typing import Callable, Optional
 import torch
 from torch import Tensor, nn
 from torch.nn.modules import module as _nn_module
+from torch.utils._device import DeviceContext
 
 from . import _lib, ops
 from .cache import B200KVCacheManager
@@ -43,11 +44,19 @@ def _stock_dropout(m: nn.Module) -> bool:
     return (_stock(m, nn.Identity) or _stock(m, nn.Dropout)) and (type(m) is nn.Identity or m.p == 0.0 or not m.training)
 
 
+def _watched() -> bool:
+    """A function or dispatch mode is active: it is to see every operation of the modules (a counter, a tracer, a rewriter).
+    The mode behind torch.set_default_device only places new tensors."""
+    C = torch._C
+    return (C._len_torch_dispatch_stack() > 0
+            or any(type(C._get_function_stack_at(i)) is not DeviceContext for i in range(C._len_torch_function_stack())))
+
+
 def _may_fuse() -> bool:
     """Whole layers run as one native call in eager inference only: under torch.compile the modules are traced, with
-    gradients enabled the Linear layers record them, and global hooks and torch.jit.trace want to see every module."""
+    gradients enabled the Linear layers record them, and global hooks, modes and torch.jit.trace want to see every module."""
     return not (torch.is_grad_enabled() or torch.compiler.is_compiling() or _nn_module._global_forward_hooks
-                or _nn_module._global_forward_pre_hooks or torch._C._get_tracing_state() is not None)
+                or _nn_module._global_forward_pre_hooks or torch._C._get_tracing_state() is not None or _watched())
 
 
 def _reference_classes():

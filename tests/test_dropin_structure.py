@@ -231,3 +231,32 @@ def test_clock_sampler_reports_samples_of_the_timed_region_only():
     got = s.stop()
     assert got["sm_mhz"] == 1900.0 and got["sm_max_mhz"] == 1965.0 and got["reasons"] == ["sw_power_cap"], got
     assert got["samples"] >= 3
+
+
+def _modes():
+    from torch._subclasses import FakeTensorMode
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Function(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    class Dispatch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    return {"function": Function, "dispatch": Dispatch, "fake": FakeTensorMode, "function under a device": Function, "device": lambda: torch.device("cpu")}
+
+
+@pytest.mark.parametrize("name", ["function", "dispatch", "fake", "function under a device", "device"])
+def test_layers_run_as_modules_under_a_mode(name):
+    """A function or dispatch mode is to see the operations of the modules, so no layer runs as one native call under it; the
+    mode behind torch.device / set_default_device, which only places new tensors, changes nothing."""
+    from contextlib import nullcontext
+    from lingbot_map_b200 import block
+    with torch.no_grad():
+        assert block._may_fuse()
+        with torch.device("cpu") if name == "function under a device" else nullcontext(), _modes()[name]():
+            assert block._may_fuse() == (name == "device")
+        assert block._may_fuse()

@@ -388,3 +388,29 @@ def test_layers_refuse_what_lies_on_another_device(monkeypatch, where, three_d):
                 fa(x, pos=pos, enable_3d_rope=three_d)
             assert answers[1:] == [("frame_layer", True)]
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("kind", ["function", "dispatch"])
+def test_a_mode_sees_the_operations_of_the_modules(kind):
+    """The four Linear layers and two norms of a block, and the two Linear layers of a frame layer, under a mode that records them."""
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+    seen = []
+
+    class Function(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append(getattr(func, "__name__", ""))
+            return func(*args, **(kwargs or {}))
+
+    class Dispatch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append({"addmm": "linear", "native_layer_norm": "layer_norm"}.get(func.overloadpacket.__name__, ""))
+            return func(*args, **(kwargs or {}))
+
+    blk, fa = _layer_pair()
+    x = torch.from_numpy(seeded.randn(11, 1, 21, 128)).to(DEV).bfloat16()
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16), (Function if kind == "function" else Dispatch)():
+        blk(x, pos=rope3d_pos(3, 1, 3, 5, 6), enable_3d_rope=True)
+        assert (seen.count("linear"), seen.count("layer_norm")) == (4, 2)
+        fa(x, pos=rope3d_pos(3, 1, 3, 5, 6), enable_3d_rope=True)
+        assert seen.count("linear") == 6
