@@ -11,9 +11,11 @@ call signatures:
 The Linear layers, LayerNorm(dim), LayerScale and the MLP stay PyTorch; q/k LayerNorm(64), RoPE, the bf16 cast,
 the K/V page append and all attention math run in the CUDA library.  Inference only (no dropout, no autograd).
 """
+from operator import attrgetter
 from typing import Callable, Optional
 
 import torch
+import torch.nn.functional as F
 from torch import Tensor, nn
 from torch.nn.modules import module as _nn_module
 from torch.utils._device import DeviceContext
@@ -52,11 +54,24 @@ def _watched() -> bool:
             or any(type(C._get_function_stack_at(i)) is not DeviceContext for i in range(C._len_torch_function_stack())))
 
 
+_layer_steps = attrgetter("_dense", "_qkv_rows", "_norm_params", "_rope_args")
+_manager_steps = attrgetter(*sorted(_MANAGER_STEPS))
+
+
+def _code() -> tuple:
+    """The functions and class methods that a native layer passes by, as they are now."""
+    return (F.linear, F.layer_norm, F.gelu, ops.prep_qkv, ops.dense_attention, rope_table_from_pos, nn.Linear.forward, nn.LayerNorm.forward,
+            nn.GELU.forward, LayerScale.forward, Mlp.forward, B200Block.ffn_residual, B200Attention.forward, B200Attention.stream_frame,
+            B200Attention._evict, *_layer_steps(B200Attention), *_layer_steps(B200FrameAttention), *_manager_steps(B200KVCacheManager))
+
+
 def _may_fuse() -> bool:
     """Whole layers run as one native call in eager inference only: under torch.compile the modules are traced, with
-    gradients enabled the Linear layers record them, and global hooks, modes and torch.jit.trace want to see every module."""
+    gradients enabled the Linear layers record them, global hooks, modes and torch.jit.trace want to see every module, and
+    a function or class method that has been replaced (by a profiler or a test) wants to be called."""
     return not (torch.is_grad_enabled() or torch.compiler.is_compiling() or _nn_module._global_forward_hooks
-                or _nn_module._global_forward_pre_hooks or torch._C._get_tracing_state() is not None or _watched())
+                or _nn_module._global_forward_pre_hooks or torch._C._get_tracing_state() is not None or _watched()
+                or _code() != _STOCK_CODE)
 
 
 def _reference_classes():
@@ -402,3 +417,6 @@ class B200Block(nn.Module):
 
     def ffn_residual(self, x: Tensor) -> Tensor:
         return x + self.ls2(self.mlp(self.norm2(x)))
+
+
+_STOCK_CODE = _code()

@@ -414,3 +414,45 @@ def test_a_mode_sees_the_operations_of_the_modules(kind):
         assert (seen.count("linear"), seen.count("layer_norm")) == (4, 2)
         fa(x, pos=rope3d_pos(3, 1, 3, 5, 6), enable_3d_rope=True)
         assert seen.count("linear") == 6
+
+
+@pytest.mark.parametrize("where", ["F.linear", "F.layer_norm", "F.gelu", "ops.prep_qkv", "ops.dense_attention", "block.LayerScale.forward", "block.Mlp.forward",
+                                   "P.B200Block.ffn_residual", "P.B200Attention.stream_frame", "P.B200Attention.forward", "P.B200Attention._evict",
+                                   "P.B200FrameAttention._dense", "P.B200KVCacheManager.append_frame", "P.B200KVCacheManager.append_frame_fused",
+                                   "P.B200KVCacheManager.evict_frames", "P.B200KVCacheManager.compute_attention", "P.B200KVCacheManager.plan",
+                                   "P.B200KVCacheManager.rollback_last_frame"])
+def test_a_replaced_function_or_method_is_called(monkeypatch, where):
+    """What a profiler or a test puts in the place of a function or class method sees the calls of a frame layer, a batch-mode block, a scale
+    pass, a keyframe and a non-keyframe; outputs as without it (two bf16 rounding steps of the largest, as everywhere here)."""
+    import torch.nn.functional as F
+    from lingbot_map_b200 import block, ops
+    blk, fa = _layer_pair()
+    pph, ppw, ns, scale = 3, 5, 6, 2
+    T = ns + pph * ppw
+    data = lambda i, n: torch.from_numpy(seeded.randn(i, 1, n * T, 128)).to(DEV).bfloat16()
+
+    def run():
+        mgr = P.B200KVCacheManager(1, scale + 2 + 16, T, 2, 64, device=DEV, scale_frames=scale, sliding_window=2, max_total_frames=40)
+        kw = dict(num_patches=T - ns, num_special=ns, enable_3d_rope=True, global_idx=0)
+        with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+            out = [fa(data(1, 1), pos=rope3d_pos(0, 1, pph, ppw, ns), enable_3d_rope=True), blk(data(2, 1), pos=rope3d_pos(0, 1, pph, ppw, ns), **kw),
+                   blk(data(3, scale), pos=rope3d_pos(0, scale, pph, ppw, ns), num_frames=scale, kv_cache=mgr, **kw)]
+            for i in range(2):
+                mgr._skip_append = i == 1
+                out.append(blk(data(4 + i, 1), pos=rope3d_pos(scale + i, 1, pph, ppw, ns), num_frames=1, kv_cache=mgr, **kw))
+        return out
+
+    want = run()
+    owner, name = where.rsplit(".", 1)
+    owner = eval(owner)
+    calls, real = [], getattr(owner, name)
+
+    def counted(*a, **k):
+        calls.append(name)
+        return real(*a, **k)
+
+    monkeypatch.setattr(owner, name, counted)
+    got = run()
+    assert calls
+    for a, b in zip(got, want):
+        assert float((a.float() - b.float()).abs().max()) <= 2 * 2 ** -7 * float(b.float().abs().max())
