@@ -531,10 +531,10 @@ Tensor rotation(const Tensor* p, int64_t mode, double base, int64_t tokens, cons
   if (mode == GCT_ROPE_NONE || p == nullptr) return Tensor();
   if (p->device() != x.device()) throw NotStock{};
   if (mode == GCT_ROPE_3D) {
-    if (!p->is_complex() || p->numel() != tokens * 32) throw NotStock{};
+    if ((p->scalar_type() != at::kComplexFloat && p->scalar_type() != at::kComplexDouble) || p->numel() != tokens * 32) throw NotStock{};
     return *p;
   }
-  if (p->scalar_type() != at::kLong || p->dim() != 3 || p->size(1) != tokens || p->size(2) != 2) throw NotStock{};
+  if (p->scalar_type() != at::kLong || p->dim() != 3 || p->size(0) < 1 || p->size(1) != tokens || p->size(2) != 2) throw NotStock{};
   Tensor cs = empty({tokens, 32, 2}, at::kFloat, *p);
   check(gct::launch_rope2d_positions(p->data_ptr<int64_t>(), p->stride(1), p->stride(2), static_cast<int>(tokens), static_cast<float>(base),
                                      cs.data_ptr<float>(), stream_of(*p)));

@@ -456,3 +456,23 @@ def test_a_replaced_function_or_method_is_called(monkeypatch, where):
     assert calls
     for a, b in zip(got, want):
         assert float((a.float() - b.float()).abs().max()) <= 2 * 2 ** -7 * float(b.float().abs().max())
+
+
+@pytest.mark.parametrize("what", ["complex32", "complex64", "no batch entry"])
+def test_layers_take_positions_as_the_modules_do(what):
+    """Half-precision complex positions are converted (the modules' result, two bf16 rounding steps of the largest output); 2-D positions
+    without a batch entry are an error before anything is launched."""
+    blk, fa = _layer_pair()
+    T = 21
+    x = torch.from_numpy(seeded.randn(11, 1, T, 128)).to(DEV).bfloat16()
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        if what == "no batch entry":
+            none = torch.zeros(0, T, 2, dtype=torch.int64, device=DEV)
+            for layer in (blk, fa):
+                with pytest.raises(IndexError):
+                    layer(x, pos=none)
+            return
+        pos = rope3d_pos(3, 1, 3, 5, 6).to(getattr(torch, what))
+        for layer in (blk, fa):
+            got, want = layer(x, pos=pos, enable_3d_rope=True), layer(x, pos=pos.to(torch.complex128), enable_3d_rope=True)
+            assert float((got.float() - want.float()).abs().max()) <= 2 * 2 ** -7 * float(want.float().abs().max())
