@@ -576,7 +576,7 @@ PyObject* py_frame_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
       if (rows.scalar_type() != at::kBFloat16) rows = rows.to(at::kBFloat16);
       Qkv r = prep(linear(rows, qkv_w, qkv_b), heads, N, norm, cs.defined() ? &cs : nullptr, cs.defined() ? mode : GCT_ROPE_NONE);
       const Tensor o = dense(r.q.view({B, N, heads, kHeadDim}), r.k.view({B, N, heads, kHeadDim}), r.v.view({B, N, heads, kHeadDim}), Tensor());
-      return linear(o.view({B * N, C}), proj_w, proj_b).view({B, N, C});
+      return linear(o.view({B * N, C}), proj_w, proj_b).view({B, N, proj_w.size(0)});
     }));
   });
 }

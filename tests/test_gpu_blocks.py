@@ -476,3 +476,19 @@ def test_layers_take_positions_as_the_modules_do(what):
         for layer in (blk, fa):
             got, want = layer(x, pos=pos, enable_3d_rope=True), layer(x, pos=pos.to(torch.complex128), enable_3d_rope=True)
             assert float((got.float() - want.float()).abs().max()) <= 2 * 2 ** -7 * float(want.float().abs().max())
+
+
+@pytest.mark.parametrize("width", [64, 128, 200])
+def test_frame_layer_with_an_output_projection_of_another_width(monkeypatch, width):
+    """proj may have been replaced by a Linear layer of another output width; as one native call and as modules (two bf16 rounding
+    steps of the largest output)."""
+    from lingbot_map_b200 import block
+    _, fa = _layer_pair()
+    fa.proj = torch.nn.Linear(128, width).to(DEV).bfloat16()
+    x, pos = torch.from_numpy(seeded.randn(11, 2, 21, 128)).to(DEV).bfloat16(), rope3d_pos(3, 1, 3, 5, 6)
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        got = fa(x, pos=pos, enable_3d_rope=True)
+        monkeypatch.setattr(block, "_may_fuse", lambda: False)
+        want = fa(x, pos=pos, enable_3d_rope=True)
+    assert got.shape == want.shape == (2, 21, width) and got.dtype == want.dtype
+    assert float((got.float() - want.float()).abs().max()) <= 2 * 2 ** -7 * float(want.float().abs().max())
