@@ -75,8 +75,8 @@ PyObject* guarded(F&& f) {
     }
   } catch (python_error& e) {
     e.restore();
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
+  } catch (...) {
+    torch::translate_exception_to_python(std::current_exception());      // what PyTorch makes of its own: OutOfMemoryError among them
   }
   return nullptr;
 }

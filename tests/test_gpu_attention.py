@@ -448,6 +448,24 @@ def test_paged_attention_query_lengths(q_len, qdtype):
     assert m.device_status() == 0
 
 
+def test_running_out_of_memory_is_an_out_of_memory_error():
+    """The operators allocate through PyTorch, within the share of the device that the process has been given: beyond it they raise
+    what PyTorch raises, which callers catch to retry with less, and work again afterwards."""
+    q = torch.zeros(1, 40000, 16, 64, dtype=torch.bfloat16, device=DEV)               # 82 MB, as large as the result
+    kv = torch.zeros(1, 130, 16, 64, dtype=torch.bfloat16, device=DEV)
+    P.ops.dense_attention(q[:, :8], kv, kv)                                           # status word
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (24 << 20)) / total)
+    try:
+        with pytest.raises(torch.cuda.OutOfMemoryError):
+            P.ops.dense_attention(q, kv, kv)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert P.ops.dense_attention(q, kv, kv).shape == q.shape
+
+
 def test_argument_errors_are_reported_not_trapped():
     m = P.B200KVCacheManager(1, 21, 26, 2, 64, device=DEV, scale_frames=2, sliding_window=3, max_total_frames=40)
     k = torch.zeros(26, 2, 64, device=DEV)
