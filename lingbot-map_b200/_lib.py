@@ -105,11 +105,14 @@ def load():
 
 def binding():
     """The PyTorch binding (csrc/gct_torch.cpp): the operators as single C calls on tensors.  Raises if it has not been
-    built."""
+    built, or was built for another torch or Python."""
     global _binding
     if _binding is None:
         load()
         import torch        # its libraries must be in the process before the binding is
+        from . import build
+        if not build.binding_matches():
+            raise ImportError(f"{build.BINDING} is missing or was not built for {build._built_for()}: run `python lingbot-map_b200/build.py`")
         from . import _gct_torch
         _gct_torch.set_classes(GctError, torch.nn.Parameter)
         _binding = _gct_torch

@@ -28,8 +28,26 @@ def _older(target, sources):
     return any(os.path.getmtime(os.path.join(HERE, s)) > t for s in sources)
 
 
+def _built_for():
+    import torch
+    return f"torch {torch.__version__}, Python {sys.version_info[0]}.{sys.version_info[1]}"
+
+
+def binding_matches():
+    """The binding in the tree was built for the torch and the Python that run now: it is linked against torch's C++ classes and
+    Python's C API, and holds what it was built for as text."""
+    if not os.path.exists(BINDING):
+        return False
+    with open(BINDING, "rb") as f:
+        return f"binding built for {_built_for()};".encode() in f.read()
+
+
+def _binding_needs_build():
+    return _older(BINDING, [BINDING_SOURCE] + HEADERS) or not binding_matches()
+
+
 def needs_build():
-    return _older(LIB, SOURCES + HEADERS) or _older(BINDING, [BINDING_SOURCE] + HEADERS)
+    return _older(LIB, SOURCES + HEADERS) or _binding_needs_build()
 
 
 def _run(cmd, what):
@@ -46,7 +64,8 @@ def _build_binding():
     from torch.utils import cpp_extension
     includes = cpp_extension.include_paths() + [sysconfig.get_paths()["include"], os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
     torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
-    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           f'-DGCT_BUILT_FOR="{_built_for()}"']
     cmd += [x for i in includes for x in ("-isystem", i)]
     cmd += [BINDING_SOURCE, "-o", BINDING, f"-L{HERE}", "-l:libgct_b200.so", "-Wl,-rpath,$ORIGIN", f"-L{torch_lib}", "-ltorch", "-ltorch_cpu",
             "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda"]
@@ -63,7 +82,7 @@ def build(force=False, verbose=False):
         log = _run(cmd, "nvcc")
         if verbose:
             print(log)
-    if force or _older(BINDING, [BINDING_SOURCE] + HEADERS):
+    if force or _binding_needs_build():
         _build_binding()
     return LIB
 

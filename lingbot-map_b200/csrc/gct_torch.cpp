@@ -25,6 +25,8 @@ namespace {
 using at::Tensor;
 using gct::kHeadDim;
 
+__attribute__((used)) const char kBuiltFor[] = "binding built for " GCT_BUILT_FOR ";";      // looked for by build.py
+
 PyObject* g_error_class = nullptr;      // _lib.GctError(code, message)
 
 // An exception of the given Python type, thrown through C++ frames and set at the boundary.

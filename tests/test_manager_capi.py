@@ -184,3 +184,17 @@ def test_launch_shape_covers_the_kv_blocks():
     assert shape(1005, 16, 136) == shape(1005, 16, 136)           # the cached plan equals the computed one
     with pytest.raises(Exception):
         _lib.check(lib.gct_attn_launch_shape(0, 16, 8, 148, 16, C.byref(C.c_int()), C.byref(C.c_int()), C.byref(C.c_int())))
+
+
+def test_binding_is_rebuilt_for_another_torch_or_python(monkeypatch):
+    """The binding links torch's C++ classes: one that was built for another torch or Python is out of date whatever its time of
+    modification, and is not loaded."""
+    from lingbot_map_b200 import build
+    assert build.binding_matches()
+    here = build._built_for()
+    for other in (here.replace("torch ", "torch 1"), here + "1", here[:-1]):
+        monkeypatch.setattr(build, "_built_for", lambda: other)
+        assert not build.binding_matches() and build.needs_build()
+        monkeypatch.setattr(_lib, "_binding", None)
+        with pytest.raises(ImportError, match="built"):
+            _lib.binding()
