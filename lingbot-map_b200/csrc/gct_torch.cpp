@@ -717,11 +717,12 @@ PyObject* py_rope3d_table(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor& out = tensor(a[4], "out");
     need_cuda(out, "out");
     const int64_t pph = integer(a[1]), ppw = integer(a[2]), ns = integer(a[3]);
-    if (out.scalar_type() != at::kFloat || !out.is_contiguous() || out.numel() < (ns + pph * ppw) * 64)
-      value_error("out must be contiguous float32 [tokens, 32, 2]");
+    // (cos, sin) pairs: as complex64 [tokens, 32] the same bytes
+    const int64_t floats = out.scalar_type() == at::kFloat ? out.numel() : out.scalar_type() == at::kComplexFloat ? 2 * out.numel() : 0;
+    if (!out.is_contiguous() || out.is_conj() || floats < (ns + pph * ppw) * 64) value_error("out must be contiguous float32 [tokens, 32, 2]");
     c10::cuda::CUDAGuard guard(out.device());
     check(gct_rope3d_table(static_cast<int>(integer(a[0])), static_cast<int>(pph), static_cast<int>(ppw), static_cast<int>(ns),
-                           out.data_ptr<float>(), stream_of(out)));
+                           static_cast<float*>(out.data_ptr()), stream_of(out)));
     Py_RETURN_NONE;
   });
 }

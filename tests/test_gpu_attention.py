@@ -448,6 +448,19 @@ def test_paged_attention_query_lengths(q_len, qdtype):
     assert m.device_status() == 0
 
 
+def test_rope3d_table_into_a_callers_buffer():
+    """[tokens, 32, 2] floats or the same bytes as complex numbers, in a buffer that may be longer; another type or layout is refused."""
+    n, args = 6 + 9 * 13, (5, 9, 13, 6, DEV)
+    want = P.ops.rope3d_table(*args)
+    for out in (torch.empty(n + 3, 32, 2, device=DEV), torch.empty(n, 32, dtype=torch.complex64, device=DEV)):
+        assert P.ops.rope3d_table(*args, out=out) is out
+        assert torch.equal((torch.view_as_real(out) if out.is_complex() else out)[:n], want)
+    for out in (torch.empty(n - 1, 32, 2, device=DEV), torch.empty(n, 32, 4, device=DEV)[..., ::2], torch.empty(n, 32, 2, dtype=torch.float64, device=DEV),
+                torch.empty(n, 31, dtype=torch.complex64, device=DEV)):
+        with pytest.raises(ValueError):
+            P.ops.rope3d_table(*args, out=out)
+
+
 def test_running_out_of_memory_is_an_out_of_memory_error():
     """The operators allocate through PyTorch, within the share of the device that the process has been given: beyond it they raise
     what PyTorch raises, which callers catch to retry with less, and work again afterwards."""
