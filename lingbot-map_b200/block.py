@@ -47,31 +47,36 @@ def _stock_dropout(m: nn.Module) -> bool:
 
 
 def _watched() -> bool:
-    """A function or dispatch mode is active: it is to see every operation of the modules (a counter, a tracer, a rewriter).
-    The mode behind torch.set_default_device only places new tensors."""
+    """An active dispatch or function mode is to see every operation of the modules (a counter, a tracer, a rewriter).  The
+    function mode behind torch.set_default_device only places new tensors."""
     C = torch._C
     return (C._len_torch_dispatch_stack() > 0
             or any(type(C._get_function_stack_at(i)) is not DeviceContext for i in range(C._len_torch_function_stack())))
 
 
+def _may_fuse() -> bool:
+    """Whole layers run as one native call in eager inference only: under torch.compile the modules are traced, with
+    gradients enabled the Linear layers record them, and global hooks, modes and torch.jit.trace want to see every module."""
+    C = torch._C
+    return not (torch.is_grad_enabled() or torch.compiler.is_compiling() or _nn_module._global_forward_hooks
+                or _nn_module._global_forward_pre_hooks or C._get_tracing_state() is not None
+                or (C._len_torch_dispatch_stack() or C._len_torch_function_stack()) and _watched())
+
+
+# The functions and class methods that a native layer passes by, as they are now.  One that has been replaced (by a profiler
+# or a test) wants to be called.
 _layer_steps = attrgetter("_dense", "_qkv_rows", "_norm_params", "_rope_args")
+_global_steps = attrgetter("forward", "stream_frame", "_evict", "_dense", "_qkv_rows", "_norm_params", "_rope_args")
 _manager_steps = attrgetter(*sorted(_MANAGER_STEPS))
 
 
-def _code() -> tuple:
-    """The functions and class methods that a native layer passes by, as they are now."""
+def _frame_code() -> tuple:
+    return F.linear, ops.prep_qkv, ops.dense_attention, rope_table_from_pos, nn.Linear.forward, _layer_steps(B200FrameAttention)
+
+
+def _block_code() -> tuple:
     return (F.linear, F.layer_norm, F.gelu, ops.prep_qkv, ops.dense_attention, rope_table_from_pos, nn.Linear.forward, nn.LayerNorm.forward,
-            nn.GELU.forward, LayerScale.forward, Mlp.forward, B200Block.ffn_residual, B200Attention.forward, B200Attention.stream_frame,
-            B200Attention._evict, *_layer_steps(B200Attention), *_layer_steps(B200FrameAttention), *_manager_steps(B200KVCacheManager))
-
-
-def _may_fuse() -> bool:
-    """Whole layers run as one native call in eager inference only: under torch.compile the modules are traced, with
-    gradients enabled the Linear layers record them, global hooks, modes and torch.jit.trace want to see every module, and
-    a function or class method that has been replaced (by a profiler or a test) wants to be called."""
-    return not (torch.is_grad_enabled() or torch.compiler.is_compiling() or _nn_module._global_forward_hooks
-                or _nn_module._global_forward_pre_hooks or torch._C._get_tracing_state() is not None or _watched()
-                or _code() != _STOCK_CODE)
+            nn.GELU.forward, LayerScale.forward, Mlp.forward, B200Block.ffn_residual, _global_steps(B200Attention), _manager_steps(B200KVCacheManager))
 
 
 def _reference_classes():
@@ -209,7 +214,7 @@ class B200FrameAttention(_AttentionBase):
 
     def forward(self, x: Tensor, pos=None, num_patches=None, num_special=None, num_frames=None,
                 enable_3d_rope=False) -> Tensor:
-        if type(self) is B200FrameAttention and _may_fuse():      # a subclass may replace any step
+        if type(self) is B200FrameAttention and _may_fuse() and _frame_code() == _STOCK_FRAME_CODE:      # a subclass may replace any step
             params = self._layer_params()
             if params is not None:
                 y = _native.frame_layer(x, params, self.num_heads, pos, *self._rope_kind(pos, enable_3d_rope))
@@ -364,7 +369,7 @@ class B200Block(nn.Module):
                 enable_3d_rope=enable_3d_rope, kv_cache=kv_cache, global_idx=global_idx,
                 num_frame_per_block=num_frame_per_block, num_frame_for_scale=num_frame_for_scale,
                 num_register_tokens=num_register_tokens)
-        if type(self) is B200Block and _may_fuse():               # a subclass may replace any step
+        if type(self) is B200Block and _may_fuse() and _block_code() == _STOCK_BLOCK_CODE:               # a subclass may replace any step
             y = self._fused_forward(x, pos, num_frames, enable_3d_rope, kv_cache, global_idx)
             if y is not NotImplemented:
                 return y
@@ -419,4 +424,4 @@ class B200Block(nn.Module):
         return x + self.ls2(self.mlp(self.norm2(x)))
 
 
-_STOCK_CODE = _code()
+_STOCK_FRAME_CODE, _STOCK_BLOCK_CODE = _frame_code(), _block_code()

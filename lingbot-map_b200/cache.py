@@ -289,7 +289,7 @@ class B200KVCacheManager:
         table is planned when block_idx == 0 and reused by the other blocks of the same frame."""
         self._require_device()
         # a plan() of a subclass, or put in its place (to attend over a page range, to time it), is the one that is called
-        stock = type(self).plan is _STOCK_PLAN and "plan" not in self.__dict__
+        stock = block_idx != 0 or (type(self).plan is _STOCK_PLAN and "plan" not in self.__dict__)
         out = self._native.attention(self._h, self._dev_index, block_idx, q, return_lse, None if stock else self.plan)
         return torch.zeros_like(q) if out is None else out          # nothing cached yet: :368-370
 
