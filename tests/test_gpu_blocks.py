@@ -191,7 +191,8 @@ def test_layers_as_one_call_equal_the_module_code(monkeypatch, dim, H, weights, 
     eight warps per row, row counts that leave warps idle, and every combination of parameter and activation precision.
 
     Both sides round the same intermediates to bf16, the native call fewer of them (scale and sum in one step), and return
-    bf16 or fp32; results may differ by two bf16 rounding steps at the largest magnitude of the output, 2 * 2^-7 * max."""
+    bf16 or fp32; results may differ by two bf16 rounding steps at the largest magnitude of the output, 2 * 2^-7 * max.  That shows a
+    missing or misplaced term; how close the sums are is measured against float64 further down."""
     from lingbot_map_b200 import block as block_mod
     pph, ppw, ns, scale, window = 3, 5, 6, 2, 2
     T = ns + pph * ppw
@@ -492,3 +493,90 @@ def test_frame_layer_with_an_output_projection_of_another_width(monkeypatch, wid
         want = fa(x, pos=pos, enable_3d_rope=True)
     assert got.shape == want.shape == (2, 21, width) and got.dtype == want.dtype
     assert float((got.float() - want.float()).abs().max()) <= 2 * 2 ** -7 * float(want.float().abs().max())
+
+
+class _In64Bits:
+    """The two layers in float64 from the module's parameters: LayerNorm, Linear, rotations and softmax attention as they are
+    defined, without a rounding in between."""
+
+    @staticmethod
+    def linear(x, m):
+        return x @ m.weight.double().t() + m.bias.double()
+
+    @staticmethod
+    def norm(x, m):
+        return torch.nn.functional.layer_norm(x, (x.shape[-1],), m.weight.double(), m.bias.double(), m.eps)
+
+    @staticmethod
+    def rotate(x, ang, three_d):                # x [N, H, 64], ang [N, 32]
+        c, s = ang.cos()[:, None], ang.sin()[:, None]
+        if three_d:
+            a, b = x[..., 0::2], x[..., 1::2]
+            return torch.stack([a * c - b * s, a * s + b * c], -1).reshape(x.shape)
+        y = x.reshape(*x.shape[:2], 2, 2, 16)
+        a, b = y[:, :, :, 0], y[:, :, :, 1]
+        c, s = c.reshape(-1, 1, 2, 16), s.reshape(-1, 1, 2, 16)
+        return torch.stack([a * c - b * s, a * s + b * c], 3).reshape(x.shape)
+
+    @classmethod
+    def attention(cls, m, x, ang, three_d, cached=None):        # x [N, C]
+        q, k, v = cls.linear(x, m.qkv).reshape(x.shape[0], 3, m.num_heads, 64).unbind(1)
+        q, k = cls.rotate(cls.norm(q, m.q_norm), ang, three_d), cls.rotate(cls.norm(k, m.k_norm), ang, three_d)
+        if cached is not None:
+            k, v = torch.cat([cached[0].double(), k]), torch.cat([cached[1].double(), v])
+        p = torch.softmax(torch.einsum("qhd,khd->hqk", q, k) / 8, -1)
+        return cls.linear(torch.einsum("hqk,khd->qhd", p, v).reshape(x.shape), m.proj)
+
+    @classmethod
+    def frame(cls, m, x, ang, three_d):
+        return torch.stack([cls.attention(m, t.double(), ang, three_d) for t in x])
+
+    @classmethod
+    def block(cls, m, x, ang, three_d, cached=None):
+        out = []
+        for t in x.double():
+            t = t + cls.attention(m.attn, cls.norm(t, m.norm1), ang, three_d, cached) * m.ls1.gamma.double()
+            out.append(t + cls.linear(torch.nn.functional.gelu(cls.linear(cls.norm(t, m.norm2), m.mlp.fc1)), m.mlp.fc2) * m.ls2.gamma.double())
+        return torch.stack(out)
+
+
+@pytest.mark.parametrize("dim,H,weights,x_dtype,three_d", [(128, 2, "bf16", "bf16", True), (192, 3, "f32", "f32", True), (1024, 16, "bf16", "bf16", False),
+                                                           (1024, 16, "bf16", "f32", True), (320, 5, "f32", "bf16", False)])
+def test_native_layers_are_no_further_from_64_bits_than_the_modules(monkeypatch, dim, H, weights, x_dtype, three_d):
+    """Error of both ways against float64, 2-norm over 2-norm.  The native call rounds the same operands to bf16 and fewer sums, so
+    its error is not larger than the modules' but for the spread of two sets of some thousand roundings of the same size (2 %; an error of
+    its own of a fifth of the roundings would show).  Neither exceeds 2^-7, which is fifty roundings of 2^-9 / sqrt(3) in quadrature: a
+    path has about ten, and those before the softmax weigh several times."""
+    from lingbot_map_b200 import block as block_mod
+    pph, ppw, ns, scale = 9, 13, 6, 2
+    T, dt = ns + pph * ppw, {"bf16": torch.bfloat16, "f32": torch.float32}
+    blk = P.B200Block(dim=dim, num_heads=H, init_values=0.5, qk_norm=True, rope=Rope2dStub(), kv_cache_sliding_window=4, kv_cache_scale_frames=scale)
+    fa = P.B200FrameAttention(dim, num_heads=H, qk_norm=True, rope=Rope2dStub())
+    blk, fa = blk.eval().to(DEV), fa.eval().to(DEV)
+    seeded.fill_module_(blk, 3)
+    seeded.fill_module_(fa, 4)
+    blk, fa = blk.to(dt[weights]), fa.to(dt[weights])
+    y, x = torch.meshgrid(torch.arange(1, pph + 1), torch.arange(1, ppw + 1), indexing="ij")
+    pos2d = torch.cat([torch.zeros(ns, 2, dtype=torch.int64), torch.stack([y, x], -1).reshape(-1, 2)])[None].to(DEV)
+    pos = lambda f, n: rope3d_pos(f, n, pph, ppw, ns) if three_d else pos2d.repeat(1, n, 1)
+    inv = 100.0 ** -(torch.arange(16, device=DEV, dtype=torch.float64) / 16)
+    ang = lambda f, n: (pos(f, n).reshape(-1, 32).angle() if three_d else (pos(f, n)[0].double()[:, :, None] * inv).reshape(-1, 32))
+    data = [torch.from_numpy(seeded.randn(i, *s, dim)).to(DEV).to(dt[x_dtype]) for i, s in enumerate([(2, T), (2, T), (1, scale * T), (1, T)])]
+
+    def run(fused):
+        monkeypatch.setattr(block_mod, "_may_fuse", lambda: fused)
+        mgr = P.B200KVCacheManager(1, scale + 4 + 16, T, H, 64, device=DEV, scale_frames=scale, sliding_window=4, max_total_frames=40)
+        kw = dict(num_patches=T - ns, num_special=ns, enable_3d_rope=three_d, global_idx=0)
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            out = [fa(data[0], pos=pos(0, 1), enable_3d_rope=three_d),
+                   blk(data[1], pos=pos(0, 1), **kw), blk(data[2], pos=pos(0, scale), num_frames=scale, kv_cache=mgr, **kw)]
+            cached = mgr._gather_kv(0)
+            out.append(blk(data[3], pos=pos(scale, 1), num_frames=1, kv_cache=mgr, **kw))
+        want = [_In64Bits.frame(fa, data[0], ang(0, 1), three_d), _In64Bits.block(blk, data[1], ang(0, 1), three_d),
+                _In64Bits.block(blk, data[2], ang(0, scale), three_d), _In64Bits.block(blk, data[3], ang(scale, 1), three_d, cached)]
+        return [float((a.double() - w).norm() / w.norm()) for a, w in zip(out, want)]
+
+    with torch.no_grad():
+        native, modules = run(True), run(False)
+    for i, (a, b) in enumerate(zip(native, modules)):
+        assert a <= 1.02 * b and a <= 2 ** -7, (i, a, b)
