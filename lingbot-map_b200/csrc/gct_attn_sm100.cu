@@ -1104,17 +1104,21 @@ void choose_attention_config(int n_q_tiles, int heads_x_batch, int total_blocks,
 #endif
   constexpr double kMergeCost = GCT_MERGE_COST;
   // Paged calls (split_len != nullptr): a call that fits one wave pays about five blocks once; in a call of several waves
-  // every wave costs about fifteen blocks beside its KV blocks (set-up, pipeline fill, epilogue, and at the board's power limit a
-  // lower clock the fuller the SMs are: idle SMs are not lost time there).  Measured, 64 (head, tile pair) items, us for 2 ranges
-  // (128 CTAs) against the 9 that a fixed cost of two blocks chose: 250 KV blocks 168 : 195, 371 242 : 268, 385 254 : 280,
-  // 527 338 : 360, 600 385 : 402.  One tile per CTA (0.6 of the work): measured for one wave only.
+  // every wave is charged fifteen blocks beside its KV blocks (set-up, pipeline fill, epilogue, and at the board's power limit a
+  // lower clock the fuller the SMs are: idle SMs are not lost time there).  Measured in back-to-back loops of this kernel, 64 (head,
+  // tile pair) items, us for 2 ranges (one wave, 128 CTAs) against the 9 (four waves) that a fixed cost of two blocks chose: 250 KV
+  // blocks 168 : 195, 371 242 : 268, 385 254 : 280, 527 338 : 360, 600 385 : 402, 1065 675 : 709.  With the five blocks of the
+  // one-wave plan these pairs imply 10 to 13 blocks per wave up to 600 blocks and 22 at 1065.  Fifteen is not a fit to them:
+  // it chooses the plan that measured faster up to a thousand blocks and keeps the nine equal ranges beyond (above 15.5 the model
+  // would take two at 1057 blocks, too).  Which is faster there inside a frame has not been measured; at 600 blocks, where two ranges
+  // win the loop, two and nine take the same time in a frame (below).  Nine blocks for one-tile CTAs is 0.6 of fifteen, not measured.
   const bool paged = split_len != nullptr;
   auto fixed = [paged](int qt, bool one_wave) { return !paged ? 2.0 : one_wave ? (qt == 2 ? 5.0 : 4.0) : (qt == 2 ? 15.0 : 9.0); };
   // Long ranges + a short one fill the SMs that equal ranges leave idle.  The paged kernel alone, back to back at the power limit,
   // takes about as long as with two equal ranges (us: 71 KV blocks 54.8 : 56.7, 193 134 : 132, 285 190 : 192, 600 392 : 385); inside
   // a frame, beside the other kernels, it is faster: 24 layers at 600 blocks 9.7-10.0 ms against 10.5 with two and with nine
-  // equal ranges, two layer pairs as modules 949-974 : 1013 us.  Not beyond a thousand blocks: nine long ranges and a short one were
-  // 0.6 % slower there than nine equal ones (1057 blocks, back to back).
+  // equal ranges, two layer pairs as modules 949-974 : 1013 us.  Not beyond a thousand blocks, on one measurement in a loop: at 1057
+  // blocks nine long ranges and a short one were 0.6 % slower than nine equal ones.  Not measured there: two long ranges and a short one.
   constexpr int kUnevenMaxBlocks = 1000;
   // the plan of the previous call with the same arguments (a frame asks 24 times for the same one)
   static thread_local SplitPlanKey last_key = {-1, -1, -1, -1, -1};

@@ -243,7 +243,8 @@ int launch_decode_attention(const float* q, const float* k_new, const float* v_n
   const int rc = device_sm_count(&sms);
   if (rc != GCT_OK) return rc;
   const int total = cached + n_q;
-  // one wave of two CTAs per SM, at least 64 keys each (two steps of the eight warps: below that the merge costs more)
+  // Two CTAs per SM, at least 64 keys each (two steps of the eight warps: below that the merge costs more): one wave for a single
+  // new token; for two to eight at D = 128 a CTA fills the registers of an SM (190 per thread) and they are two waves.
   int splits = std::max(1, std::min(2 * sms / heads, (total + 63) / 64));
   while (splits > 1 && decode_workspace_bytes(heads, head_dim, splits, n_q) > workspace_bytes) --splits;
   if (decode_workspace_bytes(heads, head_dim, splits, n_q) > workspace_bytes)

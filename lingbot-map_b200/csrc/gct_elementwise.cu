@@ -306,7 +306,8 @@ struct Raw8 {
   }
 };
 
-// v = x + gamma * y per row, stored in x's precision, and LayerNorm(v) as bf16: the residual sums and norms of a block
+// v = x + gamma * y per row, stored as sum_dtype (fp32 where x or gamma is, as the separate operations promote, else bf16), and
+// LayerNorm(v) as bf16: the residual sums and norms of a block
 // (lingbot_map/layers/block.py:217-310) in one pass over the row, which as separate tensor operations were four to
 // six launches of 2-7 us each (scale, add, norm in fp32, cast to bf16 for the next Linear).
 //

@@ -3,7 +3,7 @@
 // Restates demo_render/render_cuda_ext/frustum_cull/frustum_cull.cu:5-33 and
 // demo_render/render_cuda_ext/voxel_morton/voxel_morton.cu:5-62 of the reference (compute only; the renderer that
 // consumes them needs a graphics API and is not part of this library).  Both are streams over AoS xyz floats:
-// 13 B per point (cull: HBM bound, 19.8 us for 8 M points = 5.3 TB/s) and 24 B read + 44 B written per point (voxelise).
+// 13 B per point (cull: HBM bound, the kernel alone 19.7 us for 8 M points = 5.3 TB/s) and 24 B read + 44 B written per point (voxelise).
 // Arithmetic is written with explicitly rounded single operations (no fused multiply-add, IEEE division), so that
 // a float32 CPU restatement reproduces every mask bit and every Morton code exactly.
 #include <algorithm>
@@ -57,8 +57,9 @@ __device__ __forceinline__ bool cull_fast(float x, float y, float z, const CullA
   return in;
 }
 
-// A thread takes four points = three 16-byte loads and has the next four on their way.  Two IEEE divisions per point
-// and one load in flight: 22.6 us at 8 M points; this way 19.8 us (16 us at the measured copy rate).
+// A thread takes four points = three 16-byte loads and has the next four on their way.  The kernel alone with two IEEE divisions
+// per point and one load in flight: 22.5 us at 8 M points; this way 19.7 us (16 us at the measured copy rate; as one call
+// among others, with its launch and the allocation of the mask, 22.6 us).
 __global__ void __launch_bounds__(256) gct_frustum_cull_kernel(const float* __restrict__ pts, CullArgs a, uint8_t* __restrict__ visible,
                                                                int64_t n) {
   if (a.R_dev != nullptr) {
@@ -499,7 +500,7 @@ int frustum_cull(const float* pts, int64_t n, const float* R, const float* t, co
   axis(cx, width, &a.mid_u, &a.in_u, &a.out_u);
   axis(cy, height, &a.mid_v, &a.in_v, &a.out_v);
   a.depth_tame = near_plane > 1e-30f && far_plane < 1e30f;
-  // one wave: the camera is read once per thread
+  // The camera is read once per thread, so a thread takes many points: two waves at the most (64 registers, four CTAs per SM).
   gct_frustum_cull_kernel<<<std::min(grid_for(n / 4), 148 * 8), 256, 0, stream>>>(pts, a, visible, n);
   GCT_CUDA_CHECK(cudaGetLastError());
   return GCT_OK;

@@ -173,7 +173,8 @@ struct NormRope {
     for (int i = 0; i < 4; ++i) {
       if (t[i] == nullptr) continue;
       const at::ScalarType want = all_bf16 ? at::kBFloat16 : at::kFloat;
-      // the kernel loads 16 bytes at a time: a bf16 parameter at another address (a slice of a flat buffer) is copied
+      // the launcher takes 16-byte aligned parameters only: a bf16 one at another address (a slice of a flat buffer) is copied,
+      // as the conversion to fp32 once did; an fp32 one there was always refused and is
       const bool in_place = t[i]->is_contiguous() && (want == at::kFloat || (reinterpret_cast<uintptr_t>(t[i]->data_ptr()) & 15) == 0);
       if (t[i]->scalar_type() == want && in_place) {
         ptr[i] = t[i]->data_ptr();
