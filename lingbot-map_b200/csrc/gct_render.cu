@@ -152,8 +152,8 @@ __global__ void __launch_bounds__(256) gct_mark_unique_kernel(const int64_t* __r
 // 64-bit sort made eight radix passes over (code, index), then two gathers, a mark, a compaction and three more gathers
 // (34 launches, 240 us).  Voxel indices within +-2^nb only need a Morton key of 3 (nb + 1) bits (bits nb ... 20 of an offset
 // index all equal the complement of its sign, so leaving them out does not change the order): 24-33 bits for a room at
-// centimetres, four or five passes of eight bits.  The number of bits is found on the device and passes that are not
-// needed return at once, so the host waits only once, for the number of voxels.  Measured for 196 k points: 240 -> 67 us.
+// centimetres, four or five passes of eight bits.  The number of bits is found on the device, so the host waits only once, for
+// the number of voxels.  Measured for 196 k points: 240 us, as short-key passes 68 us, with the passes in one launch 53 us.
 constexpr int kVoxelTile = 2048;                 // keys per CTA of a pass: a frame's cloud makes about one CTA per SM
 constexpr int kVoxelThreads = 512;
 constexpr int kVoxelWarps = kVoxelThreads / 32;
@@ -161,6 +161,7 @@ constexpr int kVoxelPerThread = kVoxelTile / kVoxelThreads;
 constexpr int kVoxelMaxTiles = 256;              // every CTA of a pass adds up the digit counts of all tiles
 constexpr int kVoxelMaxPasses = 8;
 constexpr int kVoxelOffset = 1 << 20;            // voxel_morton.cu:36-38
+constexpr int32_t kVoxelPending = -1, kVoxelFailed = -2;      // in place of a tile's count
 
 struct VoxelScratch {
   uint64_t* keys0;         // Morton codes and indices, two buffers
@@ -170,6 +171,7 @@ struct VoxelScratch {
   uint32_t* extent;        // [tiles] OR of the index magnitudes of a tile
   uint32_t* hist;          // [passes][tiles][256] digit counts
   int32_t* heads;          // [tiles] first points of voxels in a tile of the sorted keys
+  uint32_t* arrived;       // CTAs that have come to the barriers of the sort, all barriers together
   int n, tiles;
   __device__ __forceinline__ uint64_t* keys(int i) const { return i & 1 ? keys1 : keys0; }
   __device__ __forceinline__ uint32_t* index(int i) const { return i & 1 ? index1 : index0; }
@@ -227,24 +229,34 @@ __global__ void __launch_bounds__(kVoxelThreads) gct_voxel_code_kernel(const flo
   if ((threadIdx.x & 31) == 0) atomicOr(&s_or, m);
   __syncthreads();
   if (threadIdx.x == 0) s.extent[blockIdx.x] = s_or;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *s.arrived = 0;
   uint32_t* hist = s.hist + static_cast<size_t>(blockIdx.x) * 256;
   for (int k = threadIdx.x; k < kVoxelMaxPasses * 256; k += kVoxelThreads)      // counts of the later passes start from zero
     hist[static_cast<size_t>(k >> 8) * s.tiles * 256 + (k & 255)] = k < 256 ? s_hist[k] : 0u;
 }
 
-// One stable pass over 8 bits.  A warp owns 128 consecutive keys of the tile and ranks them 32 at a time (one ballot per
+struct VoxelShared {
+  uint32_t warp[kVoxelWarps][256];
+  uint32_t total[256], before[256];
+  uint32_t global[256];                         // first global position of a digit of this tile, minus its first local one
+  uint32_t scan[2][8];
+  uint64_t code[kVoxelTile];
+  uint32_t index[kVoxelTile];
+  int met;
+};
+
+// One stable pass over 8 bits of one tile.  A warp owns 128 consecutive keys of the tile and ranks them 32 at a time (one ballot per
 // digit bit); the tile's base per digit is the number of smaller digits anywhere plus the number of equal ones in earlier
-// tiles.  While scattering, the digit counts of the next pass are gathered by the destination tile.
-__global__ void __launch_bounds__(kVoxelThreads) gct_voxel_pass_kernel(int pass, VoxelScratch s) {
-  pdl_wait();
-  __shared__ uint32_t s_warp[kVoxelWarps][256];
-  __shared__ uint32_t s_total[256], s_before[256];
-  __shared__ uint32_t s_global[256];                            // first global position of a digit of this tile, minus its first local one
-  __shared__ uint32_t s_scan[2][8];
-  __shared__ uint64_t s_code[kVoxelTile];
-  __shared__ uint32_t s_index[kVoxelTile];
-  const int axis_bits = voxel_axis_bits(s), passes = voxel_passes(axis_bits);
-  if (pass >= passes) return;
+// tiles.  While scattering, the digit counts of the next pass are gathered by the destination tile.  What other CTAs wrote in an
+// earlier pass is read past L1, which may hold lines of the pass before.
+__device__ __forceinline__ void voxel_pass(int pass, int passes, int tile, int axis_bits, const VoxelScratch& s, VoxelShared& sh) {
+  auto& s_warp = sh.warp;
+  auto& s_total = sh.total;
+  auto& s_before = sh.before;
+  auto& s_global = sh.global;
+  auto& s_scan = sh.scan;
+  auto& s_code = sh.code;
+  auto& s_index = sh.index;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, shift = 8 * pass;
   const uint64_t* keys = s.keys(pass);
   const uint32_t* index = s.index(pass);
@@ -252,9 +264,9 @@ __global__ void __launch_bounds__(kVoxelThreads) gct_voxel_pass_kernel(int pass,
   uint32_t idx[kVoxelPerThread], rank[kVoxelPerThread];
 #pragma unroll
   for (int u = 0; u < kVoxelPerThread; ++u) {
-    const int i = blockIdx.x * kVoxelTile + warp * (32 * kVoxelPerThread) + u * 32 + lane;
-    code[u] = i < s.n ? keys[i] : 0;
-    idx[u] = i < s.n ? index[i] : 0xffffffffu;                  // no point has this index (n <= kVoxelMaxTiles * kVoxelTile)
+    const int i = tile * kVoxelTile + warp * (32 * kVoxelPerThread) + u * 32 + lane;
+    code[u] = i < s.n ? __ldcg(keys + i) : 0;
+    idx[u] = i < s.n ? __ldcg(index + i) : 0xffffffffu;                  // no point has this index (n <= kVoxelMaxTiles * kVoxelTile)
   }
   // digit counts of all tiles: a thread adds up four digits over every eighth tile
   {
@@ -263,8 +275,8 @@ __global__ void __launch_bounds__(kVoxelThreads) gct_voxel_pass_kernel(int pass,
     uint4 total = make_uint4(0, 0, 0, 0), before = total;
 #pragma unroll 8
     for (int t = part; t < s.tiles; t += kVoxelThreads / 64) {
-      const uint4 c = hist[t * 64];
-      const uint32_t e = t < static_cast<int>(blockIdx.x) ? 0xffffffffu : 0u;
+      const uint4 c = __ldcg(hist + t * 64);
+      const uint32_t e = t < tile ? 0xffffffffu : 0u;
       total.x += c.x; total.y += c.y; total.z += c.z; total.w += c.w;
       before.x += c.x & e; before.y += c.y & e; before.z += c.z & e; before.w += c.w & e;
     }
@@ -347,7 +359,7 @@ __global__ void __launch_bounds__(kVoxelThreads) gct_voxel_pass_kernel(int pass,
   uint64_t* keys_out = s.keys(pass + 1);
   uint32_t* index_out = s.index(pass + 1);
   uint32_t* next = s.hist + static_cast<size_t>(pass + 1) * s.tiles * 256;
-  const int count = min(kVoxelTile, s.n - static_cast<int>(blockIdx.x) * kVoxelTile);
+  const int count = min(kVoxelTile, s.n - tile * kVoxelTile);
 #pragma unroll
   for (int u = 0; u < kVoxelPerThread; ++u) {
     const int local = u * kVoxelThreads + threadIdx.x;
@@ -366,22 +378,58 @@ __global__ void __launch_bounds__(kVoxelThreads) gct_voxel_pass_kernel(int pass,
   }
 }
 
-__device__ __forceinline__ bool voxel_head(const uint64_t* keys, int i, int n) { return i < n && (i == 0 || keys[i] != keys[i - 1]); }
+__device__ __forceinline__ bool voxel_head(const uint64_t* keys, int i, int n) {
+  return i < n && (i == 0 || __ldcg(keys + i) != __ldcg(keys + i - 1));
+}
 
-// First points of voxels per tile, for the gather and, with the number of passes the keys need in front, for the host
-// (`report`, in pinned host memory: [passes, count per tile ...]).
-__global__ void __launch_bounds__(kVoxelThreads) gct_voxel_count_kernel(VoxelScratch s, int32_t* report) {
-  pdl_wait();
-  const int passes = voxel_passes(voxel_axis_bits(s));
-  const uint64_t* keys = s.keys(passes);
-  int count = 0;
-#pragma unroll
-  for (int u = 0; u < kVoxelPerThread; ++u)
-    count += __syncthreads_count(voxel_head(keys, blockIdx.x * kVoxelTile + u * kVoxelThreads + threadIdx.x, s.n));
+// All CTAs of the grid (launched cooperatively: they run at the same time) meet; `target` arrivals in total.  Gives up after about
+// two seconds and returns false.
+__device__ __forceinline__ bool voxel_barrier(const VoxelScratch& s, uint32_t target, VoxelShared& sh) {
+  __syncthreads();
   if (threadIdx.x == 0) {
-    s.heads[blockIdx.x] = count;
-    report[1 + blockIdx.x] = count;
-    if (blockIdx.x == 0) report[0] = passes;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(s.arrived) : "memory");
+    const long long t0 = clock64();
+    bool met = true;
+    for (;;) {
+      uint32_t now;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(s.arrived) : "memory");
+      if (now >= target) break;
+      if (clock64() - t0 > 4000000000LL) {
+        met = false;
+        break;
+      }
+    }
+    sh.met = met;
+  }
+  __syncthreads();
+  return sh.met;
+}
+
+// The sort in one cooperative launch: as many passes as the keys need, with a barrier over the grid behind each, then the number of
+// first points of voxels per tile, for the gather and (`report`, in pinned host memory, kVoxelPending before; kVoxelFailed when a
+// barrier gave up) for the host.  As a launch per pass, five whatever the extent, one to count and a wait for the stream, a frame of 196 k
+// points took 67.9 us, this way 52.9 us: a barrier costs about a third of a dependent launch.
+__global__ void __launch_bounds__(kVoxelThreads, 2) gct_voxel_sort_kernel(VoxelScratch s, volatile int32_t* report) {
+  __shared__ VoxelShared sh;
+  const int axis_bits = voxel_axis_bits(s), passes = voxel_passes(axis_bits);
+  bool met = true;
+  for (int pass = 0; pass < passes && met; ++pass) {
+    for (int tile = blockIdx.x; tile < s.tiles; tile += gridDim.x) {
+      voxel_pass(pass, passes, tile, axis_bits, s, sh);
+      __syncthreads();
+    }
+    met = voxel_barrier(s, static_cast<uint32_t>(pass + 1) * gridDim.x, sh);
+  }
+  const uint64_t* keys = s.keys(passes);
+  for (int tile = blockIdx.x; tile < s.tiles; tile += gridDim.x) {
+    int count = 0;
+#pragma unroll
+    for (int u = 0; u < kVoxelPerThread; ++u)
+      count += __syncthreads_count(met && voxel_head(keys, tile * kVoxelTile + u * kVoxelThreads + threadIdx.x, s.n));
+    if (threadIdx.x == 0) {
+      s.heads[tile] = count;
+      report[tile] = met ? count : kVoxelFailed;
+    }
   }
 }
 
@@ -459,6 +507,7 @@ VoxelScratch voxel_scratch(void* base, int64_t n, size_t* bytes) {
   s.extent = reinterpret_cast<uint32_t*>(part(static_cast<size_t>(s.tiles) * 4));
   s.hist = reinterpret_cast<uint32_t*>(part(static_cast<size_t>(kVoxelMaxPasses) * s.tiles * 256 * 4));
   s.heads = reinterpret_cast<int32_t*>(part(static_cast<size_t>(s.tiles) * 4));
+  s.arrived = reinterpret_cast<uint32_t*>(part(sizeof(uint32_t)));
   if (bytes != nullptr) *bytes = off;
   return s;
 }
@@ -514,24 +563,42 @@ int voxel_sort_layout(int64_t n, size_t* bytes, int* tiles) {
   return GCT_OK;
 }
 
-// Five passes serve indices below 2^12 (40 bits); a wider cloud reports more and gets the rest in a second round.
-static int voxel_sort_passes(const VoxelScratch& s, int from, int to, int32_t* report, cudaStream_t stream) {
-  for (int pass = from; pass < to; ++pass) GCT_CUDA_CHECK(launch_pdl(gct_voxel_pass_kernel, dim3(s.tiles), dim3(kVoxelThreads), 0, stream, pass, s));
-  GCT_CUDA_CHECK(launch_pdl(gct_voxel_count_kernel, dim3(s.tiles), dim3(kVoxelThreads), 0, stream, s, report));
-  GCT_CUDA_CHECK(cudaStreamSynchronize(stream));
-  return GCT_OK;
-}
-
 int voxel_sort(const float* xyz, float voxel_size, int64_t n, void* scratch, int32_t* report, int64_t* voxels_out, cudaStream_t stream) {
   if (!(voxel_size > 0.f)) return fail(GCT_ERR_INVALID, "gct_voxel_morton: bad argument");
   const VoxelScratch s = voxel_scratch(scratch, n, nullptr);
-  constexpr int kFirst = 5;
-  GCT_CUDA_CHECK(launch_pdl(gct_voxel_code_kernel, dim3(s.tiles), dim3(kVoxelThreads), 0, stream, xyz, voxel_size, s));
-  int rc = voxel_sort_passes(s, 0, kFirst, report, stream);
-  if (rc == GCT_OK && report[0] > kFirst) rc = voxel_sort_passes(s, kFirst, report[0], report, stream);
+  int sms = 148;
+  const int rc = device_sm_count(&sms);
   if (rc != GCT_OK) return rc;
-  *voxels_out = 0;
-  for (int t = 0; t < s.tiles; ++t) *voxels_out += report[1 + t];
+  std::fill(report, report + s.tiles, kVoxelPending);
+  GCT_CUDA_CHECK(launch_pdl(gct_voxel_code_kernel, dim3(s.tiles), dim3(kVoxelThreads), 0, stream, xyz, voxel_size, s));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(std::min(s.tiles, 2 * sms));      // two CTAs of the sort fit an SM: all tiles at once where there are 128 SMs
+  cfg.blockDim = dim3(kVoxelThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  GCT_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gct_voxel_sort_kernel, s, static_cast<volatile int32_t*>(report)));
+  // The counts are looked for where the kernel writes them: they are there some microseconds before the stream is seen to be idle.
+  const volatile int32_t* counts = report;
+  int64_t total = 0;
+  for (int t = 0; t < s.tiles; ++t) {
+    for (uint32_t look = 1; counts[t] == kVoxelPending; ++look) {
+      if ((look & 0xfffffu) != 0) continue;
+      const cudaError_t e = cudaStreamQuery(stream);
+      if (e == cudaErrorNotReady) continue;
+      GCT_CUDA_CHECK(e);
+      if (counts[t] == kVoxelPending) return fail(GCT_ERR_DEVICE_STATUS, "voxelisation: the sort ended without a result");
+    }
+    if (counts[t] == kVoxelFailed) {
+      GCT_CUDA_CHECK(cudaStreamSynchronize(stream));
+      return fail(GCT_ERR_DEVICE_STATUS, "voxelisation: a barrier of the sort was not reached in time");
+    }
+    total += counts[t];
+  }
+  *voxels_out = total;
   return GCT_OK;
 }
 

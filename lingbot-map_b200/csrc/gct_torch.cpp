@@ -789,7 +789,7 @@ PyObject* py_voxelize_frame(PyObject*, PyObject* const* a, Py_ssize_t n) {
     int tiles = 0;
     check(gct::voxel_sort_layout(count, &bytes, &tiles));
     Tensor scratch = empty({static_cast<int64_t>(bytes)}, at::kByte, xyz);
-    Tensor report = at::empty({tiles + 1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+    Tensor report = at::empty({tiles}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
     int64_t voxels = 0;
     int rc;
     {

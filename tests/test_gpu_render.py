@@ -68,6 +68,23 @@ def test_large_cloud_properties():
     assert np.array_equal(vis[idx].cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("n", [148 * 2048 + 5, 256 * 2048 - 1, 256 * 2048])
+def test_voxelize_frame_sort_up_to_its_largest(n):
+    """More tiles than SMs, up to the largest cloud the sort takes (256 tiles meet at its barriers), again and again on one stream and on
+    two at once."""
+    rs = np.random.RandomState(n % 1000)
+    xyz = (rs.randint(-300, 301, (n, 3)) + 0.5).astype(np.float32)
+    rgb = rs.rand(n, 3).astype(np.float32)
+    wc, wcol, wcodes = R.voxelize_frame(xyz, rgb, 1.0)
+    dx, dr = torch.from_numpy(xyz).to(DEV), torch.from_numpy(rgb).to(DEV)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    for i in range(6):
+        with torch.cuda.stream(side if i % 2 else torch.cuda.current_stream()):
+            c, col, codes = RO.voxelize_frame(dx, dr, 1.0)
+            assert np.array_equal(codes.cpu().numpy(), wcodes) and np.array_equal(c.cpu().numpy(), wc) and np.array_equal(col.cpu().numpy(), wcol)
+
+
 @pytest.mark.parametrize("n", [1, 2047, 2048, 2049, 2 * 2048 + 1, 65536])
 @pytest.mark.parametrize("extent", [3, 100, 5000, 2 ** 20 - 1])
 def test_voxelize_frame_sort_edges(n, extent):
