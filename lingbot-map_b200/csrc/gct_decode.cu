@@ -25,6 +25,7 @@ namespace {
 
 constexpr int kDecodeMaxQ = 8;
 constexpr int kDecodeWarps = 8;
+constexpr int kAheadRows = 64;           // rows of a range sent for before the kernel before has ended: 19 MB over 288 CTAs at D = 128
 constexpr int kGroup = 4;                // keys per step of a warp
 constexpr float kLog2e = 1.4426950408889634f;
 
@@ -67,7 +68,6 @@ template <int D, int kQ>
 __global__ void __launch_bounds__(kDecodeWarps * 32, kQ == 1 ? 2 : 1) gct_decode_attn_kernel(const DecodeArgs a) {
   using V = typename LaneVec<D>::T;
   constexpr int kPer = D / 32;
-  pdl_wait();
   const int h = blockIdx.x, split = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_q = kQ == 1 ? 1 : a.n_q;
@@ -76,6 +76,18 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, kQ == 1 ? 2 : 1) gct_decode
   const int j1 = static_cast<int>(static_cast<long long>(split + 1) * total / a.splits);
   const size_t row_stride = static_cast<size_t>(a.heads) * D;
   const size_t head_off = static_cast<size_t>(h) * D + lane * kPer;
+  // Under the end of the kernel before, which leaves the memory idle: the first cached rows of the range on their way to L2.  A hint
+  // that reads nothing, so it may be given for rows that kernel is still writing.  Sixteen calls at 10,000 frames 499.0 -> 487.7 us.
+  {
+    constexpr int kLines = D * 4 / 128;
+    const int rows = min(min(j1, a.cached) - j0, kAheadRows);
+    for (int i = threadIdx.x; i < 2 * kLines * rows; i += kDecodeWarps * 32) {
+      const float* base = i & 1 ? a.cache_v : a.cache_k;
+      const int r = (i >> 1) / kLines, line = (i >> 1) % kLines;
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(base + static_cast<size_t>(j0 + r) * row_stride + static_cast<size_t>(h) * D + 32 * line));
+    }
+  }
+  pdl_wait();
 
   // rows [j, j + kGroup) of K and V; past the end of the range the last K row again (its weight is set to zero) and zeros for
   // V, whose last row may hold an infinity
