@@ -5,19 +5,23 @@
 //
 // One CTA owns QT (1 or 2) query tiles of 128 rows of one head and one contiguous range of KV blocks
 // (128 tokens each).  Warp roles:
-//   warps [0, 4*QT)        softmax: one thread per query row; warp w owns TMEM lanes 32*(w%4)..+31
-//   warp  4*QT             producer: TMA loads of Q once, then K and V blocks into two 4-stage rings
-//   warps 4*QT+1 .. +QT    MMA issuers, one per query tile: tcgen05.mma
+//   warps [0, 8*QT)        softmax: two threads per query row, each with 64 of a block's 128 keys; warp w owns TMEM lanes 32*(w%4)..+31
+//   warp  8*QT             producer: TMA loads of Q once, then K and V blocks into two rings of stages
+//   warps 8*QT+1 .. +QT    MMA issuers, one per query tile: tcgen05.mma
 //                              S  = Q K^T   (M128 N128 K64,  A and B from shared memory)
 //                              O += P V     (M128 N64  K128, A = P from TMEM, B = V from shared memory)
 // TMEM columns (fp32): S_t at [128t, +128), O_t at [128QT + 64t, +64), P_t (bf16 pairs) at [192QT + 64t, +64).
 // Per KV block j of tile t:
-//   softmax   wait s_full; copy the S row into 128 registers; arrive s_empty  -> S_{j+1} may overwrite S
-//             row max; the reference maximum only moves when the row max grows by more than 2^8
+//   softmax   wait s_full; copy half the S row into 64 registers; arrive s_empty  -> S_{j+1} may overwrite S
+//             row max, exchanged between the two threads; the reference maximum only moves when the row max grows by more than 2^8
 //             (then O is rescaled in TMEM, which is rare after the first blocks);
-//             P = exp2(S*c - m*c) as bf16 pairs into TMEM; arrive p_full
+//             P = exp2(S*c - m*c) as bf16 pairs into TMEM, after the previous PV; arrive p_full of the half
 //   MMA       wait s_empty, K_{j+1}: issue S_{j+1} (runs under the softmax of block j) -> s_full, k_empty
 //             wait p_full,  V_j    : issue O += P_j V_j                                -> pv_full, v_empty
+// Two threads per row make four softmax warps per sub-partition at two tiles: while two wait for S, their loads or the previous PV, the
+// others keep the exponential and FMA pipes busy.  One thread per row (two warps, 208 registers each) took 2186 active clocks per block
+// of two tiles, now 2004 (counters, 600 KV blocks, bounded mode, set-up included), and 396 us against 383 back to back at the power
+// limit; one frame of dense attention (one tile per CTA) 12.2 us, now 11.1.  Four threads per row at one tile: 11.4 us.
 // Every mbarrier wait is bounded and reports through the status word instead of spinning forever.
 //
 // Bounded mode (gct_attn_kernel<2, true>, paged attention through the cache manager).  key_norm_max[h] bounds the
@@ -26,10 +30,10 @@
 // this once per CTA from the Q tile in shared memory: they multiply their row by scale * log2(e) in place,
 // derive ref from the scaled row, and write two small operand tiles, Qx (column 0 = -ref) and Kx (column 0 = 1).
 // A fifth K16 step of the S product, S += Qx Kx^T, then subtracts ref inside the tensor core: S arrives in TMEM
-// as the finished base-2 exponent, and the sweep is exp2, row sum and bf16 packing only - no row maximum, no
-// multiply-add in front of the exponential, no rescale of O.  A CTA in which some row's ref exceeds the limit
-// (or is not finite) takes a compact two-pass softmax with a running maximum instead; the choice is made per
-// CTA inside the one launch.
+// as the finished base-2 exponent, and the sweep is exp2, row sum and bf16 packing only - no row maximum, no exchange, no
+// multiply-add in front of the exponential, no rescale of O.  The product of either half of P starts when that half is
+// there.  A CTA in which some row's ref exceeds the limit (or is not finite) takes a compact two-pass softmax with a running maximum
+// instead; the choice is made per CTA inside the one launch.
 #include <algorithm>
 #include <mutex>
 #include <vector>
@@ -52,6 +56,15 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// One arrival of the warp, by the lane with `lead` != 0.
+__device__ __forceinline__ void mbar_arrive_elected(uint32_t lead, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\t"
+      "setp.ne.b32 e, %1, 0;\n\t"
+      "@e mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}"
+      ::"r"(bar), "r"(lead)
+      : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
@@ -230,25 +243,15 @@ __device__ __forceinline__ float2 exp2_poly2(float2 x) {
   r.y = __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23));
   return r;
 }
-// Same for exponents known to lie in [-126, 1]: no clamp.  kDeg 3: relative error 7.7e-5; kDeg 2: 1.8e-3.
-// `shift` (a non-negative integer value) is subtracted from the exponent first, at no cost: it rides in the rounding
-// constant.
-template <int kDeg>
-__device__ __forceinline__ float2 exp2_poly2_inrange(float2 x, float shift = 0.f) {
+// Same for exponents known to lie in [-126, 1]: no clamp (relative error 7.7e-5).
+__device__ __forceinline__ float2 exp2_poly2_inrange(float2 x) {
   constexpr float kMagic = 12582912.f;
-  const float ms = kMagic - shift;                       // exact: both are integers below 2^24
-  const float2 t = __fadd2_rn(x, make_float2(ms, ms));   // 1.5 * 2^23 + round(x - shift)
-  const float2 n = __fadd2_rn(t, make_float2(-ms, -ms)); // round(x - shift) + shift
+  const float2 t = __fadd2_rn(x, make_float2(kMagic, kMagic));
+  const float2 n = __fadd2_rn(t, make_float2(-kMagic, -kMagic));
   const float2 f = __fadd2_rn(x, make_float2(-n.x, -n.y));
-  float2 p;
-  if constexpr (kDeg == 3) {
-    p = __ffma2_rn(make_float2(0.0551716648f, 0.0551716648f), f, make_float2(0.2426111251f, 0.2426111251f));
-    p = __ffma2_rn(p, f, make_float2(0.6932609677f, 0.6932609677f));
-    p = __ffma2_rn(p, f, make_float2(0.9999280572f, 0.9999280572f));
-  } else {
-    p = __ffma2_rn(make_float2(0.23783042f, 0.23783042f), f, make_float2(0.70339652f, 0.70339652f));
-    p = __ffma2_rn(p, f, make_float2(1.0005137f, 1.0005137f));
-  }
+  float2 p = __ffma2_rn(make_float2(0.0551716648f, 0.0551716648f), f, make_float2(0.2426111251f, 0.2426111251f));
+  p = __ffma2_rn(p, f, make_float2(0.6932609677f, 0.6932609677f));
+  p = __ffma2_rn(p, f, make_float2(0.9999280572f, 0.9999280572f));
   float2 r;
   r.x = __int_as_float(__float_as_int(p.x) + (__float_as_int(t.x) << 23));
   r.y = __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23));
@@ -281,108 +284,48 @@ struct KernelArgs {
   float bounded_limit;
 };
 
-constexpr int kKStages = 4;
-constexpr int kVStages = 4;
-#ifndef GCT_POLY_EVERY
-#define GCT_POLY_EVERY 3
-#endif
-constexpr int kPolyEvery = GCT_POLY_EVERY;   // 0: all exponentials on the special-function unit
-#ifndef GCT_FFMA_AHEAD
-#define GCT_FFMA_AHEAD 4
-#endif
-#ifndef GCT_SUM_LAG
-#define GCT_SUM_LAG 2
-#endif
-constexpr int kFfmaAhead = GCT_FFMA_AHEAD;   // software pipeline of the exponential sweep, in pairs of logits
-constexpr int kSumLag = GCT_SUM_LAG;
-#ifndef GCT_MAX_CHAINS
-#define GCT_MAX_CHAINS 4
-#endif
-#ifndef GCT_PV_WAIT_AT
-#define GCT_PV_WAIT_AT 31
-#endif
-constexpr int kPvWaitAt = GCT_PV_WAIT_AT;    // pair (31..61) after which the sweep waits for the previous PV and stores P[0,64)
-constexpr int kMaxChains = GCT_MAX_CHAINS;
-// Bounded mode: pair q of the sweep takes the polynomial when floor((q+1) * NUM / DEN) != floor(q * NUM / DEN),
-// i.e. NUM of every DEN pairs, evenly spread; the rest go to the special-function unit.
-#ifndef GCT_BOUNDED_POLY_NUM
-#define GCT_BOUNDED_POLY_NUM 2
-#endif
-#ifndef GCT_BOUNDED_POLY_DEN
-#define GCT_BOUNDED_POLY_DEN 5
-#endif
-#ifndef GCT_BOUNDED_POLY_DEG
-#define GCT_BOUNDED_POLY_DEG 3
-#endif
-#ifndef GCT_BOUNDED_HALF_AT
-#define GCT_BOUNDED_HALF_AT 30
-#endif
-constexpr int kBoundedPolyNum = GCT_BOUNDED_POLY_NUM, kBoundedPolyDen = GCT_BOUNDED_POLY_DEN;
-constexpr int kBoundedPolyDeg = GCT_BOUNDED_POLY_DEG;
-constexpr int kBoundedHalfAt = GCT_BOUNDED_HALF_AT;   // pair before which the second half of the S row must have landed
-static_assert(kBoundedHalfAt >= 0 && kBoundedHalfAt <= 32, "the second half of the row is needed from pair 32 on");
-// 1: P of a block is announced to the MMA warp as soon as its stores have completed, at the end of the block's
-// iteration; 0: by the next iteration, after it has issued its first S loads (hides the store latency, but the
-// PV product then starts later and its completion is waited for in the middle of the next sweep).
-#ifndef GCT_EARLY_P_FULL
-#define GCT_EARLY_P_FULL 1
-#endif
-// 1: the row reference is subtracted by a fifth K16 step of the S product (Qx Kx^T); 0: by the softmax threads
-// (the reference is then rounded up to an integer, which the polynomial exponentials absorb into their rounding
-// constant for free; only the pairs that go to the special-function unit pay a packed add).
-#ifndef GCT_BOUNDED_FOLD
-#define GCT_BOUNDED_FOLD 1
-#endif
-constexpr bool kBoundedFold = GCT_BOUNDED_FOLD != 0;
-constexpr bool kEarlyPFull = GCT_EARLY_P_FULL != 0;
-// 1: the waits inside the KV loop of the softmax warps end with a warp vote.  The outcome of a wait is the same in
-// every lane without it: the lanes of a converged warp poll one mbarrier phase, one clock and one abort word with the
-// same instructions, so they all see the same values; the vote costs 1.3 % of the kernel and is kept for the waits
-// outside the loop only.
-#ifndef GCT_VOTE_WAITS
-#define GCT_VOTE_WAITS 0
-#endif
-// Register budget at two query tiles per CTA: 384 threads start with 168 registers each (64512 in total);
-// the control warpgroup shrinks to kControlRegs and the two softmax warpgroups grow to kSoftmaxRegs:
-// 128 * kControlRegs + 256 * kSoftmaxRegs <= 64512, both multiples of 8.
-#ifndef GCT_CONTROL_REGS
-#define GCT_CONTROL_REGS 64
-#endif
-#ifndef GCT_SOFTMAX_REGS
-#define GCT_SOFTMAX_REGS 208
-#endif
-constexpr int kControlRegs = GCT_CONTROL_REGS;
-constexpr int kSoftmaxRegs = GCT_SOFTMAX_REGS;
-static_assert(128 * kControlRegs + 256 * kSoftmaxRegs <= 64512, "register pool of the CTA exceeded");   // power of two, independent dependency chains of the row maximum
+constexpr int kFfmaAhead = 4, kSumLag = 2;   // software pipeline of the exponential sweep, in pairs of logits
+// Register budget at two query tiles per CTA: 640 threads start with 96 registers each (61440 in total); the control
+// warpgroup shrinks to kControlRegs and the four softmax warpgroups grow to kSoftmaxRegs:
+// 128 * kControlRegs + 512 * kSoftmaxRegs <= 61440, both multiples of 8.
+constexpr int kControlRegs = 64;
+constexpr int kSoftmaxRegs = 104;      // 112 beside 32 was 2 % slower
+static_assert(128 * kControlRegs + 512 * kSoftmaxRegs <= 61440, "register pool of the CTA exceeded");
 constexpr float kRescaleThreshold = 8.0f;   // in log2 units of the scaled logits
 
-template <int QT>
+// kCtas: CTAs that share an SM (one-tile kernels only), with shorter rings so that two fit.
+template <int QT, int kCtas>
 struct SmemLayout {
+  static constexpr int kKStages = kCtas == 2 ? 2 : 4, kVStages = kCtas == 2 ? 2 : 4;
   static constexpr uint32_t q_off = 0;
   static constexpr uint32_t k_off = q_off + QT * kTileBytes;
   static constexpr uint32_t v_off = k_off + kKStages * kTileBytes;
   // bounded mode (QT == 2): one more 128B-swizzled 128 x 64 tile whose K16 column groups hold the extra operands
   // of the S product: bf16 columns [0,16) Qx of tile 0, [16,32) Qx of tile 1, [32,48) Kx
   static constexpr uint32_t x_off = v_off + kVStages * kTileBytes;
-  static constexpr uint32_t bar_off = x_off + (QT == 2 ? kTileBytes : 0);
-  // barriers: q_full, k_full[KS], k_empty[KS], v_full[VS], v_empty[VS], per tile s_full, s_empty, p_full, pv_full,
-  // then q_ready (bounded mode: Q scaled, Qx and Kx written)
-  static constexpr int n_bars = 1 + 2 * kKStages + 2 * kVStages + 4 * QT + 1;
+  // what the two threads of a row tell each other: [2 (parity of the block)][QT][2 (column half)][128 rows] floats
+  static constexpr uint32_t pair_off = x_off + (QT == 2 ? kTileBytes : 0);
+  static constexpr uint32_t bar_off = pair_off + 2 * QT * 2 * 128 * 4;
+  // barriers: q_full, k_full[KS], k_empty[KS], v_full[VS], v_empty[VS], per tile s_full, s_empty, p_full[2], pv_full[2]
+  // (per column half), then q_ready (bounded mode: Q scaled, Qx and Kx written)
+  static constexpr int n_bars = 1 + 2 * kKStages + 2 * kVStages + 6 * QT + 1;
   static constexpr uint32_t misc_off = bar_off + n_bars * 8;
   static constexpr uint32_t total = misc_off + 16;
 };
 
-// Threads per CTA: the softmax warpgroups plus one control warpgroup slot (producer + QT MMA warps; at
+// Threads per CTA: two softmax warpgroups per query tile plus the control warps (producer + QT MMA warps; at
 // QT == 2 a fourth, idle warp completes the warpgroup so that registers can be moved between
 // warpgroups with setmaxnreg).
 template <int QT>
-constexpr int kThreads = (QT == 2) ? 384 : 192;
+constexpr int kThreads = (QT == 2) ? 640 : 320;
 
-template <int QT, bool kBounded>
-__global__ void __launch_bounds__(kThreads<QT>, 1)
+template <int QT, bool kBounded, int kCtas = 1>
+__global__ void __launch_bounds__(kThreads<QT>, kCtas)
 gct_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const KernelArgs a) {
-  using L = SmemLayout<QT>;
+  using L = SmemLayout<QT, kCtas>;
+  constexpr int kKStages = L::kKStages, kVStages = L::kVStages;
+  static_assert(kCtas == 1 || QT == 1, "two tiles take all of the tensor memory");
   static_assert(!kBounded || QT == 2, "the bounded mode exists for two query tiles per CTA");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -394,19 +337,21 @@ gct_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   auto bar_v_full = [&](int s) { return bars + 8u * (1 + 2 * kKStages + s); };
   auto bar_v_empty = [&](int s) { return bars + 8u * (1 + 2 * kKStages + kVStages + s); };
   constexpr int kTileBars = 1 + 2 * kKStages + 2 * kVStages;
-  auto bar_s_full = [&](int t) { return bars + 8u * (kTileBars + 4 * t + 0); };
-  auto bar_s_empty = [&](int t) { return bars + 8u * (kTileBars + 4 * t + 1); };
-  auto bar_p_full = [&](int t) { return bars + 8u * (kTileBars + 4 * t + 2); };
-  auto bar_pv_full = [&](int t) { return bars + 8u * (kTileBars + 4 * t + 3); };
-  auto bar_q_ready = [&]() { return bars + 8u * (kTileBars + 4 * QT); };
+  auto bar_s_full = [&](int t) { return bars + 8u * (kTileBars + 6 * t + 0); };
+  auto bar_s_empty = [&](int t) { return bars + 8u * (kTileBars + 6 * t + 1); };
+  auto bar_p_full = [&](int t, int half) { return bars + 8u * (kTileBars + 6 * t + 2 + half); };
+  auto bar_pv_full = [&](int t, int half) { return bars + 8u * (kTileBars + 6 * t + 4 + half); };
+  auto bar_q_ready = [&]() { return bars + 8u * (kTileBars + 6 * QT); };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + L::misc_off);
   volatile int* cta_abort = reinterpret_cast<volatile int*>(smem + L::misc_off + 4);
   volatile int* cta_unsafe = reinterpret_cast<volatile int*>(smem + L::misc_off + 8);
 
-  const int warp = threadIdx.x >> 5;
+  // QT == 1: a warp-uniform role index keeps barriers and descriptors in uniform registers (one frame 11.0 us instead of 11.5); at two
+  // tiles the registers it takes cost more than that gives.
+  const int warp = QT == 1 ? __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0) : static_cast<int>(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  constexpr int kProducerWarp = 4 * QT;
-  constexpr int kFirstMmaWarp = 4 * QT + 1;
+  constexpr int kProducerWarp = 8 * QT;
+  constexpr int kFirstMmaWarp = 8 * QT + 1;
   constexpr uint32_t kTmemCols = (QT == 2) ? 512u : 256u;
   constexpr uint32_t kOCol = 128u * QT;
   constexpr uint32_t kPCol = 192u * QT;
@@ -449,11 +394,13 @@ gct_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
     for (int t = 0; t < QT; ++t) {
       mbar_init(bar_s_full(t), 1);
-      mbar_init(bar_s_empty(t), 4);
-      mbar_init(bar_p_full(t), 4);
-      mbar_init(bar_pv_full(t), 1);
+      mbar_init(bar_s_empty(t), 8);
+      for (int half = 0; half < 2; ++half) {
+        mbar_init(bar_p_full(t, half), 4);
+        mbar_init(bar_pv_full(t, half), 1);
+      }
     }
-    mbar_init(bar_q_ready(), 4 * QT);            // one arrival per softmax warp
+    mbar_init(bar_q_ready(), 4 * QT);       // one arrival per warp of the first column half
     *cta_abort = 0;
     *cta_unsafe = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -472,8 +419,8 @@ gct_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();      // everything above is private to the CTA; from here on global memory of earlier kernels is read
 
-  // QT == 2: 384 threads share 64K registers (168 each at launch); the control warpgroup gives most of its
-  // share to the two softmax warpgroups, whose threads hold a whole 128-column S row.
+  // QT == 2: 640 threads share 60K registers (96 each at launch); the control warpgroup gives some of its
+  // share to the softmax warpgroups, whose threads hold half an S row.
   if (warp == kProducerWarp) {
     // =========================== producer ===========================
     if constexpr (QT == 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kControlRegs));
@@ -499,7 +446,7 @@ gct_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         tma_load_4d(sbase + L::v_off + vs * kTileBytes, &tm_v, bar_v_full(vs), 0, h, jb * kBlockN, page);
       }
     }
-  } else if (warp >= kFirstMmaWarp) {
+  } else if (warp > kProducerWarp) {
     // =========================== MMA issuer of tile t ===========================
     if constexpr (QT == 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kControlRegs));
     const int t = warp - kFirstMmaWarp;
@@ -512,17 +459,18 @@ gct_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 #pragma unroll
         for (int k = 0; k < 4; ++k)   // 64 = 4 x K16; +32 B per step inside the 128 B swizzle row
           umma_ss(lead, tmem_base + t * 128, ad + 2 * k, bd + 2 * k, kIdescS, k > 0);
-        if constexpr (kBounded && kBoundedFold) {     // S += Qx_t Kx^T: subtracts the row reference (column groups t and 2 of the x tile)
+        if constexpr (kBounded) {     // S += Qx_t Kx^T: subtracts the row reference (column groups t and 2 of the x tile)
           const uint64_t xd = smem_desc(sbase + L::x_off, 16, 1024);
           umma_ss(lead, tmem_base + t * 128, xd + 2 * t, xd + 4, kIdescS, 1u);
         }
       };
-      auto issue_pv = [&](int vs, uint32_t accumulate) {
+      auto issue_pv = [&](int vs, int half, uint32_t accumulate) {
+        const uint64_t bd = smem_desc(sbase + L::v_off + vs * kTileBytes, 16, 1024);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {   // 128 tokens = 8 x K16: 8 TMEM columns of P and 16 V rows per step
-          const uint64_t bd = smem_desc(sbase + L::v_off + vs * kTileBytes + k * 2048, 16, 1024);
-          umma_ts(lead, tmem_base + kOCol + t * 64, tmem_base + kPCol + t * 64 + k * 8, bd, kIdescPV,
-                  (k > 0) ? 1u : accumulate);
+        for (int k = 0; k < 4; ++k) {   // 64 tokens = 4 x K16: 8 TMEM columns of P and 16 V rows (2 KB) per step
+          const int kk = 4 * half + k;
+          umma_ts(lead, tmem_base + kOCol + t * 64, tmem_base + kPCol + t * 64 + kk * 8, bd + kk * 128, kIdescPV,
+                  (kk > 0) ? 1u : accumulate);
         }
       };
       auto wait = [&](uint32_t bar, uint32_t parity) -> bool {
@@ -535,6 +483,7 @@ gct_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         tc_commit_elected(lead, bar_s_full(t));
         tc_commit_elected(lead, bar_k_empty(0));
       }
+      const bool both = !kBounded || *cta_unsafe != 0;      // a running maximum: see below
       for (int j = 0; ok && j < nblk; ++j) {
         if (j + 1 < nblk) {
           const int ks = (j + 1) % kKStages;
@@ -545,78 +494,95 @@ gct_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           tc_commit_elected(lead, bar_s_full(t));
           tc_commit_elected(lead, bar_k_empty(ks));
         }
+        // The two halves of P come from different warps.  With a fixed reference each half's product starts when that half
+        // is there and frees it when done; with a running maximum the threads of both halves may have rescaled O before.
         const int vs = j % kVStages;
-        if (!(ok = wait(bar_p_full(t), j & 1))) break;
+        if (!(ok = wait(bar_p_full(t, 0), j & 1))) break;
+        if (both && !(ok = wait(bar_p_full(t, 1), j & 1))) break;
         if (!(ok = wait(bar_v_full(vs), (j / kVStages) & 1))) break;
         tc_fence_after();
-        issue_pv(vs, j > 0 ? 1u : 0u);
-        tc_commit_elected(lead, bar_pv_full(t));
+        issue_pv(vs, 0, j > 0 ? 1u : 0u);
+        if (!both) {
+          tc_commit_elected(lead, bar_pv_full(t, 0));
+          if (!(ok = wait(bar_p_full(t, 1), j & 1))) break;
+          tc_fence_after();
+        }
+        issue_pv(vs, 1, 1u);
+        tc_commit_elected(lead, bar_pv_full(t, 1));
         tc_commit_elected(lead, bar_v_empty(vs));
       }
     }
   } else {
     // =========================== softmax ===========================
     if constexpr (QT == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
-    const int t = warp >> 2;                       // query tile of this warp
+    const int t = warp >> 3;                       // query tile of this warp
+    const int half = (warp >> 2) & 1;              // its 64 of the 128 columns of S, and its 32 of the 64 columns of O
     const int row = ((warp & 3) << 5) | lane;      // row inside the tile == TMEM lane
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) << 5) << 16;
-    const uint32_t s_addr = tmem_base + lane_addr + t * 128;
-    const uint32_t o_addr = tmem_base + lane_addr + kOCol + t * 64;
-    const uint32_t p_addr = tmem_base + lane_addr + kPCol + t * 64;
+    const uint32_t s_addr = tmem_base + lane_addr + t * 128 + half * 64;
+    const uint32_t o_addr = tmem_base + lane_addr + kOCol + t * 64 + half * 32;
+    const uint32_t p_addr = tmem_base + lane_addr + kPCol + t * 64 + half * 32;
+    const uint32_t pair_mine = sbase + L::pair_off + (2 * t + half) * 512 + row * 4;
+    const uint32_t pair_other = sbase + L::pair_off + (2 * t + (half ^ 1)) * 512 + row * 4;
+    const int pair_bar = 1 + 4 * t + (warp & 3);    // named barrier of this warp and the one with the other half of its rows
     const float c = kBounded ? 1.f : a.scale_log2;  // bounded mode: the Q tile already carries scale * log2(e)
-    float m = -INFINITY, l = 0.f;                   // m: reference maximum (raw logit units)
+    const uint32_t lead = lane == 0 ? 1u : 0u;
+    float m = -INFINITY, l = 0.f;                   // m: reference maximum (raw logit units); l: sum over this half
     float ref_fixed = 0.f;                          // bounded mode: upper bound of this row's exponents
     bool ok = true;
     bool running_max = false;                       // bounded kernel: this CTA fell back to the running maximum
-    // waits whose outcome the whole warp shares (the tcgen05 loads and stores that follow are warp-wide): with a
-    // vote outside the KV loop, by construction inside it (see GCT_VOTE_WAITS)
+    // Waits whose outcome the whole warp shares (the tcgen05 loads and stores that follow are warp-wide): with a
+    // vote outside the KV loop.  Inside it the outcome is the same in every lane without one: the lanes of a converged warp poll
+    // one mbarrier phase, one clock and one abort word with the same instructions.
     auto wait_v = [&](uint32_t bar, uint32_t parity) -> bool {
       return __all_sync(0xffffffffu, mbar_wait(bar, parity, cta_abort, a.status));
     };
-    auto wait_u = [&](uint32_t bar, uint32_t parity) -> bool {
-#if GCT_VOTE_WAITS
-      return __all_sync(0xffffffffu, mbar_wait(bar, parity, cta_abort, a.status));
-#else
-      return mbar_wait(bar, parity, cta_abort, a.status);
-#endif
+    auto wait_u = [&](uint32_t bar, uint32_t parity) -> bool { return mbar_wait(bar, parity, cta_abort, a.status); };
+    // The other thread's value.  Every warp meets its partner here once per KV block, also when its
+    // waits have failed (see `met` below), so that neither waits for one that has left.
+    auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory"); };
+    auto pair_exchange = [&](float x, uint32_t slot) -> float {
+      asm volatile("st.shared.f32 [%0], %1;" ::"r"(pair_mine + slot), "f"(x) : "memory");
+      pair_sync();
+      float y;
+      asm volatile("ld.shared.f32 %0, [%1];" : "=f"(y) : "r"(pair_other + slot) : "memory");
+      return y;
     };
+    constexpr uint32_t kPairSlot = QT * 2 * 128 * 4;   // slots alternate: a slow reader of one block's value and the writer of the next's
 
     if constexpr (kBounded) {
       // ---- once per CTA: scale the Q row in place, derive its reference, write Qx and Kx ----
-      ok = wait_v(bar_q_full(), 0);
       const uint32_t q_row = sbase + L::q_off + t * kTileBytes + row * 128;
       const uint32_t swz = static_cast<uint32_t>(row & 7);
-      float sq = 0.f;
-      if (ok) {
-        const float cs = a.scale_log2;
+      if (half == 0) {
+        ok = wait_v(bar_q_full(), 0);
+        float sq = 0.f;
+        if (ok) {
+          const float cs = a.scale_log2;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {              // 16-byte chunk j of the row sits at chunk j ^ (row & 7)
-          const uint32_t addr = q_row + ((static_cast<uint32_t>(j) ^ swz) << 4);
-          uint32_t w[4];
-          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(addr));
+          for (int j = 0; j < 8; ++j) {              // 16-byte chunk j of the row sits at chunk j ^ (row & 7)
+            const uint32_t addr = q_row + ((static_cast<uint32_t>(j) ^ swz) << 4);
+            uint32_t w[4];
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(addr));
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float lo = __uint_as_float(w[i] << 16) * cs, hi = __uint_as_float(w[i] & 0xffff0000u) * cs;
-            w[i] = pack_bf16x2(lo, hi);
-            const float rlo = __uint_as_float(w[i] << 16), rhi = __uint_as_float(w[i] & 0xffff0000u);
-            sq = fmaf(rlo, rlo, fmaf(rhi, rhi, sq));
+            for (int i = 0; i < 4; ++i) {
+              const float lo = __uint_as_float(w[i] << 16) * cs, hi = __uint_as_float(w[i] & 0xffff0000u) * cs;
+              w[i] = pack_bf16x2(lo, hi);
+              const float rlo = __uint_as_float(w[i] << 16), rhi = __uint_as_float(w[i] & 0xffff0000u);
+              sq = fmaf(rlo, rlo, fmaf(rhi, rhi, sq));
+            }
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
           }
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+          // rounded up to bf16 (the precision of the Qx operand) so that the value used is still an upper bound
+          const float ref = sqrtf(sq) * __ldg(a.key_norm_max + h);
+          if (!(ref <= a.bounded_limit)) *cta_unsafe = 1;            // too loose, infinite or NaN
+          ref_fixed = __uint_as_float((__float_as_uint(ref) + 0xffffu) & 0xffff0000u);
         }
-        // rounded up to bf16 (the precision of the Qx operand) so that the value used is still an upper bound
-        const float ref = sqrtf(sq) * __ldg(a.key_norm_max + h);
-        if (!(ref <= a.bounded_limit)) *cta_unsafe = 1;            // too loose, infinite or NaN
-        ref_fixed = kBoundedFold ? __uint_as_float((__float_as_uint(ref) + 0xffffu) & 0xffff0000u) : ceilf(ref);
       }
-      asm volatile("bar.sync 1, %0;" ::"n"(128 * QT) : "memory");   // all softmax threads, also after a failed wait
+      asm volatile("bar.sync 15, %0;" ::"n"(256 * QT) : "memory");   // all softmax threads, also after a failed wait
       running_max = *cta_unsafe != 0;
       if (running_max) ref_fixed = 0.f;
-      if (ok && !kBoundedFold) {
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the scaled Q rows -> tensor-core reads
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar_q_ready());
-      }
-      if (ok && kBoundedFold) {
+      if (half == 0 && ok) {
         const uint32_t x_row = sbase + L::x_off + row * 128;
         const uint32_t negref = running_max ? 0u : ((__float_as_uint(ref_fixed) >> 16) | 0x8000u);
         auto st_chunk = [&](int j, uint32_t first) {
@@ -634,55 +600,56 @@ gct_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (lane == 0) mbar_arrive(bar_q_ready());
       }
     }
-    uint32_t s[128];
 
-    int pi = g0 / a.blocks_per_page;               // page and block-in-page of block j, advanced incrementally
-    int jb = g0 - pi * a.blocks_per_page;
+    // Only the last block of a page can hold fewer than 128 tokens: `left` counts the blocks of the page from the current one on.
+    int pi = g0 / a.blocks_per_page;
+    auto blocks_of = [&](int page) { return page == a.n_pages - 1 ? a.total_blocks - page * a.blocks_per_page : a.blocks_per_page; };
+    int left = blocks_of(pi) - (g0 - pi * a.blocks_per_page);
+    auto tail_valid = [&]() -> int {               // valid tokens among this thread's 64 of a page's last block; on to the next page
+      const int valid = (pi == a.n_pages - 1 ? a.last_page_len : a.page_len) - (blocks_of(pi) - 1) * kBlockN - 64 * half;
+      left = blocks_of(++pi);
+      return valid;
+    };
+    int met = 0;                                   // KV blocks whose pair exchange this warp has taken part in
     if (kBounded && running_max) {
-      // ---- fallback of the bounded kernel: two passes over the S row in TMEM, 32 columns at a time ----
+      // ---- fallback of the bounded kernel: two passes over the half row in TMEM, 32 columns at a time ----
       // pass 1 takes the masked row maximum, pass 2 exponentiates against the running maximum (moved only when the
       // row maximum outgrows it by 2^kRescaleThreshold) and stores P; compact rather than fast.
       for (int j = 0; ok && j < nblk; ++j) {
         if (!(ok = wait_v(bar_s_full(t), j & 1))) break;
         tc_fence_after();
-        const int plen = (pi == a.n_pages - 1) ? a.last_page_len : a.page_len;
-        const int valid = min(kBlockN, plen - jb * kBlockN);
-        if (++jb == a.blocks_per_page) {
-          jb = 0;
-          ++pi;
-        }
+        const int valid = --left == 0 ? tail_valid() : 64;
         uint32_t r[32];
         float mx = -INFINITY;
 #pragma unroll 1
-        for (int ch = 0; ch < 4; ++ch) {
+        for (int ch = 0; ch < 2; ++ch) {
           tmem_ld32(s_addr + 32 * ch, r);
           tmem_wait_ld();
 #pragma unroll
           for (int i = 0; i < 32; ++i)
             if (32 * ch + i < valid) mx = fmaxf(mx, __uint_as_float(r[i]));
         }
+        mx = fmaxf(mx, pair_exchange(mx, (j & 1) * kPairSlot));
+        ++met;
         float alpha = 1.f;
         if (mx - m > kRescaleThreshold) {            // always true on the first block (m = -inf)
           alpha = fast_exp2(m - mx);
           m = mx;
         }
         if (j > 0) {
-          if (!(ok = wait_v(bar_pv_full(t), (j - 1) & 1))) break;
+          if (!(ok = wait_v(bar_pv_full(t, 1), (j - 1) & 1))) break;
           tc_fence_after();
           if (__any_sync(0xffffffffu, alpha != 1.f)) {
-#pragma unroll 1
-            for (int hh = 0; hh < 2; ++hh) {
-              tmem_ld32(o_addr + hh * 32, r);
-              tmem_wait_ld();
+            tmem_ld32(o_addr, r);
+            tmem_wait_ld();
 #pragma unroll
-              for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-              tmem_st32(o_addr + hh * 32, r);
-            }
+            for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
+            tmem_st32(o_addr, r);
           }
         }
         float sum = 0.f;
 #pragma unroll 1
-        for (int ch = 0; ch < 4; ++ch) {
+        for (int ch = 0; ch < 2; ++ch) {
           tmem_ld32(s_addr + 32 * ch, r);
           tmem_wait_ld();
           uint32_t pk16[16];
@@ -702,256 +669,160 @@ gct_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         __syncwarp();
         if (lane == 0) {
           mbar_arrive(bar_s_empty(t));               // S was read twice: only now may the next block overwrite it
-          mbar_arrive(bar_p_full(t));
+          mbar_arrive(bar_p_full(t, half));
         }
       }
-    } else
-    for (int j = 0; ok && j < nblk; ++j) {
-      if (!(ok = wait_u(bar_s_full(t), j & 1))) break;
-      tc_fence_after();
-      // valid tokens of this block
-      const int plen = (pi == a.n_pages - 1) ? a.last_page_len : a.page_len;
-      const int valid = min(kBlockN, plen - jb * kBlockN);
-      if (++jb == a.blocks_per_page) {
-        jb = 0;
-        ++pi;
-      }
-      // keys past the valid length: -inf (exp2 gives 0); bounded mode: an exponent the polynomial can take
-      // (without the fold the reference is still to be subtracted from it)
-      const uint32_t kMaskBits = !kBounded ? 0xff800000u : (kBoundedFold ? 0xc2fc0000u /* -126.f */ : __float_as_uint(ref_fixed - 126.f));
-      // masked maximum of s[lo, lo+64): four independent chains of 3-input max
-      auto half_max = [&](int lo) -> float {
-        if (valid < lo + 64) {
+      __syncwarp();
+      for (; met < nblk; ++met) pair_sync();
+    } else {
+      for (int j = 0; ok && j < nblk; ++j) {
+        if (!(ok = wait_u(bar_s_full(t), j & 1))) break;
+        tc_fence_after();
+        uint32_t s[64], pk[32];
+        tmem_ld32(s_addr, *reinterpret_cast<uint32_t(*)[32]>(&s[0]));
+        tmem_ld32(s_addr + 32, *reinterpret_cast<uint32_t(*)[32]>(&s[32]));
+        tmem_wait_ld();
+        // the S tile is in registers: the tensor core may overwrite it with the next block
+        tc_fence_before();
+        __syncwarp();
+        mbar_arrive_elected(lead, bar_s_empty(t));
+        if (--left == 0) {
+          const int valid = tail_valid();
+          if (valid < 64) {
+            // keys past the valid length: -inf (exp2 gives 0); bounded mode: an exponent the polynomial can take, -126
+            constexpr uint32_t kMaskBits = kBounded ? 0xc2fc0000u : 0xff800000u;
 #pragma unroll
-          for (int i = 0; i < 64; ++i)
-            if (lo + i >= valid) s[lo + i] = kMaskBits;
-        }
-        if constexpr (kBounded) {
-          return 0.f;                             // the reference is fixed: only the masking above is needed
-        } else {
-        // kMaxChains independent chains of 3-input max, merged by a tree at the end
-        float mxc[kMaxChains];
-#pragma unroll
-        for (int ch = 0; ch < kMaxChains; ++ch) mxc[ch] = __uint_as_float(s[lo + ch]);
-        constexpr int kRounds = (64 - kMaxChains) / (2 * kMaxChains);   // full rounds of one max3 per chain
-#pragma unroll
-        for (int r = 0; r < kRounds; ++r)
-#pragma unroll
-          for (int ch = 0; ch < kMaxChains; ++ch) {
-            const int i = kMaxChains + 2 * (r * kMaxChains + ch);
-            mxc[ch] = max3(mxc[ch], __uint_as_float(s[lo + i]), __uint_as_float(s[lo + i + 1]));
-          }
-        {
-          constexpr int kDone = kMaxChains + 2 * kRounds * kMaxChains;   // elements consumed so far
-#pragma unroll
-          for (int i = kDone; i < 64; i += 2) {
-            const int ch = ((i - kDone) / 2) % kMaxChains;
-            mxc[ch] = max3(mxc[ch], __uint_as_float(s[lo + i]), __uint_as_float(s[lo + i + 1]));
-          }
-        }
-#pragma unroll
-        for (int w = kMaxChains / 2; w >= 1; w /= 2)
-#pragma unroll
-          for (int ch = 0; ch < w; ++ch) mxc[ch] = fmaxf(mxc[ch], mxc[ch + w]);
-        return mxc[0];
-        }
-      };
-      // the second half of the row is still arriving from TMEM while the first half is reduced
-      float mx;
-      {
-        uint32_t(&s0)[32] = *reinterpret_cast<uint32_t(*)[32]>(&s[0]);
-        uint32_t(&s1)[32] = *reinterpret_cast<uint32_t(*)[32]>(&s[32]);
-        uint32_t(&s2)[32] = *reinterpret_cast<uint32_t(*)[32]>(&s[64]);
-        uint32_t(&s3)[32] = *reinterpret_cast<uint32_t(*)[32]>(&s[96]);
-        tmem_ld32(s_addr, s0);
-        tmem_ld32(s_addr + 32, s1);
-        if (j > 0 && !(kBounded && kEarlyPFull)) {
-          // P of the previous block: its stores completed while the loads above were issued
-          tmem_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar_p_full(t));
-        }
-        if constexpr (kBounded && kBoundedHalfAt == 0) {
-          // the whole row at once (a row takes under a hundred clocks to arrive): S is released right away
-          tmem_ld32(s_addr + 64, s2);
-          tmem_ld32(s_addr + 96, s3);
-          tmem_wait_ld();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar_s_empty(t));
-          if (valid < 128) {
-#pragma unroll
-            for (int i = 64; i < 128; ++i)
+            for (int i = 0; i < 64; ++i)
               if (i >= valid) s[i] = kMaskBits;
           }
-        } else {
-          tmem_wait_ld();
-          tmem_ld32(s_addr + 64, s2);
-          tmem_ld32(s_addr + 96, s3);
         }
-        const float mlo = half_max(0);
+        float alpha = 1.f;
         if constexpr (!kBounded) {
-          tmem_wait_ld();
-          // the S tile is in registers: the tensor core may overwrite it with the next block
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar_s_empty(t));
-          mx = fmaxf(mlo, half_max(64));
-        } else {
-          mx = mlo;                                // unused: the second half is masked after its load, inside the sweep
+          // four independent chains of 3-input max, merged by a tree at the end
+          float mxc[4];
+#pragma unroll
+          for (int ch = 0; ch < 4; ++ch) mxc[ch] = __uint_as_float(s[ch]);
+#pragma unroll
+          for (int i = 4; i < 64; i += 2) mxc[(i >> 1) & 3] = max3(mxc[(i >> 1) & 3], __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
+          float mx = fmaxf(fmaxf(mxc[0], mxc[1]), fmaxf(mxc[2], mxc[3]));
+          mx = fmaxf(mx, pair_exchange(mx, (j & 1) * kPairSlot));
+          ++met;
+          // move the reference maximum only when the row maximum outgrew it by more than 2^kRescaleThreshold;
+          // until then exponentials stay below 2^8 and every sum remains exact enough in fp32
+          if ((mx - m) * c > kRescaleThreshold) {      // always true on the first block (m = -inf)
+            alpha = fast_exp2((m - mx) * c);           // exp2(-inf) = 0 on the first block
+            m = mx;
+          }
         }
-      }
-      // move the reference maximum only when the row maximum outgrew it by more than 2^kRescaleThreshold;
-      // until then exponentials stay below 2^8 and every sum remains exact enough in fp32
-      float alpha = 1.f;
-      if constexpr (!kBounded) {
-        if ((mx - m) * c > kRescaleThreshold) {      // always true on the first block (m = -inf)
-          alpha = fast_exp2((m - mx) * c);           // exp2(-inf) = 0 on the first block
-          m = mx;
+        const float mc = m * c;                        // bounded mode: unused, the tensor core already subtracted ref
+        // P = exp2(S*c - m*c), software-pipelined over pairs of logits so that the exponentials (the scarce
+        // pipe) are interleaved with independent work: pair p+4 gets its packed FFMA, pair p its two EX2,
+        // pair p-2 its packed add into the row sum and its bf16 conversion (two K values per TMEM column).
+        // Bounded mode: S already is the exponent, the packed FFMA is gone.
+        const float2 c2 = make_float2(c, c), nmc2 = make_float2(-mc, -mc);
+        float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
+        auto pair_ffma = [&](int q) {
+          if constexpr (!kBounded) {
+            const float2 x = __ffma2_rn(make_float2(__uint_as_float(s[2 * q]), __uint_as_float(s[2 * q + 1])), c2, nmc2);
+            s[2 * q] = __float_as_uint(x.x);
+            s[2 * q + 1] = __float_as_uint(x.y);
+          }
+        };
+        auto pair_exp = [&](int q) {
+          // Some pairs are exponentiated on the FMA pipe: the special-function unit delivers only 16 results per
+          // clock and SM, half of what the tensor core consumes at head_dim 64.  kNum of kDen pairs, evenly spread: bounded mode, back to
+          // back at 600 KV blocks, 2 of 5 385 us, 3 of 8 389, 1 of 3 387, 3 of 7 389, 1 of 4 401; running maximum at two tiles (one
+          // more packed FMA per pair, and two clamps for the polynomial), 6264 x 6264, 2 of 7 224 us, 1 of 4 226, 1 of 3 228, 2 of 5 235;
+          // at one tile 1 of 3 (8 x 1005 x 1005 60.3 us, 2 of 7 61.3).
+          constexpr int kNum = kBounded || QT == 2 ? 2 : 1, kDen = kBounded ? 5 : QT == 2 ? 7 : 3;
+          if (((q + 1) * kNum) / kDen != (q * kNum) / kDen) {
+            const float2 x = make_float2(__uint_as_float(s[2 * q]), __uint_as_float(s[2 * q + 1]));
+            const float2 e = kBounded ? exp2_poly2_inrange(x) : exp2_poly2(x);
+            s[2 * q] = __float_as_uint(e.x);
+            s[2 * q + 1] = __float_as_uint(e.y);
+          } else {
+            s[2 * q] = __float_as_uint(fast_exp2(__uint_as_float(s[2 * q])));
+            s[2 * q + 1] = __float_as_uint(fast_exp2(__uint_as_float(s[2 * q + 1])));
+          }
+        };
+        auto pair_sum = [&](int q) {
+          const float2 e = make_float2(__uint_as_float(s[2 * q]), __uint_as_float(s[2 * q + 1]));
+          if (q & 1) acc1 = __fadd2_rn(acc1, e); else acc0 = __fadd2_rn(acc0, e);
+          pk[q] = pack_bf16x2(e.x, e.y);
+        };
+#pragma unroll
+        for (int q = 0; q < kFfmaAhead; ++q) pair_ffma(q);
+#pragma unroll
+        for (int q = 0; q < 32; ++q) {
+          if (q + kFfmaAhead < 32) pair_ffma(q + kFfmaAhead);
+          pair_exp(q);
+          if (q >= kSumLag) pair_sum(q - kSumLag);
         }
-      }
-      const float mc = m * c;                        // bounded mode: unused, the tensor core already subtracted ref
-
-      // P (and O) of this tile are free once the PV product of the previous block has completed.  The wait
-      // sits in the middle of the exponential sweep, right before the first store of P, so that the
-      // round trip softmax -> MMA warp -> tensor core -> mbarrier hides under the first half of the sweep.
-      auto wait_prev_pv_and_rescale = [&]() -> bool {
+#pragma unroll
+        for (int q = 32 - kSumLag; q < 32; ++q) pair_sum(q);
+        l = fmaf(l, alpha, (acc0.x + acc0.y) + (acc1.x + acc1.y));
+        // P (and O) of this tile are free once the PV product of the previous block has completed
         if (j > 0) {
-          if (!wait_u(bar_pv_full(t), (j - 1) & 1)) return false;
+          if (!(ok = wait_u(bar_pv_full(t, kBounded ? half : 1), (j - 1) & 1))) break;
           tc_fence_after();
-          if (!kBounded && __any_sync(0xffffffffu, alpha != 1.f)) {   // rare: rescale this warp's 32 rows of O in TMEM
+          if (!kBounded && __any_sync(0xffffffffu, alpha != 1.f)) {   // rare: rescale this warp's part of O in TMEM
             uint32_t ob[32];
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-              tmem_ld32(o_addr + hh * 32, ob);
-              tmem_wait_ld();
-#pragma unroll
-              for (int i = 0; i < 32; ++i) ob[i] = __float_as_uint(__uint_as_float(ob[i]) * alpha);
-              tmem_st32(o_addr + hh * 32, ob);
-            }
-          }
-        }
-        return true;
-      };
-      // P = exp2(S*c - m*c), software-pipelined over pairs of logits so that the exponentials (the scarce
-      // pipe) are interleaved with independent work: pair p+4 gets its packed FFMA, pair p its two EX2,
-      // pair p-2 its packed add into the row sum and its bf16 conversion (two K values per TMEM column).
-      // Bounded mode: S already is the exponent, the packed FFMA is gone.
-      const float2 c2 = make_float2(c, c), nmc2 = make_float2(-mc, -mc);
-      float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
-      uint32_t pk[kPvWaitAt > 31 ? 64 : 32];
-      auto pair_ffma = [&](int q) {
-        if constexpr (!kBounded) {
-          const float2 x = __ffma2_rn(make_float2(__uint_as_float(s[2 * q]), __uint_as_float(s[2 * q + 1])), c2, nmc2);
-          s[2 * q] = __float_as_uint(x.x);
-          s[2 * q + 1] = __float_as_uint(x.y);
-        }
-      };
-      auto pair_exp = [&](int q) {
-        // some pairs are exponentiated on the FMA pipe: the special-function unit delivers only 16 results per
-        // clock and SM, half of what the tensor core consumes at head_dim 64
-        const bool poly = kBounded ? ((q + 1) * kBoundedPolyNum) / kBoundedPolyDen != (q * kBoundedPolyNum) / kBoundedPolyDen
-                                   : (kPolyEvery > 0 && (q % (kPolyEvery > 0 ? kPolyEvery : 1)) == (kPolyEvery - 1));
-        if (poly) {
-          const float2 x = make_float2(__uint_as_float(s[2 * q]), __uint_as_float(s[2 * q + 1]));
-          float2 e;
-          if constexpr (kBounded) e = exp2_poly2_inrange<kBoundedPolyDeg>(x, kBoundedFold ? 0.f : ref_fixed);   // exponents lie in [-126, 1]
-          else e = exp2_poly2(x);
-          s[2 * q] = __float_as_uint(e.x);
-          s[2 * q + 1] = __float_as_uint(e.y);
-        } else if constexpr (kBounded && !kBoundedFold) {
-          const float2 y = __fadd2_rn(make_float2(__uint_as_float(s[2 * q]), __uint_as_float(s[2 * q + 1])),
-                                      make_float2(-ref_fixed, -ref_fixed));
-          s[2 * q] = __float_as_uint(fast_exp2(y.x));
-          s[2 * q + 1] = __float_as_uint(fast_exp2(y.y));
-        } else {
-          s[2 * q] = __float_as_uint(fast_exp2(__uint_as_float(s[2 * q])));
-          s[2 * q + 1] = __float_as_uint(fast_exp2(__uint_as_float(s[2 * q + 1])));
-        }
-      };
-      auto pair_sum = [&](int q) {
-        const float2 e = make_float2(__uint_as_float(s[2 * q]), __uint_as_float(s[2 * q + 1]));
-        if (q & 1) acc1 = __fadd2_rn(acc1, e); else acc0 = __fadd2_rn(acc0, e);
-        pk[kPvWaitAt > 31 ? q : (q & 31)] = pack_bf16x2(e.x, e.y);
-      };
-#pragma unroll
-      for (int q = 0; q < kFfmaAhead; ++q) pair_ffma(q);
-#pragma unroll
-      for (int q = 0; q < 64; ++q) {
-        if constexpr (kBounded) {
-          // bounded mode needs no row maximum: the second half of the S row arrives under the first half of the sweep
-          if (kBoundedHalfAt > 0 && q == kBoundedHalfAt) {
+            tmem_ld32(o_addr, ob);
             tmem_wait_ld();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_s_empty(t));
-            if (valid < 128) {
 #pragma unroll
-              for (int i = 64; i < 128; ++i)
-                if (i >= valid) s[i] = kMaskBits;
-            }
+            for (int i = 0; i < 32; ++i) ob[i] = __float_as_uint(__uint_as_float(ob[i]) * alpha);
+            tmem_st32(o_addr, ob);
           }
         }
-        if (q + kFfmaAhead < 64) pair_ffma(q + kFfmaAhead);
-        pair_exp(q);
-        if (q >= kSumLag) {
-          pair_sum(q - kSumLag);
-          if (q - kSumLag == kPvWaitAt) {               // at least the first 64 keys are done
-            ok = wait_prev_pv_and_rescale();
-            if (ok) tmem_st32(p_addr, *reinterpret_cast<uint32_t(*)[32]>(&pk[0]));
-          }
-        }
-      }
-#pragma unroll
-      for (int q = 64 - kSumLag; q < 64; ++q) pair_sum(q);
-      if (!ok) break;
-      tmem_st32(p_addr + 32, *reinterpret_cast<uint32_t(*)[32]>(&pk[kPvWaitAt > 31 ? 32 : 0]));
-      const float rs0 = acc0.x, rs1 = acc0.y, rs2 = acc1.x, rs3 = acc1.y;
-      l = fmaf(l, alpha, (rs0 + rs1) + (rs2 + rs3));
-      if (j + 1 == nblk || (kBounded && kEarlyPFull)) {   // otherwise the next iteration announces P after its first loads
+        tmem_st32(p_addr, pk);
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar_p_full(t));
+        mbar_arrive_elected(lead, bar_p_full(t, half));
+      }
+      if constexpr (!kBounded) {
+        __syncwarp();
+        for (; met < nblk; ++met) pair_sync();
       }
     }
 
     // ---- epilogue: O / l ----
-    if (ok && nblk > 0) ok = wait_v(bar_pv_full(t), (nblk - 1) & 1);
+    if (ok && nblk > 0) ok = wait_v(bar_pv_full(t, 1), (nblk - 1) & 1);
+    {
+      // in the order of the columns; not the slot of the last block: the partner may still be reading that
+      const float other = pair_exchange(l, (nblk & 1) * kPairSlot);
+      l = half == 0 ? l + other : other + l;
+    }
     const int qrow = (qg * QT + t) * kTileM + row;
     if (ok && nblk > 0) {
       tc_fence_after();
+      uint32_t ob[32];
+      tmem_ld32(o_addr, ob);      // warp-wide: every lane takes part, also rows past n_q
+      tmem_wait_ld();
       const float inv = 1.f / l;
       const size_t rowidx = (static_cast<size_t>(b) * a.n_q + (qrow < a.n_q ? qrow : 0)) * a.heads + h;
       const size_t prow = static_cast<size_t>(split) * a.batch * a.n_q * a.heads + rowidx;
+      if (qrow < a.n_q) {
+        if (a.final_bf16) {
+          uint4* dst = reinterpret_cast<uint4*>(a.out + rowidx * kHeadDim + half * 32);
 #pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {
-        uint32_t ob[32];
-        tmem_ld32(o_addr + hh * 32, ob);      // warp-wide: every lane takes part, also rows past n_q
-        tmem_wait_ld();
-        if (qrow < a.n_q) {
-          if (a.final_bf16) {
-            uint4* dst = reinterpret_cast<uint4*>(a.out + rowidx * kHeadDim + hh * 32);
-#pragma unroll
-            for (int q4 = 0; q4 < 4; ++q4) {
-              uint4 w;
-              w.x = pack_bf16x2(__uint_as_float(ob[q4 * 8 + 0]) * inv, __uint_as_float(ob[q4 * 8 + 1]) * inv);
-              w.y = pack_bf16x2(__uint_as_float(ob[q4 * 8 + 2]) * inv, __uint_as_float(ob[q4 * 8 + 3]) * inv);
-              w.z = pack_bf16x2(__uint_as_float(ob[q4 * 8 + 4]) * inv, __uint_as_float(ob[q4 * 8 + 5]) * inv);
-              w.w = pack_bf16x2(__uint_as_float(ob[q4 * 8 + 6]) * inv, __uint_as_float(ob[q4 * 8 + 7]) * inv);
-              dst[q4] = w;
-            }
-          } else {
-            float4* dst = reinterpret_cast<float4*>(a.part_o + prow * kHeadDim + hh * 32);
-#pragma unroll
-            for (int q4 = 0; q4 < 8; ++q4)
-              dst[q4] = make_float4(__uint_as_float(ob[q4 * 4 + 0]) * inv, __uint_as_float(ob[q4 * 4 + 1]) * inv,
-                                    __uint_as_float(ob[q4 * 4 + 2]) * inv, __uint_as_float(ob[q4 * 4 + 3]) * inv);
+          for (int q4 = 0; q4 < 4; ++q4) {
+            uint4 w;
+            w.x = pack_bf16x2(__uint_as_float(ob[q4 * 8 + 0]) * inv, __uint_as_float(ob[q4 * 8 + 1]) * inv);
+            w.y = pack_bf16x2(__uint_as_float(ob[q4 * 8 + 2]) * inv, __uint_as_float(ob[q4 * 8 + 3]) * inv);
+            w.z = pack_bf16x2(__uint_as_float(ob[q4 * 8 + 4]) * inv, __uint_as_float(ob[q4 * 8 + 5]) * inv);
+            w.w = pack_bf16x2(__uint_as_float(ob[q4 * 8 + 6]) * inv, __uint_as_float(ob[q4 * 8 + 7]) * inv);
+            dst[q4] = w;
           }
+        } else {
+          float4* dst = reinterpret_cast<float4*>(a.part_o + prow * kHeadDim + half * 32);
+#pragma unroll
+          for (int q4 = 0; q4 < 8; ++q4)
+            dst[q4] = make_float4(__uint_as_float(ob[q4 * 4 + 0]) * inv, __uint_as_float(ob[q4 * 4 + 1]) * inv,
+                                  __uint_as_float(ob[q4 * 4 + 2]) * inv, __uint_as_float(ob[q4 * 4 + 3]) * inv);
         }
       }
-      if (qrow < a.n_q && !a.final_bf16)
+      if (qrow < a.n_q && half == 0 && !a.final_bf16)
         a.part_lse[prow] = (((kBounded && !running_max) ? ref_fixed : m * c) + log2f(l)) * 0.6931471805599453f;
     }
   }
@@ -971,8 +842,8 @@ gct_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
 }  // namespace
 
-int attention_smem_bytes(int qt) {
-  return static_cast<int>((qt == 2 ? SmemLayout<2>::total : SmemLayout<1>::total) + 1024);
+int attention_smem_bytes(int qt, int ctas_per_sm) {
+  return static_cast<int>((qt == 2 ? SmemLayout<2, 1>::total : ctas_per_sm == 2 ? SmemLayout<1, 2>::total : SmemLayout<1, 1>::total) + 1024);
 }
 
 // The kernels need more dynamic shared memory than the default limit; the opt-in is a per-device attribute of each
@@ -988,10 +859,18 @@ int opt_in_shared_memory() {
   if (dev < 0 || dev >= kMaxDevices) return fail(GCT_ERR_INVALID, "attention: device ordinal out of range");
   std::lock_guard<std::mutex> lock(g_attr_mutex);
   if (!g_attr_set[dev]) {
-    const int s2 = attention_smem_bytes(2), s1 = attention_smem_bytes(1);
+    const int s2 = attention_smem_bytes(2, 1), s1 = attention_smem_bytes(1, 1), s12 = attention_smem_bytes(1, 2);
     GCT_CUDA_CHECK(cudaFuncSetAttribute(gct_attn_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, s2));
     GCT_CUDA_CHECK(cudaFuncSetAttribute(gct_attn_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, s2));
     GCT_CUDA_CHECK(cudaFuncSetAttribute(gct_attn_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, s1));
+    GCT_CUDA_CHECK(cudaFuncSetAttribute(gct_attn_kernel<1, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, s12));
+    // setmaxnreg hands out no more registers than the CTA was launched with and waits for ever for the rest: never launch such a build
+    for (const void* f : {reinterpret_cast<const void*>(&gct_attn_kernel<2, false>), reinterpret_cast<const void*>(&gct_attn_kernel<2, true>)}) {
+      cudaFuncAttributes attr;
+      GCT_CUDA_CHECK(cudaFuncGetAttributes(&attr, f));
+      if (attr.numRegs * kThreads<2> < 128 * kControlRegs + 512 * kSoftmaxRegs)
+        return fail(GCT_ERR_INVALID, "attention: the kernel was built with fewer registers than its warpgroups share");
+    }
     g_attr_set[dev] = true;
   }
   return GCT_OK;
@@ -1003,6 +882,7 @@ int launch_attention(const AttnLaunch& a, cudaStream_t stream) {
       a.last_page_len > a.page_len)
     return fail(GCT_ERR_INVALID, "attention: bad shape");
   if (a.q_tiles_per_cta != 1 && a.q_tiles_per_cta != 2) return fail(GCT_ERR_INVALID, "attention: q_tiles_per_cta");
+  if (a.ctas_per_sm != 1 && !(a.ctas_per_sm == 2 && a.q_tiles_per_cta == 1)) return fail(GCT_ERR_INVALID, "attention: ctas_per_sm");
   if (a.status == nullptr) return fail(GCT_ERR_INVALID, "attention: status word missing");
   KernelArgs k;
   k.page_table = a.page_table;
@@ -1040,7 +920,7 @@ int launch_attention(const AttnLaunch& a, cudaStream_t stream) {
     return fail(GCT_ERR_INVALID, "attention: partial buffers missing");
   const long long grid = static_cast<long long>(k.q_groups) * a.splits * a.heads * a.batch;
   if (grid <= 0 || grid > 0x7fffffffLL) return fail(GCT_ERR_INVALID, "attention: grid too large");
-  const int smem = attention_smem_bytes(a.q_tiles_per_cta);
+  const int smem = attention_smem_bytes(a.q_tiles_per_cta, a.ctas_per_sm);
   int rc = opt_in_shared_memory();
   if (rc != GCT_OK) return rc;
   const dim3 g(static_cast<unsigned>(grid));
@@ -1049,6 +929,8 @@ int launch_attention(const AttnLaunch& a, cudaStream_t stream) {
       GCT_CUDA_CHECK(launch_pdl(gct_attn_kernel<2, true>, g, dim3(kThreads<2>), smem, stream, a.tm_q, a.tm_k, a.tm_v, k));
     else
       GCT_CUDA_CHECK(launch_pdl(gct_attn_kernel<2, false>, g, dim3(kThreads<2>), smem, stream, a.tm_q, a.tm_k, a.tm_v, k));
+  } else if (a.ctas_per_sm == 2) {
+    GCT_CUDA_CHECK(launch_pdl(gct_attn_kernel<1, false, 2>, g, dim3(kThreads<1>), smem, stream, a.tm_q, a.tm_k, a.tm_v, k));
   } else {
     GCT_CUDA_CHECK(launch_pdl(gct_attn_kernel<1, false>, g, dim3(kThreads<1>), smem, stream, a.tm_q, a.tm_k, a.tm_v, k));
   }

@@ -80,6 +80,7 @@ struct AttnLaunch {
   int last_page_len = 0;
   int n_q = 0, heads = 0, batch = 1;
   int q_tiles_per_cta = 2;           // 1 or 2
+  int ctas_per_sm = 1;               // 2: one-tile CTAs two to an SM
   int splits = 1;
   int split_len = 0;                 // 0: `splits` equal ranges of KV blocks; > 0: splits - 1 ranges of split_len blocks, the last
                                      // one takes the (shorter) rest and its CTAs are launched last
@@ -95,7 +96,7 @@ struct AttnLaunch {
   float bounded_limit = 0.f;
 };
 int launch_attention(const AttnLaunch& a, cudaStream_t stream);
-int attention_smem_bytes(int q_tiles_per_cta);
+int attention_smem_bytes(int q_tiles_per_cta, int ctas_per_sm);
 
 // Encode a 4-D bf16 tensor map {64, heads, tokens, pages} with the given element strides
 // (head, token, page) and the box {64,1,128,1}.
@@ -155,12 +156,15 @@ const gct_mgr_config_t& mgr_config(const gct_mgr_t* m);
 // src: q_src / k_src / v_src, strides, dtypes, norm parameters, rotation and q_out filled in; the destination pages come
 // from the bookkeeping of this append.
 int mgr_append(gct_mgr_t* m, int block, PrepLaunch src, cudaStream_t stream);
-// (q tiles per CTA, splits) of a dense attention call with at most max_splits partial results.
-int dense_attention_plan(int batch, int n_q, int n_kv, int heads, int max_splits, int* q_tiles_per_cta, int* splits);
+// How a dense attention call with at most max_splits partial results is cut.
+struct DensePlan {
+  int q_tiles_per_cta = 1, ctas_per_sm = 1, splits = 1;
+};
+int dense_attention_plan(int batch, int n_q, int n_kv, int heads, int max_splits, DensePlan* plan);
 // splits > 1: part_o [splits, batch * n_q * heads, 64] and part_lse [splits, batch * n_q * heads] are scratch.
 int dense_attention_run(const void* q, const void* k, const void* v, void* out, int batch, int n_q, int n_kv, int heads,
-                        const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3], int q_tiles_per_cta,
-                        int splits, float* part_o, float* part_lse, int* status, cudaStream_t stream);
+                        const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3], const DensePlan& plan,
+                        float* part_o, float* part_lse, int* status, cudaStream_t stream);
 
 
 // Residual sum and LayerNorm of rows: v = x + gamma * y to sum_out (y null: v = x, nothing stored), LayerNorm(v) to norm_out

@@ -807,19 +807,33 @@ int gct_attn_launch_shape(int n_q, int heads, int kv_blocks, int num_sms, int ma
 }  // extern "C"
 
 namespace gct {
-int dense_attention_plan(int batch, int n_q, int n_kv, int heads, int max_splits, int* q_tiles_per_cta, int* splits) {
+int dense_attention_plan(int batch, int n_q, int n_kv, int heads, int max_splits, DensePlan* plan) {
   if (batch <= 0 || n_q <= 0 || n_kv <= 0 || heads <= 0) return fail(GCT_ERR_INVALID, "dense attention: bad shape");
   int sms = 148;
   const int rc = device_sm_count(&sms);
   if (rc != GCT_OK) return rc;
-  choose_attention_config((n_q + kTileM - 1) / kTileM, heads * batch, (n_kv + kBlockN - 1) / kBlockN, sms, std::max(max_splits, 1),
-                          q_tiles_per_cta, splits);
+  const int q_tiles = (n_q + kTileM - 1) / kTileM, blocks = (n_kv + kBlockN - 1) / kBlockN;
+  choose_attention_config(q_tiles, heads * batch, blocks, sms, std::max(max_splits, 1), &plan->q_tiles_per_cta, &plan->splits);
+  plan->ctas_per_sm = 1;
+  // A call of several waves over few KV blocks spends much of its time on set-up and epilogue of its CTAs.  Two one-tile CTAs on an SM run
+  // these under each other's KV loop, but read K and V twice.  Time per wave, in KV blocks of a two-tile CTA, with b blocks (from 8 x
+  // 1005 x 1005, b = 8: two tiles 67.7 us, two CTAs 60.3 us; 6264 x 6264, b = 49: 224 us and 243 us; one tile alone: b = 1 5.8 us, b = 8
+  // 11.1 us): two tiles b + 4.0, two CTAs 1.14 b + 1.56, one tile alone 0.52 b + 3.7.
+  const long long tiles = static_cast<long long>(q_tiles) * heads * batch, pairs = static_cast<long long>((q_tiles + 1) / 2) * heads * batch;
+  if (plan->splits == 1 && tiles > sms) {
+    auto waves = [](long long ctas, long long slots) { return static_cast<double>((ctas + slots - 1) / slots); };
+    const double chosen = plan->q_tiles_per_cta == 2 ? waves(pairs, sms) * (blocks + 4.0) : waves(tiles, sms) * (0.52 * blocks + 3.7);
+    if (waves(tiles, 2ll * sms) * (1.14 * blocks + 1.56) < 0.97 * chosen) {
+      plan->q_tiles_per_cta = 1;
+      plan->ctas_per_sm = 2;
+    }
+  }
   return GCT_OK;
 }
 
 int dense_attention_run(const void* q, const void* k, const void* v, void* out, int batch, int n_q, int n_kv, int heads,
-                        const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3], int q_tiles_per_cta,
-                        int splits, float* part_o, float* part_lse, int* status, cudaStream_t stream) {
+                        const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3], const DensePlan& plan,
+                        float* part_o, float* part_lse, int* status, cudaStream_t stream) {
   AttnLaunch a;
   // strides are (batch, token, head) in elements
   int rc = make_tensor_map(&a.tm_q, q, heads, n_q, batch, q_strides[2], q_strides[1], q_strides[0]);
@@ -836,15 +850,16 @@ int dense_attention_run(const void* q, const void* k, const void* v, void* out, 
   a.heads = heads;
   a.batch = batch;
   a.status = status;
-  a.q_tiles_per_cta = q_tiles_per_cta;
-  a.splits = splits;
-  a.final_bf16 = splits == 1;
+  a.q_tiles_per_cta = plan.q_tiles_per_cta;
+  a.ctas_per_sm = plan.ctas_per_sm;
+  a.splits = plan.splits;
+  a.final_bf16 = plan.splits == 1;
   a.out = static_cast<__nv_bfloat16*>(out);
   a.part_o = part_o;
   a.part_lse = part_lse;
   rc = launch_attention(a, stream);
-  if (rc != GCT_OK || splits == 1) return rc;
-  return launch_merge(part_o, part_lse, splits, static_cast<int64_t>(batch) * n_q * heads, a.out, nullptr, nullptr, stream);
+  if (rc != GCT_OK || plan.splits == 1) return rc;
+  return launch_merge(part_o, part_lse, plan.splits, static_cast<int64_t>(batch) * n_q * heads, a.out, nullptr, nullptr, stream);
 }
 }  // namespace gct
 
@@ -861,13 +876,13 @@ int gct_attn_dense(const void* q_dev, const void* k_dev, const void* v_dev, void
     return fail(GCT_ERR_CAPACITY, "gct_attn_dense: needs a 256-byte aligned workspace of at least 256 bytes (status word)");
   const size_t rows = static_cast<size_t>(batch) * n_q * heads;
   const size_t per_split = rows * kHeadDim * 4 + rows * 4;
-  int qt = 1, splits = 1;
+  DensePlan plan;
   const int rc = dense_attention_plan(batch, n_q, n_kv, heads,
-                                      static_cast<int>(std::min<size_t>((workspace_bytes - 256) / per_split, kMaxSplitsCap)), &qt, &splits);
+                                      static_cast<int>(std::min<size_t>((workspace_bytes - 256) / per_split, kMaxSplitsCap)), &plan);
   if (rc != GCT_OK) return rc;
   float* part_o = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace_dev) + 256);
-  return dense_attention_run(q_dev, k_dev, v_dev, out_dev, batch, n_q, n_kv, heads, q_strides, k_strides, v_strides, qt, splits, part_o,
-                             part_o + static_cast<size_t>(splits) * rows * kHeadDim, static_cast<int*>(workspace_dev),
+  return dense_attention_run(q_dev, k_dev, v_dev, out_dev, batch, n_q, n_kv, heads, q_strides, k_strides, v_strides, plan, part_o,
+                             part_o + static_cast<size_t>(plan.splits) * rows * kHeadDim, static_cast<int*>(workspace_dev),
                              static_cast<cudaStream_t>(stream));
 }
 

@@ -276,21 +276,20 @@ Tensor dense(const Tensor& q, const Tensor& k, const Tensor& v, Tensor out) {
   if (k.sizes() != v.sizes() || k.size(0) != B || k.size(2) != H) value_error("k/v shape mismatch");
   c10::cuda::CUDAGuard guard(q.device());
   if (!out.defined()) out = empty({B, Nq, H, kHeadDim}, at::kBFloat16, q);
-  int qt = 1, splits = 1;
-  check(gct::dense_attention_plan(static_cast<int>(B), static_cast<int>(Nq), static_cast<int>(Nkv), static_cast<int>(H), kDenseMaxSplits, &qt,
-                                  &splits));
+  gct::DensePlan plan;
+  check(gct::dense_attention_plan(static_cast<int>(B), static_cast<int>(Nq), static_cast<int>(Nkv), static_cast<int>(H), kDenseMaxSplits, &plan));
   const int64_t rows = B * Nq * H;
   Tensor scratch;
   float* part = nullptr;
-  if (splits > 1) {
-    scratch = empty({splits * rows * (kHeadDim + 1)}, at::kFloat, q);
+  if (plan.splits > 1) {
+    scratch = empty({plan.splits * rows * (kHeadDim + 1)}, at::kFloat, q);
     part = scratch.data_ptr<float>();
   }
   const int64_t qs[3] = {q.stride(0), q.stride(1), q.stride(2)}, ks[3] = {k.stride(0), k.stride(1), k.stride(2)},
                 vs[3] = {v.stride(0), v.stride(1), v.stride(2)};
   check(gct::dense_attention_run(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), static_cast<int>(B), static_cast<int>(Nq),
-                                 static_cast<int>(Nkv), static_cast<int>(H), qs, ks, vs, qt, splits, part,
-                                 part == nullptr ? nullptr : part + splits * rows * kHeadDim, status_of(q), stream_of(q)));
+                                 static_cast<int>(Nkv), static_cast<int>(H), qs, ks, vs, plan, part,
+                                 part == nullptr ? nullptr : part + plan.splits * rows * kHeadDim, status_of(q), stream_of(q)));
   return out;
 }
 

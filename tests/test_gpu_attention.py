@@ -148,6 +148,21 @@ def test_dense_attention_vs_oracle(B, Nq, Nkv, H):
     assert P.ops.device_status(DEV) == 0
 
 
+@pytest.mark.parametrize("Nkv", [1, 31, 32, 33, 63, 64, 65, 127, 128, 129, 192, 193, 320])
+@pytest.mark.parametrize("B,Nq,H", [(1, 1, 1), (1, 129, 3), (1, 200, 160), (2, 385, 60)])
+def test_dense_attention_at_the_edges_of_a_block(B, Nq, H, Nkv):
+    """Two threads share a row of 128 keys: lengths around their boundary and the block's, for one-tile CTAs (one wave, or two to an SM when
+    there are more than one wave of them), two-tile CTAs and split ranges; keys that grow, so that the running maximum moves."""
+    q, k, v = seeded.randn(1, B, Nq, H, 64), seeded.randn(2, B, Nkv, H, 64), seeded.randn(3, B, Nkv, H, 64)
+    k = k * np.linspace(0.2, 2.0, Nkv, dtype=np.float32)[None, :, None, None]
+    out = P.ops.dense_attention(bf(q), bf(k), bf(v))
+    heads = sorted({0, 1 % H, H // 2, H - 1})
+    for b in range(B):
+        want = O.attention(r(q[b][:, heads]), r(k[b][:, heads]), r(v[b][:, heads]))[0]
+        assert_close(out[b][:, heads], want, f"b={b}")
+    assert P.ops.device_status(DEV) == 0
+
+
 def test_dense_attention_strided_views():
     """q/k/v as views into one qkv buffer [B, N, 3, H, 64] (the layout the qkv Linear produces)."""
     B, N, H = 2, 200, 4
