@@ -123,6 +123,13 @@ int voxel_gather(const float* xyz, const float* rgb, float voxel_size, int64_t n
                  int64_t* codes, cudaStream_t stream);
 
 // ---- elementwise kernels ---------------------------------------------------------------
+// Pages and slots of one frame's K/V rows.
+struct PageSlots {
+  int patch_page = -1;               // tokens >= num_special go to row (token - num_special) of this page
+  int sp_page0 = -1, sp_off0 = 0, sp_n0 = 0, sp_page1 = -1;   // specials: first sp_n0 at sp_off0 of page0, rest at row 0.. of page1
+};
+constexpr int kAppendFrames = 8;     // frames of one paged launch
+
 struct PrepLaunch {
   // sources: rows of 64 elements; element strides between tokens and heads
   const void* q_src = nullptr; const void* k_src = nullptr; const void* v_src = nullptr;
@@ -142,8 +149,7 @@ struct PrepLaunch {
   // K/V destination, paged (k_out == null): pool [pages, 2, page_size, H, 64]
   __nv_bfloat16* pool = nullptr;
   int page_size = 0, num_pages = 0, num_special = 0;
-  int patch_page = -1;               // tokens >= num_special go to row (token - num_special) of this page
-  int sp_page0 = -1, sp_off0 = 0, sp_n0 = 0, sp_page1 = -1;   // specials: first sp_n0 at sp_off0 of page0, rest at row 0.. of page1
+  PageSlots dst[kAppendFrames];      // of frame token / tokens_per_frame
   int* status = nullptr;
   float* key_norm_max = nullptr;     // [H] running maximum of the 2-norms of the K rows written (paged destination)
 };
@@ -156,6 +162,9 @@ const gct_mgr_config_t& mgr_config(const gct_mgr_t* m);
 // src: q_src / k_src / v_src, strides, dtypes, norm parameters, rotation and q_out filled in; the destination pages come
 // from the bookkeeping of this append.
 int mgr_append(gct_mgr_t* m, int block, PrepLaunch src, cudaStream_t stream);
+// `frames` times gct_mgr_append and gct_mgr_evict for the frames of k and v (bf16 [frames * tokens_per_frame, H, 64], contiguous), with
+// up to kAppendFrames frames per launch.
+int mgr_append_frames(gct_mgr_t* m, int block, const __nv_bfloat16* k, const __nv_bfloat16* v, int frames, int sliding_window, cudaStream_t stream);
 // How a dense attention call with at most max_splits partial results is cut.
 struct DensePlan {
   int q_tiles_per_cta = 1, ctas_per_sm = 1, splits = 1;
@@ -186,6 +195,8 @@ struct RowLaunch {
   __nv_bfloat16* norm_out = nullptr;
 };
 int launch_residual_norm(const RowLaunch& p, cudaStream_t stream);
+// GELU (the erf form) of n contiguous values in place.
+int launch_gelu(__nv_bfloat16* x, int64_t n, cudaStream_t stream);
 // Table of the 2-D rotation [tokens, 32, 2] from integer positions [tokens, 2] with the given strides.
 int launch_rope2d_positions(const int64_t* pos, int64_t token_stride, int64_t axis_stride, int tokens, float base, float* cs, cudaStream_t stream);
 

@@ -174,7 +174,6 @@ __device__ __forceinline__ void rotate16(float (&x)[16], const float2 (&cs)[8]) 
 template <int kMode, bool kQkF32, bool kVF32>
 __global__ void __launch_bounds__(kPrepThreads) gct_prep_kernel(const PrepLaunch p) {
   __shared__ __align__(16) float s_norm[4][kHeadDim];       // q weight, q bias, k weight, k bias
-  pdl_wait();
   const int part = threadIdx.x & 3, e0 = 32 * (part >> 1) + 8 * (part & 1);
   const int rows = p.tokens * p.heads;
   const int row = (blockIdx.x * kPrepThreads + threadIdx.x) >> 2;
@@ -183,6 +182,7 @@ __global__ void __launch_bounds__(kPrepThreads) gct_prep_kernel(const PrepLaunch
   const int token = r / p.heads, h = r - token * p.heads;
   const bool do_q = p.q_src != nullptr && p.q_out != nullptr, do_kv = p.k_out != nullptr || p.pool != nullptr;
   const size_t src = static_cast<size_t>(token) * p.src_token_stride + static_cast<size_t>(h) * p.src_head_stride + e0;
+  pdl_wait();
   RawRow<kQkF32> rq, rk;
   RawRow<kVF32> rv;
   if (do_q) rq.load(p.q_src, src);
@@ -232,15 +232,17 @@ __global__ void __launch_bounds__(kPrepThreads) gct_prep_kernel(const PrepLaunch
     v_row = p.v_out + static_cast<size_t>(token) * p.heads * kHeadDim;
   } else if (p.pool != nullptr) {
     int page, slot;
-    if (token >= p.num_special) {
-      page = p.patch_page;
-      slot = token - p.num_special;
-    } else if (token < p.sp_n0) {
-      page = p.sp_page0;
-      slot = p.sp_off0 + token;
+    const int frame = token < p.tokens_per_frame ? 0 : token / p.tokens_per_frame, in_frame = token - frame * p.tokens_per_frame;
+    const PageSlots& to = p.dst[frame];
+    if (in_frame >= p.num_special) {
+      page = to.patch_page;
+      slot = in_frame - p.num_special;
+    } else if (in_frame < to.sp_n0) {
+      page = to.sp_page0;
+      slot = to.sp_off0 + in_frame;
     } else {
-      page = p.sp_page1;
-      slot = token - p.sp_n0;
+      page = to.sp_page1;
+      slot = in_frame - to.sp_n0;
     }
     if (page < 0 || page >= p.num_pages || slot < 0 || slot >= p.page_size) {
       if (active && part == 0) atomicCAS(p.status, 0, kStatusBadIndex);
@@ -392,6 +394,24 @@ __global__ void __launch_bounds__(kThreads > 128 ? kThreads : 128) gct_residual_
 #pragma unroll
   for (int i = 0; i < 8; ++i) r.v[i] = fmaf(v.v[i] * rstd, ww.v[i], bb.v[i]);
   store8(p.norm_out + at, r);
+}
+
+// x = 0.5 x (1 + erf(x / sqrt 2)) of bf16 values in place, in fp32: the activation between the two Linear layers of a block.  A frame is
+// 1005 x 4096 values (8 MB, just written: they lie in L2), so the time is the launch, which overlaps the end of the product before,
+// and one round trip.  In place of a tensor operation (6.5 us, out of place, and its dispatch), together with the appends of a scale
+// pass in one launch: a sequence's first sixteen frames through two layer pairs 3668 -> 3617 us.
+__global__ void __launch_bounds__(256) gct_gelu_kernel(__nv_bfloat16* __restrict__ x, int64_t n) {
+  pdl_wait();
+  auto gelu = [](float v) { return 0.5f * v * (1.f + erff(v * 0.70710678118654752f)); };
+  const int64_t i = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) * 8;
+  if (i + 8 <= n) {
+    Row8 r = load8(x, GCT_BF16, i);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) r.v[e] = gelu(r.v[e]);
+    store8(x + i, r);
+  } else {
+    for (int64_t e = i; e < n; ++e) x[e] = __float2bfloat16_rn(gelu(__bfloat162float(x[e])));
+  }
 }
 
 // cos/sin table of the 2-D rotation from integer (y, x) positions [tokens, 2] (lingbot_map/layers/rope.py:105-119): entry
@@ -603,6 +623,8 @@ int launch_prep(const PrepLaunch& p, cudaStream_t stream) {
       misaligned(p.v_out) || misaligned(p.pool) || misaligned(p.qn_w) || misaligned(p.qn_b) || misaligned(p.kn_w) ||
       misaligned(p.kn_b) || misaligned(p.rope_cs))
     return fail(GCT_ERR_INVALID, "prep: tensors must be 16-byte aligned");
+  if (p.k_out == nullptr && p.pool != nullptr && p.tokens > static_cast<long long>(kAppendFrames) * p.tokens_per_frame)
+    return fail(GCT_ERR_INVALID, "prep: more frames than one launch takes");
   const long long rows = static_cast<long long>(p.tokens) * p.heads;
   if (rows > (1ll << 28)) return fail(GCT_ERR_INVALID, "prep: too many rows");
   const dim3 grid(static_cast<unsigned>((rows * 4 + kPrepThreads - 1) / kPrepThreads)), block(kPrepThreads);
@@ -633,6 +655,14 @@ int launch_residual_norm(const RowLaunch& p, cudaStream_t stream) {
   auto kernel = threads == 32 ? gct_residual_norm_kernel<32> : threads == 64 ? gct_residual_norm_kernel<64>
                 : threads == 128 ? gct_residual_norm_kernel<128> : gct_residual_norm_kernel<256>;
   GCT_CUDA_CHECK(launch_pdl(kernel, grid, block, 0, stream, p));
+  return GCT_OK;
+}
+
+int launch_gelu(__nv_bfloat16* x, int64_t n, cudaStream_t stream) {
+  const int64_t ctas = (n + 2047) / 2048;
+  if (n < 0 || ctas > 0x7fffffff || (reinterpret_cast<uintptr_t>(x) & 15) != 0) return fail(GCT_ERR_INVALID, "gelu: bad argument");
+  if (n == 0) return GCT_OK;
+  GCT_CUDA_CHECK(launch_pdl(gct_gelu_kernel, dim3(static_cast<unsigned>(ctas)), dim3(256), 0, stream, x, n));
   return GCT_OK;
 }
 

@@ -299,12 +299,8 @@ int gct_mgr_bind(gct_mgr_t* m, void* const* pools_dev, void* workspace_dev, size
   return GCT_OK;
 }
 
-// Where one frame's K/V rows go; the bookkeeping half of append_frame.
-struct AppendPlan {
-  int patch_page, sp_page0, sp_off0, sp_n0, sp_page1;
-};
-
-static int append_bookkeeping(gct_mgr* m, int block, AppendPlan* plan) {
+// The bookkeeping half of append_frame; *plan: where the frame's K/V rows go.
+static int append_bookkeeping(gct_mgr* m, int block, PageSlots* plan) {
   if (m == nullptr) return fail(GCT_ERR_INVALID, "null manager");
   if (block < 0 || block >= m->cfg.num_blocks) return fail(GCT_ERR_INVALID, "block index out of range");
   BlockState& b = m->blocks[block];
@@ -322,7 +318,7 @@ static int append_bookkeeping(gct_mgr* m, int block, AppendPlan* plan) {
       return fail(GCT_ERR_POOL_EXHAUSTED, "block " + std::to_string(block) + ": special page pool exhausted at special_token_count=" +
                                               std::to_string(b.special_token_count) + ". Increase max_total_frames.");
   }
-  AppendPlan pl{-1, -1, 0, 0, -1};
+  PageSlots pl;
   pl.patch_page = b.free_patch.back();                       // LIFO pop (:496)
   b.free_patch.pop_back();
   if (static_cast<int>(b.scale_pages.size()) < m->cfg.scale_frames)   // :507-510
@@ -411,18 +407,14 @@ static int track_key_norms(gct_mgr* m, int block, PrepLaunch* p, cudaStream_t st
   return GCT_OK;
 }
 
-static void fill_paged_dst(const gct_mgr* m, int block, const AppendPlan& pl, PrepLaunch* p) {
+static void fill_paged_dst(const gct_mgr* m, int block, const PageSlots* frames, int count, PrepLaunch* p) {
   p->pool = m->pools[block];
   p->page_size = m->geo.page_size;
   p->num_pages = m->geo.max_num_pages;
   p->num_special = m->cfg.num_special_tokens;
-  p->patch_page = pl.patch_page;
-  p->sp_page0 = pl.sp_page0;
-  p->sp_off0 = pl.sp_off0;
-  p->sp_n0 = pl.sp_n0;
-  p->sp_page1 = pl.sp_page1;
+  std::copy(frames, frames + count, p->dst);
   p->status = m->status_dev;
-  p->tokens = m->cfg.tokens_per_frame;
+  p->tokens = count * m->cfg.tokens_per_frame;
   p->tokens_per_frame = m->cfg.tokens_per_frame;
   p->heads = m->cfg.num_heads;
 }
@@ -435,14 +427,55 @@ const gct_mgr_config_t& mgr_config(const gct_mgr_t* m) { return m->cfg; }
 int mgr_append(gct_mgr_t* m, int block, PrepLaunch p, cudaStream_t stream) {
   int rc = check_bound(m);
   if (rc != GCT_OK) return rc;
-  AppendPlan pl;
+  PageSlots pl;
   rc = append_bookkeeping(m, block, &pl);
   if (rc != GCT_OK) return rc;
-  fill_paged_dst(m, block, pl, &p);
+  fill_paged_dst(m, block, &pl, 1, &p);
   rc = track_key_norms(m, block, &p, stream);
   if (rc != GCT_OK) return rc;
   m->launches += 1;
   return launch_prep(p, stream);
+}
+
+// A launch per frame took 4 us each on top of what the frames of a scale pass need together.  A batch ends where a frame would write a
+// page that a frame of the batch writes (evicted in between and handed out again): the rows of a launch are written in any order.
+int mgr_append_frames(gct_mgr_t* m, int block, const __nv_bfloat16* k, const __nv_bfloat16* v, int frames, int sliding_window, cudaStream_t stream) {
+  int rc = check_bound(m);
+  if (rc != GCT_OK) return rc;
+  const int64_t token = static_cast<int64_t>(m->cfg.num_heads) * kHeadDim, frame = m->cfg.tokens_per_frame * token;
+  PageSlots batch[kAppendFrames];
+  int first = 0, count = 0;
+  auto flush = [&]() -> int {
+    if (count == 0) return GCT_OK;
+    PrepLaunch p;
+    p.k_src = k + first * frame;
+    p.v_src = v + first * frame;
+    p.src_token_stride = token;
+    p.src_head_stride = kHeadDim;
+    fill_paged_dst(m, block, batch, count, &p);
+    first += count;
+    count = 0;
+    const int r = track_key_norms(m, block, &p, stream);
+    if (r != GCT_OK) return r;
+    m->launches += 1;
+    return launch_prep(p, stream);
+  };
+  for (int f = 0; f < frames; ++f) {
+    PageSlots next;
+    const int appended = append_bookkeeping(m, block, &next);
+    bool taken = count == kAppendFrames;
+    for (int i = 0; i < count; ++i) taken |= batch[i].patch_page == next.patch_page;
+    if (appended != GCT_OK || taken) {
+      const std::string error = g_last_error;
+      rc = flush();
+      if (rc != GCT_OK) return rc;
+      if (appended != GCT_OK) return fail(appended, error);      // the frames before are in, as they would be one by one
+    }
+    batch[count++] = next;
+    rc = gct_mgr_evict(m, block, sliding_window);
+    if (rc != GCT_OK) return rc;
+  }
+  return flush();
 }
 }  // namespace gct
 

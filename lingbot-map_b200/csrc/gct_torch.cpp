@@ -656,19 +656,15 @@ PyObject* py_block_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
       } else {
         Qkv r = prep(qkv, heads, N, norm, cs, rope);
         o = dense(r.q.view({B, N, heads, kHeadDim}), r.k.view({B, N, heads, kHeadDim}), r.v.view({B, N, heads, kHeadDim}), Tensor());
-        if (m != nullptr) {
-          const int64_t step = gct::mgr_config(m).tokens_per_frame * C;
-          for (int64_t f = 0; f < frames; ++f) {
-            check(gct_mgr_append(m, blk, bf16(r.k) + f * step, GCT_BF16, bf16(r.v) + f * step, GCT_BF16, stream_of(x)));
-            check(gct_mgr_evict(m, blk, static_cast<int>(window)));
-          }
-        }
+        if (m != nullptr)
+          check(gct::mgr_append_frames(m, blk, bf16(r.k), bf16(r.v), static_cast<int>(frames), static_cast<int>(window), stream_of(x)));
       }
       const Tensor attn = linear(o.view({B * N, C}), proj_w, proj_b);
       Tensor sum;
       const Tensor normed2 = residual_norm(x, &attn, g1, &sum, n2w, n2b, eps2);
       if (with_ffn) {
-        const Tensor h = at::gelu(linear(normed2, fc1_w, fc1_b));
+        const Tensor h = linear(normed2, fc1_w, fc1_b);
+        check(gct::launch_gelu(static_cast<__nv_bfloat16*>(h.data_ptr()), h.numel(), stream_of(h)));
         const Tensor f = linear(h, fc2_w, fc2_b);
         Tensor out;
         residual_norm(sum, &f, g2, &out, nullptr, nullptr, 0.0);

@@ -256,6 +256,38 @@ def test_layers_as_one_call_equal_the_module_code(monkeypatch, dim, H, weights, 
         assert d <= 2 * 2 ** -7 * top, (i, d, top)
 
 
+@pytest.mark.parametrize("frames,scale,window", [(2, 2, 1), (8, 8, 4), (9, 16, 4), (17, 17, 2), (11, 2, 1), (20, 3, 2)])
+def test_scale_pass_appends_its_frames_as_one_by_one(monkeypatch, frames, scale, window):
+    """The native scale pass appends up to eight frames per launch, and ends a launch where an evicted page comes back: page tables and
+    pages as the modules make them, which append and evict frame by frame (K and V differ by the rounding steps of the test above).  The
+    hidden layer has 33 columns, so that the activation ends in the middle of eight values."""
+    from lingbot_map_b200 import block as block_mod
+    pph, ppw, ns, dim, H = 3, 5, 6, 128, 2
+    T = ns + pph * ppw
+    blk = P.B200Block(dim=dim, num_heads=H, mlp_ratio=33 / 128, init_values=0.5, qk_norm=True, rope=Rope2dStub(), kv_cache_sliding_window=window,
+                      kv_cache_scale_frames=scale).eval().to(DEV)
+    seeded.fill_module_(blk, 3)
+    blk = blk.to(torch.bfloat16)
+    x = torch.from_numpy(seeded.randn(3, 1, frames * T, dim)).to(DEV).to(torch.bfloat16)
+
+    def run(fused):
+        monkeypatch.setattr(block_mod, "_may_fuse", lambda: fused)
+        mgr = P.B200KVCacheManager(1, scale + window + 16, T, H, 64, device=DEV, scale_frames=scale, sliding_window=window, max_total_frames=40)
+        y = blk(x, pos=rope3d_pos(0, frames, pph, ppw, ns), num_frames=frames, kv_cache=mgr, num_patches=T - ns, num_special=ns,
+                enable_3d_rope=True, global_idx=0, num_frame_for_scale=scale)
+        assert mgr.device_status() == 0
+        return [y, *mgr._gather_kv(0)], mgr.build_visible_page_table(0), mgr.key_norm_max.clone()
+
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        got, table, norms = run(True)
+        want, wtable, wnorms = run(False)
+    assert table == wtable
+    assert torch.allclose(norms, wnorms, rtol=2 ** -7)
+    for a, b in zip(got, want):
+        assert a.dtype == b.dtype and a.shape == b.shape
+        assert float((a.float() - b.float()).abs().max()) <= 2 * 2 ** -7 * float(b.float().abs().max())
+
+
 def _layer_pair(dim=128, H=2):
     blk = P.B200Block(dim=dim, num_heads=H, init_values=0.5, qk_norm=True, rope=Rope2dStub()).eval().to(DEV)
     fa = P.B200FrameAttention(dim, num_heads=H, qk_norm=True, rope=Rope2dStub()).eval().to(DEV)
