@@ -572,7 +572,6 @@ int voxel_sort(const float* xyz, float voxel_size, int64_t n, void* scratch, int
   std::fill(report, report + s.tiles, kVoxelPending);
   GCT_CUDA_CHECK(launch_pdl(gct_voxel_code_kernel, dim3(s.tiles), dim3(kVoxelThreads), 0, stream, xyz, voxel_size, s));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(std::min(s.tiles, 2 * sms));      // two CTAs of the sort fit an SM: all tiles at once where there are 128 SMs
   cfg.blockDim = dim3(kVoxelThreads);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -580,7 +579,19 @@ int voxel_sort(const float* xyz, float voxel_size, int64_t n, void* scratch, int
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  GCT_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gct_voxel_sort_kernel, s, static_cast<volatile int32_t*>(report)));
+  // Two CTAs of the sort fit an SM: all tiles at once where there are 128 SMs.  The stream may own fewer than the device has (a green
+  // context, a share of the device); the driver then refuses the launch, and half as many CTAs take twice as many tiles each.
+  int grid = std::min(s.tiles, 2 * sms);
+  for (;;) {
+    cfg.gridDim = dim3(grid);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gct_voxel_sort_kernel, s, static_cast<volatile int32_t*>(report));
+    if (e != cudaErrorCooperativeLaunchTooLarge || grid == 1) {
+      GCT_CUDA_CHECK(e);
+      break;
+    }
+    cudaGetLastError();                                // answered by the smaller launch
+    grid /= 2;
+  }
   // The counts are looked for where the kernel writes them: they are there some microseconds before the stream is seen to be idle.
   const volatile int32_t* counts = report;
   int64_t total = 0;

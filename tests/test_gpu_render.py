@@ -85,6 +85,30 @@ def test_voxelize_frame_sort_up_to_its_largest(n):
             assert np.array_equal(codes.cpu().numpy(), wcodes) and np.array_equal(c.cpu().numpy(), wc) and np.array_equal(col.cpu().numpy(), wcol)
 
 
+@pytest.mark.parametrize("sms", [8, 16, 72])
+@pytest.mark.parametrize("n", [2048, 40 * 2048 + 1, 256 * 2048])
+def test_voxelize_frame_on_part_of_the_gpu(sms, n):
+    """A stream that owns a few of the SMs: the sort's tiles do not all run at once there, and a CTA takes several."""
+    from torch.cuda import green_contexts
+    if not green_contexts.SUPPORTED:
+        pytest.skip("PyTorch was built without green contexts")
+    rs = np.random.RandomState(sms + n % 1000)
+    xyz = (rs.randint(-300, 301, (n, 3)) + 0.5).astype(np.float32)
+    rgb = rs.rand(n, 3).astype(np.float32)
+    wc, wcol, wcodes = R.voxelize_frame(xyz, rgb, 1.0)
+    dx, dr = torch.from_numpy(xyz).to(DEV), torch.from_numpy(rgb).to(DEV)
+    torch.cuda.synchronize()
+    part = torch.cuda.GreenContext.create(sms, 0)
+    part.set_context()
+    try:
+        got = RO.voxelize_frame(dx, dr, 1.0)
+        torch.cuda.synchronize()
+    finally:
+        part.pop_context()
+    for a, b in zip(got, (wc, wcol, wcodes)):
+        assert np.array_equal(a.cpu().numpy(), b)
+
+
 @pytest.mark.parametrize("n", [1, 2047, 2048, 2049, 2 * 2048 + 1, 65536])
 @pytest.mark.parametrize("extent", [3, 100, 5000, 2 ** 20 - 1])
 def test_voxelize_frame_sort_edges(n, extent):
