@@ -114,8 +114,8 @@ void choose_attention_config(int n_q_tiles, int heads_x_batch, int total_blocks,
 // strides (row and column of R, step of t).
 int frustum_cull(const float* pts, int64_t n, const float* R, const float* t, const int* device_strides, float fx, float fy, float cx,
                  float cy, int width, int height, float near_plane, float far_plane, uint8_t* visible, cudaStream_t stream);
-// Voxelisation of up to kVoxelMaxPoints points: sort (scratch of `bytes`; `report`: pinned host memory of an int per tile;
-// waits for the stream), then, with outputs sized by the number of voxels, gather.
+// Voxelisation of up to kVoxelMaxPoints points: sort (scratch of `bytes`; `report`: pinned host memory of an int per tile; waits
+// for the number of voxels only, so its kernel may still be ending), then, with outputs sized by that number and on the same stream, gather.
 constexpr int64_t kVoxelMaxPoints = 256 * 2048;
 int voxel_sort_layout(int64_t n, size_t* bytes, int* tiles);
 int voxel_sort(const float* xyz, float voxel_size, int64_t n, void* scratch, int32_t* report, int64_t* voxels_out, cudaStream_t stream);

@@ -7,6 +7,7 @@
 // Arithmetic is written with explicitly rounded single operations (no fused multiply-add, IEEE division), so that
 // a float32 CPU restatement reproduces every mask bit and every Morton code exactly.
 #include <algorithm>
+#include <chrono>
 
 #include "gct_common.h"
 
@@ -163,6 +164,7 @@ constexpr int kVoxelMaxTiles = 256;              // every CTA of a pass adds up 
 constexpr int kVoxelMaxPasses = 8;
 constexpr int kVoxelOffset = 1 << 20;            // voxel_morton.cu:36-38
 constexpr int32_t kVoxelPending = -1, kVoxelFailed = -2;      // in place of a tile's count
+constexpr std::chrono::microseconds kVoxelLook{150};          // the largest cloud of the sort: up to 126 us from the call to its counts
 
 struct VoxelScratch {
   uint64_t* keys0;         // Morton codes and indices, two buffers
@@ -569,6 +571,8 @@ int voxel_sort(const float* xyz, float voxel_size, int64_t n, void* scratch, int
   int sms = 148;
   const int rc = device_sm_count(&sms);
   if (rc != GCT_OK) return rc;
+  unsigned flags = 0;
+  GCT_CUDA_CHECK(cudaGetDeviceFlags(&flags));
   std::fill(report, report + s.tiles, kVoxelPending);
   GCT_CUDA_CHECK(launch_pdl(gct_voxel_code_kernel, dim3(s.tiles), dim3(kVoxelThreads), 0, stream, xyz, voxel_size, s));
   cudaLaunchConfig_t cfg = {};
@@ -593,14 +597,17 @@ int voxel_sort(const float* xyz, float voxel_size, int64_t n, void* scratch, int
     grid /= 2;
   }
   // The counts are looked for where the kernel writes them: they are there some microseconds before the stream is seen to be idle.
+  // Only for as long as the largest sort takes with nothing queued before it, and only in a program whose threads spin in waits anyway;
+  // otherwise, and behind earlier work, the wait is the stream's, as the program chose it for the device.
   const volatile int32_t* counts = report;
+  const unsigned schedule = flags & cudaDeviceScheduleMask;
+  bool look = schedule == cudaDeviceScheduleAuto || schedule == cudaDeviceScheduleSpin;
+  const auto until = std::chrono::steady_clock::now() + kVoxelLook;
   int64_t total = 0;
   for (int t = 0; t < s.tiles; ++t) {
-    for (uint32_t look = 1; counts[t] == kVoxelPending; ++look) {
-      if ((look & 0xfffffu) != 0) continue;
-      const cudaError_t e = cudaStreamQuery(stream);
-      if (e == cudaErrorNotReady) continue;
-      GCT_CUDA_CHECK(e);
+    while (look && counts[t] == kVoxelPending) look = std::chrono::steady_clock::now() < until;
+    if (counts[t] == kVoxelPending) {
+      GCT_CUDA_CHECK(cudaStreamSynchronize(stream));
       if (counts[t] == kVoxelPending) return fail(GCT_ERR_DEVICE_STATUS, "voxelisation: the sort ended without a result");
     }
     if (counts[t] == kVoxelFailed) {

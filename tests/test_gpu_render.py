@@ -2,6 +2,10 @@
 code and voxel centre equal (the kernels use single rounded float operations for that reason).  Covers empty input,
 sizes that are not a multiple of the four points a thread takes, points behind the camera / outside the planes /
 on image borders, negative coordinates, and a multi-million point cloud through properties."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -107,6 +111,30 @@ def test_voxelize_frame_on_part_of_the_gpu(sms, n):
         part.pop_context()
     for a, b in zip(got, (wc, wcol, wcodes)):
         assert np.array_equal(a.cpu().numpy(), b)
+
+
+def test_voxelize_frame_waits_as_the_program_chose():
+    """The wait for the number of voxels, behind half a second of earlier work on the stream, in a process that has its threads sleep in
+    waits for the GPU: the thread spends next to no processor time in it."""
+    code = """
+import ctypes, time
+cu = ctypes.CDLL("libcuda.so.1")
+assert cu.cuInit(0) == 0 and cu.cuDevicePrimaryCtxSetFlags_v2(0, 4) == 0           # CU_CTX_SCHED_BLOCKING_SYNC
+import torch
+from lingbot_map_b200 import render_ops as RO
+xyz, rgb = torch.rand(50000, 3, device="cuda:0"), torch.rand(50000, 3, device="cuda:0")
+want = RO.voxelize_frame(xyz, rgb, 0.05)
+torch.cuda.synchronize()
+torch.cuda._sleep(900_000_000)
+wall, busy = time.perf_counter(), time.thread_time()
+got = RO.voxelize_frame(xyz, rgb, 0.05)
+wall, busy = time.perf_counter() - wall, time.thread_time() - busy
+assert all(torch.equal(a, b) for a, b in zip(got, want))
+assert wall > 0.2, wall
+assert busy < 0.25 * wall, (busy, wall)
+"""
+    r = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
 
 
 @pytest.mark.parametrize("n", [1, 2047, 2048, 2049, 2 * 2048 + 1, 65536])
