@@ -173,6 +173,11 @@ int gct_mgr_launch_count(const gct_mgr_t* m, int64_t* count_out);
 int gct_attn_launch_shape(int n_q, int heads, int kv_blocks, int num_sms, int max_splits, int* q_tiles_per_cta_out,
                           int* splits_out, int* split_len_out);
 
+/* The same for a dense attention call: query tiles per CTA, CTAs that share an SM (2 only with one tile each) and KV ranges.  The
+ * PyTorch operator has max_splits = 8. */
+int gct_attn_dense_launch_shape(int batch, int n_q, int n_kv, int heads, int num_sms, int max_splits, int* q_tiles_per_cta_out,
+                                int* ctas_per_sm_out, int* splits_out);
+
 /* ---- stand-alone operators --------------------------------------------------------- */
 
 /* Dense non-causal attention, the F.scaled_dot_product_attention call of Attention.forward

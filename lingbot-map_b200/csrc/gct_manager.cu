@@ -840,27 +840,48 @@ int gct_attn_launch_shape(int n_q, int heads, int kv_blocks, int num_sms, int ma
 }  // extern "C"
 
 namespace gct {
+// A call takes its time in waves of CTAs.  In KV blocks of a two-tile CTA (1.33 us), a wave over ranges of b blocks takes, measured back
+// to back (150 shapes, 1 to 86 blocks, within 6 % (rms) where a plan is among the better ones):
+//   two tiles per CTA      b + 4.8          one tile          0.64 b + 2.8
+//   two one-tile CTAs on an SM  1.08 b + 3.8 (1.19 b + 3.5 when there is no other wave), and what is left over for at most one CTA per
+//   SM  0.64 b + 2.2
+// and the merge of partial results 3.2 + 0.004 per CTA that writes one.  Two CTAs on an SM run the set-up and epilogue of one under the
+// other's KV loop and read K and V twice: in a call of one wave they are slower from six blocks on (1570 x 1664 x 16 heads 24.9 us, two
+// tiles 23.4), with more waves they are faster (2566 x 2688 57 us, two tiles 66, three ranges 76; 8 x 1005 x 1024 57, 68) unless the pairs
+// of tiles save a wave (6264 x 6264 231 us, two tiles 224).
+static DensePlan choose_dense_plan(int batch, int n_q, int n_kv, int heads, int sms, int max_splits) {
+  const long long q_tiles = (n_q + kTileM - 1) / kTileM, tiles = q_tiles * heads * batch, pairs = (q_tiles + 1) / 2 * heads * batch;
+  const int blocks = (n_kv + kBlockN - 1) / kBlockN;
+  DensePlan plan;
+  double best = 1e300;
+  for (int qt = 2; qt >= 1; --qt) {
+    for (int s = 1; s <= std::min(blocks, max_splits); ++s) {
+      const long long ctas = (qt == 2 ? pairs : tiles) * s;
+      const int len = s > 1 ? std::max((blocks + s - 1) / s, 2) : blocks;       // a range of one block takes as long as one of two
+      const double cost = static_cast<double>((ctas + sms - 1) / sms) * (qt == 2 ? len + 4.8 : 0.64 * len + 2.8) + (s > 1 ? 3.2 + 0.004 * ctas : 0.0);
+      if (cost < best - 1e-9) {
+        best = cost;
+        plan.q_tiles_per_cta = qt;
+        plan.splits = s;
+      }
+    }
+  }
+  if (tiles > sms) {
+    const long long waves = tiles / (2ll * sms), rest = tiles % (2ll * sms);
+    const double cost = tiles <= 2ll * sms ? 1.19 * blocks + 3.5
+                                           : static_cast<double>(waves + (rest > sms ? 1 : 0)) * (1.08 * blocks + 3.8) +
+                                                 (rest > 0 && rest <= sms ? 0.64 * blocks + 2.2 : 0.0);
+    if (cost < 0.98 * best) plan = {1, 2, 1};
+  }
+  return plan;
+}
+
 int dense_attention_plan(int batch, int n_q, int n_kv, int heads, int max_splits, DensePlan* plan) {
   if (batch <= 0 || n_q <= 0 || n_kv <= 0 || heads <= 0) return fail(GCT_ERR_INVALID, "dense attention: bad shape");
   int sms = 148;
   const int rc = device_sm_count(&sms);
   if (rc != GCT_OK) return rc;
-  const int q_tiles = (n_q + kTileM - 1) / kTileM, blocks = (n_kv + kBlockN - 1) / kBlockN;
-  choose_attention_config(q_tiles, heads * batch, blocks, sms, std::max(max_splits, 1), &plan->q_tiles_per_cta, &plan->splits);
-  plan->ctas_per_sm = 1;
-  // A call of several waves over few KV blocks spends much of its time on set-up and epilogue of its CTAs.  Two one-tile CTAs on an SM run
-  // these under each other's KV loop, but read K and V twice.  Time per wave, in KV blocks of a two-tile CTA, with b blocks (from 8 x
-  // 1005 x 1005, b = 8: two tiles 67.7 us, two CTAs 60.3 us; 6264 x 6264, b = 49: 224 us and 243 us; one tile alone: b = 1 5.8 us, b = 8
-  // 11.1 us): two tiles b + 4.0, two CTAs 1.14 b + 1.56, one tile alone 0.52 b + 3.7.
-  const long long tiles = static_cast<long long>(q_tiles) * heads * batch, pairs = static_cast<long long>((q_tiles + 1) / 2) * heads * batch;
-  if (plan->splits == 1 && tiles > sms) {
-    auto waves = [](long long ctas, long long slots) { return static_cast<double>((ctas + slots - 1) / slots); };
-    const double chosen = plan->q_tiles_per_cta == 2 ? waves(pairs, sms) * (blocks + 4.0) : waves(tiles, sms) * (0.52 * blocks + 3.7);
-    if (waves(tiles, 2ll * sms) * (1.14 * blocks + 1.56) < 0.97 * chosen) {
-      plan->q_tiles_per_cta = 1;
-      plan->ctas_per_sm = 2;
-    }
-  }
+  *plan = choose_dense_plan(batch, n_q, n_kv, heads, sms, std::max(max_splits, 1));
   return GCT_OK;
 }
 
@@ -897,6 +918,18 @@ int dense_attention_run(const void* q, const void* k, const void* v, void* out, 
 }  // namespace gct
 
 extern "C" {
+
+int gct_attn_dense_launch_shape(int batch, int n_q, int n_kv, int heads, int num_sms, int max_splits, int* q_tiles_per_cta_out,
+                                int* ctas_per_sm_out, int* splits_out) {
+  if (batch <= 0 || n_q <= 0 || n_kv <= 0 || heads <= 0 || num_sms <= 0 || max_splits <= 0 || q_tiles_per_cta_out == nullptr ||
+      ctas_per_sm_out == nullptr || splits_out == nullptr)
+    return fail(GCT_ERR_INVALID, "gct_attn_dense_launch_shape: bad argument");
+  const DensePlan plan = choose_dense_plan(batch, n_q, n_kv, heads, num_sms, max_splits);
+  *q_tiles_per_cta_out = plan.q_tiles_per_cta;
+  *ctas_per_sm_out = plan.ctas_per_sm;
+  *splits_out = plan.splits;
+  return GCT_OK;
+}
 
 int gct_attn_dense(const void* q_dev, const void* k_dev, const void* v_dev, void* out_dev, int batch, int n_q, int n_kv,
                    int heads, const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3],

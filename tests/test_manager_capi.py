@@ -186,6 +186,31 @@ def test_launch_shape_covers_the_kv_blocks():
         _lib.check(lib.gct_attn_launch_shape(0, 16, 8, 148, 16, C.byref(C.c_int()), C.byref(C.c_int()), C.byref(C.c_int())))
 
 
+def _dense_shape(batch, n_q, n_kv, heads, sms=148, max_splits=8):
+    import ctypes as C
+    out = [C.c_int() for _ in range(3)]
+    _lib.check(_lib.load().gct_attn_dense_launch_shape(batch, n_q, n_kv, heads, sms, max_splits, *(C.byref(x) for x in out)))
+    return tuple(x.value for x in out)
+
+
+@pytest.mark.parametrize("shape,want", [
+    ((1, 1005, 1005, 16), (1, 1, 1)), ((8, 1005, 1005, 16), (1, 2, 1)), ((1, 6264, 6264, 16), (2, 1, 1)), ((1, 1005, 8000, 16), (2, 1, 2)),
+    # the pairs of tiles fit one wave: two CTAs on an SM are slower, from six KV blocks on
+    ((1, 1570, 253, 16), (1, 2, 1)), ((1, 1570, 1570, 16), (2, 1, 1)), ((2, 783, 783, 16), (2, 1, 1)), ((3, 573, 1382, 16), (2, 1, 1)),
+    # ranges of a few blocks per two-tile CTA are slower than one range in two CTAs on an SM, or than one tile per CTA
+    ((1, 2349, 2349, 16), (1, 2, 1)), ((1, 2566, 2685, 16), (1, 2, 1)), ((5, 1005, 2685, 16), (1, 2, 1)), ((1, 2536, 2536, 3), (1, 1, 2)),
+    ((1, 450, 1660, 8), (1, 1, 4))])
+def test_dense_launch_shape(shape, want):
+    """Host arithmetic of the dense attention launch: query tiles per CTA, CTAs per SM and KV ranges, where each measured faster."""
+    assert _dense_shape(*shape) == want
+    for sms in (8, 132, 148):
+        for most in (1, 2, 8, 32):
+            qt, ctas, splits = _dense_shape(*shape, sms=sms, max_splits=most)
+            assert qt in (1, 2) and ctas in (1, 2) and qt * ctas <= 2 and 1 <= splits <= min(most, -(-shape[2] // 128)) and (ctas == 1 or splits == 1)
+    with pytest.raises(Exception):
+        _dense_shape(0, *shape[1:])
+
+
 def test_binding_is_rebuilt_for_another_torch_or_python(monkeypatch):
     """The binding links torch's C++ classes: one that was built for another torch or Python is out of date whatever its time of
     modification, and is not loaded."""
