@@ -151,8 +151,8 @@ def test_dense_attention_vs_oracle(B, Nq, Nkv, H):
 @pytest.mark.parametrize("Nkv", [1, 31, 32, 33, 63, 64, 65, 127, 128, 129, 192, 193, 320])
 @pytest.mark.parametrize("B,Nq,H", [(1, 1, 1), (1, 129, 3), (1, 200, 160), (2, 385, 60)])
 def test_dense_attention_at_the_edges_of_a_block(B, Nq, H, Nkv):
-    """Two threads share a row of 128 keys: lengths around their boundary and the block's, for one-tile CTAs (one wave, or two to an SM when
-    there are more than one wave of them), two-tile CTAs and split ranges; keys that grow, so that the running maximum moves."""
+    """Two threads share a row of 128 keys: lengths around their boundary and the block's, for one-tile CTAs, alone on an SM or two to an SM
+    when there is more than one wave of them (the test below reaches the other plans); keys that grow, so that the running maximum moves."""
     q, k, v = seeded.randn(1, B, Nq, H, 64), seeded.randn(2, B, Nkv, H, 64), seeded.randn(3, B, Nkv, H, 64)
     k = k * np.linspace(0.2, 2.0, Nkv, dtype=np.float32)[None, :, None, None]
     out = P.ops.dense_attention(bf(q), bf(k), bf(v))
@@ -160,6 +160,35 @@ def test_dense_attention_at_the_edges_of_a_block(B, Nq, H, Nkv):
     for b in range(B):
         want = O.attention(r(q[b][:, heads]), r(k[b][:, heads]), r(v[b][:, heads]))[0]
         assert_close(out[b][:, heads], want, f"b={b}")
+    assert P.ops.device_status(DEV) == 0
+
+
+def _dense_plan(B, Nq, Nkv, H):
+    import ctypes as C
+    out = [C.c_int() for _ in range(3)]
+    sms = torch.cuda.get_device_properties(DEV).multi_processor_count
+    _lib.check(_lib.load().gct_attn_dense_launch_shape(B, Nq, Nkv, H, sms, 8, *(C.byref(x) for x in out)))
+    return tuple(x.value for x in out)
+
+
+@pytest.mark.parametrize("tail", [1, 63, 64, 65, 127, 128])
+@pytest.mark.parametrize("B,Nq,H,blocks,plan", [(1, 256, 140, 8, (2, 1, 1)), (1, 1005, 16, 63, (2, 1, 2)), (1, 450, 8, 13, (1, 1, 4)), (2, 385, 60, 3, (1, 2, 1))])
+def test_dense_attention_plans_at_the_edges_of_a_block(B, Nq, H, blocks, plan, tail):
+    """Every plan of a dense call (tiles per CTA, CTAs per SM, KV ranges) with a last block of `tail` keys, on a few heads and rows of each
+    query tile; keys that grow, so that the running maximum moves in the last block too."""
+    Nkv = 128 * (blocks - 1) + tail
+    if torch.cuda.get_device_properties(DEV).multi_processor_count == 148:
+        assert _dense_plan(B, Nq, Nkv, H) == plan
+    g = torch.Generator(device=DEV).manual_seed(tail)
+    q, k, v = (torch.randn(B, n, H, 64, device=DEV, generator=g) for n in (Nq, Nkv, Nkv))
+    k = k * torch.linspace(0.2, 2.0, Nkv, device=DEV)[None, :, None, None]
+    q, k, v = (x.to(torch.bfloat16) for x in (q, k, v))
+    out = P.ops.dense_attention(q, k, v)
+    heads, rows = sorted({0, H // 2, H - 1}), sorted({i for t in range(0, Nq, 128) for i in (t, min(t + 33, Nq - 1), min(t + 127, Nq - 1))})
+    pick = lambda x: x[:, heads].float().cpu().numpy().astype(np.float64)
+    for b in range(B):
+        want = O.attention(pick(q[b, rows]), pick(k[b]), pick(v[b]))[0]
+        assert_close(out[b, rows][:, heads], want, f"b={b}")
     assert P.ops.device_status(DEV) == 0
 
 
@@ -773,6 +802,48 @@ def test_rows_past_the_valid_length_of_the_last_page_do_not_leak():
     for bounded in (True, False):
         m.set_bounded_mode(bounded)
         assert_close(m.compute_attention(0, bf(q)), want, f"garbage tail, bounded={bounded}")
+    assert m.device_status() == 0
+
+
+@pytest.mark.parametrize("mode", ["bounded", "fallback", "exact"])
+@pytest.mark.parametrize("last", [1, 63, 64, 65, 127, 128, 129, 192])
+@pytest.mark.parametrize("page", [261, 192])
+def test_page_tails_of_the_two_tile_kernels(page, last, mode):
+    """The two threads of a row mask the tail of a page's last block, each its 64 keys: every length of the last page around their
+    boundary and the block's, pages that end five and 64 keys into a block, with the fixed reference, with the running maximum that a
+    CTA of that kernel falls back to (a key far beyond the others in a page that is not visible makes the bound too loose), and with
+    the running maximum from the start.  Rows past the last valid one hold values that would show."""
+    import ctypes as C
+    tpf, H = page + 1, 70 if page > 256 else 140                  # pairs of query tiles for one wave, twice as many tiles
+    m = P.B200KVCacheManager(1, 1 + 1 + 16, tpf, H, 64, num_special_tokens=1, device=DEV, scale_frames=1, sliding_window=1, max_total_frames=page)
+    for _ in range(last):
+        m.append_frame_bookkeeping(0)
+        m.evict_frames(0, 1, 1)
+    table = m.build_visible_page_table(0)
+    assert m.compute_last_page_len(0) == last
+    qt, splits, ln = C.c_int(), C.c_int(), C.c_int()
+    blocks = (len(table) - 1) * -(-page // 128) + -(-last // 128)
+    _lib.check(_lib.load().gct_attn_launch_shape(tpf, H, blocks, 148, 16, C.byref(qt), C.byref(splits), C.byref(ln)))
+    assert qt.value == 2
+    g = torch.Generator(device=DEV).manual_seed(last)
+    pool = m.kv_caches[0]
+    pool.normal_(generator=g)
+    if mode == "fallback":
+        pool[next(i for i in range(pool.shape[0]) if i not in table), 0, 0] = 100.0
+    m.rescan_key_norms()
+    m.set_bounded_mode(mode != "exact")
+    pool[table[-1], 0, last:] = 3.0e3
+    pool[table[-1], 1, last:] = -7.0e4
+    q = torch.randn(tpf, H, 64, device=DEV, generator=g).to(torch.bfloat16)
+    bound = float(q.float().norm(dim=-1).max() * m.key_norm_max.max()) * 0.125 * 1.4427
+    assert bound < 40 if mode == "bounded" else mode == "exact" or bound > 200
+    out, lse = m.compute_attention(0, q, return_lse=True)
+    kk, vv = m._gather_kv(0)
+    assert kk.shape[0] == (len(table) - 1) * page + last
+    for h in (0, H // 2, H - 1):
+        want, wl = O.attention(*(x[:, h:h + 1].float().cpu().numpy().astype(np.float64) for x in (q, kk, vv)))
+        assert_close(out[:, h:h + 1], want, f"head {h}")
+        assert np.abs(lse[:, h].cpu().numpy() - wl[:, 0]).max() < 4e-3      # the Q tile rounded after its scale; as for the headline cache
     assert m.device_status() == 0
 
 

@@ -81,16 +81,21 @@ def test_one_process_drives_two_gpus():
     """The shared-memory opt-in of the attention kernels and the SM count are per-device state: a process that has
     used GPU 0 must be able to launch the 2-tile kernel (176 KB of dynamic shared memory) on GPU 1 as well.  Small
     cases only: dense attention with one and two query tiles per CTA, and a paged call through a manager."""
-    import numpy as np
+    import ctypes as C
     sys.path.insert(0, ROOT)
     import lingbot_map_b200 as P
+    from lingbot_map_b200 import _lib
     outs = []
     for dev in ("cuda:0", "cuda:1"):
         g = torch.Generator().manual_seed(3)                          # host generator: identical inputs on both devices
-        q = torch.randn(1, 300, 4, 64, generator=g).to(dev).to(torch.bfloat16)
-        k = torch.randn(1, 700, 4, 64, generator=g).to(dev).to(torch.bfloat16)
-        small = P.ops.dense_attention(q[:, :100], k, k)               # one tile per CTA
-        big = P.ops.dense_attention(q, k, k)                          # two tiles per CTA
+        q = torch.randn(1, 256, 140, 64, generator=g).to(dev).to(torch.bfloat16)
+        k = torch.randn(1, 900, 140, 64, generator=g).to(dev).to(torch.bfloat16)
+        for n_q, tiles in ((100, 1), (256, 2)):                       # query tiles per CTA
+            shape = [C.c_int() for _ in range(3)]
+            _lib.check(_lib.load().gct_attn_dense_launch_shape(1, n_q, 900, 140, 148, 8, *(C.byref(x) for x in shape)))
+            assert shape[0].value == tiles
+        small = P.ops.dense_attention(q[:, :100], k, k)
+        big = P.ops.dense_attention(q, k, k)
         ref = torch.nn.functional.scaled_dot_product_attention(q.float().permute(0, 2, 1, 3), k.float().permute(0, 2, 1, 3),
                                                                k.float().permute(0, 2, 1, 3)).permute(0, 2, 1, 3)
         assert float((big.float() - ref).abs().max()) < 2e-2 and float((small.float() - ref[:, :100]).abs().max()) < 2e-2

@@ -2,6 +2,7 @@
 code and voxel centre equal (the kernels use single rounded float operations for that reason).  Covers empty input,
 sizes that are not a multiple of the four points a thread takes, points behind the camera / outside the planes /
 on image borders, negative coordinates, and a multi-million point cloud through properties."""
+import concurrent.futures
 import os
 import subprocess
 import sys
@@ -74,19 +75,25 @@ def test_large_cloud_properties():
 
 @pytest.mark.parametrize("n", [148 * 2048 + 5, 256 * 2048 - 1, 256 * 2048])
 def test_voxelize_frame_sort_up_to_its_largest(n):
-    """More tiles than SMs, up to the largest cloud the sort takes (256 tiles meet at its barriers), again and again on one stream and on
-    two at once."""
+    """More tiles than SMs, up to the largest cloud the sort takes (256 tiles meet at its barriers), again and again from two threads at
+    once, each on its stream."""
     rs = np.random.RandomState(n % 1000)
     xyz = (rs.randint(-300, 301, (n, 3)) + 0.5).astype(np.float32)
     rgb = rs.rand(n, 3).astype(np.float32)
     wc, wcol, wcodes = R.voxelize_frame(xyz, rgb, 1.0)
     dx, dr = torch.from_numpy(xyz).to(DEV), torch.from_numpy(rgb).to(DEV)
-    side = torch.cuda.Stream()
-    side.wait_stream(torch.cuda.current_stream())
-    for i in range(6):
-        with torch.cuda.stream(side if i % 2 else torch.cuda.current_stream()):
-            c, col, codes = RO.voxelize_frame(dx, dr, 1.0)
-            assert np.array_equal(codes.cpu().numpy(), wcodes) and np.array_equal(c.cpu().numpy(), wc) and np.array_equal(col.cpu().numpy(), wcol)
+    torch.cuda.synchronize()
+
+    def calls(_):
+        with torch.cuda.stream(torch.cuda.Stream(DEV)):
+            got = [RO.voxelize_frame(dx, dr, 1.0) for _ in range(12)]
+            torch.cuda.current_stream().synchronize()
+            return got
+
+    with concurrent.futures.ThreadPoolExecutor(2) as pool:
+        results = [r for part in pool.map(calls, range(2)) for r in part]
+    for c, col, codes in results:
+        assert np.array_equal(codes.cpu().numpy(), wcodes) and np.array_equal(c.cpu().numpy(), wc) and np.array_equal(col.cpu().numpy(), wcol)
 
 
 @pytest.mark.parametrize("sms", [8, 16, 72])
@@ -140,8 +147,8 @@ assert busy < 0.25 * wall, (busy, wall)
 @pytest.mark.parametrize("n", [1, 2047, 2048, 2049, 2 * 2048 + 1, 65536])
 @pytest.mark.parametrize("extent", [3, 100, 5000, 2 ** 20 - 1])
 def test_voxelize_frame_sort_edges(n, extent):
-    """The frame-sized sort at the edges of its tiles (2048 points) and for clouds whose voxel indices need from one pass
-    (within +-7) over the five that are launched first (below 2^12) to all eight (2^20); every index twice, so that the
+    """The frame-sized sort at the edges of its tiles (2048 points) and for clouds whose voxel indices need from two passes
+    (within +-7) over five (below 2^12) to all eight (2^20); every index twice, so that the
     order among equal keys shows in the colours."""
     rs = np.random.RandomState(n + extent)
     idx = rs.randint(-extent, extent + 1, (n, 3))
