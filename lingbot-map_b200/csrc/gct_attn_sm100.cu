@@ -289,7 +289,7 @@ constexpr int kFfmaAhead = 4, kSumLag = 2;   // software pipeline of the exponen
 // warpgroup shrinks to kControlRegs and the four softmax warpgroups grow to kSoftmaxRegs:
 // 128 * kControlRegs + 512 * kSoftmaxRegs <= 61440, both multiples of 8.
 constexpr int kControlRegs = 64;
-constexpr int kSoftmaxRegs = 104;      // 112 beside 32 was 2 % slower
+constexpr int kSoftmaxRegs = 104;      // 112 beside 32 was 2 % slower; of <2, true>'s 528 bytes of spill loads all but 76 go with the fallback
 static_assert(128 * kControlRegs + 512 * kSoftmaxRegs <= 61440, "register pool of the CTA exceeded");
 constexpr float kRescaleThreshold = 8.0f;   // in log2 units of the scaled logits
 
@@ -614,7 +614,8 @@ gct_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     if (kBounded && running_max) {
       // ---- fallback of the bounded kernel: two passes over the half row in TMEM, 32 columns at a time ----
       // pass 1 takes the masked row maximum, pass 2 exponentiates against the running maximum (moved only when the
-      // row maximum outgrows it by 2^kRescaleThreshold) and stores P; compact rather than fast.
+      // row maximum outgrows it by 2^kRescaleThreshold) and stores P; compact rather than fast (600 KV blocks, every CTA here: 700 us
+      // per call, with the fixed reference 369).
       for (int j = 0; ok && j < nblk; ++j) {
         if (!(ok = wait_v(bar_s_full(t), j & 1))) break;
         tc_fence_after();
@@ -787,6 +788,9 @@ gct_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
 
     // ---- epilogue: O / l ----
+    // With the fixed reference the warps of the first half have only waited for their own half's products inside the loop, so for them
+    // this wait can end one phase early, on the block before the last.  What orders their read of O behind the last products is the
+    // exchange below: the partner comes to it after its own waits, which followed every phase of this barrier.
     if (ok && nblk > 0) ok = wait_v(bar_pv_full(t, 1), (nblk - 1) & 1);
     {
       // in the order of the columns; not the slot of the last block: the partner may still be reading that
@@ -986,21 +990,23 @@ void choose_attention_config(int n_q_tiles, int heads_x_batch, int total_blocks,
 #endif
   constexpr double kMergeCost = GCT_MERGE_COST;
   // Paged calls (split_len != nullptr): a call that fits one wave pays about five blocks once; in a call of several waves
-  // every wave is charged fifteen blocks beside its KV blocks (set-up, pipeline fill, epilogue, and at the board's power limit a
-  // lower clock the fuller the SMs are: idle SMs are not lost time there).  Measured in back-to-back loops of this kernel, 64 (head,
-  // tile pair) items, us for 2 ranges (one wave, 128 CTAs) against the 9 (four waves) that a fixed cost of two blocks chose: 250 KV
-  // blocks 168 : 195, 371 242 : 268, 385 254 : 280, 527 338 : 360, 600 385 : 402, 1065 675 : 709.  With the five blocks of the
-  // one-wave plan these pairs imply 10 to 13 blocks per wave up to 600 blocks and 22 at 1065.  Fifteen is not a fit to them:
-  // it chooses the plan that measured faster up to a thousand blocks and keeps the nine equal ranges beyond (above 15.5 the model
-  // would take two at 1057 blocks, too).  Which is faster there inside a frame has not been measured; at 600 blocks, where two ranges
-  // win the loop, two and nine take the same time in a frame (below).  Nine blocks for one-tile CTAs is 0.6 of fifteen, not measured.
+  // every wave is charged fifteen blocks beside its KV blocks (set-up, pipeline fill, epilogue).  The constants were set with one thread
+  // per row; with two, the plans they choose between measure (64 (head, tile pair) items; us per call in a loop, and ms of a frame of 24
+  // layers with the other kernels; each plan was forced in turn):
+  //   KV blocks    2 equal ranges     2 long + a short one     9 equal ranges       (frames cached)
+  //     600         394   10.2           371    9.5               395   10.0               320
+  //     760         495   12.5           468   11.8               490   12.3             3,500
+  //     928         600   15.1           572   14.3               590   14.8             7,000
+  //    1057         693   17.4           659   16.5               678   16.9            10,000
+  // Fifteen blocks per wave keep several equal waves off where long ranges and a short one are faster; that these win beyond a thousand
+  // blocks as well is not used yet.  At 41 blocks (4 frames) two equal ranges take 31.9 us where the plan chosen takes 34.7.  Nine blocks
+  // for one-tile CTAs is 0.6 of fifteen, not measured.  Calls without split_len (the static entry point) take equal ranges at two blocks
+  // per wave, as measured with one thread per row.
   const bool paged = split_len != nullptr;
   auto fixed = [paged](int qt, bool one_wave) { return !paged ? 2.0 : one_wave ? (qt == 2 ? 5.0 : 4.0) : (qt == 2 ? 15.0 : 9.0); };
-  // Long ranges + a short one fill the SMs that equal ranges leave idle.  The paged kernel alone, back to back at the power limit,
-  // takes about as long as with two equal ranges (us: 71 KV blocks 54.8 : 56.7, 193 134 : 132, 285 190 : 192, 600 392 : 385); inside
-  // a frame, beside the other kernels, it is faster: 24 layers at 600 blocks 9.7-10.0 ms against 10.5 with two and with nine
-  // equal ranges, two layer pairs as modules 949-974 : 1013 us.  Not beyond a thousand blocks, on one measurement in a loop: at 1057
-  // blocks nine long ranges and a short one were 0.6 % slower than nine equal ones.  Not measured there: two long ranges and a short one.
+  // Long ranges + a short one fill the SMs that equal ranges leave idle (the table above).  The line at a thousand blocks was drawn with
+  // one thread per row, where nine long ranges and a short one were 0.6 % slower than nine equal ones at 1057 blocks; two long ranges
+  // and a short one, 2.5 % faster there now, were not measured then.
   constexpr int kUnevenMaxBlocks = 1000;
   // the plan of the previous call with the same arguments (a frame asks 24 times for the same one)
   static thread_local SplitPlanKey last_key = {-1, -1, -1, -1, -1};

@@ -77,7 +77,8 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, kQ == 1 ? 2 : 1) gct_decode
   const size_t row_stride = static_cast<size_t>(a.heads) * D;
   const size_t head_off = static_cast<size_t>(h) * D + lane * kPer;
   // Under the end of the kernel before, which leaves the memory idle: the first cached rows of the range on their way to L2.  A hint
-  // that reads nothing, so it may be given for rows that kernel is still writing.  Sixteen calls at 10,000 frames 499.0 -> 487.7 us.
+  // that reads nothing, so it may be given for rows that kernel is still writing.  Sixteen calls at 10,000 frames 491.7 -> 477.7 us,
+  // at 1,000 frames 139 -> 119; with a Linear layer of the library before each call, which lets no launch begin early, 262.7 -> 262.2.
   {
     constexpr int kLines = D * 4 / 128;
     const int rows = min(min(j1, a.cached) - j0, kAheadRows);
